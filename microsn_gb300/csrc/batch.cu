@@ -259,7 +259,7 @@ static const char* profile_cache(mlc_ctx* ctx, BatchIO* b, const FftPlan2D& p, i
     MLC_CUDA(cudaMemGetInfo(&fr, &tot));
     budget = tot / 4;
   }
-  const size_t stride = (size_t)round_up((long)p.spec_bytes(), 256);
+  const size_t stride = (size_t)round_up((long)profile_spectrum_bytes(p), 256);
   if ((size_t)nprof * stride > budget) return nullptr;
   b->kcache_key.clear();  // invalid until the new spectra are queued
   char* kc = (char*)grow_dev(ctx, b, b->kcache, b->kcache_cap, (size_t)nprof * stride);

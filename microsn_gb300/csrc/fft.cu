@@ -91,13 +91,13 @@ void set_max_smem(const void* func, size_t bytes) {
 }
 
 FftPlan2D::~FftPlan2D() {
-  if (twx) cudaFree(twx);
-  if (twy) cudaFree(twy);
+  for (void* t : {twx, twy, twx3, twy3, twl3})
+    if (t) cudaFree(t);
 }
 
 // exp(-2 pi i m / N), m in [0, N), evaluated in long double with the angle reduced to
 // the first octant so that each entry is correctly rounded to FP64 in practice.
-static void twiddle_table(int N, std::vector<double>& re, std::vector<double>& im) {
+static void twiddle_table(int N, std::vector<long double>& re, std::vector<long double>& im) {
   re.resize(N);
   im.resize(N);
   const long double TWO_PI = 6.283185307179586476925286766559005768L;
@@ -130,21 +130,60 @@ static void twiddle_table(int N, std::vector<double>& re, std::vector<double>& i
       c = (k == 0) ? 1 : (k == 2) ? -1 : 0;
       s = (k == 1) ? 1 : (k == 3) ? -1 : 0;
     }
-    re[m] = (double)c;
-    im[m] = -(double)s;  // forward sign
+    re[m] = c;
+    im[m] = -s;  // forward sign
   }
 }
 
 template <typename T>
 static void* upload_twiddles(int N) {
-  std::vector<double> re, im;
+  std::vector<long double> re, im;
   twiddle_table(N, re, im);
   std::vector<C2<T>> h(N);
-  for (int m = 0; m < N; m++) h[m] = C2<T>{(T)re[m], (T)im[m]};
+  for (int m = 0; m < N; m++) h[m] = C2<T>{(T)(double)re[m], (T)(double)im[m]};
   void* d = nullptr;
   MLC_CUDA(cudaMalloc(&d, sizeof(C2<T>) * N));
   MLC_CUDA(cudaMemcpy(d, h.data(), sizeof(C2<T>) * N, cudaMemcpyHostToDevice));
   return d;
+}
+
+// The same table in three limbs: a plane of (re, im) high and middle limbs, then one of low
+// limbs.  The high limb is cut to multiples of 2^-24 (limb.cuh); the sum keeps what long
+// double holds on this host (64 bits or more).
+static void* upload_limbs3(const std::vector<long double>& re, const std::vector<long double>& im) {
+  const size_t N = re.size();
+  std::vector<float> h(N * 6);
+  float* lo = h.data() + N * 4;
+  for (size_t m = 0; m < N; m++)
+    for (int k = 0; k < 2; k++) {
+      const long double v = k ? im[m] : re[m];
+      const float a = (float)(rintl(v * 16777216.0L) / 16777216.0L);
+      const float b = (float)(v - (long double)a);
+      h[m * 4 + k] = a;
+      h[m * 4 + 2 + k] = b;
+      lo[m * 2 + k] = (float)(v - (long double)a - (long double)b);
+    }
+  void* d = nullptr;
+  MLC_CUDA(cudaMalloc(&d, h.size() * sizeof(float)));
+  MLC_CUDA(cudaMemcpy(d, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice));
+  return d;
+}
+static void* upload_twiddles3(int N) {
+  std::vector<long double> re, im;
+  twiddle_table(N, re, im);
+  return upload_limbs3(re, im);
+}
+// Level 0 of the row transforms: W_M^(m q) for q = 1 .. R0 - 1, m < M / R0.
+static void* upload_level0(int M) {
+  const int R0 = limb_first_radix(M), J = M / R0;
+  std::vector<long double> re, im, lr, li;
+  twiddle_table(M, re, im);
+  for (int q = 1; q < R0; q++)
+    for (int m = 0; m < J; m++) {
+      lr.push_back(re[(size_t)m * q]);
+      li.push_back(im[(size_t)m * q]);
+    }
+  return upload_limbs3(lr, li);
 }
 
 static void split_columns(int Ny, int& N1, int& N2) {
@@ -182,6 +221,9 @@ FftPlan2D* plan_get(mlc_ctx* ctx, int Nx, int Ny, int prec) {
   if (prec == MLC_F64) {
     p->twx = upload_twiddles<double>(Nx);
     p->twy = upload_twiddles<double>(Ny);
+    p->twx3 = upload_twiddles3(Nx);
+    p->twy3 = upload_twiddles3(Ny);
+    if (limb_first_radix(p->M)) p->twl3 = upload_level0(p->M);
   } else if (prec_is_ff(prec)) {
     p->twx = upload_twiddles<ff>(Nx);
     p->twy = upload_twiddles<ff>(Ny);
@@ -206,7 +248,7 @@ void conv_fused(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, const double
   if (p.prec == PREC_FFS) {  // P0-P2 to the half-spectrum, then P3 into FP32 pixels
     void* tmp = ws_get(ctx, WS_SPEC_TMP, p.spec_bytes());
     conv_fused_impl<ff>(ctx, p, Fmap, prof, pN, nullptr, tmp, WS_KX);
-    rows_c2r_impl<ff, float>(ctx, p, tmp, out);
+    if (!limb2_rows_c2r(ctx, p, tmp, out)) rows_c2r_impl<ff, float>(ctx, p, tmp, out);
   } else if (p.prec == PREC_FF) conv_fused_impl<ff>(ctx, p, Fmap, prof, pN, out);
   else if (p.prec == MLC_F64) conv_fused_impl<double>(ctx, p, Fmap, prof, pN, out);
   else conv_fused_impl<float>(ctx, p, Fmap, prof, pN, out);
@@ -225,6 +267,10 @@ bool profile_spectrum_supported(const FftPlan2D& p) {
   return profile_spectrum_supported_impl<float>(p);
 }
 
+size_t profile_spectrum_bytes(const FftPlan2D& p) {
+  return p.prec == MLC_F64 ? limb3_profile_spectrum_bytes(p) : p.spec_bytes();
+}
+
 void profile_spectrum(mlc_ctx* ctx, const FftPlan2D& p, const double* prof, int pN, void* ks) {
   if (prec_is_ff(p.prec)) profile_spectrum_impl<ff>(ctx, p, prof, pN, ks);
   else if (p.prec == MLC_F64) profile_spectrum_impl<double>(ctx, p, prof, pN, ks);
@@ -241,7 +287,7 @@ void conv_cached(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, const void*
   if (p.prec == PREC_FFS) {
     void* tmp = ws_get(ctx, WS_SPEC_TMP, p.spec_bytes());
     conv_cached_impl<ff>(ctx, p, Fmap, ks, tmp);
-    rows_c2r_impl<ff, float>(ctx, p, tmp, out);
+    if (!limb2_rows_c2r(ctx, p, tmp, out)) rows_c2r_impl<ff, float>(ctx, p, tmp, out);
   } else if (p.prec == PREC_FF) conv_cached_real_impl<ff>(ctx, p, Fmap, ks, out);
   else if (p.prec == MLC_F64) conv_cached_real_impl<double>(ctx, p, Fmap, ks, out);
   else conv_cached_real_impl<float>(ctx, p, Fmap, ks, out);
@@ -253,9 +299,10 @@ bool rows_c2r_interleave_supported(const FftPlan2D& p) {
 
 bool rows_c2r_interleave(mlc_ctx* ctx, const FftPlan2D& p, const void* specs, long spec_stride, int nm, int S,
                          void* out, unsigned planar) {
-  if (p.prec == PREC_FFS) return c2r_interleave_impl<ff, float>(ctx, p, specs, spec_stride, nm, S, out, planar);
+  if (!rows_c2r_interleave_supported(p)) return false;
+  if (p.prec == PREC_FFS) return limb2_rows_c2r_il(ctx, p, specs, spec_stride, nm, S, out, planar);
   if (p.prec == PREC_FF) return c2r_interleave_impl<ff>(ctx, p, specs, spec_stride, nm, S, out, planar);
-  if (p.prec == MLC_F64) return c2r_interleave_impl<double>(ctx, p, specs, spec_stride, nm, S, out, planar);
+  if (p.prec == MLC_F64) return limb3_rows_c2r_il(ctx, p, specs, spec_stride, nm, S, out, planar);
   return c2r_interleave_impl<float>(ctx, p, specs, spec_stride, nm, S, out, planar);
 }
 

@@ -3,7 +3,7 @@
 // the column passes (a 128-byte strip of columns per CTA, four-step split N = N1*N2).
 #pragma once
 
-#include "mlc_common.cuh"
+#include "limb.cuh"
 
 namespace mlc {
 
@@ -82,8 +82,8 @@ struct Dft<T, 5, INV> {
     C2<T> u = C2<T>{x0.x - scale2(t1.x, 0.25f), x0.y - scale2(t1.y, 0.25f)};
     C2<T> m = C2<T>{b * t2.x, b * t2.y};
     C2<T> p1 = cadd(u, m), p2 = csub(u, m);
-    C2<T> q1 = C2<T>{s1 * da.x + s2 * db.x, s1 * da.y + s2 * db.y};
-    C2<T> q2 = C2<T>{s2 * da.x - s1 * db.x, s2 * da.y - s1 * db.y};
+    C2<T> q1 = C2<T>{lin2(s1, da.x, s2, db.x), lin2(s1, da.y, s2, db.y)};
+    C2<T> q2 = C2<T>{lin2(s2, da.x, -s1, db.x), lin2(s2, da.y, -s1, db.y)};
     C2<T> iq1 = mul_mi<T, INV>(q1), iq2 = mul_mi<T, INV>(q2);
     v[0] = cadd(x0, t1);
     v[1] = cadd(p1, iq1);
@@ -136,7 +136,7 @@ __device__ __forceinline__ void dft_split2(C2<T>* v, const T* wr, const T* wi) {
   for (int k = 1; k < H; k++) {
     // W^k o with W^k = (wr, -wi) forward, (wr, wi) inverse
     const T sr = INV ? -wi[k] : wi[k];
-    const C2<T> t = C2<T>{wr[k] * o[k].x + sr * o[k].y, wr[k] * o[k].y - sr * o[k].x};
+    const C2<T> t = C2<T>{lin2(wr[k], o[k].x, sr, o[k].y), lin2(wr[k], o[k].y, -sr, o[k].x)};
     v[k] = cadd(e[k], t);
     v[k + H] = csub(e[k], t);
   }

@@ -1,4 +1,5 @@
-// FP64 instantiations of the FFT and convolution passes of fft_impl.cuh.
+// FP64 instantiations of the FFT and convolution passes of fft_impl.cuh: the plain form, and
+// the sizes without a limb kernel (fft_limb.cuh).
 #include "fft_impl.cuh"
 
 namespace mlc {
@@ -10,6 +11,5 @@ template void profile_spectrum_impl<double>(mlc_ctx*, const FftPlan2D&, const do
 template void conv_cached_impl<double>(mlc_ctx*, const FftPlan2D&, const void*, const void*, void*);
 template void conv_cached_real_impl<double>(mlc_ctx*, const FftPlan2D&, const void*, const void*, void*);
 template void conv_plain_impl<double>(mlc_ctx*, const FftPlan2D&, const void*, const double*, int, void*);
-template bool c2r_interleave_impl<double, double>(mlc_ctx*, const FftPlan2D&, const void*, long, int, int, void*, unsigned);
 
 }  // namespace mlc

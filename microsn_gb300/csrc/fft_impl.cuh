@@ -910,7 +910,7 @@ static void launch_rows_r2c(mlc_ctx* ctx, const FftPlan2D& p, const Loader& ld, 
         MLC_CHECK_LAUNCH();
         return;
       }
-    } else {
+    } else if constexpr (!std::is_same<Loader, ProfileRows<double>>::value) {  // (those: limb3_rows_r2c_profile)
       switch (p.M) {
         case 5000: k3 = k_rows_r2c3<T, 8, 25, 25, Loader>; J = 625; break;
         case 4096: k3 = k_rows_r2c3<T, 16, 16, 16, Loader>; J = 256; break;
@@ -942,7 +942,7 @@ static void launch_rows_r2c(mlc_ctx* ctx, const FftPlan2D& p, const Loader& ld, 
 
 template <typename T, typename TO = typename RealOut<T>::type>
 static void launch_rows_c2r(mlc_ctx* ctx, const FftPlan2D& p, const void* in, void* out) {
-  {
+  if constexpr (!(std::is_same<T, ff>::value && std::is_same<TO, float>::value)) {  // (those: limb2_rows_c2r)
     using K3 = void (*)(const C2<T>*, long, TO*, long, const C2<T>*);
     K3 k3 = nullptr;
     int J = 0;
@@ -985,8 +985,10 @@ constexpr int strip_width() {
 }
 
 // kind 'A': row sets {n2 + N2*j}, length N1; kind 'B': row blocks {k1*N2 + j}, length N2.
+// limbs: FP64 passes, and the inverse ones of FP32 maps' float-float plans, in limb arithmetic
+// where the length has a kernel (the plain convolution keeps the plan's own arithmetic).
 template <typename T, bool INV>
-static void launch_colpass(mlc_ctx* ctx, const FftPlan2D& p, void* buf, char kind, int post_tw) {
+static void launch_colpass(mlc_ctx* ctx, const FftPlan2D& p, void* buf, char kind, int post_tw, bool limbs = true) {
   constexpr int CW = strip_width<T>();
   const int nstrips = ceil_div(p.Wc, CW);
   int L, nsets, tw_stride;
@@ -998,6 +1000,10 @@ static void launch_colpass(mlc_ctx* ctx, const FftPlan2D& p, void* buf, char kin
     L = p.N2; nsets = p.N1; set_mul = p.N2; j_mul = 1; tw_stride = p.N1; rl = p.rlN2;
   }
   if (L == 1 && !post_tw) return;
+  if constexpr (std::is_same<T, double>::value)
+    if (limbs && limb3_colpass(ctx, p, buf, kind, INV, post_tw)) return;
+  if constexpr (std::is_same<T, ff>::value && INV)
+    if (limbs && p.prec == PREC_FFS && limb2_colpass_inverse(ctx, p, buf, kind, post_tw)) return;
   // two-level register kernels for the lengths that split into two supported factors
   using K2 = void (*)(C2<T>*, long, long, long, const C2<T>*, int, int);
   K2 k2 = nullptr;
@@ -1035,13 +1041,45 @@ static void launch_colpass(mlc_ctx* ctx, const FftPlan2D& p, void* buf, char kin
 // ---------------------------------------------------------------- entry templates
 
 template <typename T>
-void forward_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* in, int in_dtype, void* spec) {
-  if (in_dtype == MLC_F64)
+static void forward_passes(mlc_ctx* ctx, const FftPlan2D& p, const void* in, int in_dtype, void* spec, bool limbs) {
+  bool done = false;
+  if constexpr (std::is_same<T, double>::value) done = limbs && limb3_rows_r2c_map(ctx, p, in, in_dtype, spec);
+  if (done) {
+  } else if (in_dtype == MLC_F64)
     launch_rows_r2c<T>(ctx, p, RealRows<T, double>{(const double*)in, p.Nx}, p.Ny, spec);
   else
     launch_rows_r2c<T>(ctx, p, RealRows<T, float>{(const float*)in, p.Nx}, p.Ny, spec);
-  launch_colpass<T, false>(ctx, p, spec, 'A', 1);
-  launch_colpass<T, false>(ctx, p, spec, 'B', 0);
+  launch_colpass<T, false>(ctx, p, spec, 'A', 1, limbs);
+  launch_colpass<T, false>(ctx, p, spec, 'B', 0, limbs);
+}
+
+template <typename T>
+void forward_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* in, int in_dtype, void* spec) {
+  forward_passes<T>(ctx, p, in, in_dtype, spec, true);
+}
+
+// Workspace of P0's rows; FP64 keeps them in three limbs (24 bytes) beside the FP64 ones, with
+// an exponent per column (LimbProfileBuffer in fft_limb.cuh).
+template <typename T>
+static size_t profile_rows_bytes(const FftPlan2D& p, int rows) {
+  const size_t n = (size_t)(rows > 0 ? rows : 1) * p.Wp;
+  return n * sizeof(C2<T>) + (std::is_same<T, double>::value ? n * 24 + (size_t)p.Wp * sizeof(int) : 0);
+}
+
+// P0: the profile's 2h non-zero rows.
+template <typename T>
+static void profile_rows(mlc_ctx* ctx, const FftPlan2D& p, const double* prof, int pN, void* kx) {
+  if constexpr (std::is_same<T, double>::value)
+    if (limb3_rows_r2c_profile(ctx, p, prof, pN, kx)) return;
+  const int h = pN / 2;
+  launch_rows_r2c<T>(ctx, p, ProfileRows<T>{prof, pN, h, p.Nx}, 2 * h, kx);
+}
+// P3 of a single convolution into pixels of the plan's default type.
+template <typename T>
+static void real_rows(mlc_ctx* ctx, const FftPlan2D& p, const void* in, void* out) {
+  if constexpr (std::is_same<T, double>::value)
+    if (limb3_rows_c2r(ctx, p, in, out)) return;
+  launch_rows_c2r<T>(ctx, p, in, out);
 }
 
 // spec_out: stop after P2 and leave the inverse half-spectrum there (pitch Wp) instead of
@@ -1053,18 +1091,28 @@ void conv_fused_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, const d
   const int h = pN / 2;
   MLC_REQUIRE(pN % 2 == 0 && 2 * h <= p.Ny && 2 * h <= p.Nx, MLC_ERR_LIMIT,
               "profile raster larger than the map");
-  void* kx = ws_get(ctx, kx_slot, (size_t)(2 * h > 0 ? 2 * h : 1) * p.Wp * sizeof(C2<T>));
+  void* kx = ws_get(ctx, kx_slot, profile_rows_bytes<T>(p, 2 * h));
   void* tmp = spec_out ? spec_out : ws_get(ctx, WS_SPEC_TMP, p.spec_bytes());
-  launch_rows_r2c<T>(ctx, p, ProfileRows<T>{prof, pN, h, p.Nx}, 2 * h, kx);
+  profile_rows<T>(ctx, p, prof, pN, kx);
+  {
+    bool done = false;
+    if constexpr (std::is_same<T, double>::value) done = limb3_conv(ctx, p, Fmap, tmp, kx, h);
+    if constexpr (std::is_same<T, ff>::value) done = p.prec == PREC_FFS && limb2_conv(ctx, p, Fmap, tmp, kx, h);
+    if (done) {
+      launch_colpass<T, true>(ctx, p, tmp, 'A', 0);
+      if (!spec_out) real_rows<T>(ctx, p, tmp, out);
+      return;
+    }
+  }
   const int nstrips = ceil_div(p.Wc, CW);
   const T scale = (T)(1.0 / ((double)p.Nx * (double)p.Ny));
-  {
+  if constexpr (!std::is_same<T, double>::value) {  // (FP64: limb3_conv has taken these lengths)
     // two-level register kernel where N2 splits into two supported factors
     using K2 = void (*)(const C2<T>*, C2<T>*, long, const C2<T>*, int, int, int, const C2<T>*, T, C2<T>*);
     K2 k2 = nullptr;
     int nthr = 0;
-    // float-float and FP64 at N2 = 100: the map-spectrum tile prefetched into L2, or staged in
-    // shared memory (chosen per map size by the autotuner, or pinned with mlc_ctx_tune_set)
+    // float-float at N2 = 100: the map-spectrum tile prefetched into L2, or staged in shared
+    // memory (chosen per map size by the autotuner, or pinned with mlc_ctx_tune_set)
     K2 k2s = nullptr;
     if constexpr (sizeof(C2<T>) == 16)
       if (p.N2 == 100) k2s = k_conv_fused2<T, CW, 10, 10, true>;
@@ -1097,7 +1145,7 @@ void conv_fused_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, const d
       }
       MLC_CHECK_LAUNCH();
       launch_colpass<T, true>(ctx, p, tmp, 'A', 0);
-      if (!spec_out) launch_rows_c2r<T>(ctx, p, tmp, out);
+      if (!spec_out) real_rows<T>(ctx, p, tmp, out);
       return;
     }
   }
@@ -1112,7 +1160,7 @@ void conv_fused_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, const d
   }
   MLC_CHECK_LAUNCH();
   launch_colpass<T, true>(ctx, p, tmp, 'A', 0);
-  if (!spec_out) launch_rows_c2r<T>(ctx, p, tmp, out);
+  if (!spec_out) real_rows<T>(ctx, p, tmp, out);
 }
 
 // P1's register kernel in mode MODE for the plan's N2 (nullptr where there is none): the
@@ -1133,8 +1181,7 @@ static auto p1_mode_kernel(int N2, int& nthr) {
 
 template <typename T>
 bool profile_spectrum_supported_impl(const FftPlan2D& p) {
-  int nthr = 0;
-  return p1_mode_kernel<T, 1>(p.N2, nthr) != nullptr;
+  return p.N2 == 100 || p.N2 == 128;
 }
 
 // The profile's spectrum as P1 holds it before the product (P0, then P1 up to forward
@@ -1144,21 +1191,25 @@ void profile_spectrum_impl(mlc_ctx* ctx, const FftPlan2D& p, const double* prof,
   constexpr int CW = strip_width<T>();
   const int h = pN / 2;
   MLC_REQUIRE(pN % 2 == 0 && 2 * h <= p.Ny && 2 * h <= p.Nx, MLC_ERR_LIMIT, "profile raster larger than the map");
-  int nthr = 0;
-  const auto k = p1_mode_kernel<T, 1>(p.N2, nthr);
-  MLC_REQUIRE(k != nullptr, MLC_ERR_LIMIT, "no cached profile spectra for this map size");
-  void* kx = ws_get(ctx, WS_KX, (size_t)(2 * h > 0 ? 2 * h : 1) * p.Wp * sizeof(C2<T>));
-  launch_rows_r2c<T>(ctx, p, ProfileRows<T>{prof, pN, h, p.Nx}, 2 * h, kx);
-  const size_t smem = ((size_t)p.N2 * CW + p.N1 + 2 * (size_t)p.N2) * sizeof(C2<T>);
-  set_max_smem((const void*)k, smem);
-  const T scale = (T)(1.0 / ((double)p.Nx * (double)p.Ny));  // stored with the spectrum
-  {
-    MLC_KSCOPE(ctx, "conv_profile_spectrum");
-    k<<<dim3(ceil_div(p.Wc, CW), p.N1), nthr, smem, ctx->stream>>>(nullptr, nullptr, p.Wp, (const C2<T>*)kx, h,
-                                                                     p.Ny, p.N1, (const C2<T>*)p.twy, scale,
-                                                                     (C2<T>*)ks);
+  MLC_REQUIRE(profile_spectrum_supported_impl<T>(p), MLC_ERR_LIMIT, "no cached profile spectra for this map size");
+  void* kx = ws_get(ctx, WS_KX, profile_rows_bytes<T>(p, 2 * h));
+  profile_rows<T>(ctx, p, prof, pN, kx);
+  if constexpr (std::is_same<T, double>::value) {
+    limb3_conv_profile(ctx, p, kx, h, ks);
+  } else {
+    int nthr = 0;
+    const auto k = p1_mode_kernel<T, 1>(p.N2, nthr);
+    const size_t smem = ((size_t)p.N2 * CW + p.N1 + 2 * (size_t)p.N2) * sizeof(C2<T>);
+    set_max_smem((const void*)k, smem);
+    const T scale = (T)(1.0 / ((double)p.Nx * (double)p.Ny));  // stored with the spectrum
+    {
+      MLC_KSCOPE(ctx, "conv_profile_spectrum");
+      k<<<dim3(ceil_div(p.Wc, CW), p.N1), nthr, smem, ctx->stream>>>(nullptr, nullptr, p.Wp, (const C2<T>*)kx, h,
+                                                                       p.Ny, p.N1, (const C2<T>*)p.twy, scale,
+                                                                       (C2<T>*)ks);
+    }
+    MLC_CHECK_LAUNCH();
   }
-  MLC_CHECK_LAUNCH();
 }
 
 // conv_fused_impl up to P2 (the inverse half-spectrum into spec_out) from a profile
@@ -1167,19 +1218,27 @@ void profile_spectrum_impl(mlc_ctx* ctx, const FftPlan2D& p, const double* prof,
 template <typename T>
 void conv_cached_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, const void* ks, void* spec_out) {
   constexpr int CW = strip_width<T>();
-  int nthr = 0;
-  const auto k = p1_mode_kernel<T, 2>(p.N2, nthr);
-  MLC_REQUIRE(k != nullptr, MLC_ERR_LIMIT, "no cached profile spectra for this map size");
-  const T scale = (T)(1.0 / ((double)p.Nx * (double)p.Ny));
-  const size_t smem = ((size_t)p.N2 * CW + p.N1 + 2 * (size_t)p.N2) * sizeof(C2<T>);
-  set_max_smem((const void*)k, smem);
-  {
-    MLC_KSCOPE(ctx, "conv_cached_spectrum");
-    k<<<dim3(ceil_div(p.Wc, CW), p.N1), nthr, smem, ctx->stream>>>((const C2<T>*)Fmap, (C2<T>*)spec_out, p.Wp,
-                                                                     nullptr, 0, p.Ny, p.N1, (const C2<T>*)p.twy,
-                                                                     scale, (C2<T>*)ks);
+  MLC_REQUIRE(profile_spectrum_supported_impl<T>(p), MLC_ERR_LIMIT, "no cached profile spectra for this map size");
+  if constexpr (std::is_same<T, double>::value) {
+    limb3_conv_cached(ctx, p, Fmap, spec_out, ks);
+  } else {
+    bool done = false;
+    if constexpr (std::is_same<T, ff>::value) done = p.prec == PREC_FFS && limb2_conv_cached(ctx, p, Fmap, spec_out, ks);
+    if (!done) {
+      int nthr = 0;
+      const auto k = p1_mode_kernel<T, 2>(p.N2, nthr);
+      const T scale = (T)(1.0 / ((double)p.Nx * (double)p.Ny));
+      const size_t smem = ((size_t)p.N2 * CW + p.N1 + 2 * (size_t)p.N2) * sizeof(C2<T>);
+      set_max_smem((const void*)k, smem);
+      {
+        MLC_KSCOPE(ctx, "conv_cached_spectrum");
+        k<<<dim3(ceil_div(p.Wc, CW), p.N1), nthr, smem, ctx->stream>>>((const C2<T>*)Fmap, (C2<T>*)spec_out, p.Wp,
+                                                                         nullptr, 0, p.Ny, p.N1, (const C2<T>*)p.twy,
+                                                                         scale, (C2<T>*)ks);
+      }
+      MLC_CHECK_LAUNCH();
+    }
   }
-  MLC_CHECK_LAUNCH();
   launch_colpass<T, true>(ctx, p, spec_out, 'A', 0);
 }
 
@@ -1188,7 +1247,7 @@ template <typename T>
 void conv_cached_real_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, const void* ks, void* out) {
   void* tmp = ws_get(ctx, WS_SPEC_TMP, p.spec_bytes());
   conv_cached_impl<T>(ctx, p, Fmap, ks, tmp);
-  launch_rows_c2r<T>(ctx, p, tmp, out);
+  real_rows<T>(ctx, p, tmp, out);
 }
 
 template <typename T>
@@ -1204,7 +1263,8 @@ void conv_plain_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, const d
     k_wrap_full<T><<<grid, 256, 0, ctx->stream>>>(prof, pN, p.Nx, p.Ny, (T*)kreal);
   }
   MLC_CHECK_LAUNCH();
-  forward_impl<T>(ctx, p, kreal, sizeof(T) == 8 ? MLC_F64 : MLC_F32, kspec);
+  // (its own transforms stay in the map's precision: this form is what the fused one is measured against)
+  forward_passes<T>(ctx, p, kreal, sizeof(T) == 8 ? MLC_F64 : MLC_F32, kspec, false);
   const long n = (long)p.Ny * p.Wp;
   const T scale = (T)(1.0 / ((double)p.Nx * (double)p.Ny));
   grid = (int)std::min<long>((n + 255) / 256, (long)ctx->sm_count * 16);
@@ -1213,8 +1273,8 @@ void conv_plain_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, const d
     k_multiply<T><<<grid, 256, 0, ctx->stream>>>((const C2<T>*)Fmap, (C2<T>*)kspec, n, scale);
   }
   MLC_CHECK_LAUNCH();
-  launch_colpass<T, true>(ctx, p, kspec, 'B', 1);
-  launch_colpass<T, true>(ctx, p, kspec, 'A', 0);
+  launch_colpass<T, true>(ctx, p, kspec, 'B', 1, false);
+  launch_colpass<T, true>(ctx, p, kspec, 'A', 0, false);
   launch_rows_c2r<T>(ctx, p, kspec, out);
 }
 

@@ -1,0 +1,398 @@
+// Fixed-grid sums of two or three FP32 numbers ("limbs") for the transforms.
+//
+// GB300 issues FP32 about sixty times faster than FP64 (measured: 39 against 0.63 T
+// operations/s), and a Fourier transform is mostly additions.  A float-float sum needs the
+// two-sum (8 FP32 operations) because its parts float: where the exponents of the operands
+// are not known, the rounding error of the high parts has to be recovered.  Here every value
+// of one transform is first scaled by one power of two so that |x| < 1, and its high limb
+// is a multiple of one fixed grid, 2^-22.  High limbs then add exactly in a single FP32
+// addition, and a sum costs one addition per limb:
+//
+//   lf2  h (multiple of 2^-22) + l                          two limbs, about 46 bits
+//   lf3  h (multiple of 2^-22) + m (multiple of 2^-39) + l   three limbs, about 62 bits
+//
+// Why |x| < 1 holds throughout a transform: the scale comes from S, the sum of |re| + |im|
+// over all of its inputs, and every intermediate value of an FFT is a sum of distinct inputs
+// times factors of modulus one, so its modulus is at most S -- whatever the inputs.  The
+// absolute error of an operation is about 2^-46 S (lf2) or 2^-62 S (lf3); against the
+// rms of the values that is about 2^-40 and 2^-56 in the passes here, so lf2 results
+// rounded to FP32 and lf3 results rounded to FP64 carry the rounding of the last step.
+//
+// Products return to the grid with the additive constant 3 = 1.5 * 2: t = 3 + x c is
+// rounded to 2^-22 (t lies in [2, 4)), t - 3 is the high limb, and fma(x, c, -(t - 3)) is the
+// rest, exactly.  The same with 1.5 * 2^-16 for the second limb.  All operations are
+// explicitly rounded intrinsics: nothing may be contracted or reassociated.
+#pragma once
+
+#include "mlc_common.cuh"
+
+namespace mlc {
+
+constexpr float LIMB_G1 = 3.0f;         // 1.5 * 2: rounds to multiples of 2^-22
+constexpr float LIMB_G2 = 0x1.8p-16f;   // rounds to multiples of 2^-39
+constexpr float LIMB_G3 = 0x1.8p-39f;   // rounds to multiples of 2^-62
+
+struct lf2 {
+  float h, l;
+  lf2() = default;
+  __host__ __device__ constexpr lf2(float h_, float l_) : h(h_), l(l_) {}
+  __host__ __device__ constexpr lf2(double d) : h((float)d), l((float)(d - (double)(float)d)) {}
+};
+
+// A constant's high limb is cut to multiples of 2^-24, so that its product with a value's
+// high limb leaves an exact remainder.
+__host__ __device__ constexpr double limb_cut24(double d) {
+  return (double)(long long)(d * 16777216.0 + (d < 0 ? -0.5 : 0.5)) / 16777216.0;
+}
+
+struct lf3 {
+  float h, m, l;
+  lf3() = default;
+  __host__ __device__ constexpr lf3(float h_, float m_, float l_) : h(h_), m(m_), l(l_) {}
+  __host__ __device__ constexpr lf3(double d)
+      : h((float)limb_cut24(d)),
+        m((float)(d - limb_cut24(d))),
+        l((float)((d - limb_cut24(d)) - (double)(float)(d - limb_cut24(d)))) {}
+};
+
+template <>
+struct C2<lf3> {
+  lf3 x, y;
+};
+
+template <typename T>
+struct is_limb {
+  static constexpr bool value = false;
+};
+template <>
+struct is_limb<lf2> {
+  static constexpr bool value = true;
+};
+template <>
+struct is_limb<lf3> {
+  static constexpr bool value = true;
+};
+
+// ---------------------------------------------------------------- lf2
+
+__device__ __forceinline__ lf2 operator+(lf2 a, lf2 b) { return lf2(__fadd_rn(a.h, b.h), __fadd_rn(a.l, b.l)); }
+__device__ __forceinline__ lf2 operator-(lf2 a, lf2 b) { return lf2(__fsub_rn(a.h, b.h), __fsub_rn(a.l, b.l)); }
+__device__ __forceinline__ lf2 operator-(lf2 a) { return lf2(-a.h, -a.l); }
+__device__ __forceinline__ lf2 operator*(lf2 a, lf2 b) {
+  const float h = __fsub_rn(__fmaf_rn(a.h, b.h, LIMB_G1), LIMB_G1);
+  float e = __fmaf_rn(a.h, b.h, -h);
+  e = __fmaf_rn(a.h, b.l, e);
+  return lf2(h, __fmaf_rn(a.l, b.h, e));
+}
+__device__ __forceinline__ lf2 scale2(lf2 a, float s) {
+  const float h = __fsub_rn(__fmaf_rn(a.h, s, LIMB_G1), LIMB_G1);
+  return lf2(h, __fmaf_rn(a.l, s, __fmaf_rn(a.h, s, -h)));
+}
+// c x + d y with one trip over the grid (12 operations).  NORM carries what has gathered in
+// the low limb back into the high one (3 more).
+template <bool NORM>
+__device__ __forceinline__ lf2 limb_lin2(lf2 c, lf2 x, lf2 d, lf2 y) {
+  const float t1 = __fmaf_rn(c.h, x.h, LIMB_G1), t2 = __fmaf_rn(d.h, y.h, t1);
+  float e = __fmaf_rn(c.h, x.h, -__fsub_rn(t1, LIMB_G1));
+  float f = __fmaf_rn(d.h, y.h, -__fsub_rn(t2, t1));
+  e = __fmaf_rn(c.l, x.h, e);
+  f = __fmaf_rn(d.l, y.h, f);
+  e = __fmaf_rn(c.h, x.l, e);
+  f = __fmaf_rn(d.h, y.l, f);
+  e = __fadd_rn(e, f);
+  if (!NORM) return lf2(__fsub_rn(t2, LIMB_G1), e);
+  const float t3 = __fadd_rn(t2, e);
+  return lf2(__fsub_rn(t3, LIMB_G1), __fsub_rn(e, __fsub_rn(t3, t2)));
+}
+__device__ __forceinline__ lf2 limb_norm(lf2 a) {
+  const float q = __fsub_rn(__fadd_rn(a.l, LIMB_G1), LIMB_G1);
+  return lf2(__fadd_rn(a.h, q), __fsub_rn(a.l, q));
+}
+
+// ---------------------------------------------------------------- lf3
+
+__device__ __forceinline__ lf3 operator+(lf3 a, lf3 b) {
+  return lf3(__fadd_rn(a.h, b.h), __fadd_rn(a.m, b.m), __fadd_rn(a.l, b.l));
+}
+__device__ __forceinline__ lf3 operator-(lf3 a, lf3 b) {
+  return lf3(__fsub_rn(a.h, b.h), __fsub_rn(a.m, b.m), __fsub_rn(a.l, b.l));
+}
+__device__ __forceinline__ lf3 operator-(lf3 a) { return lf3(-a.h, -a.m, -a.l); }
+__device__ __forceinline__ lf3 operator*(lf3 a, lf3 b) {
+  const float h = __fsub_rn(__fmaf_rn(a.h, b.h, LIMB_G1), LIMB_G1);
+  const float r = __fmaf_rn(a.h, b.h, -h);  // a multiple of 2^-46 below 2^-22: exact
+  const float u0 = __fadd_rn(r, LIMB_G2), u1 = __fmaf_rn(a.h, b.m, u0), u2 = __fmaf_rn(a.m, b.h, u1);
+  float e = __fsub_rn(r, __fsub_rn(u0, LIMB_G2));
+  float f = __fmaf_rn(a.h, b.m, -__fsub_rn(u1, u0));
+  f = __fadd_rn(f, __fmaf_rn(a.m, b.h, -__fsub_rn(u2, u1)));
+  e = __fmaf_rn(a.h, b.l, e);
+  f = __fmaf_rn(a.l, b.h, f);
+  e = __fmaf_rn(a.m, b.m, e);
+  return lf3(h, __fsub_rn(u2, LIMB_G2), __fadd_rn(e, f));
+}
+// s a power of two, at least 2^-16: the remainder of the high limb is on the second grid.
+__device__ __forceinline__ lf3 scale2(lf3 a, float s) {
+  const float h = __fsub_rn(__fmaf_rn(a.h, s, LIMB_G1), LIMB_G1);
+  const float r = __fmaf_rn(a.h, s, -h);
+  const float p = __fsub_rn(__fmaf_rn(a.m, s, LIMB_G2), LIMB_G2);
+  return lf3(h, __fadd_rn(r, p), __fmaf_rn(a.l, s, __fmaf_rn(a.m, s, -p)));
+}
+// c x + d y (34 operations).  NORM carries the lower limbs' excess upwards (6 more): between
+// two carries a limb may gather up to 2^7 of its own grid steps, the exact range of an FP32
+// addition, so every twiddle product carries and the additions between them do not.
+template <bool NORM>
+__device__ __forceinline__ lf3 limb_lin2(lf3 c, lf3 x, lf3 d, lf3 y) {
+  const float t1 = __fmaf_rn(c.h, x.h, LIMB_G1), t2 = __fmaf_rn(d.h, y.h, t1);
+  const float r = __fadd_rn(__fmaf_rn(c.h, x.h, -__fsub_rn(t1, LIMB_G1)), __fmaf_rn(d.h, y.h, -__fsub_rn(t2, t1)));
+  const float u0 = __fadd_rn(r, LIMB_G2), u1 = __fmaf_rn(c.m, x.h, u0), u2 = __fmaf_rn(c.h, x.m, u1);
+  const float u3 = __fmaf_rn(d.m, y.h, u2), u4 = __fmaf_rn(d.h, y.m, u3);
+  float e = __fsub_rn(r, __fsub_rn(u0, LIMB_G2));
+  float f = __fmaf_rn(c.m, x.h, -__fsub_rn(u1, u0));
+  e = __fadd_rn(e, __fmaf_rn(c.h, x.m, -__fsub_rn(u2, u1)));
+  f = __fadd_rn(f, __fmaf_rn(d.m, y.h, -__fsub_rn(u3, u2)));
+  e = __fadd_rn(e, __fmaf_rn(d.h, y.m, -__fsub_rn(u4, u3)));
+  e = __fmaf_rn(c.l, x.h, e);
+  f = __fmaf_rn(d.l, y.h, f);
+  e = __fmaf_rn(c.m, x.m, e);
+  f = __fmaf_rn(d.m, y.m, f);
+  e = __fmaf_rn(c.h, x.l, e);
+  f = __fmaf_rn(d.h, y.l, f);
+  e = __fadd_rn(e, f);
+  if (!NORM) return lf3(__fsub_rn(t2, LIMB_G1), __fsub_rn(u4, LIMB_G2), e);
+  const float u5 = __fadd_rn(u4, e);
+  const float m = __fsub_rn(u5, LIMB_G2), t3 = __fadd_rn(t2, m);
+  return lf3(__fsub_rn(t3, LIMB_G1), __fsub_rn(m, __fsub_rn(t3, t2)), __fsub_rn(e, __fsub_rn(u5, u4)));
+}
+__device__ __forceinline__ lf3 limb_norm(lf3 a) {
+  const float q = __fsub_rn(__fadd_rn(a.l, LIMB_G2), LIMB_G2);
+  const float m = __fadd_rn(a.m, q);
+  const float p = __fsub_rn(__fadd_rn(m, LIMB_G1), LIMB_G1);
+  return lf3(__fadd_rn(a.h, p), __fsub_rn(m, p), __fsub_rn(a.l, q));
+}
+
+// ---------------------------------------------------------------- complex products
+
+// a x + b y of the small DFTs' constants: the limb forms make one trip over the grid.
+template <typename T>
+__device__ __forceinline__ T lin2(T a, T x, T b, T y) {
+  return a * x + b * y;
+}
+__device__ __forceinline__ lf2 lin2(lf2 a, lf2 x, lf2 b, lf2 y) { return limb_lin2<false>(a, x, b, y); }
+__device__ __forceinline__ lf3 lin2(lf3 a, lf3 x, lf3 b, lf3 y) { return limb_lin2<false>(a, x, b, y); }
+
+// v w or v conj(w) with the carry of limb_lin2 where NORM (lf3: always).
+template <bool CONJ, bool NORM, typename T>
+__device__ __forceinline__ C2<T> limb_tw(C2<T> v, C2<T> w) {
+  constexpr bool N = NORM || sizeof(T) == sizeof(lf3);
+  if (CONJ) return C2<T>{limb_lin2<N>(w.x, v.x, w.y, v.y), limb_lin2<N>(w.x, v.y, -w.y, v.x)};
+  return C2<T>{limb_lin2<N>(w.x, v.x, -w.y, v.y), limb_lin2<N>(w.x, v.y, w.y, v.x)};
+}
+template <typename T>
+__device__ __forceinline__ C2<T> limb_cnorm(C2<T> v) {
+  return C2<T>{limb_norm(v.x), limb_norm(v.y)};
+}
+
+// ---------------------------------------------------------------- scale of one transform
+
+// Partial sum of |re| + |im| over the inputs of one transform.  FP64: s 2^(e - 1023) with
+// the exponent field e kept apart (in place, bits 20..30), s from the high words alone.
+template <typename S>
+struct LimbSum;
+template <>
+struct LimbSum<ff> {
+  float s;
+};
+template <>
+struct LimbSum<double> {
+  int e;
+  float s;
+};
+
+// 2^(a - b) for exponent fields a <= b in place (bits 20..30); 0 where it underflows FP32.
+__device__ __forceinline__ float limb_pow_diff(int a, int b) {
+  return __int_as_float(max(a - b + (127 << 20), 0) << 3);
+}
+template <int N>
+__device__ __forceinline__ LimbSum<ff> limb_sum(const C2<ff>* v) {
+  float s = 0.f;
+#pragma unroll
+  for (int i = 0; i < N; i++) s = __fadd_rn(s, __fadd_rn(fabsf(v[i].x.hi), fabsf(v[i].y.hi)));
+  return LimbSum<ff>{s};
+}
+template <int N>
+__device__ __forceinline__ LimbSum<double> limb_sum(const C2<double>* v) {
+  int top = 0;
+#pragma unroll
+  for (int i = 0; i < N; i++)
+    top = max(top, max(__double2hiint(v[i].x) & 0x7fffffff, __double2hiint(v[i].y) & 0x7fffffff));
+  const int e = top & 0x7ff00000;
+  float s = 0.f;
+#pragma unroll
+  for (int i = 0; i < N; i++) {
+    s = __fadd_rn(s, limb_pow_diff(__double2hiint(v[i].x) & 0x7fffffff, e));
+    s = __fadd_rn(s, limb_pow_diff(__double2hiint(v[i].y) & 0x7fffffff, e));
+  }
+  return LimbSum<double>{e, s};
+}
+__device__ __forceinline__ LimbSum<ff> limb_sum_add(LimbSum<ff> a, LimbSum<ff> b) {
+  return LimbSum<ff>{__fadd_rn(a.s, b.s)};
+}
+__device__ __forceinline__ LimbSum<double> limb_sum_add(LimbSum<double> a, LimbSum<double> b) {
+  const int e = max(a.e, b.e);
+  return LimbSum<double>{e, __fmaf_rn(a.s, limb_pow_diff(a.e, e), __fmul_rn(b.s, limb_pow_diff(b.e, e)))};
+}
+__device__ __forceinline__ LimbSum<ff> limb_sum_warp(LimbSum<ff> a) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) a.s = __fadd_rn(a.s, __shfl_xor_sync(0xffffffffu, a.s, o));
+  return a;
+}
+__device__ __forceinline__ LimbSum<double> limb_sum_warp(LimbSum<double> a) {
+  const int e = __reduce_max_sync(0xffffffffu, a.e);
+  a.s = __fmul_rn(a.s, limb_pow_diff(a.e, e));
+  a.e = e;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) a.s = __fadd_rn(a.s, __shfl_xor_sync(0xffffffffu, a.s, o));
+  return a;
+}
+
+// The power of two that brings a transform below 1/2 and back.  lf2: two FP32 factors;
+// lf3: the exponent fields to add to a double before its conversion to a 62-bit fixed-point
+// integer and after the way back.  A sum that is not finite makes every output NaN.
+template <typename T>
+struct LimbScale;
+template <>
+struct LimbScale<lf2> {
+  float down, up;
+};
+template <>
+struct LimbScale<lf3> {
+  int e;  // x < 2^(e - 1)
+  bool bad;
+};
+// extra: the transform's values may grow to 2^extra times the sum.  lf2 takes the least power of
+// two above the sum; lf3 one more, as limb_out needs |x| < 1 and the sum is cut to high words.
+__device__ __forceinline__ LimbScale<lf2> limb_scale(LimbSum<ff> a, int extra) {
+  const int b = __float_as_int(a.s) >> 23;  // (a.s >= 0, so no sign bit)
+  if (b >= 255) return LimbScale<lf2>{__int_as_float(0x7fffffff), __int_as_float(0x7fffffff)};
+  const int e = min(max(b - 127 + 1 + extra, -100), 126);
+  return LimbScale<lf2>{__int_as_float((127 - e) << 23), __int_as_float((127 + e) << 23)};
+}
+// (values below 2^-1022 of a transform whose sum is below 2^-960 count as zero)
+__device__ __forceinline__ LimbScale<lf3> limb_scale(LimbSum<double> a, int extra) {
+  const int e = (a.e >> 20) - 1023 + ((__float_as_int(a.s) >> 23) - 127) + 2 + extra;
+  return LimbScale<lf3>{max(e, -960), a.e >= 0x7ff00000};
+}
+
+// ---------------------------------------------------------------- in and out
+
+__device__ __forceinline__ lf2 limb_in(ff v, LimbScale<lf2> s) {
+  const float hi = __fmul_rn(v.hi, s.down);
+  const float h = __fsub_rn(__fadd_rn(hi, LIMB_G1), LIMB_G1);
+  return lf2(h, __fmaf_rn(v.lo, s.down, __fsub_rn(hi, h)));
+}
+__device__ __forceinline__ ff limb_out(lf2 v, LimbScale<lf2> s) {
+  return ff(__fmul_rn(v.h, s.up), __fmul_rn(v.l, s.up));
+}
+__device__ __forceinline__ float limb_round(lf2 v, LimbScale<lf2> s) { return __fmul_rn(__fadd_rn(v.h, v.l), s.up); }
+
+// FP64 in: the exponent moved by an integer addition, one conversion to a fixed-point
+// integer of 62 fractional bits, and its bit fields 22 | 17 | 23 as the three limbs.
+__device__ __forceinline__ lf3 limb_in(double v, LimbScale<lf3> s) {
+  const int hi = __double2hiint(v), d = (62 - s.e) << 20;
+  const int ex = hi & 0x7ff00000;
+  const bool z = ex == 0 || ex + d <= 0;
+  const long long q = __double2ll_rn(z ? 0.0 : __hiloint2double(hi + d, __double2loint(v)));
+  const int qh = (int)(q >> 32);
+  const unsigned ql = (unsigned)q;
+  const float h = __fsub_rn(__int_as_float(0x40400000 + (qh >> 8)), LIMB_G1);
+  const float m = __fsub_rn(__int_as_float(0x37800000 | (int)(__funnelshift_r(ql, (unsigned)qh, 23) & 0x1ffffu)), 0x1p-16f);
+  const float l = __fsub_rn(__int_as_float(0x2C000000 | (int)(ql & 0x7fffffu)), 0x1p-39f);
+  return lf3(h, m, l);
+}
+__device__ __forceinline__ double limb_out(lf3 v, LimbScale<lf3> s) {
+  const float c = __fsub_rn(__fadd_rn(v.l, LIMB_G2), LIMB_G2);
+  const float mm = __fadd_rn(v.m, c), ll = __fsub_rn(v.l, c);
+  const int ih = __float_as_int(__fadd_rn(v.h, LIMB_G1)) - 0x40400000;
+  const int im = __float_as_int(__fadd_rn(mm, LIMB_G2)) - 0x37C00000;
+  const int il = __float_as_int(__fadd_rn(ll, LIMB_G3)) - 0x2C400000;
+  const long long q = ((long long)ih << 40) + ((long long)im << 23) + il;
+  const double d = __ll2double_rn(q);
+  if (s.bad) return __longlong_as_double(0x7ff8000000000000ll);
+  const int hi = __double2hiint(d), ex = hi & 0x7ff00000, r = ex + ((s.e - 62) << 20);
+  if (ex == 0 || r <= 0) return 0.0;
+  if (r >= 0x7ff00000) return __hiloint2double((hi & 0x80000000) | 0x7ff00000, 0);
+  return __hiloint2double(hi + ((s.e - 62) << 20), __double2loint(d));
+}
+__device__ __forceinline__ double limb_round(lf3 v, LimbScale<lf3> s) { return limb_out(v, s); }
+
+template <typename S, typename T>
+__device__ __forceinline__ C2<T> limb_cin(C2<S> v, LimbScale<T> s) {
+  return C2<T>{limb_in(v.x, s), limb_in(v.y, s)};
+}
+template <typename S, typename T>
+__device__ __forceinline__ C2<S> limb_cout(C2<T> v, LimbScale<T> s) {
+  return C2<S>{limb_out(v.x, s), limb_out(v.y, s)};
+}
+
+// ---------------------------------------------------------------- arrays of limbs
+
+// Complex limbs in shared memory: lf2 as one 16-byte word, lf3 as 16 bytes (high and middle
+// limbs) and 8 bytes (low limbs) in two planes, so that every access is one aligned vector.
+template <typename T>
+struct LimbArr {
+  C2<T>* p;
+  static __host__ __device__ constexpr size_t bytes(long n) { return (size_t)n * sizeof(C2<T>); }
+  static __device__ __forceinline__ LimbArr at(unsigned char* raw, long) { return LimbArr{reinterpret_cast<C2<T>*>(raw)}; }
+  __device__ __forceinline__ C2<T> ld(int i) const { return p[i]; }
+  __device__ __forceinline__ void st(int i, C2<T> v) const { p[i] = v; }
+};
+template <>
+struct LimbArr<lf3> {
+  float4* a;
+  float2* b;
+  static __host__ __device__ constexpr size_t bytes(long n) { return (size_t)((n + 1) & ~1L) * 24; }
+  static __device__ __forceinline__ LimbArr at(unsigned char* raw, long n) {
+    return LimbArr{reinterpret_cast<float4*>(raw), reinterpret_cast<float2*>(raw + (size_t)((n + 1) & ~1L) * 16)};
+  }
+  __device__ __forceinline__ C2<lf3> ld(int i) const {
+    const float4 u = a[i];
+    const float2 v = b[i];
+    return C2<lf3>{lf3(u.x, u.z, v.x), lf3(u.y, u.w, v.y)};
+  }
+  __device__ __forceinline__ void st(int i, C2<lf3> v) const {
+    a[i] = make_float4(v.x.h, v.y.h, v.x.m, v.y.m);
+    b[i] = make_float2(v.x.l, v.y.l);
+  }
+};
+
+// Twiddle tables in global memory: the float-float table for ff and lf2, two planes for lf3.
+template <typename T>
+struct LimbTab;
+template <>
+struct LimbTab<ff> {
+  const float4* p;
+  __device__ __forceinline__ C2<ff> ld(long i) const {
+    const float4 v = __ldg(p + i);
+    return C2<ff>{ff(v.x, v.y), ff(v.z, v.w)};
+  }
+};
+template <>
+struct LimbTab<lf2> {
+  const float4* p;
+  __device__ __forceinline__ C2<lf2> ld(long i) const {
+    const float4 v = __ldg(p + i);
+    return C2<lf2>{lf2(v.x, v.y), lf2(v.z, v.w)};
+  }
+};
+template <>
+struct LimbTab<lf3> {
+  const float4* a;
+  const float2* b;
+  __device__ __forceinline__ C2<lf3> ld(long i) const {
+    const float4 u = __ldg(a + i);
+    const float2 v = __ldg(b + i);
+    return C2<lf3>{lf3(u.x, u.z, v.x), lf3(u.y, u.w, v.y)};
+  }
+};
+
+}  // namespace mlc

@@ -26,10 +26,20 @@ struct FftPlan2D {
   RadixList rlM{}, rlN1{}, rlN2{};
   void* twx = nullptr;  // Nx-entry table exp(-2 pi i m / Nx)
   void* twy = nullptr;  // Ny-entry table exp(-2 pi i m / Ny)
+  void* twx3 = nullptr;  // the same tables in three limbs (FP64 plans; see LimbTab)
+  void* twy3 = nullptr;
+  void* twl3 = nullptr;  // W_M^(m q), [q - 1][m]: level 0 of the row transforms (limb_first_radix)
   size_t elem = 0;      // sizeof(C2<T>)
   size_t spec_bytes() const { return (size_t)Ny * Wp * elem; }
   ~FftPlan2D();
 };
+
+// First radix of the limb row transforms of M points (fft_limb.cuh), 0 where there is none.
+inline int limb_first_radix(int M) { return M == 5000 || M == 1000 ? 10 : M == 4096 || M == 2000 ? 8 : 0; }
+inline int limb_level0_entries(int M) {
+  const int r = limb_first_radix(M);
+  return r ? (r - 1) * (M / r) : 0;
+}
 
 // Internal plan precisions (mlc_map_set_fft): FFTs in float-float arithmetic of FP64 maps
 // (FP64 outputs), and of FP32 maps (float-float spectra, FP32 outputs).
@@ -205,9 +215,10 @@ void selftest_wait_timeout(mlc_ctx* ctx, unsigned polls, unsigned* report_host);
 bool p1_staged_choice(mlc_ctx* ctx, const FftPlan2D& p, const std::function<void(bool)>& run);
 // Cached profile spectra: the profile's spectrum as the fused convolution's P1 holds it
 // before the product with the map spectrum (Ny x Wp complex of the plan's arithmetic, the
-// map spectrum's layout), and conv_fused_spectrum starting from it.  Supported where P1 has
-// its register form for N2 = 100 or 128.
+// map spectrum's layout; profile_spectrum_bytes), and conv_fused_spectrum starting from it.
+// Supported where P1 has its register form for N2 = 100 or 128.
 bool profile_spectrum_supported(const FftPlan2D& p);
+size_t profile_spectrum_bytes(const FftPlan2D& p);
 void profile_spectrum(mlc_ctx* ctx, const FftPlan2D& p, const double* prof, int pN, void* ks);
 void conv_cached_spectrum(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, const void* ks, void* spec_out);
 void conv_cached(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, const void* ks, void* out);
@@ -246,6 +257,26 @@ bool c2r_interleave_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* specs, lo
                          void* out, unsigned planar);
 template <typename T, typename TO>
 void rows_c2r_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* spec, void* out);
+
+// The passes in fixed-grid limb arithmetic (fft_limb.cuh): FP64 plans in three limbs, the
+// inverse passes of FP32 maps' float-float plans in two.  Each returns false, with nothing
+// launched, where it has no kernel for the plan's sizes.
+bool limb3_rows_r2c_map(mlc_ctx* ctx, const FftPlan2D& p, const void* in, int in_dtype, void* out);
+bool limb3_rows_r2c_profile(mlc_ctx* ctx, const FftPlan2D& p, const double* prof, int pN, void* out);
+bool limb3_rows_c2r(mlc_ctx* ctx, const FftPlan2D& p, const void* in, void* out);
+bool limb3_rows_c2r_il(mlc_ctx* ctx, const FftPlan2D& p, const void* specs, long spec_stride, int nm, int S,
+                       void* out, unsigned planar);
+bool limb3_colpass(mlc_ctx* ctx, const FftPlan2D& p, void* buf, char kind, bool inverse, int post_tw);
+bool limb3_conv(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, void* out, void* kx, int h);
+bool limb3_conv_profile(mlc_ctx* ctx, const FftPlan2D& p, void* kx, int h, void* ks);
+size_t limb3_profile_spectrum_bytes(const FftPlan2D& p);  // of ks
+bool limb3_conv_cached(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, void* out, const void* ks);
+bool limb2_colpass_inverse(mlc_ctx* ctx, const FftPlan2D& p, void* buf, char kind, int post_tw);
+bool limb2_conv(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, void* out, const void* kx, int h);
+bool limb2_conv_cached(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, void* out, const void* ks);
+bool limb2_rows_c2r(mlc_ctx* ctx, const FftPlan2D& p, const void* in, void* out);
+bool limb2_rows_c2r_il(mlc_ctx* ctx, const FftPlan2D& p, const void* specs, long spec_stride, int nm, int S,
+                       void* out, unsigned planar);
 
 // Host profile rasters (profile.cpp)
 int profile_dims(const mlc_profile& p);

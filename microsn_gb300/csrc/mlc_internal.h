@@ -65,6 +65,7 @@ enum WsSlot {
   WS_BATCH_MAPS,  // convolved maps of one profile group (mlc_convolve_sample_tracks)
   WS_BATCH_IMAP,  // their profile-interleaved copy
   WS_SAMPLE_ORDER,  // the sampler's epoch chunks in map-cell order
+  WS_EXP_TAB,       // 2^(j/4096) of the pair stage's exponentials
   WS_NSLOTS
 };
 

@@ -12,10 +12,12 @@
 #include <vector>
 
 #include "mlc_internal.h"
+#include "radix.cuh"
 
 namespace mlc {
 
 void radix_sort_u64_u32(mlc_ctx* ctx, long n, uint64_t* keys, uint32_t* vals);
+bool radix_sort_range_u64_u32(mlc_ctx* ctx, long n, uint64_t* keys, uint32_t* vals, const unsigned long long* range);
 
 // The key of the reference's z sort (thrust::stable_sort_by_key on doubles, a radix sort):
 // the order of the bit patterns with the sign folded in, -0.0 taken as +0.0 (the radix sort
@@ -32,23 +34,65 @@ __device__ __forceinline__ double value_of(uint64_t k) {
   return __longlong_as_double((k & 0x8000000000000000ull) ? (k & 0x7fffffffffffffffull) : ~k);
 }
 
-// z keys and pair indices for the stable rank sort.
-__global__ void k_pair_z(const double* __restrict__ LCA, const double* __restrict__ LCB, int Nloc, int Nprof,
-                         uint64_t* __restrict__ keys, uint32_t* __restrict__ idx) {
-  const long P = (long)Nloc * Nloc;
-  for (long p = blockIdx.x * (long)blockDim.x + threadIdx.x; p < P; p += (long)gridDim.x * blockDim.x) {
-    const int a = (int)(p / Nloc), b = (int)(p % Nloc);
-    const double z = __ldg(LCA + (long)a * Nprof) / __ldg(LCB + (long)b * Nprof);
-    keys[p] = key_of(z);
-    idx[p] = (uint32_t)p;
+// Correctly rounded a / b from y = 1/b as a pair (yh = RN(1/b), yl the rest): q = RN(a yh +
+// RN(a yl)) is within one ulp of a/b, its residual a - q b is exact with an FMA, and
+// RN(q + r yh) is then the correctly rounded quotient (Markstein's theorem; the first step as
+// in Brisebarre, Muller and Raina, "Accelerating correctly rounded floating-point division
+// when the divisor is known in advance", IEEE Trans. Comput. 53, 2004).  Four FP64 operations
+// instead of a division's dozen, for operands of moderate exponent (no step over- or
+// underflows); others divide.
+struct Reciprocal {
+  double b, h, l;
+  bool plain;
+  static __device__ __forceinline__ bool moderate(double v) {
+    const int e = (__double2hiint(v) >> 20) & 0x7ff;
+    return e > 1023 - 400 && e < 1023 + 400;
   }
+  __device__ __forceinline__ explicit Reciprocal(double b_) : b(b_) {
+    plain = !moderate(b);
+    h = 1.0 / b;
+    l = h * __fma_rn(-b, h, 1.0);
+  }
+  __device__ __forceinline__ double quotient(double a) const {
+    if (plain || !moderate(a)) return a / b;
+    const double q = __fma_rn(a, h, __dmul_rn(a, l));
+    return __fma_rn(__fma_rn(-q, b, a), h, q);
+  }
+};
+
+// z keys and pair indices for the stable rank sort: a thread per b, Z_ROWS rows a each; and the
+// least key and least ~key of all (range).
+constexpr int Z_ROWS = 32;
+__global__ void __launch_bounds__(256) k_pair_z(const double* __restrict__ LCA, const double* __restrict__ LCB, int Nloc,
+                                                int Nprof, uint64_t* __restrict__ keys, uint32_t* __restrict__ idx,
+                                                unsigned long long* __restrict__ range) {
+  __shared__ unsigned long long least[2];
+  if (threadIdx.x < 2) least[threadIdx.x] = ~0ull;
+  __syncthreads();
+  const int b = blockIdx.x * 256 + threadIdx.x;
+  if (b < Nloc) {
+    const Reciprocal rb(__ldg(LCB + (long)b * Nprof));
+    const int a1 = min(Nloc, (int)(blockIdx.y + 1) * Z_ROWS);
+    uint64_t lo = ~0ull, nhi = ~0ull;
+    for (int a = blockIdx.y * Z_ROWS; a < a1; a++) {
+      const long p = (long)a * Nloc + b;
+      const uint64_t k = key_of(rb.quotient(__ldg(LCA + (long)a * Nprof)));
+      keys[p] = k;
+      idx[p] = (uint32_t)p;
+      lo = min(lo, k);
+      nhi = min(nhi, ~k);
+    }
+    atomicMin(&least[0], (unsigned long long)lo);
+    atomicMin(&least[1], (unsigned long long)nhi);
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) atomicMin(&range[threadIdx.x], least[threadIdx.x]);
 }
 
 // rank[perm[r]] = r
-__global__ void k_invert_perm(const uint32_t* __restrict__ perm, long P, uint32_t* __restrict__ rank) {
-  for (long r = blockIdx.x * (long)blockDim.x + threadIdx.x; r < P; r += (long)gridDim.x * blockDim.x)
-    rank[perm[r]] = (uint32_t)r;
-}
+struct LoadOwnIndex {
+  __device__ __forceinline__ uint32_t operator()(long i) const { return (uint32_t)i; }
+};
 
 // upper_bound of each edge in the sorted z: the reference's binary search
 // (thrust::upper_bound, gpu_functions.cu:388) step for step -- the same midpoints and the
@@ -69,53 +113,74 @@ __global__ void k_upper_bound(const uint64_t* __restrict__ sorted, long P, const
   upper[i] = (uint32_t)lo;
 }
 
-// mA[i*Nloc + a] = LC[a*Nprof + ind_i] + fac_i * DLC[a*(Nprof-1) + ind_i], or 1 (ind_i = -1);
-// with invert, its correctly rounded reciprocal (the B side: one division per (epoch,
-// location) instead of one per pair)
+// m[i*Nloc + a] = LC[a*Nprof + ind_i] + fac_i * DLC[a*(Nprof-1) + ind_i], or 1 (ind_i = -1).
+// The B side (rho given) as rho_i / m, rho_i = rho[i] + rho[Njp + i], rounded once: one division
+// per (epoch, location) instead of one per pair.
 __global__ void k_interp(const double* __restrict__ LC, const double* __restrict__ DLC, int Nloc, int Nprof,
-                         int Njp, const int* __restrict__ ind, const double* __restrict__ fac, int invert,
-                         double* __restrict__ m) {
+                         int Njp, const int* __restrict__ ind, const double* __restrict__ fac,
+                         const double* __restrict__ rho, double* __restrict__ m) {
   const long n = (long)Nloc * Njp;
   for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) {
     const int i = (int)(q / Nloc), a = (int)(q % Nloc);
     const int k = ind[i];
-    const double v = (k == -1) ? 1.0 : LC[(long)a * Nprof + k] + fac[i] * DLC[(long)a * (Nprof - 1) + k];
-    m[q] = invert ? 1.0 / v : v;
+    double v = (k == -1) ? 1.0 : LC[(long)a * Nprof + k] + fac[i] * DLC[(long)a * (Nprof - 1) + k];
+    if (rho) {
+      const double h = rho[i] / v, r = __fma_rn(-h, v, rho[i]) + rho[Njp + i];
+      // (a quotient that is 0, infinite or NaN has no residual)
+      v = isfinite(h) && h != 0.0 && isfinite(r) ? h + r / v : h;
+    }
+    m[q] = v;
   }
 }
 
-// Point-source values for the fused binning's float pre-search: zA[a] = (float)LCA[a*Nprof],
-// zB[b] = (float)(1 / LCB[b*Nprof]).
-__global__ void k_zfloat(const double* __restrict__ LCA, const double* __restrict__ LCB, int Nloc, int Nprof,
-                         float* __restrict__ zA, float* __restrict__ zB) {
+// Point-source values of the fused binning: the FP64 values z[a], and FP32 ones of z (side A) or
+// 1/z (side B) for the search.
+__global__ void k_zvalues(const double* __restrict__ LC, int Nloc, int Nprof, int invert, double* __restrict__ z,
+                          float* __restrict__ zf) {
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < Nloc; q += gridDim.x * blockDim.x) {
-    zA[q] = (float)LCA[(long)q * Nprof];
-    zB[q] = (float)(1.0 / LCB[(long)q * Nprof]);
+    const double v = LC[(long)q * Nprof];
+    z[q] = v;
+    zf[q] = invert ? (float)(1.0 / v) : (float)v;
   }
 }
-
-struct Chi2Consts {
-  const double* d;
-  const double* s;
+// chi2 of pair (a, b) = sum_i ((d_i - mA_i/mB_i)/s_i)^2 in FP64.  The kernels that sum it are
+// bound by the FP64 pipe (0.63 T operations/s), so each term is two FMAs:
+//   t = ds_i - mA_i B_i,  c += t^2,  ds_i = RN(d_i/s_i),  B_i = RN(rho_i / mB_i),  rho_i = ds_i / d_i
+// (to twice the precision).  d_i/s_i is rounded, but rho_i follows it, so that t = rho_i (d_i -
+// mA_i/mB_i) with the one rounding of B_i inside the difference -- as 1/mB_i's would be -- and
+// a factor rho_i within one ulp of 1/s_i.  Where d_i or s_i is zero, not finite or of an extreme
+// exponent (PLAIN) the terms are (d_i - mA_i RN(1/mB_i)) RN(1/s_i).
+template <bool PLAIN>
+struct RatioChi2 {
+  const double* mA;
+  const double* iB;
+  const double* d;   // ds_i, or d_i
+  const double* is;  // 1 / s_i (PLAIN)
+  int Nloc, Njp;
+  __device__ __forceinline__ double operator()(int a, int b) const {
+    double c = 0.0;
+    for (int i = 0; i < Njp; i++) {
+      double t = __fma_rn(-__ldg(mA + (long)i * Nloc + a), __ldg(iB + (long)i * Nloc + b), __ldg(d + i));
+      if (PLAIN) t *= __ldg(is + i);
+      c = __fma_rn(t, t, c);
+    }
+    return c;
+  }
+  __device__ __forceinline__ double operator()(long p) const {  // pair index a Nloc + b, below 2^32
+    const uint32_t a = (uint32_t)p / (uint32_t)Nloc;
+    return (*this)((int)a, (int)((uint32_t)p - a * (uint32_t)Nloc));
+  }
 };
 
-// One pair per thread: chi2 = sum_i ((d_i - mA_i/mB_i)/s_i)^2 in FP64, the divisions as
-// products with the correctly rounded reciprocals iB_i = 1/mB_i and is_i = 1/s_i (each term
-// within a few ulp of the divided form; GB300's FP64 divide is a long instruction sequence).
-__global__ void __launch_bounds__(256) k_pair_chi2_ratio(const double* __restrict__ mA, const double* __restrict__ iB,
-                                                         int Nloc, int Njp, const double* __restrict__ d,
-                                                         const double* __restrict__ is, const uint32_t* __restrict__ rank,
+// One pair per thread, in pair order, or at its rank.
+template <bool PLAIN>
+__global__ void __launch_bounds__(256) k_pair_chi2_ratio(RatioChi2<PLAIN> f, const uint32_t* __restrict__ rank,
                                                          double* __restrict__ chi2) {
   const int b = blockIdx.x * 32 + (threadIdx.x & 31);
   const int a = blockIdx.y * 8 + (threadIdx.x >> 5);
-  if (a >= Nloc || b >= Nloc) return;
-  double c = 0.0;
-  for (int i = 0; i < Njp; i++) {
-    const double tmp = (__ldg(d + i) - __ldg(mA + (long)i * Nloc + a) * __ldg(iB + (long)i * Nloc + b)) * __ldg(is + i);
-    c += tmp * tmp;
-  }
-  const long p = (long)a * Nloc + b;
-  chi2[rank ? rank[p] : p] = c;
+  if (a >= f.Nloc || b >= f.Nloc) return;
+  const long p = (long)a * f.Nloc + b;
+  chi2[rank ? rank[p] : p] = f(a, b);
 }
 
 // Bin means of the rank-ordered chi2 (bin_chi2_GPU): every bin's slice is cut into pieces
@@ -123,39 +188,85 @@ __global__ void __launch_bounds__(256) k_pair_chi2_ratio(const double* __restric
 // second kernel adds each bin's pieces in order -- a fixed summation order (the result does
 // not depend on timing), and a bin of millions of pairs is spread over many CTAs (one CTA
 // per bin left most SMs idle behind the largest bins).
+//
+// exp(-c/2), the FP64 pipe's largest part of this kernel, from a table: exp(-c/2) =
+// 2^(k/4096) e^r with k = RN(-c 2048/ln 2) and |r| <= ln 2/8192, where three terms of the
+// series for e^r - 1 leave less than 2^-58; 2^(j/4096) for the 4096 fractions lies in shared
+// memory.  Eight FP64 operations, within 1.02 ulp (bin means of 8.5e7 pairs 3.24 -> 2.03 ms); outside [0, 1400] (NaN, results near or
+// below the smallest normal) the library's exp, and 0 where that underflows.
+constexpr int EXP_TAB = 4096;
+__device__ __forceinline__ double exp_neg_half(double c, const double* tab) {
+  // (compared by its high word: FP64 comparisons run on the FP64 pipe, and a negative or NaN c
+  // has a larger one)
+  const unsigned hi = (unsigned)__double2hiint(c);
+  if (hi >= 0x4095E000u) return hi - 0x40977000u < 0x7FF00000u - 0x40977000u ? 0.0 : exp(-0.5 * c);  // 1400; 1500 to below inf
+  const double magic = 6755399441055744.0;                  // 1.5 * 2^52: the sum's low word is k
+  const double t = __fma_rn(c, -2954.639443740597, magic);  // 2048 / ln 2
+  const double k = __dsub_rn(t, magic);
+  double r = __fma_rn(k, 0x1.62e42fe8p-12, c);  // r' = -2 r = c + k ln 2/2048; 30 bits of it: exact
+  r = __fma_rn(k, 0x1.e8e7bcd5e4f1ep-42, r);
+  const int ki = __double2loint(t);
+  const double p = __fma_rn(r, __fma_rn(r, -1.0 / 48.0, 0.125), -0.5);
+  const double s = tab[ki & (EXP_TAB - 1)];
+  const double e = __fma_rn(s, __dmul_rn(r, p), s);
+  return __hiloint2double(__double2hiint(e) + ((ki >> 12) << 20), __double2loint(e));
+}
+
+// 2^(j/4096) on the device, made once per context.
+static const double* exp_table(mlc_ctx* ctx) {
+  if (!ctx->ws_ptr[WS_EXP_TAB]) {
+    std::vector<double> h(EXP_TAB);
+    for (int j = 0; j < EXP_TAB; j++) h[j] = (double)exp2l((long double)j / EXP_TAB);
+    void* d = ws_get(ctx, WS_EXP_TAB, sizeof(double) * EXP_TAB);
+    MLC_CUDA(cudaMemcpy(d, h.data(), sizeof(double) * EXP_TAB, cudaMemcpyHostToDevice));
+  }
+  return (const double*)ctx->ws_ptr[WS_EXP_TAB];
+}
+__device__ __forceinline__ void load_exp_table(const double* __restrict__ src, double* dst) {
+  for (int i = threadIdx.x; i < EXP_TAB / 2; i += blockDim.x)
+    reinterpret_cast<double2*>(dst)[i] = __ldg(reinterpret_cast<const double2*>(src) + i);
+}
 constexpr uint32_t BIN_PIECE = 1u << 15;
 struct BinPiece {
   uint32_t first, count;
 };
 
 __global__ void __launch_bounds__(256) k_bin_piece_sums(const double* __restrict__ chi2,
-                                                        const BinPiece* __restrict__ pieces,
-                                                        double* __restrict__ psum, double* __restrict__ pexp) {
-  const BinPiece pc = pieces[blockIdx.x];
-  double sc = 0.0, se = 0.0;
-  for (uint32_t k = threadIdx.x; k < pc.count; k += blockDim.x) {
-    const double c = chi2[(long)pc.first + k];
-    sc += c;
-    se += exp(-0.5 * c);
-  }
+                                                        const BinPiece* __restrict__ pieces, int npieces,
+                                                        const double* __restrict__ etab, double* __restrict__ psum,
+                                                        double* __restrict__ pexp) {
+  __shared__ __align__(16) double tab[EXP_TAB];
   __shared__ double r1[8], r2[8];
-  for (int o = 16; o > 0; o >>= 1) {
-    sc += __shfl_xor_sync(0xffffffffu, sc, o);
-    se += __shfl_xor_sync(0xffffffffu, se, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    r1[threadIdx.x >> 5] = sc;
-    r2[threadIdx.x >> 5] = se;
-  }
+  load_exp_table(etab, tab);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double a = 0.0, b = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
-      a += r1[w];
-      b += r2[w];
+  for (int pi = blockIdx.x; pi < npieces; pi += gridDim.x) {  // (one table for many pieces)
+    const BinPiece pc = pieces[pi];
+    double sc = 0.0, se = 0.0;
+#pragma unroll 4
+    for (uint32_t k = threadIdx.x; k < pc.count; k += blockDim.x) {
+      const double c = chi2[(long)pc.first + k];
+      sc += c;
+      se += exp_neg_half(c, tab);
     }
-    psum[blockIdx.x] = a;
-    pexp[blockIdx.x] = b;
+    for (int o = 16; o > 0; o >>= 1) {
+      sc += __shfl_xor_sync(0xffffffffu, sc, o);
+      se += __shfl_xor_sync(0xffffffffu, se, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+      r1[threadIdx.x >> 5] = sc;
+      r2[threadIdx.x >> 5] = se;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double a = 0.0, b = 0.0;
+      for (int w = 0; w < (int)(blockDim.x >> 5); w++) {
+        a += r1[w];
+        b += r2[w];
+      }
+      psum[pi] = a;
+      pexp[pi] = b;
+    }
+    __syncthreads();  // r1, r2 are rewritten by the next piece
   }
 }
 
@@ -186,83 +297,141 @@ __global__ void k_bin_combine(const uint32_t* __restrict__ pfirst, const uint32_
 // 1.8e-7 of z, float edges within 6e-8 of the edges): when z32 is more than 2^-20 z32
 // away from both neighbouring float edges the float order is the FP64 order; otherwise
 // (and for zero, non-finite or extreme z32) the exact FP64 quotient is searched in the
-// FP64 edges.  chi2 as k_pair_chi2_ratio.  Sums in FP64 shared-memory accumulators, one
-// flush per CTA.  Each CTA covers 16 A curves x 256 B curves.
-constexpr int FUSED_A = 16;
-__global__ void __launch_bounds__(256) k_pair_bin_fused(const double* __restrict__ mA, const double* __restrict__ iB,
-                                                        const float* __restrict__ zA, const float* __restrict__ zB,
-                                                        const double* __restrict__ LCA, const double* __restrict__ LCB,
-                                                        int Nloc, int Nprof, int Njp, const double* __restrict__ d,
-                                                        const double* __restrict__ is, int nb,
-                                                        const double* __restrict__ edges, double* __restrict__ gsum,
-                                                        double* __restrict__ gexp, unsigned long long* __restrict__ gcnt) {
-  extern __shared__ double sm[];
-  double* e_s = sm;
-  double* sum_s = sm + nb;
-  double* exp_s = sum_s + nb;
-  float* ef_s = reinterpret_cast<float*>(exp_s + nb);
-  unsigned int* cnt_s = reinterpret_cast<unsigned int*>(ef_s + nb);
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) {
-    e_s[i] = edges[i];
-    ef_s[i] = (float)edges[i];
-    sum_s[i] = 0.0;
-    exp_s[i] = 0.0;
-    cnt_s[i] = 0u;
+// FP64 edges.
+//
+// A thread goes through na places a of its b and keeps the sums of its present bin in registers;
+// when the bin changes they go to the bin's accumulators in global memory: an add there costs
+// the SM no FP64 operation, where an FP64 add to shared memory is a compare-and-swap loop of
+// them.  There are up to 1024 copies of the accumulators, so that each sums a thousand
+// values or so (the rounding of one running sum of all 10^6 pairs of a bin would show), and
+// k_fused_combine adds the copies up in pairs.  (With the accumulators there, having both
+// sides sorted, so that bins change once in tens of pairs, measures the same.)  The next pair's
+// bin is the last one's while z32 is clear of that bin's two edges.  What is left is the FP64
+// pipe: 2 Njp operations for chi2, 8 for the exponential, 2 for the sums (9216 locations,
+// Njp = 5: 6.24 -> 3.56 ms; the pipe needs 2.7).  A CTA: 256 b x na (at most FUSED_A) a.
+constexpr int FUSED_A = 64;
+struct FusedSide {
+  const double* z;
+  const float* zf;
+};
+__device__ __forceinline__ int edge_search(const double* e, int nb, double z) {
+  int lo = 0, hi = nb;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (e[mid] < z) lo = mid + 1;
+    else hi = mid;
   }
+  return lo;
+}
+
+template <bool PLAIN>
+__global__ void __launch_bounds__(256) k_pair_bin_fused(RatioChi2<PLAIN> f, FusedSide A, FusedSide B, int na, int nb,
+                                                        const double* __restrict__ edges,
+                                                        const double* __restrict__ etab, int copies,
+                                                        double* __restrict__ gsum, double* __restrict__ gexp,
+                                                        unsigned long long* __restrict__ gcnt) {
+  extern __shared__ __align__(16) double sm[];
+  double* tab = sm;
+  float* ef_s = reinterpret_cast<float*>(tab + EXP_TAB);
+  load_exp_table(etab, tab);
+  for (int i = threadIdx.x; i < nb; i += blockDim.x) ef_s[i] = (float)edges[i];
   __syncthreads();
+  const long copy = (long)((blockIdx.y * gridDim.x + blockIdx.x) % copies) * nb;
+  auto flush = [&](int bin, double sc, double se, unsigned cn) {
+    atomicAdd(gsum + copy + bin, sc);
+    atomicAdd(gexp + copy + bin, se);
+    atomicAdd(gcnt + copy + bin, (unsigned long long)cn);
+  };
   const int b = blockIdx.x * 256 + threadIdx.x;
-  const int a0 = blockIdx.y * FUSED_A;
-  if (b < Nloc) {
-    const float zb = __ldg(zB + b);
-    for (int a = a0; a < a0 + FUSED_A && a < Nloc; a++) {
-      const float z32 = __ldg(zA + a) * zb;
-      int lo = 0, hi = nb;  // first float edge >= z32
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (ef_s[mid] < z32) lo = mid + 1;
-        else hi = mid;
-      }
-      bool exact = !(z32 > 0x1p-100f && z32 < 0x1p100f);
-      if (!exact) {
-        const float tol = z32 * 0x1p-20f;
-        exact = (lo < nb && ef_s[lo] - z32 <= tol) || (lo > 0 && z32 - ef_s[lo - 1] <= tol);
-      }
-      if (exact) {
-        double z = __ldg(LCA + (long)a * Nprof) / __ldg(LCB + (long)b * Nprof);
-        // NaN: the rank order puts a negative one (the GPU's 0/0) before every z, in the
-        // first bin, and a positive one (from a NaN light-curve value) after +inf, counted
-        // here in no bin
-        if (z != z) {
-          if (!signbit(z)) continue;
-          z = -INFINITY;
-        }
-        lo = 0;
-        hi = nb;
+  if (b < f.Nloc) {
+    const float zb = __ldg(B.zf + b);
+    const int a0 = blockIdx.y * na, a1 = min(a0 + na, f.Nloc);
+    int bin = -1;                   // bin of the sums below
+    float below = 0.f, above = 0.f;  // z32 strictly between them: certainly this bin
+    double sc = 0.0, se = 0.0;
+    unsigned cn = 0;
+    for (int a = a0; a < a1; a++) {
+      const float z32 = __ldg(A.zf + a) * zb;
+      if (!(z32 > below && z32 < above)) {
+        int lo = 0, hi = nb;  // first float edge >= z32
         while (lo < hi) {
           const int mid = (lo + hi) >> 1;
-          if (e_s[mid] < z) lo = mid + 1;
+          if (ef_s[mid] < z32) lo = mid + 1;
           else hi = mid;
         }
+        bool exact = !(z32 > 0x1p-100f && z32 < 0x1p100f);
+        if (!exact) {
+          const float tol = z32 * 0x1p-20f;
+          exact = (lo < nb && ef_s[lo] - z32 <= tol) || (lo > 0 && z32 - ef_s[lo - 1] <= tol);
+        }
+        if (exact) {
+          // NaN: the rank order puts a negative one (the GPU's 0/0) before every z, in the
+          // first bin, and a positive one (from a NaN light-curve value) after +inf, counted
+          // here in no bin
+          const double z = __ldg(A.z + a) / __ldg(B.z + b);
+          if (z != z) lo = signbit(z) ? 0 : nb;
+          else lo = edge_search(edges, nb, z);
+        }
+        if (lo != bin) {
+          if (cn) flush(bin, sc, se, cn);
+          bin = lo;
+          sc = se = 0.0;
+          cn = 0;
+        }
+        // the bin's float edges, moved in by twice the tolerance (an empty interval where that
+        // leaves nothing, or beyond the exponents the float search answers for)
+        below = bin > 0 ? ef_s[bin - 1] * (1.f + 0x1p-19f) : 0x1p-100f;
+        above = bin < nb ? ef_s[bin] * (1.f - 0x1p-19f) : 0x1p100f;
+        below = fmaxf(below, 0x1p-100f);
+        above = fminf(above, 0x1p100f);
       }
-      if (lo >= nb) continue;
-      double c = 0.0;
-      for (int i = 0; i < Njp; i++) {
-        const double tmp =
-            (__ldg(d + i) - __ldg(mA + (long)i * Nloc + a) * __ldg(iB + (long)i * Nloc + b)) * __ldg(is + i);
-        c += tmp * tmp;
-      }
-      atomicAdd(&sum_s[lo], c);
-      atomicAdd(&exp_s[lo], exp(-0.5 * c));
-      atomicAdd(&cnt_s[lo], 1u);
+      if (bin >= nb) continue;
+      const double c = f(a, b);
+      sc += c;
+      se += exp_neg_half(c, tab);
+      cn++;
     }
+    // what the threads hold at the end: neighbours mostly hold the same bin
+    const unsigned act = __activemask();
+    int same = 0;
+    __match_all_sync(act, bin, &same);
+    if (same && act == 0xffffffffu) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        sc += __shfl_xor_sync(0xffffffffu, sc, o);
+        se += __shfl_xor_sync(0xffffffffu, se, o);
+        cn += __shfl_xor_sync(0xffffffffu, cn, o);
+      }
+      if (threadIdx.x & 31) cn = 0;
+    }
+    if (cn) flush(bin, sc, se, cn);
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) {
-    if (cnt_s[i]) {
-      atomicAdd(&gsum[i], sum_s[i]);
-      atomicAdd(&gexp[i], exp_s[i]);
-      atomicAdd(&gcnt[i], (unsigned long long)cnt_s[i]);
-    }
+}
+
+// The copies' sums: a warp per bin, each lane the copies 32 apart, then the lanes in pairs.
+__global__ void __launch_bounds__(256) k_fused_combine(int nb, int copies, double* __restrict__ gsum,
+                                                       double* __restrict__ gexp,
+                                                       unsigned long long* __restrict__ gcnt) {
+  const int i = (blockIdx.x * 256 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (i >= nb) return;
+  double s = 0.0, e = 0.0;
+  unsigned long long n = 0;
+  for (int c = lane; c < copies; c += 32) {
+    const long q = (long)c * nb + i;
+    s += gsum[q];
+    e += gexp[q];
+    n += gcnt[q];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, o);
+    e += __shfl_xor_sync(0xffffffffu, e, o);
+    n += __shfl_xor_sync(0xffffffffu, n, o);
+  }
+  if (lane == 0) {
+    gsum[i] = s;
+    gexp[i] = e;
+    gcnt[i] = n;
   }
 }
 
@@ -272,25 +441,32 @@ static int grid_for(mlc_ctx* ctx, long n) {
   return (int)std::max<long>(1, std::min<long>((n + 255) / 256, (long)ctx->sm_count * 16));
 }
 
+constexpr long RANGE_SORT_FROM = 1l << 20;  // (fewer keys are bound by the launches of either form)
+
 void pair_setup(mlc_ctx* ctx, int Nloc, int Nprof, const double* LCA, const double* LCB, int Nbins,
                 const double* edges_host, uint32_t* rank, uint32_t* lower_host, uint32_t* nper_host) {
   const long P = (long)Nloc * Nloc;
   MLC_REQUIRE(P <= 0xFFFFFFFFl, MLC_ERR_LIMIT, "Nloc^2 above 2^32-1");
   uint64_t* keys = (uint64_t*)ws_get(ctx, WS_PAIR_ACC, sizeof(uint64_t) * P + sizeof(uint32_t) * P + 4096);
   uint32_t* idx = reinterpret_cast<uint32_t*>(keys + P);
-  {
-    MLC_KSCOPE(ctx, "pair_z");
-    k_pair_z<<<grid_for(ctx, P), 256, 0, ctx->stream>>>(LCA, LCB, Nloc, Nprof, keys, idx);
-  }
-  MLC_CHECK_LAUNCH();
-  radix_sort_u64_u32(ctx, P, keys, idx);
-  if (rank) {
+  unsigned long long* range = reinterpret_cast<unsigned long long*>(keys + P + (P + 1) / 2);
+  auto make_keys = [&] {
+    MLC_CUDA(cudaMemsetAsync(range, 0xff, 2 * sizeof(*range), ctx->stream));
     {
-      MLC_KSCOPE(ctx, "pair_rank");
-      k_invert_perm<<<grid_for(ctx, P), 256, 0, ctx->stream>>>(idx, P, rank);
+      MLC_KSCOPE(ctx, "pair_z");
+      k_pair_z<<<dim3(ceil_div(Nloc, 256), ceil_div(Nloc, Z_ROWS)), 256, 0, ctx->stream>>>(LCA, LCB, Nloc, Nprof, keys,
+                                                                                         idx, range);
     }
     MLC_CHECK_LAUNCH();
+  };
+  make_keys();
+  // by the top of the keys' range where the keys are many and that decides their order (8.5e7: 3.7
+  // ms, by all bits 7.7); outliers, infinities or NaN may stretch the range: then by all bits
+  if (P < RANGE_SORT_FROM || !radix_sort_range_u64_u32(ctx, P, keys, idx, range)) {
+    if (P >= RANGE_SORT_FROM) make_keys();
+    radix_sort_u64_u32(ctx, P, keys, idx);
   }
+  if (rank) put_by_index(ctx, "pair_rank", idx, LoadOwnIndex{}, P, rank);
   if (Nbins > 0) {
     double* dedge = (double*)ws_get(ctx, WS_SMALL, sizeof(double) * Nbins + sizeof(uint32_t) * Nbins);
     uint32_t* dup = reinterpret_cast<uint32_t*>(dedge + Nbins);
@@ -313,17 +489,27 @@ void pair_setup(mlc_ctx* ctx, int Nloc, int Nprof, const double* LCA, const doub
 
 struct Interp {
   double* mA;
-  double* iB;  // 1 / mB
+  double* iB;  // B_i (see RatioChi2), 1 / mB_i where plain
   double* d;
-  double* is;  // 1 / s
+  double* is;
+  bool plain;
 };
+
+static bool moderate_host(double v) {
+  int e = 0;
+  return std::isfinite(v) && v != 0.0 && (std::frexp(v, &e), e > -400 && e < 400);
+}
 
 static Interp build_interp(mlc_ctx* ctx, int Njp, const int* indA, const int* indB, const double* facA,
                            const double* facB, const double* d, const double* s, int Nloc, int Nprof,
                            const double* LCA, const double* DLCA, const double* LCB, const double* DLCB) {
   const long n = (long)Nloc * Njp;
-  // small tables: ind A/B (int), fac A/B, d, s
-  size_t small = sizeof(double) * 4 * Njp + sizeof(int) * 2 * Njp + 64;
+  for (int i = 0; i < Njp; i++) {
+    MLC_REQUIRE(indA[i] >= -1 && indA[i] < Nprof - 1 && indB[i] >= -1 && indB[i] < Nprof - 1, MLC_ERR_ARG,
+                "interpolation index out of the profile range");
+  }
+  // small tables: fac A/B, d (ds), 1/s, rho (two rows); ind A/B (int)
+  size_t small = sizeof(double) * 6 * Njp + sizeof(int) * 2 * Njp + 64;
   char* sm = (char*)ws_get(ctx, WS_LOC, sizeof(double) * 2 * n + small);
   Interp I;
   I.mA = (double*)sm;
@@ -332,47 +518,64 @@ static Interp build_interp(mlc_ctx* ctx, int Njp, const int* indA, const int* in
   double* fB = fA + Njp;
   I.d = fB + Njp;
   I.is = I.d + Njp;
-  int* iA = reinterpret_cast<int*>(I.is + Njp);
+  double* rho = I.is + Njp;
+  int* iA = reinterpret_cast<int*>(rho + 2 * Njp);
   int* iB = iA + Njp;
-  std::vector<char> h(sizeof(double) * 4 * Njp + sizeof(int) * 2 * Njp);
+  I.plain = false;
+  for (int i = 0; i < Njp; i++) I.plain |= !moderate_host(d[i]) || !moderate_host(s[i]);
+  std::vector<char> h(sizeof(double) * 6 * Njp + sizeof(int) * 2 * Njp);
   double* hd = reinterpret_cast<double*>(h.data());
   std::copy(facA, facA + Njp, hd);
   std::copy(facB, facB + Njp, hd + Njp);
-  std::copy(d, d + Njp, hd + 2 * Njp);
-  for (int i = 0; i < Njp; i++) hd[3 * Njp + i] = 1.0 / s[i];
-  int* hi = reinterpret_cast<int*>(hd + 4 * Njp);
+  for (int i = 0; i < Njp; i++) {
+    const double ds = d[i] / s[i];
+    hd[2 * Njp + i] = I.plain ? d[i] : ds;
+    hd[3 * Njp + i] = 1.0 / s[i];
+    // rho = ds / d to twice the precision: its rounding, then the exact residual over d
+    const double rh = I.plain ? 1.0 : ds / d[i];
+    hd[4 * Njp + i] = rh;
+    hd[5 * Njp + i] = I.plain ? 0.0 : std::fma(-rh, d[i], ds) / d[i];
+  }
+  int* hi = reinterpret_cast<int*>(hd + 6 * Njp);
   std::copy(indA, indA + Njp, hi);
   std::copy(indB, indB + Njp, hi + Njp);
   MLC_CUDA(cudaMemcpy(fA, h.data(), h.size(), cudaMemcpyHostToDevice));
-  for (int i = 0; i < Njp; i++) {
-    MLC_REQUIRE(indA[i] >= -1 && indA[i] < Nprof - 1 && indB[i] >= -1 && indB[i] < Nprof - 1, MLC_ERR_ARG,
-                "interpolation index out of the profile range");
-  }
   if (n > 0) {
     {
       MLC_KSCOPE(ctx, "pair_interp");
-      k_interp<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(LCA, DLCA, Nloc, Nprof, Njp, iA, fA, 0, I.mA);
+      k_interp<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(LCA, DLCA, Nloc, Nprof, Njp, iA, fA, nullptr, I.mA);
     }
     MLC_CHECK_LAUNCH();
     {
       MLC_KSCOPE(ctx, "pair_interp");
-      k_interp<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(LCB, DLCB, Nloc, Nprof, Njp, iB, fB, 1, I.iB);
+      k_interp<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(LCB, DLCB, Nloc, Nprof, Njp, iB, fB, rho, I.iB);
     }
     MLC_CHECK_LAUNCH();
   }
   return I;
 }
 
+template <bool PLAIN>
+static void pair_chi2_run(mlc_ctx* ctx, const Interp& I, int Nloc, int Njp, const uint32_t* rank, double* chi2) {
+  const RatioChi2<PLAIN> f{I.mA, I.iB, I.d, I.is, Nloc, Njp};
+  if (rank && (long)Nloc * Nloc <= 0xFFFFFFFFl) {
+    put_by_index(ctx, "pair_chi2_ratio", rank, f, (long)Nloc * Nloc, chi2);
+    return;
+  }
+  {
+    MLC_KSCOPE(ctx, "pair_chi2_ratio");
+    k_pair_chi2_ratio<PLAIN><<<dim3(ceil_div(Nloc, 32), ceil_div(Nloc, 8)), 256, 0, ctx->stream>>>(f, rank, chi2);
+  }
+  MLC_CHECK_LAUNCH();
+}
+
 void pair_chi2_ratio(mlc_ctx* ctx, int Njp, const int* indA, const int* indB, const double* facA,
                      const double* facB, const double* d, const double* s, int Nloc, int Nprof, const double* LCA,
                      const double* DLCA, const double* LCB, const double* DLCB, const uint32_t* rank, double* chi2) {
+  if (Nloc <= 0) return;
   Interp I = build_interp(ctx, Njp, indA, indB, facA, facB, d, s, Nloc, Nprof, LCA, DLCA, LCB, DLCB);
-  dim3 grid(ceil_div(Nloc, 32), ceil_div(Nloc, 8));
-  {
-    MLC_KSCOPE(ctx, "pair_chi2_ratio");
-    k_pair_chi2_ratio<<<grid, 256, 0, ctx->stream>>>(I.mA, I.iB, Nloc, Njp, I.d, I.is, rank, chi2);
-  }
-  MLC_CHECK_LAUNCH();
+  if (I.plain) pair_chi2_run<true>(ctx, I, Nloc, Njp, rank, chi2);
+  else pair_chi2_run<false>(ctx, I, Nloc, Njp, rank, chi2);
 }
 
 void bin_chi2(mlc_ctx* ctx, int Nbins, const uint32_t* lower_host, const uint32_t* nper_host,
@@ -400,9 +603,11 @@ void bin_chi2(mlc_ctx* ctx, int Nbins, const uint32_t* lower_host, const uint32_
     MLC_CUDA(cudaMemcpyAsync(dp, pieces.data(), sizeof(BinPiece) * pieces.size(), cudaMemcpyHostToDevice, ctx->stream));
   MLC_CUDA(cudaMemcpyAsync(dfirst, pfirst.data(), sizeof(uint32_t) * (Nbins + 1), cudaMemcpyHostToDevice, ctx->stream));
   MLC_CUDA(cudaMemcpyAsync(dn, nper.data(), sizeof(uint32_t) * Nbins, cudaMemcpyHostToDevice, ctx->stream));
+  const double* etab = exp_table(ctx);
   if (!pieces.empty()) {
     MLC_KSCOPE(ctx, "pair_bin_means");
-    k_bin_piece_sums<<<(unsigned)pieces.size(), 256, 0, ctx->stream>>>(chi2_sorted, dp, ps, pe);
+    const unsigned grid = (unsigned)std::min<size_t>(pieces.size(), (size_t)ctx->sm_count * 6);
+    k_bin_piece_sums<<<grid, 256, 0, ctx->stream>>>(chi2_sorted, dp, (int)pieces.size(), etab, ps, pe);
   }
   MLC_CHECK_LAUNCH();
   {
@@ -420,28 +625,47 @@ void pair_bin_fused(mlc_ctx* ctx, int Njp, const int* indA, const int* indB, con
                     const double* DLCA, const double* LCB, const double* DLCB, int Nbins, const double* edges_host,
                     double* bchi2_host, double* bexp_host, uint32_t* nper_host) {
   MLC_REQUIRE(Nbins > 0 && Nbins <= 6000, MLC_ERR_LIMIT, "fused pair binning supports 1..6000 bins");
-  Interp I = build_interp(ctx, Njp, indA, indB, facA, facB, d, s, Nloc, Nprof, LCA, DLCA, LCB, DLCB);
-  char* sm = (char*)ws_get(ctx, WS_PAIR_ACC, (sizeof(double) * 3 + 8) * Nbins + 2 * sizeof(float) * Nloc + 128);
+  // edges, sums, counts; both sides' FP64 and FP32 point-source values
+  const int copies = std::max(16, std::min(1024, (1 << 19) / Nbins));
+  const size_t N = (size_t)Nloc, NC = (size_t)copies * Nbins;
+  char* sm = (char*)ws_get(ctx, WS_PAIR_ACC, 8 * (3 * NC + Nbins) + 2 * (8 + 4) * N + 512);
   double* de = (double*)sm;
   double* gs = de + Nbins;
-  double* ge = gs + Nbins;
-  unsigned long long* gc = reinterpret_cast<unsigned long long*>(ge + Nbins);
-  float* zA = reinterpret_cast<float*>(gc + Nbins);
-  float* zB = zA + Nloc;
-  {
+  double* ge = gs + NC;
+  unsigned long long* gc = reinterpret_cast<unsigned long long*>(ge + NC);
+  double* z = reinterpret_cast<double*>(gc + NC);
+  float* zf = reinterpret_cast<float*>(z + 2 * N);
+  if (Nloc > 0) {
     MLC_KSCOPE(ctx, "pair_interp");
-    k_zfloat<<<grid_for(ctx, Nloc), 256, 0, ctx->stream>>>(LCA, LCB, Nloc, Nprof, zA, zB);
+    k_zvalues<<<grid_for(ctx, Nloc), 256, 0, ctx->stream>>>(LCA, Nloc, Nprof, 0, z, zf);
+    k_zvalues<<<grid_for(ctx, Nloc), 256, 0, ctx->stream>>>(LCB, Nloc, Nprof, 1, z + N, zf + N);
   }
   MLC_CHECK_LAUNCH();
+  Interp I = build_interp(ctx, Njp, indA, indB, facA, facB, d, s, Nloc, Nprof, LCA, DLCA, LCB, DLCB);
   MLC_CUDA(cudaMemcpyAsync(de, edges_host, sizeof(double) * Nbins, cudaMemcpyHostToDevice, ctx->stream));
-  MLC_CUDA(cudaMemsetAsync(gs, 0, (sizeof(double) * 2 + 8) * Nbins, ctx->stream));
-  const size_t smem = (sizeof(double) * 3 + sizeof(float) + sizeof(unsigned)) * Nbins;
-  set_max_smem((const void*)k_pair_bin_fused, smem);
-  dim3 grid(ceil_div(Nloc, 256), ceil_div(Nloc, FUSED_A));
-  {
-    MLC_KSCOPE(ctx, "pair_bin_fused");
-    k_pair_bin_fused<<<grid, 256, smem, ctx->stream>>>(I.mA, I.iB, zA, zB, LCA, LCB, Nloc, Nprof, Njp, I.d, I.is,
-                                                      Nbins, de, gs, ge, gc);
+  MLC_CUDA(cudaMemsetAsync(gs, 0, 8 * 3 * NC, ctx->stream));
+  const size_t smem = sizeof(double) * EXP_TAB + sizeof(float) * Nbins;
+  const double* etab = exp_table(ctx);
+  if (Nloc > 0) {
+    const void* k = I.plain ? (const void*)k_pair_bin_fused<true> : (const void*)k_pair_bin_fused<false>;
+    set_max_smem(k, smem);
+    // A places per CTA: as many as leave four CTAs for every SM
+    const int cols = ceil_div(Nloc, 256);
+    const int na = (int)std::max<long>(4, std::min<long>(FUSED_A, (long)Nloc * cols / (4 * ctx->sm_count)));
+    dim3 grid(cols, ceil_div(Nloc, na));
+    const FusedSide A{z, zf}, B{z + N, zf + N};
+    {
+      MLC_KSCOPE(ctx, "pair_bin_fused");
+      if (I.plain)
+        k_pair_bin_fused<true><<<grid, 256, smem, ctx->stream>>>(RatioChi2<true>{I.mA, I.iB, I.d, I.is, Nloc, Njp}, A, B,
+                                                                 na, Nbins, de, etab, copies, gs, ge, gc);
+      else
+        k_pair_bin_fused<false><<<grid, 256, smem, ctx->stream>>>(RatioChi2<false>{I.mA, I.iB, I.d, I.is, Nloc, Njp},
+                                                                  A, B, na, Nbins, de, etab, copies, gs, ge, gc);
+    }
+    MLC_CHECK_LAUNCH();
+    MLC_KSCOPE(ctx, "pair_bin_combine");
+    k_fused_combine<<<ceil_div(Nbins, 8), 256, 0, ctx->stream>>>(Nbins, copies, gs, ge, gc);
   }
   MLC_CHECK_LAUNCH();
   std::vector<double> hs(Nbins), he(Nbins);

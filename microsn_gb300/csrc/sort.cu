@@ -1,33 +1,38 @@
 // Hand-written stable LSD radix sort (8-bit digits) of 64-bit keys carrying 32-bit
-// values, and warp-aggregated shared-memory histograms.
+// values, a stable-order scatter through bins for random writes, and warp-aggregated
+// shared-memory histograms.
 //
-// Up front, k_digit_hist counts all eight digits of every tile in one read of the keys;
+// Up to 16384 keys: one CTA sorts them in shared memory, all passes in one launch
+// (10^4 keys: 0.25 ms of launches, scans and a host round trip before, 64 us now).
+//
+// More: k_digit_hist counts all eight digits of every tile in one read of the keys;
 // their totals give each digit's global start and let passes where all keys share a
 // digit be skipped.  Then one pass per remaining digit: (1) per-tile counts of that
 // digit in the keys' current order (the up-front counts serve the first pass only,
 // since each scatter permutes the keys); (2) k_scan_digit turns them into scatter
 // offsets; (3) k_scatter ranks each key inside its tile with __match_any_sync in
-// element order (stable) and scatters key and value.  Every scatter address is checked
-// against n; a violation sets an error flag instead of writing.
+// element order (stable), puts the tile in digit order in shared memory and writes it
+// from there: the keys of one digit are consecutive, 32 on average in a tile of 8192, so
+// a warp writes a few whole runs (writing each key from the thread that ranked it cost
+// 2.4 ms a pass for 8.5e7 keys, this 0.64; see k_scatter).  Every scatter address is checked against
+// n; a violation sets an error flag instead of writing.
 
 #include <mutex>
 #include <unordered_map>
 
 #include "mlc_internal.h"
-#include "scan.cuh"
+#include "radix.cuh"
 
 namespace mlc {
 
-static constexpr int SORT_THREADS = 256;
-static constexpr int SORT_ITEMS = 16;
-static constexpr int SORT_TILE = SORT_THREADS * SORT_ITEMS;  // 4096
-static constexpr int SORT_WARPS = SORT_THREADS / 32;
-
-// Order-preserving map of an IEEE double to an unsigned key.
+// Order-preserving map of an IEEE double to an unsigned key, and back.
 __host__ __device__ __forceinline__ uint64_t f64_key(double d) {
   uint64_t u;
   memcpy(&u, &d, 8);
   return (u & 0x8000000000000000ull) ? ~u : (u | 0x8000000000000000ull);
+}
+__device__ __forceinline__ double key_f64(uint64_t k) {
+  return __longlong_as_double((k & 0x8000000000000000ull) ? (k & 0x7fffffffffffffffull) : ~k);
 }
 
 uint64_t f64_to_key(double d) { return f64_key(d); }
@@ -54,130 +59,176 @@ __global__ void __launch_bounds__(SORT_THREADS) k_digit_hist(const uint64_t* __r
   }
 }
 
-// Exclusive scan, in digit-major order, of hist[pass] (256 x ntiles) -> offsets (same
-// layout).  One CTA per digit scans that digit's tiles, starting from the digit's
-// global base (the count of all keys with a smaller digit, from the host).
-__global__ void __launch_bounds__(1024) k_scan_digit(const uint32_t* __restrict__ hist, int ntiles,
-                                                     const uint32_t* __restrict__ digit_base,
-                                                     uint32_t* __restrict__ offs) {
+// The longest run of keys with equal sorted bits that one thread puts in order.
+constexpr int FIX_RUN = 64;
+
+// Insertion of elements [b, e): a key passes only larger ones.
+__device__ __forceinline__ void fix_run(uint64_t* ks, uint32_t* vals, int b, int e) {
+  for (int i = b + 1; i < e; i++) {
+    const uint64_t k = ks[i];
+    if (ks[i - 1] <= k) continue;
+    const uint32_t v = vals[i];
+    int j = i;
+    for (; j > b && ks[j - 1] > k; j--) {
+      ks[j] = ks[j - 1];
+      vals[j] = vals[j - 1];
+    }
+    ks[j] = k;
+    vals[j] = v;
+  }
+}
+
+// First place of the run of equal bits (key >> sh) that the descent at i (ks[i] > ks[i + 1])
+// belongs to; -1 where an earlier descent of the run exists (which lists it), -2 where the run
+// is too long.
+__device__ __forceinline__ int run_of_descent(const uint64_t* ks, int i, uint64_t lo, int sh) {
+  const uint64_t tp = (ks[i] - lo) >> sh;
+  int b = i;
+  while (b > 0 && i - b <= FIX_RUN && (ks[b - 1] - lo) >> sh == tp) {
+    if (ks[b - 1] > ks[b]) return -1;
+    b--;
+  }
+  return i - b > FIX_RUN ? -2 : b;
+}
+
+// Up to 1024 ITEMS keys in one CTA: stable LSD passes, keys and values in shared memory, held in
+// registers while they change places.  Four passes over the 32 bits below the highest in
+// which keys differ, then runs of equal bits that are out of order put right by a thread
+// each; all other digits too where a run is too long for that (equal keys never are out of
+// order).  F64: the keys are doubles, mapped on the way in and back out.
+constexpr int SMALL_THREADS = 1024, SMALL_WARPS = SMALL_THREADS / 32, SMALL_MAX_ITEMS = 16;
+constexpr long SMALL_MAX = (long)SMALL_THREADS * SMALL_MAX_ITEMS;
+
+template <int ITEMS, bool F64>
+__global__ void __launch_bounds__(SMALL_THREADS) k_sort_small(uint64_t* __restrict__ keys, uint32_t* __restrict__ vals,
+                                                              int n) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int CAP = SMALL_THREADS * ITEMS;
+  uint64_t* ks = reinterpret_cast<uint64_t*>(smem_raw);
+  uint32_t* vs = reinterpret_cast<uint32_t*>(ks + CAP);
+  uint32_t (*wcnt)[256] = reinterpret_cast<uint32_t (*)[256]>(vs + CAP);
+  uint16_t* list = reinterpret_cast<uint16_t*>(vs + CAP);  // (the counters' space, after the passes)
+  __shared__ uint32_t base[256];
   __shared__ uint32_t wsum[32];
-  const int d = blockIdx.x;
-  uint32_t running = digit_base[d];
-  for (int t0 = 0; t0 < ntiles; t0 += blockDim.x) {
-    const int t = t0 + threadIdx.x;
-    const uint32_t v = (t < ntiles) ? hist[(long)d * ntiles + t] : 0;
-    uint32_t agg;
-    const uint32_t ex = block_exclusive_sum(v, &agg, wsum);
-    if (t < ntiles) offs[(long)d * ntiles + t] = running + ex;
-    running += agg;
-    __syncthreads();  // wsum is rewritten by the next round
-  }
-}
-
-// Per-tile counts of one digit position in the current key order: hist [digit][tile].
-__global__ void __launch_bounds__(SORT_THREADS) k_tile_hist(const uint64_t* __restrict__ keys, long n, int ntiles,
-                                                            int shift, uint32_t* __restrict__ hist) {
-  __shared__ uint32_t cnt[256];
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) cnt[i] = 0;
-  __syncthreads();
-  const long t0 = (long)blockIdx.x * SORT_TILE;
-  for (int q = 0; q < SORT_ITEMS; q++) {
-    const long i = t0 + (long)q * SORT_THREADS + threadIdx.x;
-    if (i < n) atomicAdd(&cnt[(keys[i] >> shift) & 0xff], 1u);
-  }
-  __syncthreads();
-  for (int d = threadIdx.x; d < 256; d += blockDim.x) hist[(long)d * ntiles + blockIdx.x] = cnt[d];
-}
-
-// totals[p*256 + d] = number of keys whose digit p is d
-__global__ void __launch_bounds__(256) k_digit_totals(const uint32_t* __restrict__ hist, int ntiles,
-                                                      unsigned long long* __restrict__ totals) {
-  const long row = blockIdx.x;  // p*256 + d
-  unsigned long long s = 0;
-  for (int t = threadIdx.x; t < ntiles; t += blockDim.x) s += hist[row * ntiles + t];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  __shared__ unsigned long long red[8];
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned long long t = 0;
-    for (int w = 0; w < 8; w++) t += red[w];
-    totals[row] = t;
-  }
-}
-
-__global__ void __launch_bounds__(SORT_THREADS) k_scatter(const uint64_t* __restrict__ kin,
-                                                          const uint32_t* __restrict__ vin, uint64_t* __restrict__ kout,
-                                                          uint32_t* __restrict__ vout, long n, int ntiles, int shift,
-                                                          const uint32_t* __restrict__ offs, int* __restrict__ err) {
-  __shared__ uint32_t wcnt[SORT_WARPS][256];  // per-warp running digit counts, then warp bases
-  __shared__ uint32_t gbase[256];
+  __shared__ unsigned long long differ;
+  __shared__ int nlist, too_long;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int i = threadIdx.x; i < SORT_WARPS * 256; i += blockDim.x) (&wcnt[0][0])[i] = 0;
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) gbase[i] = offs[(long)i * ntiles + blockIdx.x];
-  __syncthreads();
-  // warp w owns tile elements [w*512, (w+1)*512): item q of lane l is element w*512 + 32q + l
-  const long t0 = (long)blockIdx.x * SORT_TILE + (long)warp * (SORT_ITEMS * 32);
-  uint64_t key[SORT_ITEMS];
-  uint32_t rank[SORT_ITEMS];
   const unsigned lt = (1u << lane) - 1u;
-#pragma unroll
-  for (int q = 0; q < SORT_ITEMS; q++) {
-    const long i = t0 + q * 32 + lane;
-    const bool ok = i < n;
-    key[q] = ok ? kin[i] : ~0ull;
-    const unsigned d = ok ? (unsigned)((key[q] >> shift) & 0xff) : 256u;
-    const unsigned act = __ballot_sync(0xffffffffu, ok);
-    const unsigned peers = __match_any_sync(0xffffffffu, d) & act;
-    uint32_t r = 0;
-    if (ok) {
-      const uint32_t before = wcnt[warp][d];
-      r = before + __popc(peers & lt);
-    }
-    __syncwarp();
-    if (ok && (peers & lt) == 0) wcnt[warp][d] += __popc(peers);
-    __syncwarp();
-    rank[q] = r;
-  }
+  const int e0 = warp * (ITEMS * 32) + lane;  // item q is element e0 + 32 q
+  if (threadIdx.x == 0) differ = 0, nlist = 0, too_long = 0;
   __syncthreads();
-  // exclusive scan of the per-warp counts for each digit -> warp bases
-  for (int d = threadIdx.x; d < 256; d += blockDim.x) {
-    uint32_t s = 0;
-    for (int w = 0; w < SORT_WARPS; w++) {
-      const uint32_t c = wcnt[w][d];
-      wcnt[w][d] = s;
-      s += c;
-    }
-  }
-  __syncthreads();
+  uint64_t first = keys[0];
+  if (F64) first = f64_key(__longlong_as_double((long long)first));
+  uint64_t key[ITEMS];
+  uint64_t m = 0;
 #pragma unroll
-  for (int q = 0; q < SORT_ITEMS; q++) {
-    const long i = t0 + q * 32 + lane;
-    if (i < n) {
-      const unsigned d = (unsigned)((key[q] >> shift) & 0xff);
-      const uint64_t dst = (uint64_t)gbase[d] + wcnt[warp][d] + rank[q];
-      if (dst < (uint64_t)n) {
-        kout[dst] = key[q];
-        vout[dst] = vin[i];
-      } else {
-        atomicExch(err, 1);
-      }
+  for (int q = 0; q < ITEMS; q++) {
+    const int e = e0 + 32 * q;
+    key[q] = ~0ull;  // (places past n: all bits set, and after the others of their digit, so they stay last)
+    if (e < n) {
+      const uint64_t k = keys[e];
+      key[q] = F64 ? f64_key(__longlong_as_double((long long)k)) : k;
+      m |= key[q] ^ first;
+      vs[e] = vals[e];
+    }
+    ks[e] = key[q];
+  }
+  if (m) atomicOr(&differ, (unsigned long long)m);
+  __syncthreads();
+  const uint64_t diff = differ;
+  auto pass = [&](int shift) {
+    for (int i = threadIdx.x; i < SMALL_WARPS * 256; i += SMALL_THREADS) (&wcnt[0][0])[i] = 0;
+#pragma unroll
+    for (int q = 0; q < ITEMS; q++) key[q] = ks[e0 + 32 * q];
+    __syncthreads();
+    uint32_t pos[ITEMS];
+#pragma unroll
+    for (int q = 0; q < ITEMS; q++) pos[q] = warp_digit_rank((unsigned)(key[q] >> shift) & 0xffu, true, wcnt[warp], lt);
+    __syncthreads();
+    digit_places<SMALL_WARPS>(wcnt, base, wsum);
+#pragma unroll
+    for (int q = 0; q < ITEMS; q++) {
+      pos[q] += wcnt[warp][(unsigned)(key[q] >> shift) & 0xffu];
+      ks[pos[q]] = key[q];
+    }
+    uint32_t v[ITEMS];
+#pragma unroll
+    for (int q = 0; q < ITEMS; q++) v[q] = vs[e0 + 32 * q];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < ITEMS; q++) vs[pos[q]] = v[q];
+    __syncthreads();
+  };
+  const int sh = diff ? max(0, 32 - __clzll((long long)diff)) : 64;  // the lowest sorted bit
+#pragma unroll 1
+  for (int shift = sh; shift < min(64, sh + 32); shift += 8)
+    if ((diff >> shift) & 0xff) pass(shift);
+  if (sh > 0 && sh < 64) {
+    for (int i = threadIdx.x; i + 1 < n; i += SMALL_THREADS) {
+      if (!(ks[i] > ks[i + 1])) continue;
+      const int b = run_of_descent(ks, i, 0, sh);
+      if (b >= 0) list[atomicAdd(&nlist, 1)] = (uint16_t)b;
+      else if (b == -2) too_long = 1;
+    }
+    __syncthreads();
+    for (int r = threadIdx.x; r < nlist; r += SMALL_THREADS) {
+      const int b = list[r];
+      int e = b + 1;
+      while (e < n && e - b <= FIX_RUN && (ks[e] >> sh) == (ks[b] >> sh)) e++;
+      if (e - b > FIX_RUN) too_long = 1;
+      else fix_run(ks, vs, b, e);
+    }
+    __syncthreads();
+    if (too_long) {
+#pragma unroll 1
+      for (int shift = 0; shift < 64; shift += 8)
+        if ((diff >> shift) & 0xff) pass(shift);
     }
   }
+#pragma unroll
+  for (int q = 0; q < ITEMS; q++) {
+    const int e = e0 + 32 * q;
+    if (e < n) {
+      const uint64_t k = ks[e];
+      keys[e] = F64 ? (uint64_t)__double_as_longlong(key_f64(k)) : k;
+      vals[e] = vs[e];
+    }
+  }
+}
+
+template <bool F64>
+static void sort_small(mlc_ctx* ctx, int n, uint64_t* keys, uint32_t* vals) {
+  using K = void (*)(uint64_t*, uint32_t*, int);
+  const int items = (n + SMALL_THREADS - 1) / SMALL_THREADS;
+  K k = k_sort_small<16, F64>;
+  int cap = 16;
+  if (items <= 1) k = k_sort_small<1, F64>, cap = 1;
+  else if (items <= 2) k = k_sort_small<2, F64>, cap = 2;
+  else if (items <= 4) k = k_sort_small<4, F64>, cap = 4;
+  else if (items <= 8) k = k_sort_small<8, F64>, cap = 8;
+  const size_t smem = (size_t)cap * SMALL_THREADS * 12 + sizeof(uint32_t) * SMALL_WARPS * 256;
+  set_max_smem((const void*)k, smem);
+  {
+    MLC_KSCOPE(ctx, "sort_small");
+    k<<<1, SMALL_THREADS, smem, ctx->stream>>>(keys, vals, n);
+  }
+  MLC_CHECK_LAUNCH();
 }
 
 // Sorts keys/vals (device, n) stably; uses two workspace buffers.  Result in place.
 void radix_sort_u64_u32(mlc_ctx* ctx, long n, uint64_t* keys, uint32_t* vals) {
   if (n <= 1) return;
+  if (n <= SMALL_MAX) {
+    sort_small<false>(ctx, (int)n, keys, vals);
+    return;
+  }
   MLC_REQUIRE(n <= 0xFFFFFFFFl, MLC_ERR_LIMIT, "sort length above 2^32-1");
   const int ntiles = (int)((n + SORT_TILE - 1) / SORT_TILE);
   uint64_t* k2 = (uint64_t*)ws_get(ctx, WS_SORT_KEYS, sizeof(uint64_t) * n);
   uint32_t* v2 = (uint32_t*)ws_get(ctx, WS_SORT_VALS, sizeof(uint32_t) * n);
-  uint32_t* hist = (uint32_t*)ws_get(ctx, WS_SORT_HIST,
-                                     sizeof(uint32_t) * (256 * (size_t)ntiles * 9 + 8 * 256) + 8 * 256 * 8 + 64);
+  uint32_t* hist = (uint32_t*)ws_get(ctx, WS_SORT_HIST, sizeof(uint32_t) * 256 * (size_t)ntiles * 9 + 8 * 256 * 8 + 64);
   uint32_t* offs = hist + (size_t)8 * 256 * ntiles;
-  uint32_t* dbase = offs + (size_t)256 * ntiles;
-  unsigned long long* dtot = reinterpret_cast<unsigned long long*>(dbase + 8 * 256);
+  unsigned long long* dtot = reinterpret_cast<unsigned long long*>(offs + (size_t)256 * ntiles);
   int* derr = reinterpret_cast<int*>(dtot + 8 * 256);
   MLC_CUDA(cudaMemsetAsync(derr, 0, sizeof(int), ctx->stream));
   {
@@ -190,46 +241,33 @@ void radix_sort_u64_u32(mlc_ctx* ctx, long n, uint64_t* keys, uint32_t* vals) {
     k_digit_totals<<<8 * 256, 256, 0, ctx->stream>>>(hist, ntiles, dtot);
   }
   MLC_CHECK_LAUNCH();
-  // Digit totals to the host: digit bases, and positions where all keys agree are skipped.
+  // Digit totals to the host: positions where all keys agree are skipped.
   std::vector<unsigned long long> h(8 * 256);
   MLC_CUDA(cudaMemcpyAsync(h.data(), dtot, h.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                            ctx->stream));
   MLC_CUDA(cudaStreamSynchronize(ctx->stream));
-  std::vector<uint32_t> base(8 * 256);
-  std::vector<char> trivial(8, 0);
-  for (int p = 0; p < 8; p++) {
-    uint64_t run = 0;
-    for (int d = 0; d < 256; d++) {
-      const uint64_t tot = h[p * 256 + d];
-      base[p * 256 + d] = (uint32_t)run;
-      run += tot;
-      if (tot == (uint64_t)n) trivial[p] = 1;
-    }
-  }
-  MLC_CUDA(cudaMemcpy(dbase, base.data(), base.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
   uint64_t* ka = keys;
   uint32_t* va = vals;
   uint64_t* kb = k2;
   uint32_t* vb = v2;
   bool first = true;
   for (int p = 0; p < 8; p++) {
-    if (trivial[p]) continue;
+    bool trivial = false;
+    for (int d = 0; d < 256; d++) trivial |= h[p * 256 + d] == (unsigned long long)n;
+    if (trivial) continue;
     if (!first) {  // per-tile counts of digit p in the current order
       MLC_KSCOPE(ctx, "sort_tile_hist");
-      k_tile_hist<<<ntiles, SORT_THREADS, 0, ctx->stream>>>(ka, n, ntiles, 8 * p, hist + (size_t)p * 256 * ntiles);
+      k_tile_hist<uint64_t, ShiftDigit><<<ntiles, SORT_THREADS, 0, ctx->stream>>>(ka, n, ntiles, ShiftDigit{8 * p},
+                                                                                  hist + (size_t)p * 256 * ntiles);
     }
     MLC_CHECK_LAUNCH();
     first = false;
     {
       MLC_KSCOPE(ctx, "sort_scan");
-      k_scan_digit<<<256, 1024, 0, ctx->stream>>>(hist + (size_t)p * 256 * ntiles, ntiles, dbase + p * 256, offs);
+      k_scan_digit<<<256, 1024, 0, ctx->stream>>>(hist + (size_t)p * 256 * ntiles, ntiles, dtot + p * 256, offs);
     }
     MLC_CHECK_LAUNCH();
-    {
-      MLC_KSCOPE(ctx, "sort_scatter");
-      k_scatter<<<ntiles, SORT_THREADS, 0, ctx->stream>>>(ka, va, kb, vb, n, ntiles, 8 * p, offs, derr);
-    }
-    MLC_CHECK_LAUNCH();
+    scatter(ctx, "sort_scatter", ka, LoadU32{va}, kb, vb, n, ntiles, ShiftDigit{8 * p}, offs, derr);
     std::swap(ka, kb);
     std::swap(va, vb);
   }
@@ -243,6 +281,124 @@ void radix_sort_u64_u32(mlc_ctx* ctx, long n, uint64_t* keys, uint32_t* vals) {
   MLC_REQUIRE(herr == 0, MLC_ERR_CUDA, "radix sort: scatter offset out of range (inconsistent digit counts)");
 }
 
+// ---- keys spread over their range: four passes instead of eight
+//
+// Of the 64 key bits of values that fill a range, the top 32 of (key - least key) almost
+// decide the order: of 8.5e7 quotients over some twenty octaves about one key in six has a
+// neighbour of the same 32 bits.  Four stable passes order the keys by them; where two
+// neighbours of the same top bits then stand in the wrong order (a descent), their run is
+// sorted by its full keys, stably, by one thread: within tiles of the keys in shared memory
+// (k_fix_tiles), then across the tiles' edges (k_fix_edges).  Runs of equal keys are in order
+// as they stand, however long.  A run with a descent that is longer than FIX_RUN is
+// reported instead: the caller makes the keys again and takes radix_sort_u64_u32.
+constexpr int FIX_TILE = 4096, FIX_THREADS = 256;
+
+__global__ void __launch_bounds__(FIX_THREADS) k_fix_tiles(uint64_t* __restrict__ keys, uint32_t* __restrict__ vals,
+                                                           long n, const unsigned long long* __restrict__ range,
+                                                           int* __restrict__ give_up) {
+  __shared__ uint64_t ks[FIX_TILE];
+  __shared__ uint16_t list[FIX_TILE / 2];  // first elements of the runs to sort (two keys or more each)
+  __shared__ int nlist;
+  const uint64_t lo = range[0];
+  const int sh = RangeDigit::base_shift(range);
+  const long t0 = (long)blockIdx.x * FIX_TILE;
+  const int cnt = (int)min((long)FIX_TILE, n - t0);
+  if (threadIdx.x == 0) nlist = 0;
+  for (int i = threadIdx.x; i < cnt; i += FIX_THREADS) ks[i] = keys[t0 + i];
+  __syncthreads();
+  auto top = [&](uint64_t k) { return (k - lo) >> sh; };
+  for (int i = threadIdx.x; i + 1 < cnt; i += FIX_THREADS) {
+    if (!(ks[i] > ks[i + 1])) continue;  // (a descent has equal top bits: the keys are in their order)
+    const int b = run_of_descent(ks, i, lo, sh);
+    if (b >= 0) list[atomicAdd(&nlist, 1)] = (uint16_t)b;
+    else if (b == -2) atomicExch(give_up, 1);
+  }
+  __syncthreads();
+  for (int r = threadIdx.x; r < nlist; r += FIX_THREADS) {
+    const int b = list[r];
+    const uint64_t tp = top(ks[b]);
+    int e = b + 1;
+    while (e < cnt && e - b <= FIX_RUN && top(ks[e]) == tp) e++;
+    if (e - b > FIX_RUN) {
+      atomicExch(give_up, 1);
+      continue;
+    }
+    // (a run that goes on in a neighbouring tile is k_fix_edges')
+    if ((b == 0 && t0 > 0 && top(keys[t0 - 1]) == tp) || (e == cnt && t0 + e < n && top(keys[t0 + e]) == tp)) continue;
+    fix_run(ks, vals + t0, b, e);
+    for (int i = b; i < e; i++) keys[t0 + i] = ks[i];
+  }
+}
+
+// The runs across the edge at the start of tile 1, 2, ...: a thread each.
+__global__ void __launch_bounds__(256) k_fix_edges(uint64_t* __restrict__ keys, uint32_t* __restrict__ vals, long n,
+                                                   const unsigned long long* __restrict__ range,
+                                                   int* __restrict__ give_up) {
+  const uint64_t lo = range[0];
+  const int sh = RangeDigit::base_shift(range);
+  const long j = ((long)blockIdx.x * blockDim.x + threadIdx.x + 1) * FIX_TILE;
+  if (j >= n) return;
+  const uint64_t tp = (keys[j] - lo) >> sh;
+  long b = j, e = j;
+  while (b > 0 && j - b <= FIX_RUN && ((keys[b - 1] - lo) >> sh) == tp) b--;
+  while (e < n && e - j <= FIX_RUN && ((keys[e] - lo) >> sh) == tp) e++;
+  if (b == j) return;
+  bool descent = false;
+  for (long i = b; i + 1 < e; i++) descent |= keys[i] > keys[i + 1];
+  if (!descent) return;
+  if (j - b > FIX_RUN || e - j > FIX_RUN) atomicExch(give_up, 1);
+  else fix_run(keys + b, vals + b, 0, (int)(e - b));
+}
+
+// Sorts keys/vals stably by the top of their range, then fixes what that leaves.  range (device):
+// the least key, and the least ~key.  False: the keys have to be sorted by all their bits, and
+// are in no order.
+bool radix_sort_range_u64_u32(mlc_ctx* ctx, long n, uint64_t* keys, uint32_t* vals, const unsigned long long* range) {
+  MLC_REQUIRE(n <= 0xFFFFFFFFl, MLC_ERR_LIMIT, "sort length above 2^32-1");
+  const int ntiles = (int)((n + SORT_TILE - 1) / SORT_TILE);
+  uint64_t* k2 = (uint64_t*)ws_get(ctx, WS_SORT_KEYS, sizeof(uint64_t) * n);
+  uint32_t* v2 = (uint32_t*)ws_get(ctx, WS_SORT_VALS, sizeof(uint32_t) * n);
+  uint32_t* hist = (uint32_t*)ws_get(ctx, WS_SORT_HIST, sizeof(uint32_t) * 256 * (size_t)ntiles * 2 + 256 * 8 + 64);
+  uint32_t* offs = hist + (size_t)256 * ntiles;
+  unsigned long long* dtot = reinterpret_cast<unsigned long long*>(offs + (size_t)256 * ntiles);
+  int* derr = reinterpret_cast<int*>(dtot + 256);  // [0] scatter error, [1] runs too long to fix
+  MLC_CUDA(cudaMemsetAsync(derr, 0, 2 * sizeof(int), ctx->stream));
+  uint64_t* ka = keys;
+  uint32_t* va = vals;
+  uint64_t* kb = k2;
+  uint32_t* vb = v2;
+  for (int p = 0; p < 4; p++) {
+    const RangeDigit dg{range, p};
+    {
+      MLC_KSCOPE(ctx, "sort_tile_hist");
+      k_tile_hist<uint64_t, RangeDigit><<<ntiles, SORT_THREADS, 0, ctx->stream>>>(ka, n, ntiles, dg, hist);
+    }
+    MLC_CHECK_LAUNCH();
+    {
+      MLC_KSCOPE(ctx, "sort_scan");
+      k_digit_totals<<<256, 256, 0, ctx->stream>>>(hist, ntiles, dtot);
+      k_scan_digit<<<256, 1024, 0, ctx->stream>>>(hist, ntiles, dtot, offs);
+    }
+    MLC_CHECK_LAUNCH();
+    scatter(ctx, "sort_scatter", ka, LoadU32{va}, kb, vb, n, ntiles, dg, offs, derr);
+    std::swap(ka, kb);
+    std::swap(va, vb);
+  }
+  // (four passes: the result is back in keys)
+  {
+    MLC_KSCOPE(ctx, "sort_fix");
+    const long tiles = (n + FIX_TILE - 1) / FIX_TILE;
+    k_fix_tiles<<<(unsigned)tiles, FIX_THREADS, 0, ctx->stream>>>(keys, vals, n, range, derr + 1);
+    k_fix_edges<<<(unsigned)((tiles + 255) / 256), 256, 0, ctx->stream>>>(keys, vals, n, range, derr + 1);
+  }
+  MLC_CHECK_LAUNCH();
+  int h[2] = {};
+  MLC_CUDA(cudaMemcpyAsync(h, derr, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
+  MLC_CUDA(cudaStreamSynchronize(ctx->stream));
+  MLC_REQUIRE(h[0] == 0, MLC_ERR_CUDA, "radix sort: scatter offset out of range (inconsistent digit counts)");
+  return h[1] == 0;
+}
+
 __global__ void k_f64_to_keys(double* __restrict__ v, long n) {
   uint64_t* u = reinterpret_cast<uint64_t*>(v);
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
@@ -250,17 +406,16 @@ __global__ void k_f64_to_keys(double* __restrict__ v, long n) {
 }
 __global__ void k_keys_to_f64(double* __restrict__ v, long n) {
   uint64_t* u = reinterpret_cast<uint64_t*>(v);
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-    uint64_t k = u[i];
-    uint64_t b = (k & 0x8000000000000000ull) ? (k & 0x7fffffffffffffffull) : ~k;
-    double d;
-    memcpy(&d, &b, 8);
-    v[i] = d;
-  }
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
+    v[i] = key_f64(u[i]);
 }
 
 void sort_f64_u32(mlc_ctx* ctx, long n, double* keys, uint32_t* vals) {
   if (n <= 1) return;
+  if (n <= SMALL_MAX) {
+    sort_small<true>(ctx, (int)n, reinterpret_cast<uint64_t*>(keys), vals);
+    return;
+  }
   const int grid = (int)std::min<long>((n + 255) / 256, (long)ctx->sm_count * 16);
   {
     MLC_KSCOPE(ctx, "sort_keys_in");

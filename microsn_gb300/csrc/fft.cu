@@ -91,7 +91,7 @@ void set_max_smem(const void* func, size_t bytes) {
 }
 
 FftPlan2D::~FftPlan2D() {
-  for (void* t : {twx, twy, twx3, twy3, twl3})
+  for (void* t : {twx, twy, twx3, twy3, twl3, twl})
     if (t) cudaFree(t);
 }
 
@@ -174,16 +174,30 @@ static void* upload_twiddles3(int N) {
   return upload_limbs3(re, im);
 }
 // Level 0 of the row transforms: W_M^(m q) for q = 1 .. R0 - 1, m < M / R0.
-static void* upload_level0(int M) {
-  const int R0 = limb_first_radix(M), J = M / R0;
-  std::vector<long double> re, im, lr, li;
+static void level0_table(int M, int R0, std::vector<long double>& lr, std::vector<long double>& li) {
+  const int J = M / R0;
+  std::vector<long double> re, im;
   twiddle_table(M, re, im);
   for (int q = 1; q < R0; q++)
     for (int m = 0; m < J; m++) {
       lr.push_back(re[(size_t)m * q]);
       li.push_back(im[(size_t)m * q]);
     }
+}
+static void* upload_level0_limbs3(int M) {
+  std::vector<long double> lr, li;
+  level0_table(M, limb_first_radix(M), lr, li);
   return upload_limbs3(lr, li);
+}
+static void* upload_level0_f32(int M) {
+  std::vector<long double> lr, li;
+  level0_table(M, row3_first_radix(M), lr, li);
+  std::vector<C2<float>> h(lr.size());
+  for (size_t i = 0; i < h.size(); i++) h[i] = C2<float>{(float)(double)lr[i], (float)(double)li[i]};
+  void* d = nullptr;
+  MLC_CUDA(cudaMalloc(&d, h.size() * sizeof(C2<float>)));
+  MLC_CUDA(cudaMemcpy(d, h.data(), h.size() * sizeof(C2<float>), cudaMemcpyHostToDevice));
+  return d;
 }
 
 static void split_columns(int Ny, int& N1, int& N2) {
@@ -223,13 +237,14 @@ FftPlan2D* plan_get(mlc_ctx* ctx, int Nx, int Ny, int prec) {
     p->twy = upload_twiddles<double>(Ny);
     p->twx3 = upload_twiddles3(Nx);
     p->twy3 = upload_twiddles3(Ny);
-    if (limb_first_radix(p->M)) p->twl3 = upload_level0(p->M);
+    if (limb_first_radix(p->M)) p->twl3 = upload_level0_limbs3(p->M);
   } else if (prec_is_ff(prec)) {
     p->twx = upload_twiddles<ff>(Nx);
     p->twy = upload_twiddles<ff>(Ny);
   } else {
     p->twx = upload_twiddles<float>(Nx);
     p->twy = upload_twiddles<float>(Ny);
+    if (row3_first_radix(p->M)) p->twl = upload_level0_f32(p->M);
   }
   FftPlan2D* raw = p.get();
   ctx->plans[key] = std::move(p);

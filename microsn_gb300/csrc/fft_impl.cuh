@@ -83,16 +83,44 @@ __global__ void __launch_bounds__(512) k_rows_r2c(Loader ld, C2<T>* __restrict__
 // then the split into Nx/2+1 spectrum values and the zero padding up to Wp.  FP32: four
 // CTAs per SM (three for 16^3, whose 80 registers would spill at 64), like k_rows_c2r3;
 // FP64 keeps the compiler's allocation (its 90 KB rows fit two CTAs per SM anyway).
+// Level 1's twiddle W_M^(j q) of the three-level rows.  FP32 plans hold these in the order [q - 1][j]
+// (tw1), which consecutive lanes read as whole lines: out of the table of W_Nx they are 2 q
+// entries apart, a sector per lane (with row_block: rows of 4096 points at 8192^2, c2r 207 -> 146 us and 133
+// with level 2 read as below and the points written from registers; r2c 201 -> 130).
+template <typename T, int J>
+__device__ __forceinline__ C2<T> level1_tw(const C2<T>* __restrict__ twx, const C2<T>* __restrict__ tw1, int j, int q) {
+  if constexpr (std::is_same<T, float>::value) return ldc(tw1 + (q - 1) * J + j);
+  else return ldc(twx + 2L * j * q);
+}
+
+// Level 2's twiddles W_J^(m q) = W_Nx^(2 L1 m q) in shared memory as [q - 1][m] (in the order of
+// W_J a warp would read them q entries apart).
+template <typename T, int L1, int L2, int L3>
+__device__ __forceinline__ void fill_level2_tw(C2<T>* wJ, const C2<T>* __restrict__ twx) {
+  for (int e = threadIdx.x; e < (L2 - 1) * L3; e += blockDim.x) {
+    const int q = e / L3 + 1, m = e - (q - 1) * L3;
+    wJ[e] = ldc(twx + 2L * L1 * m * q);
+  }
+}
+
+// Elements between the blocks of level 1 in shared memory.  Level 3 reads block after block
+// with consecutive lanes: a power-of-two stride (16^3) would put the lanes' 8 bytes in two
+// banks.
+template <int J>
+constexpr int row_block() {
+  return J % 16 == 0 ? J + 1 : J;
+}
+
 template <typename T, int L1, int L2, int L3, typename Loader>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (L1 == 16 ? 3 : 4) : 0)
-    k_rows_r2c3(Loader ld, C2<T>* __restrict__ out, long pitch,
-                                                   const C2<T>* __restrict__ twx) {
-  constexpr int J = L2 * L3, M = L1 * J;
+    k_rows_r2c3(Loader ld, C2<T>* __restrict__ out, long pitch, const C2<T>* __restrict__ twx,
+                const C2<T>* __restrict__ tw1) {
+  constexpr int J = L2 * L3, M = L1 * J, JP = row_block<J>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C2<T>* s = reinterpret_cast<C2<T>*>(smem_raw);
-  C2<T>* wJ = s + M;  // W_J^e = W_Nx^(2 L1 e), e < J
+  C2<T>* wJ = s + L1 * JP;  // (L2 - 1) L3 < J entries
   const int tid = threadIdx.x, row = blockIdx.x;
-  for (int e = tid; e < J; e += blockDim.x) wJ[e] = ldc(twx + 2L * L1 * e);
+  fill_level2_tw<T, L1, L2, L3>(wJ, twx);
   for (int j = tid; j < J; j += blockDim.x) {
     C2<T> v[L1];
 #pragma unroll
@@ -100,7 +128,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (L1 == 16 ? 3 : 4) : 0)
     Dft<T, L1, false>::run(v);
     s[j] = v[0];
 #pragma unroll
-    for (int k1 = 1; k1 < L1; k1++) s[k1 * J + j] = cmul(v[k1], ldc(twx + 2L * j * k1));  // W_M^(j k1)
+    for (int k1 = 1; k1 < L1; k1++) s[k1 * JP + j] = cmul(v[k1], level1_tw<T, J>(twx, tw1, j, k1));  // W_M^(j k1)
   }
   __syncthreads();
   {
@@ -109,15 +137,15 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (L1 == 16 ? 3 : 4) : 0)
     C2<T> u[L2];
     if (act) {
 #pragma unroll
-      for (int b = 0; b < L2; b++) u[b] = s[k1 * J + L3 * b + m];
+      for (int b = 0; b < L2; b++) u[b] = s[k1 * JP + L3 * b + m];
       Dft<T, L2, false>::run(u);
 #pragma unroll
-      for (int k2 = 1; k2 < L2; k2++) u[k2] = cmul(u[k2], wJ[m * k2]);
+      for (int k2 = 1; k2 < L2; k2++) u[k2] = cmul(u[k2], wJ[(k2 - 1) * L3 + m]);
     }
     __syncthreads();
     if (act) {
 #pragma unroll
-      for (int k2 = 0; k2 < L2; k2++) s[k1 * J + k2 * L3 + m] = u[k2];
+      for (int k2 = 0; k2 < L2; k2++) s[k1 * JP + k2 * L3 + m] = u[k2];
     }
   }
   __syncthreads();
@@ -127,7 +155,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (L1 == 16 ? 3 : 4) : 0)
     C2<T> w[L3];
     if (act) {
 #pragma unroll
-      for (int m = 0; m < L3; m++) w[m] = s[k1 * J + k2 * L3 + m];
+      for (int m = 0; m < L3; m++) w[m] = s[k1 * JP + k2 * L3 + m];
       Dft<T, L3, false>::run(w);
     }
     __syncthreads();
@@ -175,16 +203,17 @@ __global__ void __launch_bounds__(512) k_rows_c2r(const C2<T>* __restrict__ in, 
 //   level 2, item (n1, m < L3): DFT^-1_L2 over b of s[n1 J + L3 b + m], twiddle W_J^-(m n2)
 //                                                                      -> s[n1 J + n2 L3 + m]
 //   level 3, item (n1, n2):     DFT^-1_L3 over m                      -> z[n1 + L1 (n2 + L2 n3)]
-// and one coalesced copy of z to the output row.  Levels 2 and 3 read all their inputs
-// before a barrier and then overwrite the same buffer (M complex values, 40 KB at
-// M = 5000 in FP32).  Items of levels 2 and 3 fit in one pass of the CTA (L1 L3 and
-// L1 L2 <= blockDim).
-template <typename T, int L1, int L2, int L3>
-__device__ __forceinline__ void c2r3_row(const C2<T>* __restrict__ a, const C2<T>* __restrict__ twx, C2<T>* s) {
-  constexpr int J = L2 * L3, M = L1 * J;
-  C2<T>* wJ = s + M;  // W_J^e = W_Nx^(2 L1 e), e < J
+// and z from the registers of level 3 to put: to the output row, or over the shared buffer.
+// Level 2 reads all its inputs before a barrier and then overwrites the same buffer (M
+// complex values, 40 KB at M = 5000 in FP32).  Items of levels 2 and 3 fit in one pass of the
+// CTA (L1 L3 and L1 L2 <= blockDim).
+template <typename T, int L1, int L2, int L3, typename Put>
+__device__ __forceinline__ void c2r3_row(const C2<T>* __restrict__ a, const C2<T>* __restrict__ twx,
+                                         const C2<T>* __restrict__ tw1, C2<T>* s, Put put) {
+  constexpr int J = L2 * L3, M = L1 * J, JP = row_block<J>();
+  C2<T>* wJ = s + L1 * JP;  // (L2 - 1) L3 < J entries
   const int tid = threadIdx.x;
-  for (int e = tid; e < J; e += blockDim.x) wJ[e] = ldc(twx + 2L * L1 * e);
+  fill_level2_tw<T, L1, L2, L3>(wJ, twx);
   for (int j = tid; j < J; j += blockDim.x) {
     C2<T> v[L1];
 #pragma unroll
@@ -198,7 +227,7 @@ __device__ __forceinline__ void c2r3_row(const C2<T>* __restrict__ a, const C2<T
     Dft<T, L1, true>::run(v);
     s[j] = v[0];
 #pragma unroll
-    for (int n1 = 1; n1 < L1; n1++) s[n1 * J + j] = cmulc(v[n1], ldc(twx + 2L * j * n1));  // W_M^-(j n1)
+    for (int n1 = 1; n1 < L1; n1++) s[n1 * JP + j] = cmulc(v[n1], level1_tw<T, J>(twx, tw1, j, n1));  // W_M^-(j n1)
   }
   __syncthreads();
   {
@@ -207,47 +236,44 @@ __device__ __forceinline__ void c2r3_row(const C2<T>* __restrict__ a, const C2<T
     C2<T> u[L2];
     if (act) {
 #pragma unroll
-      for (int b = 0; b < L2; b++) u[b] = s[n1 * J + L3 * b + m];
+      for (int b = 0; b < L2; b++) u[b] = s[n1 * JP + L3 * b + m];
       Dft<T, L2, true>::run(u);
 #pragma unroll
-      for (int n2 = 1; n2 < L2; n2++) u[n2] = cmulc(u[n2], wJ[m * n2]);
+      for (int n2 = 1; n2 < L2; n2++) u[n2] = cmulc(u[n2], wJ[(n2 - 1) * L3 + m]);
     }
     __syncthreads();
     if (act) {
 #pragma unroll
-      for (int n2 = 0; n2 < L2; n2++) s[n1 * J + n2 * L3 + m] = u[n2];
+      for (int n2 = 0; n2 < L2; n2++) s[n1 * JP + n2 * L3 + m] = u[n2];
     }
   }
   __syncthreads();
-  {
-    const bool act = tid < L1 * L2;
-    const int n2 = tid / L1, n1 = tid - n2 * L1;  // n1 fastest: the writes below are contiguous
-    C2<T> w[L3];
-    if (act) {
+  // (thread tid = n1 + L1 n2 holds points tid + L1 L2 n3: whole lines of the row)
+  const bool act = tid < L1 * L2;
+  const int n2 = tid / L1, n1 = tid - n2 * L1;
+  C2<T> w[L3];
+  if (act) {
 #pragma unroll
-      for (int m = 0; m < L3; m++) w[m] = s[n1 * J + n2 * L3 + m];
-      Dft<T, L3, true>::run(w);
-    }
-    __syncthreads();
-    if (act) {
-#pragma unroll
-      for (int n3 = 0; n3 < L3; n3++) s[n1 + L1 * (n2 + L2 * n3)] = w[n3];
-    }
+    for (int m = 0; m < L3; m++) w[m] = s[n1 * JP + n2 * L3 + m];
+    Dft<T, L3, true>::run(w);
   }
-  __syncthreads();
+  put(act, tid, w);
 }
 
 template <typename T, int L1, int L2, int L3, typename TO>
 __global__ void __launch_bounds__(256) k_rows_c2r3(const C2<T>* __restrict__ in, long pitch,
                                                    TO* __restrict__ out, long ldo,
-                                                   const C2<T>* __restrict__ twx) {
-  constexpr int M = L1 * L2 * L3;
+                                                   const C2<T>* __restrict__ twx, const C2<T>* __restrict__ tw1) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C2<T>* s = reinterpret_cast<C2<T>*>(smem_raw);
   const int row = blockIdx.x;
-  c2r3_row<T, L1, L2, L3>(in + (long)row * pitch, twx, s);
   C2<TO>* dst = reinterpret_cast<C2<TO>*>(out + (long)row * ldo);
-  for (int n = threadIdx.x; n < M; n += blockDim.x) dst[n] = C2<TO>{out_cvt<TO>(s[n].x), out_cvt<TO>(s[n].y)};
+  c2r3_row<T, L1, L2, L3>(in + (long)row * pitch, twx, tw1, s, [&](bool act, int n0, const C2<T>* w) {
+    if (act) {
+#pragma unroll
+      for (int n3 = 0; n3 < L3; n3++) dst[n0 + L1 * L2 * n3] = C2<TO>{out_cvt<TO>(w[n3].x), out_cvt<TO>(w[n3].y)};
+    }
+  });
 }
 
 // P3 of four profiles with the interleave fused in.  A cluster of four CTAs takes one row
@@ -263,7 +289,8 @@ __global__ void __launch_bounds__(256) k_rows_c2r3(const C2<T>* __restrict__ in,
 template <typename T, int L1, int L2, int L3, typename TO>
 __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(256)
     k_rows_c2r3_il(const C2<T>* __restrict__ specs, long spec_stride, long pitch, int nm,
-                   TO* __restrict__ out, int S, const C2<T>* __restrict__ twx, unsigned planar) {
+                   TO* __restrict__ out, int S, const C2<T>* __restrict__ twx, const C2<T>* __restrict__ tw1,
+                   unsigned planar) {
   constexpr int J = L2 * L3, M = L1 * J, NX = 2 * M;
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
@@ -276,7 +303,15 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(256)
     T* d = reinterpret_cast<T*>(s);
     for (int n = threadIdx.x; n < NX; n += blockDim.x) d[n] = T(src[n]);
   } else if (q < nm) {
-    c2r3_row<T, L1, L2, L3>(specs + (long)q * spec_stride + (long)row * pitch, twx, s);
+    c2r3_row<T, L1, L2, L3>(specs + (long)q * spec_stride + (long)row * pitch, twx, tw1, s,
+                            [&](bool act, int n0, const C2<T>* w) {
+                              __syncthreads();
+                              if (act) {
+#pragma unroll
+                                for (int n3 = 0; n3 < L3; n3++) s[n0 + L1 * L2 * n3] = w[n3];
+                              }
+                              __syncthreads();
+                            });
   } else {
     for (int n = threadIdx.x; n < M; n += blockDim.x) s[n] = C2<T>{T(0), T(0)};
   }
@@ -433,7 +468,7 @@ __device__ __forceinline__ void c2r5_row(const C2<T>* __restrict__ a, const C2<T
 template <typename T, typename TO>
 __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(512, 2)
     k_rows_c2r5_il(const C2<T>* __restrict__ specs, long spec_stride, long pitch, int nm, TO* __restrict__ out,
-                   int S, const C2<T>* __restrict__ twx, unsigned planar) {
+                   int S, const C2<T>* __restrict__ twx, const C2<T>*, unsigned planar) {
   constexpr int NX = 10000;
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
@@ -893,7 +928,7 @@ static void launch_rows_r2c(mlc_ctx* ctx, const FftPlan2D& p, const Loader& ld, 
   // the profile's 2h rows (P0) timed apart from the map's rows
   const char* name = std::is_same<Loader, ProfileRows<T>>::value ? "fft_profile_rows" : "fft_rows_r2c";
   {
-    using K3 = void (*)(Loader, C2<T>*, long, const C2<T>*);
+    using K3 = void (*)(Loader, C2<T>*, long, const C2<T>*, const C2<T>*);
     K3 k3 = nullptr;
     int J = 0;
     // float-float: the five-level kernel of 5000-point rows (the three-level ones would
@@ -920,11 +955,11 @@ static void launch_rows_r2c(mlc_ctx* ctx, const FftPlan2D& p, const Loader& ld, 
       }
     }
     if (k3) {
-      const size_t smem3 = ((size_t)p.M + J) * sizeof(C2<T>);
+      const size_t smem3 = ((size_t)p.M + J + 16) * sizeof(C2<T>);  // (16: row_block)
       set_max_smem((const void*)k3, smem3);
       {
         MLC_KSCOPE(ctx, name);
-        k3<<<nrows, 256, smem3, ctx->stream>>>(ld, (C2<T>*)out, p.Wp, (const C2<T>*)p.twx);
+        k3<<<nrows, 256, smem3, ctx->stream>>>(ld, (C2<T>*)out, p.Wp, (const C2<T>*)p.twx, (const C2<T>*)p.twl);
       }
       MLC_CHECK_LAUNCH();
       return;
@@ -943,7 +978,7 @@ static void launch_rows_r2c(mlc_ctx* ctx, const FftPlan2D& p, const Loader& ld, 
 template <typename T, typename TO = typename RealOut<T>::type>
 static void launch_rows_c2r(mlc_ctx* ctx, const FftPlan2D& p, const void* in, void* out) {
   if constexpr (!(std::is_same<T, ff>::value && std::is_same<TO, float>::value)) {  // (those: limb2_rows_c2r)
-    using K3 = void (*)(const C2<T>*, long, TO*, long, const C2<T>*);
+    using K3 = void (*)(const C2<T>*, long, TO*, long, const C2<T>*, const C2<T>*);
     K3 k3 = nullptr;
     int J = 0;
     switch (p.M) {
@@ -954,11 +989,12 @@ static void launch_rows_c2r(mlc_ctx* ctx, const FftPlan2D& p, const void* in, vo
       default: break;
     }
     if (k3) {
-      const size_t smem3 = ((size_t)p.M + J) * sizeof(C2<T>);
+      const size_t smem3 = ((size_t)p.M + J + 16) * sizeof(C2<T>);  // (16: row_block)
       set_max_smem((const void*)k3, smem3);
       {
         MLC_KSCOPE(ctx, "fft_rows_c2r");
-        k3<<<p.Ny, 256, smem3, ctx->stream>>>((const C2<T>*)in, p.Wp, (TO*)out, p.Nx, (const C2<T>*)p.twx);
+        k3<<<p.Ny, 256, smem3, ctx->stream>>>((const C2<T>*)in, p.Wp, (TO*)out, p.Nx, (const C2<T>*)p.twx,
+                                              (const C2<T>*)p.twl);
       }
       MLC_CHECK_LAUNCH();
       return;
@@ -1287,7 +1323,7 @@ void rows_c2r_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* spec, void* out
 template <typename T, typename TO>
 bool c2r_interleave_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* specs, long spec_stride, int nm, int S,
                          void* out, unsigned planar) {
-  using K = void (*)(const C2<T>*, long, long, int, TO*, int, const C2<T>*, unsigned);
+  using K = void (*)(const C2<T>*, long, long, int, TO*, int, const C2<T>*, const C2<T>*, unsigned);
   K k = nullptr;
   int J = 0, nthr = 256;
   switch (p.M) {
@@ -1306,13 +1342,13 @@ bool c2r_interleave_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* specs, lo
     default: return false;
   }
   if (!rows_c2r_interleave_supported(p)) return false;
-  const size_t smem = ((size_t)p.M + J) * sizeof(C2<T>);
+  const size_t smem = ((size_t)p.M + J + 16) * sizeof(C2<T>);  // (16: row_block)
   set_max_smem((const void*)k, smem);
   const int quads = (nm + 3) / 4;
   {
     MLC_KSCOPE(ctx, "fft_rows_c2r_interleave");
     k<<<dim3(4 * quads, p.Ny), nthr, smem, ctx->stream>>>((const C2<T>*)specs, spec_stride, p.Wp, nm, (TO*)out, S,
-                                                           (const C2<T>*)p.twx, planar);
+                                                           (const C2<T>*)p.twx, (const C2<T>*)p.twl, planar);
   }
   MLC_CHECK_LAUNCH();
   return true;

@@ -28,7 +28,8 @@ struct FftPlan2D {
   void* twy = nullptr;  // Ny-entry table exp(-2 pi i m / Ny)
   void* twx3 = nullptr;  // the same tables in three limbs (FP64 plans; see LimbTab)
   void* twy3 = nullptr;
-  void* twl3 = nullptr;  // W_M^(m q), [q - 1][m]: level 0 of the row transforms (limb_first_radix)
+  void* twl3 = nullptr;  // W_M^(m q), [q - 1][m]: level 0 of the limb row transforms (limb_first_radix)
+  void* twl = nullptr;   // the same for level 1 of FP32 three-level rows (row3_first_radix)
   size_t elem = 0;      // sizeof(C2<T>)
   size_t spec_bytes() const { return (size_t)Ny * Wp * elem; }
   ~FftPlan2D();
@@ -40,6 +41,9 @@ inline int limb_level0_entries(int M) {
   const int r = limb_first_radix(M);
   return r ? (r - 1) * (M / r) : 0;
 }
+
+// First radix of the three-level row transforms of M points (fft_impl.cuh), 0 where there is none.
+inline int row3_first_radix(int M) { return M == 5000 || M == 2000 ? 8 : M == 4096 ? 16 : M == 1000 ? 10 : 0; }
 
 // Internal plan precisions (mlc_map_set_fft): FFTs in float-float arithmetic of FP64 maps
 // (FP64 outputs), and of FP32 maps (float-float spectra, FP32 outputs).

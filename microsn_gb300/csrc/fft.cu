@@ -25,6 +25,7 @@
 // kernels and launch sequences are in fft_impl.cuh.
 #include <algorithm>
 #include <cmath>
+#include <functional>
 #include <map>
 #include <mutex>
 #include <unordered_map>
@@ -75,6 +76,50 @@ RadixList factor_radices(int L, int tw_stride) {
   return rl;
 }
 
+// Few and large radices: a level's twiddle products and its trip through shared memory cost more
+// than the additions of a larger small transform.
+AnyLevels any_levels(int L, bool pad) {
+  AnyLevels lv;
+  lv.L = L;
+  if (L < 2 || L > 65535) return lv;
+  int e2 = 0, e3 = 0, e5 = 0, n = L;
+  while (n % 2 == 0) e2++, n /= 2;
+  while (n % 3 == 0) e3++, n /= 3;
+  while (n % 5 == 0) e5++, n /= 5;
+  if (n != 1) return lv;
+  std::vector<int> r;
+  while (e2 > 0 && e5 > 0) r.push_back(10), e2--, e5--;
+  while (e3 > 1) r.push_back(9), e3 -= 2;
+  while (e2 > 2 && e2 != 4) r.push_back(8), e2 -= 3;
+  while (e2 > 1) r.push_back(4), e2 -= 2;
+  if (e2 > 0 && e3 > 0) r.push_back(6), e2--, e3--;
+  for (; e5 > 0; e5--) r.push_back(5);
+  for (; e3 > 0; e3--) r.push_back(3);
+  for (; e2 > 0; e2--) r.push_back(2);
+  std::sort(r.begin(), r.end(), std::greater<int>());
+  if ((int)r.size() > AnyLevels::MAX) return lv;
+  lv.n = (int)r.size();
+  auto magic = [](int d) { return d > 1 ? (uint32_t)((0x100000000ull + d - 1) / d) : 0u; };
+  int b = L;
+  for (int i = 0; i < lv.n; i++) {
+    lv.r[i] = r[i];
+    b /= r[i];
+    lv.bn[i] = b;
+    lv.tw[i] = lv.ntw;
+    if (i + 1 < lv.n) lv.ntw += (r[i] - 1) * b;
+    lv.mr[i] = magic(r[i]);
+    lv.mbn[i] = magic(b);
+  }
+  int t = 1;  // places of one sub-block, from the innermost outwards, odd where they are padded
+  for (int i = lv.n - 1; i >= 0; i--) {
+    lv.tn[i] = t;
+    t *= r[i];
+    if (pad && i > 0) t |= 1;
+  }
+  lv.places = t;
+  return lv;
+}
+
 // The attribute belongs to the function on the current device: a process holding contexts
 // on several GPUs sets it once per (device, function).
 void set_max_smem(const void* func, size_t bytes) {
@@ -91,7 +136,7 @@ void set_max_smem(const void* func, size_t bytes) {
 }
 
 FftPlan2D::~FftPlan2D() {
-  for (void* t : {twx, twy, twx3, twy3, twl3, twl})
+  for (void* t : {twx, twy, twx3, twy3, twl3, twl, anyM_tw, any1_tw, any2_tw})
     if (t) cudaFree(t);
 }
 
@@ -200,6 +245,29 @@ static void* upload_level0_f32(int M) {
   return d;
 }
 
+// The levels' twiddles W_{B_i}^(m q), [q - 1][m], one level after another.
+static void* upload_any(const AnyLevels& lv, bool limbs3) {
+  if (lv.n < 2) return nullptr;
+  std::vector<long double> re, im, lr, li;
+  twiddle_table(lv.L, re, im);
+  int f = 1;  // W_{B_i} = W_L^f
+  for (int i = 0; i + 1 < lv.n; i++) {
+    for (int q = 1; q < lv.r[i]; q++)
+      for (int m = 0; m < lv.bn[i]; m++) {
+        lr.push_back(re[(size_t)m * q * f]);
+        li.push_back(im[(size_t)m * q * f]);
+      }
+    f *= lv.r[i];
+  }
+  if (limbs3) return upload_limbs3(lr, li);
+  std::vector<C2<ff>> h(lr.size());
+  for (size_t i = 0; i < h.size(); i++) h[i] = C2<ff>{ff((double)lr[i]), ff((double)li[i])};
+  void* d = nullptr;
+  MLC_CUDA(cudaMalloc(&d, h.size() * sizeof(C2<ff>)));
+  MLC_CUDA(cudaMemcpy(d, h.data(), h.size() * sizeof(C2<ff>), cudaMemcpyHostToDevice));
+  return d;
+}
+
 static void split_columns(int Ny, int& N1, int& N2) {
   int best = 1;
   for (int d = 1; (long)d * d <= Ny; d++)
@@ -245,6 +313,16 @@ FftPlan2D* plan_get(mlc_ctx* ctx, int Nx, int Ny, int prec) {
     p->twx = upload_twiddles<float>(Nx);
     p->twy = upload_twiddles<float>(Ny);
     if (row3_first_radix(p->M)) p->twl = upload_level0_f32(p->M);
+  }
+  if (prec == MLC_F64 || prec == PREC_FFS) {
+    p->anyM = any_levels(p->M, true);
+    p->anyM_tw = upload_any(p->anyM, prec == MLC_F64);
+  }
+  if (prec == MLC_F64) {
+    p->any1 = any_levels(p->N1, false);
+    p->any2 = any_levels(p->N2, false);
+    p->any1_tw = upload_any(p->any1, true);
+    p->any2_tw = upload_any(p->any2, true);
   }
   FftPlan2D* raw = p.get();
   ctx->plans[key] = std::move(p);

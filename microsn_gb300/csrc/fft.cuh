@@ -45,7 +45,7 @@ struct Dft<T, 3, INV> {
     const T h = (T)0.86602540378443864676372317075294;  // sin(2 pi / 3)
     C2<T> s = cadd(v[1], v[2]);
     C2<T> d = csub(v[1], v[2]);
-    C2<T> m = C2<T>{v[0].x - (T)0.5 * s.x, v[0].y - (T)0.5 * s.y};
+    C2<T> m = C2<T>{v[0].x - scale2(s.x, 0.5f), v[0].y - scale2(s.y, 0.5f)};
     C2<T> id = mul_mi<T, INV>(d);  // -i d (forward) / +i d (inverse)
     v[0] = cadd(v[0], s);
     v[1] = C2<T>{m.x + h * id.x, m.y + h * id.y};
@@ -162,6 +162,61 @@ struct Dft<T, 10, INV> {
     for (int k2 = 0; k2 < 5; k2++) {
       v[(6 * k2) % 10] = a[k2];
       v[(5 + 6 * k2) % 10] = b[k2];
+    }
+  }
+};
+
+// 6 points by the prime-factor split 6 = 2 x 3: n = (3 n1 + 2 n2) mod 6, k = (3 k1 + 4 k2) mod 6.
+template <typename T, bool INV>
+struct Dft<T, 6, INV> {
+  static __device__ __forceinline__ void run(C2<T>* v) {
+    C2<T> a[3], b[3];
+#pragma unroll
+    for (int n2 = 0; n2 < 3; n2++) {
+      const C2<T> x0 = v[(2 * n2) % 6], x1 = v[(3 + 2 * n2) % 6];
+      a[n2] = cadd(x0, x1);
+      b[n2] = csub(x0, x1);
+    }
+    Dft<T, 3, INV>::run(a);
+    Dft<T, 3, INV>::run(b);
+#pragma unroll
+    for (int k2 = 0; k2 < 3; k2++) {
+      v[(4 * k2) % 6] = a[k2];
+      v[(3 + 4 * k2) % 6] = b[k2];
+    }
+  }
+};
+
+// 9 points as 3 x 3: DFT3 over n1 of x[3 n1 + n2], twiddle W9^(n2 k1), DFT3 over n2 -> X[k1 + 3 k2].
+template <typename T, bool INV>
+struct Dft<T, 9, INV> {
+  static __device__ __forceinline__ void run(C2<T>* v) {
+    // cos, sin(2 pi m / 9), m = 1, 2, 4
+    const T cr[3] = {(T)0.76604444311897803520239265055541668, (T)0.17364817766693034885171662676931480,
+                     (T)-0.93969262078590838405410927732473147};
+    const T ci[3] = {(T)0.64278760968653932632264340990726343, (T)0.98480775301220805936674302458952303,
+                     (T)0.34202014332566873304409961468225958};
+    C2<T> y[3][3];
+#pragma unroll
+    for (int n2 = 0; n2 < 3; n2++) {
+#pragma unroll
+      for (int n1 = 0; n1 < 3; n1++) y[n2][n1] = v[3 * n1 + n2];
+      Dft<T, 3, INV>::run(y[n2]);
+#pragma unroll
+      for (int k1 = 1; k1 < 3; k1++) {
+        if (n2 == 0) continue;
+        const int m = n2 * k1 == 4 ? 2 : n2 * k1 - 1;  // m = 1, 2, 4 -> 0, 1, 2
+        const T sr = INV ? -ci[m] : ci[m];
+        const C2<T> q = y[n2][k1];
+        y[n2][k1] = C2<T>{lin2(cr[m], q.x, sr, q.y), lin2(cr[m], q.y, -sr, q.x)};
+      }
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < 3; k1++) {
+      C2<T> u[3] = {y[0][k1], y[1][k1], y[2][k1]};
+      Dft<T, 3, INV>::run(u);
+#pragma unroll
+      for (int k2 = 0; k2 < 3; k2++) v[k1 + 3 * k2] = u[k2];
     }
   }
 };

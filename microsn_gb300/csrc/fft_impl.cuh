@@ -73,16 +73,6 @@ __global__ void __launch_bounds__(512) k_rows_r2c(Loader ld, C2<T>* __restrict__
   for (int k = M + 1 + threadIdx.x; k < pitch; k += blockDim.x) o[k] = C2<T>{(T)0, (T)0};
 }
 
-// Real FFT of one row per CTA with M = L1 L2 L3 (J = L2 L3) in three register levels, the
-// forward counterpart of c2r3_row below (same item shapes, forward DFTs and twiddles):
-//   level 1, item j < J:        z[J a + j] (a < L1) from the loader, DFT_L1 over a,
-//                               twiddle W_M^(j k1)                    -> s[k1 J + j]
-//   level 2, item (k1, m < L3): DFT_L2 over b of s[k1 J + L3 b + m], twiddle W_J^(m k2)
-//                                                                      -> s[k1 J + k2 L3 + m]
-//   level 3, item (k1, k2):     DFT_L3 over m                      -> Z[k1 + L1 (k2 + L2 k3)]
-// then the split into Nx/2+1 spectrum values and the zero padding up to Wp.  FP32: four
-// CTAs per SM (three for 16^3, whose 80 registers would spill at 64), like k_rows_c2r3;
-// FP64 keeps the compiler's allocation (its 90 KB rows fit two CTAs per SM anyway).
 // Level 1's twiddle W_M^(j q) of the three-level rows.  FP32 plans hold these in the order [q - 1][j]
 // (tw1), which consecutive lanes read as whole lines: out of the table of W_Nx they are 2 q
 // entries apart, a sector per lane (with row_block: rows of 4096 points at 8192^2, c2r 207 -> 146 us and 133
@@ -111,6 +101,16 @@ constexpr int row_block() {
   return J % 16 == 0 ? J + 1 : J;
 }
 
+// Real FFT of one row per CTA with M = L1 L2 L3 (J = L2 L3) in three register levels, the
+// forward counterpart of c2r3_row below (same item shapes, forward DFTs and twiddles):
+//   level 1, item j < J:        z[J a + j] (a < L1) from the loader, DFT_L1 over a,
+//                               twiddle W_M^(j k1)                    -> s[k1 J + j]
+//   level 2, item (k1, m < L3): DFT_L2 over b of s[k1 J + L3 b + m], twiddle W_J^(m k2)
+//                                                                      -> s[k1 J + k2 L3 + m]
+//   level 3, item (k1, k2):     DFT_L3 over m                      -> Z[k1 + L1 (k2 + L2 k3)]
+// then the split into Nx/2+1 spectrum values and the zero padding up to Wp.  FP32: four
+// CTAs per SM (three for 16^3, whose 80 registers would spill at 64), like k_rows_c2r3;
+// FP64 keeps the compiler's allocation (its 90 KB rows fit two CTAs per SM anyway).
 template <typename T, int L1, int L2, int L3, typename Loader>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? (L1 == 16 ? 3 : 4) : 0)
     k_rows_r2c3(Loader ld, C2<T>* __restrict__ out, long pitch, const C2<T>* __restrict__ twx,

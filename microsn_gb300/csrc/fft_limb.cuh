@@ -867,6 +867,17 @@ constexpr int limb_cw(int g) {
   return sizeof(T) == sizeof(lf2) || g == 16 ? 16 : 32;
 }
 
+// The same passes for other lengths (fft_limb_any.cu).
+template <bool INV>
+bool any_colpass_impl(mlc_ctx* ctx, const FftPlan2D& p, void* buf, char kind, int post_tw);
+template <typename T>
+bool any_rows_c2r_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* in, void* out);
+template <typename T, typename Loader>
+bool any_rows_r2c_impl(mlc_ctx* ctx, const FftPlan2D& p, const Loader& ld, int nrows, void* out, const char* name);
+bool any3_conv_fits(const FftPlan2D& p);
+void any3_conv(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, void* out, const LimbSpectrum& rows, int h, lf3 r,
+               int rexp);
+
 template <typename T, bool INV>
 bool limb_colpass_impl(mlc_ctx* ctx, const FftPlan2D& p, void* buf, char kind, int post_tw) {
   using S = typename LimbTraits<T>::S;
@@ -883,7 +894,10 @@ bool limb_colpass_impl(mlc_ctx* ctx, const FftPlan2D& p, void* buf, char kind, i
     case 80: k = k_limb_colpass2<S, T, limb_cw<T>(10), 8, 10, INV>; g = 10; break;
     case 50: k = k_limb_colpass2<S, T, limb_cw<T>(10), 5, 10, INV>; g = 10; break;
     case 40: k = k_limb_colpass2<S, T, limb_cw<T>(8), 5, 8, INV>; g = 8; break;
-    default: return false;
+    default:
+      // (lf2: the float-float kernel is as fast, 42 and 53 us at 2400^2)
+      if constexpr (sizeof(T) == sizeof(lf3)) return any_colpass_impl<INV>(ctx, p, buf, kind, post_tw);
+      return false;
   }
   const int cw = limb_cw<T>(g);
   const size_t smem = LimbArr<T>::bytes(L * cw) + 2 * LimbArr<T>::bytes(L);
@@ -924,10 +938,7 @@ bool limb3_conv_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, void* o
       default: break;
     }
   }
-  if (!k) return false;
-  const int cw = limb_cw<lf3>(g);
-  const size_t smem = LimbArr<lf3>::bytes(p.N2 * cw) + 3 * LimbArr<lf3>::bytes(p.N2) + LimbArr<lf3>::bytes(p.N1);
-  set_max_smem((const void*)k, smem);
+  if (!k && !(MODE == 0 && any3_conv_fits(p))) return false;
   const LimbSpectrum rows = limb3_profile_rows(p, kx, 2 * h);
   if constexpr (MODE != 2) {
     MLC_KSCOPE(ctx, "conv_profile_columns");
@@ -942,6 +953,13 @@ bool limb3_conv_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, void* o
   const float a = (float)(rintl(m * 16777216.0L) / 16777216.0L);
   const float b = (float)(m - (long double)a);
   const lf3 r(a, b, (float)(m - (long double)a - (long double)b));
+  if (!k) {
+    any3_conv(ctx, p, Fmap, out, rows, h, r, -e);
+    return true;
+  }
+  const int cw = limb_cw<lf3>(g);
+  const size_t smem = LimbArr<lf3>::bytes(p.N2 * cw) + 3 * LimbArr<lf3>::bytes(p.N2) + LimbArr<lf3>::bytes(p.N1);
+  set_max_smem((const void*)k, smem);
   {
     MLC_KSCOPE(ctx, name);
     k<<<dim3(ceil_div(p.Wc, cw), p.N1), g * cw, smem, ctx->stream>>>((const C2<double>*)Fmap, (C2<double>*)out, p.Wp,
@@ -1005,7 +1023,7 @@ template <typename T>
 bool limb_rows_c2r_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* in, void* out) {
   using S = typename LimbTraits<T>::S;
   using TO = typename LimbTraits<T>::TO;
-  return limb_row_dispatch<T>(p.M, [&](auto lv, auto nt) {
+  const bool done = limb_row_dispatch<T>(p.M, [&](auto lv, auto nt) {
     using LV = decltype(lv);
     auto k = k_limb_rows_c2r<S, T, TO, decltype(nt)::value, LV>;
     const size_t smem = limb_row_smem<T, LV>();
@@ -1016,6 +1034,7 @@ bool limb_rows_c2r_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* in, void* 
     }
     MLC_CHECK_LAUNCH();
   });
+  return done || any_rows_c2r_impl<T>(ctx, p, in, out);
 }
 
 template <typename T>
@@ -1040,7 +1059,7 @@ bool limb_rows_c2r_il_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* specs, 
 template <typename T, typename Loader>
 bool limb_rows_r2c_impl(mlc_ctx* ctx, const FftPlan2D& p, const Loader& ld, int nrows, void* out, const char* name) {
   using S = typename LimbTraits<T>::S;
-  return limb_row_dispatch<T>(p.M, [&](auto lv, auto nt) {
+  const bool done = limb_row_dispatch<T>(p.M, [&](auto lv, auto nt) {
     using LV = decltype(lv);
     auto k = k_limb_rows_r2c<S, T, decltype(nt)::value, LV, Loader>;
     const size_t smem = limb_row_smem<T, LV>();
@@ -1051,6 +1070,7 @@ bool limb_rows_r2c_impl(mlc_ctx* ctx, const FftPlan2D& p, const Loader& ld, int 
     }
     MLC_CHECK_LAUNCH();
   });
+  return done || any_rows_r2c_impl<T>(ctx, p, ld, nrows, out, name);
 }
 
 }  // namespace mlc

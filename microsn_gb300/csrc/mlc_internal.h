@@ -13,6 +13,19 @@
 
 namespace mlc {
 
+// An in-place transform of L points in shared memory by any radices (fft_limb_any.cu): level i
+// works on blocks of r[0] ... r[i-1] parts, each of r[i] sub-blocks of bn[i] points that lie
+// tn[i] places apart; its twiddles [q - 1][m] start at entry tw[i] of the table.
+struct AnyLevels {
+  static constexpr int MAX = 10;
+  int L = 0, n = 0;  // n = 0: none (L = 1, or a factor other than 2, 3 and 5)
+  int r[MAX] = {}, bn[MAX] = {}, tn[MAX] = {}, tw[MAX] = {};
+  uint32_t mr[MAX] = {}, mbn[MAX] = {};  // multipliers that divide by r[i], bn[i] (numerators below 2^16)
+  int places = 0;                        // places the points take
+  int ntw = 0;                           // entries of the whole table
+};
+AnyLevels any_levels(int L, bool pad);
+
 // Plan for 2-D real transforms of an Ny x Nx image: rows are real FFTs of length Nx
 // (a complex FFT of length M = Nx/2 plus the split post-process); columns are complex
 // FFTs of length Ny = N1 * N2 done as two in-place sub-passes over row sets.
@@ -29,7 +42,11 @@ struct FftPlan2D {
   void* twx3 = nullptr;  // the same tables in three limbs (FP64 plans; see LimbTab)
   void* twy3 = nullptr;
   void* twl3 = nullptr;  // W_M^(m q), [q - 1][m]: level 0 of the limb row transforms (limb_first_radix)
-  void* twl = nullptr;   // the same for level 1 of FP32 three-level rows (row3_first_radix)
+  AnyLevels anyM{}, any1{}, any2{};  // M, N1 and N2 points by any radices, and their tables
+  void* anyM_tw = nullptr;           // (the arithmetic's own layout: float-float, or three limbs)
+  void* any1_tw = nullptr;
+  void* any2_tw = nullptr;
+  void* twl = nullptr;   // the same as twl3 for level 1 of FP32 three-level rows (row3_first_radix)
   size_t elem = 0;      // sizeof(C2<T>)
   size_t spec_bytes() const { return (size_t)Ny * Wp * elem; }
   ~FftPlan2D();

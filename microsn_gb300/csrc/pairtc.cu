@@ -16,16 +16,24 @@
 //
 // Kernel layout (one persistent CTA per SM, 4 + 12..24 warps):
 //   warp 0      TMA producer: the work item's 128 A rows (3 slices x Kp, resident in shared
-//               memory) and, double-buffered, each 48-row B tile
-//   warp 1      MMA issuer (one thread): 9 slice pairs x Kp/16 tcgen05.mma per tile into one
-//               of two TMEM buffers (5 accumulators x 48 columns each; buffers at columns
-//               0 and 256 of the 512 allocated)
+//               memory) and, double-buffered, each 48-row B tile, its three slices stacked
+//               into 144 rows
+//   warp 1      MMA issuer: per K step one tcgen05.mma of each A slice against the stacked B
+//               slices (N = 144), into one of two TMEM buffers (5 accumulators x 48 columns,
+//               d ascending, so the three products of a slice are side by side; buffers at
+//               columns 0 and 256 of the 512 allocated)
 //   warp 2      TMEM allocation / release
 //   warps 4..    epilogue (12, 16 or 24 warps, the same number per TMEM lane quadrant; the
 //               autotuner picks the count): TMEM ->
 //               registers, chi2 assembly, log10-chi2 histogram in shared memory, top-k
 //               candidates below a threshold, refinement list, optional matrix
 // Every barrier wait is bounded; a timeout sets the error flag and all roles unwind.
+//
+// Measured, 10^10 pairs of 128 epochs: 15.8 ms.  The MMAs alone take 12.6 ms (loads and waits
+// kept, the arithmetic after them left out; 9.7 ms at the tensor pipe's rate), the epilogue is
+// the rest: 34 instructions a pair.  One MMA per slice pair (N = 48, 72 a tile, issued by a
+// lone thread) took 33.5 ms, bound by the issue of an MMA, some 50 cycles whatever its shape;
+// the epilogue's scalar form (56 instructions) was hidden behind it.
 #include <cuda.h>
 
 #include <algorithm>
@@ -48,13 +56,13 @@ constexpr int TM = PD_TILE_M, TN = PD_TILE_N;
 constexpr int NSTAGE = 2;
 // Epilogue shapes: EPIW warps (a multiple of 4: the same number per TMEM lane quadrant, one
 // per SM sub-partition each), each taking WCOLS of the 48 tile columns, CCH per TMEM load.
-// 12 warps: 16 columns (loads of 8); 16: 12 (loads of 4); 24: 8 (one load of 8).
+// 12 warps: 16 columns; 16: 12; 24: 8.
 template <int EPIW>
 struct Epi {
   static constexpr int warps = EPIW;
   static constexpr int per_q = EPIW / 4;
   static constexpr int wcols = TN / per_q;
-  static constexpr int cch = wcols % 8 == 0 ? 8 : 4;
+  static constexpr int cch = 4;
   static constexpr int threads = (4 + EPIW) * 32;
   static_assert(EPIW % 4 == 0 && wcols * per_q == TN && wcols % cch == 0 && wcols <= 16, "epilogue column split");
 };
@@ -100,6 +108,47 @@ size_t smem_bytes(int nkb, int nbins) {
 
 // 2^k for k in [-126, 127]; 0 below (the terms it scales are then negligible)
 __device__ __forceinline__ float pow2f(int k) { return k < -126 ? 0.f : __int_as_float((k + 127) << 23); }
+
+// Two FP32 values in one 64-bit register pair, and the packed operations on them: each half
+// rounds as the scalar operation does, for one issue slot instead of two.
+struct f2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ f2 f2_pack(float a, float b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 f2_split(f2 a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
+  return r;
+}
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ f2 f2_sub(f2 a, f2 b) {
+  f2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ float lg2_approx(float x) {
+  float r;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
 
 // Error-free sum s + e = a + b.
 __device__ __forceinline__ float two_sum(float a, float b, float& e) {
@@ -147,10 +196,11 @@ __global__ void __launch_bounds__(Epi<EPIW>::threads, 1) k_pairdiff_tc(const __g
   volatile int* abort_s = (volatile int*)(tmem_slot + 1);
   uint32_t* hist_s = tmem_slot + 4;
   // counters: below lo, the nbins bins, at or above hi (flushed to the global layout: bins, below, above)
-  float4* colv = (float4*)(hist_s + ((P.nbins + 2 + 3) & ~3));  // [EPIW][16] column constants
+  float* colv = (float*)(hist_s + ((P.nbins + 2 + 3) & ~3));  // [EPIW][8 pairs][8] column constants
   const uint32_t hist_sa = tc::smem_u32(hist_s);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // (the warp's number as a uniform value)
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     tc::mbar_init(a_full, 1);
     tc::mbar_init(a_empty, 1);
@@ -168,7 +218,7 @@ __global__ void __launch_bounds__(Epi<EPIW>::threads, 1) k_pairdiff_tc(const __g
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
   auto fail = [&]() {
     *abort_s = 1;
@@ -190,51 +240,60 @@ __global__ void __launch_bounds__(Epi<EPIW>::threads, 1) k_pairdiff_tc(const __g
         const uint32_t s = cB & 1, u = cB >> 1;
         if (*abort_s || !tc::mbar_wait(b_empty + s, (u & 1) ^ 1)) { fail(); break; }
         tc::mbar_arrive_expect_tx(b_full + s, 3 * nkb * B_BOX);
-        for (int bx = 0; bx < 3 * nkb; bx++)
-          tc::tma_load_2d(B_s + (s * 3 * nkb + bx) * B_BOX, &tmB, b_full + s, bx * 64, jt * TN);
+        for (int b = 0; b < 3; b++)  // a K box's three slices one below the other: 3 TN rows
+          for (int kb = 0; kb < nkb; kb++)
+            tc::tma_load_2d(B_s + (s * 3 * nkb + kb * 3 + b) * B_BOX, &tmB, b_full + s, (b * nkb + kb) * 64, jt * TN);
       }
     }
-  } else if (warp == 1 && lane == 0) {
-    // ------------------------------------------------ MMA issuer
-    const uint32_t idesc = tc::idesc_bf16(TM, TN);
+  } else if (warp == 1) {
+    // ------------------------------------------------ MMA issuer (the whole warp; lane 0 issues)
+    const uint32_t issue = lane == 0;
     uint32_t cB = 0, ct = 0, n = 0;
     // Descriptors of the box starts: the start-address field holds (address >> 4) in its low
     // 14 bits and shared-memory addresses stay below 2^18, so a descriptor for
-    // base + offset is the base descriptor plus offset >> 4 (no carry).
-    const uint64_t dA = tc::desc_sw128(tc::smem_u32(A_s));
-    const uint64_t dB0 = tc::desc_sw128(tc::smem_u32(B_s)), dB1 = tc::desc_sw128(tc::smem_u32(B_s + 3 * nkb * B_BOX));
+    // base + offset is the base descriptor plus offset >> 4 in its low word (no carry).
+    const uint64_t dA = tc::desc_sw128(tc::smem_u32(A_s)), dB = tc::desc_sw128(tc::smem_u32(B_s));
+    const uint32_t a_hi = (uint32_t)(dA >> 32), a_lo = (uint32_t)dA, b_hi = (uint32_t)(dB >> 32), b_lo = (uint32_t)dB;
     for (int it = blockIdx.x; it < P.nitems && !*abort_s; it += gridDim.x, n++) {
       const int jc = it % P.njc;
       const int j0 = jc * P.jchunk, j1 = min(P.nj, j0 + P.jchunk);
-      if (!tc::mbar_wait(a_full, n & 1)) { fail(); break; }
+      if (!__all_sync(0xffffffffu, tc::mbar_wait(a_full, n & 1))) { fail(); break; }
       for (int jt = j0; jt < j1; jt++, cB++, ct++) {
         const uint32_t s = cB & 1, u = cB >> 1, tb = ct & 1, tu = ct >> 1;
-        if (*abort_s || !tc::mbar_wait(b_full + s, u & 1) || !tc::mbar_wait(t_empty + tb, (tu & 1) ^ 1)) {
+        if (!__all_sync(0xffffffffu, !*abort_s && tc::mbar_wait(b_full + s, u & 1) &&
+                                         tc::mbar_wait(t_empty + tb, (tu & 1) ^ 1))) {
           fail();
           break;
         }
         tc::fence_after_sync();
         const uint32_t dbase = tmem + tb * TBUF;
-        const uint64_t dBs = s ? dB1 : dB0;
-        // slice pairs ordered so that each accumulator's first MMA clears it
+        const uint32_t bs_lo = b_lo + s * (uint32_t)((3 * nkb * B_BOX) >> 4);
+        // Slice a of A against the three stacked slices of B, N = 3 TN, lands in the accumulators
+        // d = a, a+1, a+2, which lie side by side.  The first K step clears an accumulator where
+        // its first pair is formed: d = 0..2 together, d = 3 and 4 by (a, b) = (1, 2), (2, 2).
 #pragma unroll
-        for (int a = 0; a < 3; a++)
+        for (int kk = 0; kk < nkb * 4; kk++) {
+          const int kb = kk >> 2, ko = (kk & 3) * 32;
 #pragma unroll
-          for (int b = 0; b < 3; b++) {
-            const int d = a + b;
-            const bool first_of_d = (a == 0) || (b == 2);  // (0,b) opens d <= 2; (a,2) opens d = 3, 4
-#pragma unroll
-            for (int kk = 0; kk < nkb * 4; kk++) {
-              const int kb = kk >> 2, ko = (kk & 3) * 32;
-              const uint64_t ad = dA + (uint64_t)((((a * nkb + kb) * A_BOX) + ko) >> 4);
-              const uint64_t bd = dBs + (uint64_t)((((b * nkb + kb) * B_BOX) + ko) >> 4);
-              tc::mma_bf16(dbase + d * TN, ad, bd, idesc, (first_of_d && kk == 0) ? 0u : 1u);
+          for (int a = 0; a < 3; a++) {
+            const uint32_t al = a_lo + (uint32_t)((((a * nkb + kb) * A_BOX) + ko) >> 4);
+            const uint32_t bl = bs_lo + (uint32_t)(((kb * 3 * B_BOX) + ko) >> 4);
+            if (kk > 0 || a == 0) {
+              tc::mma_bf16(issue, dbase + a * TN, a_hi, al, b_hi, bl, tc::idesc_bf16(TM, 3 * TN), kk > 0 ? 1u : 0u);
+            } else {
+              tc::mma_bf16(issue, dbase + a * TN, a_hi, al, b_hi, bl, tc::idesc_bf16(TM, 2 * TN), 1u);
+              tc::mma_bf16(issue, dbase + (a + 2) * TN, a_hi, al, b_hi, bl + (2 * B_BOX >> 4), tc::idesc_bf16(TM, TN), 0u);
             }
           }
-        tc::mma_commit(b_empty + s);
-        tc::mma_commit(t_full + tb);
+        }
+        if (lane == 0) {
+          tc::mma_commit(b_empty + s);
+          tc::mma_commit(t_full + tb);
+        }
+        __syncwarp();
       }
-      tc::mma_commit(a_empty);
+      if (lane == 0) tc::mma_commit(a_empty);
+      __syncwarp();
     }
   } else if (warp >= 4) {
     // ------------------------------------------------ epilogue
@@ -243,6 +302,10 @@ __global__ void __launch_bounds__(Epi<EPIW>::threads, 1) k_pairdiff_tc(const __g
     // Every epilogue warp walks the same items and reaches the two named-barrier syncs per
     // item the same number of times; after an abort it only skips the work.
     uint32_t ct = 0;
+    constexpr float FLOOR_ADD = 12582912.f;  // 1.5 2^23
+    constexpr int FLOOR_BITS = 0x4B400000;   // its bits
+    const f2 k8 = f2_pack(0x1p-8f, 0x1p-8f), k16 = f2_pack(0x1p-16f, 0x1p-16f), k14 = f2_pack(0x1p-14f, 0x1p-14f);
+    const f2 hsc = f2_pack(P.hscale, P.hscale), hof = f2_pack(P.hoff, P.hoff);
     for (int it = blockIdx.x; it < P.nitems; it += gridDim.x) {
       const int itile = it / P.njc, jc = it % P.njc;
       const int j0 = jc * P.jchunk, j1 = min(P.nj, j0 + P.jchunk);
@@ -251,7 +314,8 @@ __global__ void __launch_bounds__(Epi<EPIW>::threads, 1) k_pairdiff_tc(const __g
       const float2 aff = irow ? P.alpha_ff[i] : make_float2(0.f, 0.f);
       const int ei = irow ? P.ea[i] : PD_EMIN;
       const float pa = pow2f(ei);  // 2^ei
-      float4* cv = colv + (warp - 4) * 16;
+      const f2 ax = f2_pack(aff.x, aff.x), ay = f2_pack(aff.y, aff.y), npa = f2_pack(-pa, -pa);
+      float* cv = colv + (warp - 4) * 64;
       // this warp's WCOLS columns h*WCOLS + c of a tile: (beta_ff, 2^(ej+33)) fetched one tile ahead
       // (the loads run while the previous tile is processed), staged in shared memory and read
       // back as one broadcast load per element
@@ -268,7 +332,12 @@ __global__ void __launch_bounds__(Epi<EPIW>::threads, 1) k_pairdiff_tc(const __g
         const uint32_t tb = ct & 1, tu = ct >> 1;
         if (*abort_s) break;
         // (the previous tile's reads of cv ended at the __syncwarp closing it)
-        if (lane < WCOLS) cv[lane] = make_float4(nb.x, nb.y, pow2f(ne + 33), 0.f);  // 2 x 2^(ei+ej) x 2^32 with pa
+        if (lane < WCOLS) {
+          float* bp = cv + lane / 2 * 8 + (lane & 1);
+          bp[0] = nb.x;
+          bp[2] = nb.y;
+          bp[4] = pow2f(ne + 33);  // 2 x 2^(ei+ej) x 2^32 with pa
+        }
         fetch(jt + 1);
         __syncwarp();
         if (!tc::mbar_wait(t_full + tb, tu & 1)) {
@@ -276,81 +345,133 @@ __global__ void __launch_bounds__(Epi<EPIW>::threads, 1) k_pairdiff_tc(const __g
           break;
         }
         tc::fence_after_sync();
-        // full tiles (every row and column real) skip the per-element range tests
-        const bool fast = irow && (jt + 1) * TN <= P.NB;
+        const bool full = irow && (jt + 1) * TN <= P.NB;  // the row and every column are real
+        const uint32_t ta0 = tmem + tb * TBUF + lane_addr + h * WCOLS;
+        // a chunk's accumulators d = 0..3 are loaded while the previous chunk is worked on
+        uint32_t x[2][4][CCH];
+        auto load = [&](int ch, uint32_t (&r)[4][CCH]) {
+#pragma unroll
+          for (int d = 0; d < 4; d++) tc::tmem_ld<CCH>(ta0 + ch * CCH + d * TN, r[d]);
+        };
+        load(0, x[0]);
+#pragma unroll
         for (int ch = 0; ch < WCOLS / CCH; ch++) {
-          const int col0 = h * WCOLS + ch * CCH;
-          uint32_t r0[CCH], r1[CCH], r2[CCH], r3[CCH], r4[CCH];
-          const uint32_t ta = tmem + tb * TBUF + lane_addr + col0;
-          tc::tmem_ld<CCH>(ta, r0);
-          tc::tmem_ld<CCH>(ta + TN, r1);
-          tc::tmem_ld<CCH>(ta + 2 * TN, r2);
-          tc::tmem_ld<CCH>(ta + 3 * TN, r3);
-          tc::tmem_ld<CCH>(ta + 4 * TN, r4);
           tc::tmem_wait_ld();
 #pragma unroll
-          for (int c = 0; c < CCH; c++) {
-            const int j = jt * TN + col0 + c;
-            if (!fast && (!irow || j >= P.NB)) continue;
-            const float4 b = cv[ch * CCH + c];
-            // 2 x 2^(ei+ej) = sum_d 2^(ei+ej+33-8d) X_d; s0 = 2^(ei+ej+33) is an exact product
-            const float s0 = pa * b.z;
-            const float X0 = __uint_as_float(r0[c]), X1 = __uint_as_float(r1[c]);
-            const float X2 = __uint_as_float(r2[c]), X3 = __uint_as_float(r3[c]);
+          for (int d = 0; d < 4; d++) tc::reg_fence<CCH>(x[ch & 1][d]);
+          if (ch + 1 < WCOLS / CCH) load(ch + 1, x[(ch + 1) & 1]);
+          const uint32_t(&r)[4][CCH] = x[ch & 1];
+          auto pair = [&](int d, int c) { return f2_pack(__uint_as_float(r[d][c]), __uint_as_float(r[d][c + 1])); };
+          float chi2[CCH], lim[CCH];
+          bool rare = !full;
+#pragma unroll
+          for (int c = 0; c < CCH; c += 2) {
+            // both columns of a pair: beta's high parts, low parts, and 2^(ej+33)
+            const float* bp = cv + (ch * CCH + c) / 2 * 8;
+            const ulonglong2 bxy = *reinterpret_cast<const ulonglong2*>(bp);
+            const f2 bx{bxy.x}, by{bxy.y}, bz{*reinterpret_cast<const unsigned long long*>(bp + 4)};
+            // 2 x 2^(ei+ej) = sum_d 2^(ei+ej+33-8d) X_d; s0 = -2^(ei+ej+33) is an exact product.
             // FP32 assembly from the largest term down: ab + e = |P|^2 + |Q|^2 (high parts)
-            // exactly; s0 X0 is exact (integer < 2^24 times a power of two), so ab - s0 X0 is
+            // exactly; s0 X0 is exact (integer < 2^24 times a power of two), so ab + s0 X0 is
             // rounded once, relative to itself, then the X1 term, then the small rest.  Error
             // about 3 2^-24 chi2 + 2^-32 (|P|^2+|Q|^2) (the left-out X4 term below 2^-30 of it):
             // within 4e-6 of chi2 whenever chi2 >= 2^-14 (|P|^2+|Q|^2)
-            float e;
-            const float ab = two_sum(aff.x, b.x, e);
-            const float t1 = fmaf(-X0, s0, ab);
-            const float t2 = fmaf(-X1, s0 * 0x1p-8f, t1);
-            const float w = fmaf(X3, 0x1p-8f, X2);
-            float chi2 = t2 + fmaf(-w, s0 * 0x1p-16f, e + (aff.y + b.y));
+            const f2 s0 = f2_mul(npa, bz);
+            const f2 ab = f2_add(ax, bx), bb = f2_sub(ab, ax);
+            const f2 e = f2_add(f2_sub(ax, f2_sub(ab, bb)), f2_sub(bx, bb));
+            const f2 t1 = f2_fma(pair(0, c), s0, ab);
+            const f2 t2 = f2_fma(pair(1, c), f2_mul(s0, k8), t1);
+            const f2 w = f2_fma(pair(3, c), k8, pair(2, c));
+            const f2 chi = f2_add(t2, f2_fma(w, f2_mul(s0, k16), f2_add(e, f2_add(ay, by))));
+            const float2 v = f2_split(chi), l = f2_split(f2_mul(ab, k14));
+            chi2[c] = v.x;
+            chi2[c + 1] = v.y;
             // One test for the rare cases: lim is at least every bound below, so a value at or
             // above it needs neither the float-float form nor the exact list.
-            float lim = fmaxf(0x1p-14f * ab, P.thr);
-            float qbound = 0.f;
+            lim[c] = fmaxf(l.x, P.thr);
+            lim[c + 1] = fmaxf(l.y, P.thr);
             if constexpr (OUT) {
-              const float q = pa + b.z * 0x1p-33f;
-              qbound = P.refine_f * q * q;
-              lim = fmaxf(lim, qbound);
+              const float2 z = f2_split(bz);
+              const float q0 = pa + z.x * 0x1p-33f, q1 = pa + z.y * 0x1p-33f;
+              lim[c] = fmaxf(lim[c], P.refine_f * q0 * q0);
+              lim[c + 1] = fmaxf(lim[c + 1], P.refine_f * q1 * q1);
             }
-            if (chi2 < lim) {
-              // below 2^-14 (|P|^2+|Q|^2) the float-float form: with this assembly almost no
-              // warp enters it (the earlier form, good to (|P|^2+|Q|^2)/16, sent some lane of
-              // most warps there)
-              if (chi2 < 0x1p-14f * ab)
-                chi2 = chi2_assemble(aff, make_float2(b.x, b.y), X0 * s0, X1 * (s0 * 0x1p-8f), X2 * (s0 * 0x1p-16f),
-                                     X3 * (s0 * 0x1p-24f), __uint_as_float(r4[c]) * (s0 * 0x1p-32f));
-              // below 1e-7 (|P|^2+|Q|^2) the float-float rounding (about 2^-40 of it) could
-              // exceed 1e-5 relative; those, the top-k candidates and (matrix mode) pairs within
-              // the quantisation-error bound go to the exact FP64 list (which also histograms
-              // them)
-              const float bound = fmaxf(fmaxf(1e-7f * ab, P.thr), qbound);
-              if (chi2 < bound) {
-                const unsigned k = atomicAdd(P.nref, 1u);
-                if (k < P.rcap) {
-                  P.ri[k] = i;
-                  P.rj[k] = j;
-                }
-                continue;
+            rare |= !(chi2[c] >= lim[c]) || !(chi2[c + 1] >= lim[c + 1]);  // (NaN: rare)
+          }
+          // the tile's last loads are done: the next MMAs may have its buffer while this goes on
+          auto release = [&]() {
+            tc::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(t_empty + tb);
+          };
+          if (!__any_sync(0xffffffffu, rare)) {
+            if (ch + 1 == WCOLS / CCH) release();
+#pragma unroll
+            for (int c = 0; c < CCH; c += 2) {
+              const int col = jt * TN + h * WCOLS + ch * CCH + c;
+              if constexpr (OUT) {
+                P.out[(long)i * P.NB + col] = chi2[c];
+                P.out[(long)i * P.NB + col + 1] = chi2[c + 1];
+              }
+              // shared counters: [below lo, bins 0 .. nbins-1, at or above hi].  floor(t) stands in
+              // the low bits of t + 1.5 2^23 rounded down, ordered like t also where |t| >= 2^22
+              // (chi2 is positive and no NaN here; a subnormal one, of flat curves, is -inf: below)
+              const float2 t = f2_split(f2_fma(f2_pack(lg2_approx(chi2[c]), lg2_approx(chi2[c + 1])), hsc, hof));
+#pragma unroll
+              for (int k = 0; k < 2; k++) {
+                const int f = __float_as_int(__fadd_rd(k ? t.y : t.x, FLOOR_ADD));
+                const uint32_t slot = (uint32_t)min(max(f, FLOOR_BITS - 1), FLOOR_BITS + P.nbins);
+                asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(hist_sa + 4u * (slot - (FLOOR_BITS - 1))) : "memory");
               }
             }
-            if constexpr (OUT) P.out[(long)i * P.NB + j] = chi2;
-            // chi2 >= 1e-7 (|P|^2+|Q|^2) > 0 here; a subnormal one (flat curves) falls out of range
-            float lg;
-            asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(lg) : "f"(chi2));
-            const int bin = __float2int_rd(fmaf(lg, P.hscale, P.hoff));
-            // shared counters: [below lo, bins 0 .. nbins-1, at or above hi]
-            const uint32_t slot = (uint32_t)(min(max(bin, -1), P.nbins) + 1);
-            asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(hist_sa + 4u * slot) : "memory");
+          } else {
+            uint32_t r4[CCH];
+            tc::tmem_ld<CCH>(ta0 + ch * CCH + 4 * TN, r4);
+            tc::tmem_wait_ld();
+            tc::reg_fence<CCH>(r4);
+            if (ch + 1 == WCOLS / CCH) release();
+#pragma unroll
+            for (int c = 0; c < CCH; c++) {
+              const int j = jt * TN + h * WCOLS + ch * CCH + c;
+              if (!irow || j >= P.NB) continue;
+              float v = chi2[c];
+              if (v < lim[c]) {
+                const float* bp = cv + (ch * CCH + c) / 2 * 8 + (c & 1);
+                const float2 bff = make_float2(bp[0], bp[2]);
+                const float ab = aff.x + bff.x, s0 = pa * bp[4];
+                // below 2^-14 (|P|^2+|Q|^2) the float-float form
+                if (v < 0x1p-14f * ab)
+                  v = chi2_assemble(aff, bff, __uint_as_float(r[0][c]) * s0, __uint_as_float(r[1][c]) * (s0 * 0x1p-8f),
+                                    __uint_as_float(r[2][c]) * (s0 * 0x1p-16f), __uint_as_float(r[3][c]) * (s0 * 0x1p-24f),
+                                    __uint_as_float(r4[c]) * (s0 * 0x1p-32f));
+                // below 1e-7 (|P|^2+|Q|^2) the float-float rounding (about 2^-40 of it) could
+                // exceed 1e-5 relative; those, the top-k candidates and (matrix mode) pairs within
+                // the quantisation-error bound go to the exact FP64 list (which also histograms
+                // them)
+                float bound = fmaxf(1e-7f * ab, P.thr);
+                if constexpr (OUT) {
+                  const float qs = pa + bp[4] * 0x1p-33f;
+                  bound = fmaxf(bound, P.refine_f * qs * qs);
+                }
+                if (v < bound) {
+                  const unsigned k = atomicAdd(P.nref, 1u);
+                  if (k < P.rcap) {
+                    P.ri[k] = i;
+                    P.rj[k] = j;
+                  }
+                  continue;
+                }
+              }
+              if constexpr (OUT) P.out[(long)i * P.NB + j] = v;
+              // v >= 1e-7 (|P|^2+|Q|^2) > 0 here; a subnormal one (flat curves) falls out of range
+              const int bin = __float2int_rd(fmaf(lg2_approx(v), P.hscale, P.hoff));
+              const uint32_t slot = (uint32_t)(min(max(bin, -1), P.nbins) + 1);
+              asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(hist_sa + 4u * slot) : "memory");
+            }
+            __syncwarp();
           }
         }
-        tc::fence_before_sync();
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive(t_empty + tb);
       }
       // flush this item's histogram (per item, so the 32-bit shared counters cannot overflow)
       epi_sync<EPIW>();

@@ -101,13 +101,17 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
-// D[tmem] (+)= A[smem] * B[smem]^T, issued by one thread.
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                         uint32_t accumulate) {
+// D[tmem] (+)= A[smem] * B[smem]^T, issued by the one lane whose issue != 0 while its whole warp
+// runs here: the operands are then warp-uniform and stay in uniform registers.  (Issued from a
+// branch that one lane took, each MMA first moved its descriptors there: some 50 cycles an
+// MMA, whatever its shape.)  a, b: descriptors as (high, low) words.
+__device__ __forceinline__ void mma_bf16(uint32_t issue, uint32_t d_tmem, uint32_t a_hi, uint32_t a_lo, uint32_t b_hi,
+                                         uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(
-          d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      "{\n .reg .pred p, q;\n .reg .b64 a, b;\n setp.ne.b32 q, %0, 0;\n setp.ne.b32 p, %7, 0;\n"
+      " mov.b64 a, {%3, %2};\n mov.b64 b, {%5, %4};\n"
+      " @q tcgen05.mma.cta_group::1.kind::f16 [%1], a, b, %6, p;\n}" ::"r"(issue),
+      "r"(d_tmem), "r"(a_hi), "r"(a_lo), "r"(b_hi), "r"(b_lo), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 

@@ -529,11 +529,16 @@ __global__ void __launch_bounds__(256) k_pd_refine(const double* __restrict__ ce
   }
 }
 
-// chi2 of pseudo-random pairs (integer hash of the sample index) for the top-k threshold.
+// chi2 of pseudo-random pairs (integer hash of the sample index) for the top-k threshold.  Eight
+// lanes per pair, so that a warp reads whole sectors of four pairs' curves: bound by the FP64
+// pipe (2^20 pairs of 128 epochs; a thread per pair, reading rows alone, took 905 us).
 __global__ void __launch_bounds__(256) k_pd_sample(const double* __restrict__ cenA, const double* __restrict__ cenB,
                                                    int NA, int NB, int T, long S,
                                                    uint64_t* __restrict__ keys, uint32_t* __restrict__ vals) {
-  for (long p = blockIdx.x * (long)blockDim.x + threadIdx.x; p < S; p += (long)gridDim.x * blockDim.x) {
+  constexpr int L = 8;
+  const int l = threadIdx.x % L;
+  // (whole warps stay in the loop: S and the stride are multiples of a warp's four pairs)
+  for (long p = (blockIdx.x * (long)blockDim.x + threadIdx.x) / L; p < S; p += (long)gridDim.x * blockDim.x / L) {
     uint64_t z = (uint64_t)p * 0x9E3779B97F4A7C15ull + 0x632BE59BD9B4E019ull;
     z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
     z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
@@ -542,13 +547,17 @@ __global__ void __launch_bounds__(256) k_pd_sample(const double* __restrict__ ce
     const double* a = cenA + (long)i * T;
     const double* b = cenB + (long)j * T;
     double s = 0.0;
-    for (int t = 0; t < T; t++) {
+#pragma unroll 4
+    for (int t = l; t < T; t += L) {
       const double r = b[t] - a[t];
       s += r * r;
     }
-    uint64_t u = __double_as_longlong(s);  // s >= 0: the bit pattern orders like the value
-    keys[p] = u;
-    vals[p] = (uint32_t)p;
+#pragma unroll
+    for (int o = L / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (l == 0) {
+      keys[p] = __double_as_longlong(s);  // s >= 0: the bit pattern orders like the value
+      vals[p] = (uint32_t)p;
+    }
   }
 }
 
@@ -735,10 +744,12 @@ static void pairdiff_core(mlc_ctx* ctx, int method, const float* A, const float*
   const unsigned cap = (unsigned)std::min<long long>(P, 8LL * k + (1LL << 20));
   double thr = -1.0;  // no candidates unless k > 0
   if (k > 0) {
-    // 2^20 sampled pairs: the threshold only filters candidates (the top-k itself is exact),
-    // and with the 4x + 16 rank margin below it stays above the k-th value (a rerun of the
-    // pass when it does not); 2^22 samples cost 3.5 ms of a 41 ms 10^10-pair step in FP64
-    const long S = 1L << 20;
+    // Sampled pairs: the threshold only filters candidates (the top-k itself is exact), and with
+    // the 4x + 16 rank margin below it stays above the k-th value (a rerun of the pass when it
+    // does not).  64 samples expected among the top k are plenty for that margin; 2^20 at most
+    // (2^22 cost 3.5 ms in FP64), 2^14 at least.
+    long S = 1L << 14;
+    while (S < (1L << 20) && (double)S * k < 64.0 * (double)P) S *= 2;
     uint64_t* sk = (uint64_t*)ws_get(ctx, WS_LOC, (sizeof(uint64_t) + sizeof(uint32_t)) * S);
     uint32_t* sv = (uint32_t*)(sk + S);
     {

@@ -245,8 +245,9 @@ static void* upload_level0_f32(int M) {
   return d;
 }
 
-// The levels' twiddles W_{B_i}^(m q), [q - 1][m], one level after another.
-static void* upload_any(const AnyLevels& lv, bool limbs3) {
+// The levels' twiddles W_{B_i}^(m q), [q - 1][m], one level after another, in the plan's own
+// arithmetic (FP64: three limbs).
+static void* upload_any(const AnyLevels& lv, int prec) {
   if (lv.n < 2) return nullptr;
   std::vector<long double> re, im, lr, li;
   twiddle_table(lv.L, re, im);
@@ -259,13 +260,17 @@ static void* upload_any(const AnyLevels& lv, bool limbs3) {
       }
     f *= lv.r[i];
   }
-  if (limbs3) return upload_limbs3(lr, li);
-  std::vector<C2<ff>> h(lr.size());
-  for (size_t i = 0; i < h.size(); i++) h[i] = C2<ff>{ff((double)lr[i]), ff((double)li[i])};
-  void* d = nullptr;
-  MLC_CUDA(cudaMalloc(&d, h.size() * sizeof(C2<ff>)));
-  MLC_CUDA(cudaMemcpy(d, h.data(), h.size() * sizeof(C2<ff>), cudaMemcpyHostToDevice));
-  return d;
+  if (prec == MLC_F64) return upload_limbs3(lr, li);
+  auto upload = [&](auto zero) {
+    using T = decltype(zero);
+    std::vector<C2<T>> h(lr.size());
+    for (size_t i = 0; i < h.size(); i++) h[i] = C2<T>{T((double)lr[i]), T((double)li[i])};
+    void* d = nullptr;
+    MLC_CUDA(cudaMalloc(&d, h.size() * sizeof(C2<T>)));
+    MLC_CUDA(cudaMemcpy(d, h.data(), h.size() * sizeof(C2<T>), cudaMemcpyHostToDevice));
+    return d;
+  };
+  return prec_is_ff(prec) ? upload(ff(0.0)) : upload(0.f);
 }
 
 static void split_columns(int Ny, int& N1, int& N2) {
@@ -314,16 +319,12 @@ FftPlan2D* plan_get(mlc_ctx* ctx, int Nx, int Ny, int prec) {
     p->twy = upload_twiddles<float>(Ny);
     if (row3_first_radix(p->M)) p->twl = upload_level0_f32(p->M);
   }
-  if (prec == MLC_F64 || prec == PREC_FFS) {
-    p->anyM = any_levels(p->M, true);
-    p->anyM_tw = upload_any(p->anyM, prec == MLC_F64);
-  }
-  if (prec == MLC_F64) {
-    p->any1 = any_levels(p->N1, false);
-    p->any2 = any_levels(p->N2, false);
-    p->any1_tw = upload_any(p->any1, true);
-    p->any2_tw = upload_any(p->any2, true);
-  }
+  p->anyM = any_levels(p->M, true);
+  p->any1 = any_levels(p->N1, false);
+  p->any2 = any_levels(p->N2, false);
+  p->anyM_tw = upload_any(p->anyM, prec);
+  p->any1_tw = upload_any(p->any1, prec);
+  p->any2_tw = upload_any(p->any2, prec);
   FftPlan2D* raw = p.get();
   ctx->plans[key] = std::move(p);
   return raw;

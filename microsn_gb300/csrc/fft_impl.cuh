@@ -922,6 +922,15 @@ __global__ void k_multiply(const C2<T>* __restrict__ Fmap, C2<T>* __restrict__ F
 
 // ---------------------------------------------------------------- host orchestration
 
+// The passes of lengths without an unrolled kernel (fft_any_real.cuh); false, with nothing
+// launched, where the length has one level only or its rows do not fit.
+template <typename T, typename Loader>
+bool any_real_r2c(mlc_ctx* ctx, const FftPlan2D& p, const Loader& ld, int nrows, void* out, const char* name);
+template <typename T, typename TO>
+bool any_real_c2r(mlc_ctx* ctx, const FftPlan2D& p, const void* in, void* out);
+template <typename T, bool INV>
+bool any_real_colpass(mlc_ctx* ctx, const FftPlan2D& p, void* buf, char kind, int post_tw);
+
 template <typename T, typename Loader>
 static void launch_rows_r2c(mlc_ctx* ctx, const FftPlan2D& p, const Loader& ld, int nrows, void* out) {
   if (nrows <= 0) return;
@@ -965,6 +974,8 @@ static void launch_rows_r2c(mlc_ctx* ctx, const FftPlan2D& p, const Loader& ld, 
       return;
     }
   }
+  if constexpr (!std::is_same<T, double>::value)
+    if (any_real_r2c<T>(ctx, p, ld, nrows, out, name)) return;
   size_t smem = 2 * (size_t)(p.M + 1) * sizeof(C2<T>);
   auto kern = k_rows_r2c<T, Loader>;
   set_max_smem((const void*)kern, smem);
@@ -1000,6 +1011,8 @@ static void launch_rows_c2r(mlc_ctx* ctx, const FftPlan2D& p, const void* in, vo
       return;
     }
   }
+  if constexpr (!std::is_same<T, double>::value && std::is_same<TO, typename RealOut<T>::type>::value)
+    if (any_real_c2r<T, TO>(ctx, p, in, out)) return;
   size_t smem = 2 * (size_t)(p.M + 1) * sizeof(C2<T>);
   auto kern = k_rows_c2r<T, TO>;
   set_max_smem((const void*)kern, smem);
@@ -1062,6 +1075,8 @@ static void launch_colpass(mlc_ctx* ctx, const FftPlan2D& p, void* buf, char kin
     MLC_CHECK_LAUNCH();
     return;
   }
+  if constexpr (!std::is_same<T, double>::value)
+    if (any_real_colpass<T, INV>(ctx, p, buf, kind, post_tw)) return;
   size_t smem = (2 * (size_t)L * CW + rl.tlen + L) * sizeof(C2<T>);
   auto kern = k_colpass<T, CW, INV>;
   set_max_smem((const void*)kern, smem);

@@ -3,42 +3,10 @@
 // are unrolled; the places of their points come from a few integer multiplications per item,
 // little beside the arithmetic of its points.  Inputs wait in shared memory, as they were read,
 // for the sum that scales them.
+#include "fft_any.cuh"
 #include "fft_limb.cuh"
 
 namespace mlc {
-
-__device__ __forceinline__ int any_div(int x, int d, uint32_t magic) { return d == 1 ? x : (int)__umulhi((uint32_t)x, magic); }
-
-// Place of sub-block `blk` of level i: its digits over r[0 .. i-1], the last one fastest.
-__device__ __forceinline__ int any_outer(const AnyLevels& lv, int i, int blk) {
-  int p = 0;
-  for (int j = i - 1; j >= 0; j--) {
-    const int q = any_div(blk, lv.r[j], lv.mr[j]);
-    p += (blk - q * lv.r[j]) * lv.tn[j];
-    blk = q;
-  }
-  return p;
-}
-// Place of point m of a block of level i (level i = 0: of the whole transform).
-__device__ __forceinline__ int any_inner(const AnyLevels& lv, int i, int m) {
-  int p = 0;
-  for (int j = i; j < lv.n - 1; j++) {
-    const int q = any_div(m, lv.bn[j], lv.mbn[j]);
-    p += q * lv.tn[j];
-    m -= q * lv.bn[j];
-  }
-  return p + m;
-}
-// Place of output k: output digit j (radix r[j], digit 0 fastest) is the place's digit j.
-__device__ __forceinline__ int any_output(const AnyLevels& lv, int k) {
-  int p = 0;
-  for (int j = 0; j < lv.n; j++) {
-    const int q = any_div(k, lv.r[j], lv.mr[j]);
-    p += (k - q * lv.r[j]) * lv.tn[j];
-    k = q;
-  }
-  return p;
-}
 
 // Level i, radix R, over CW interleaved columns.  DIT false: the small transform, then the
 // twiddles; true (the way back, levels in the opposite order): conjugate twiddles, then it.
@@ -77,16 +45,7 @@ __device__ __forceinline__ void any_level(const LimbArr<T>& s, const AnyLevels& 
 
 template <typename T, bool INV, bool DIT, int CW, typename Tw>
 __device__ __forceinline__ void any_level_r(const LimbArr<T>& s, const AnyLevels& lv, int i, Tw tw) {
-  switch (lv.r[i]) {
-    case 10: any_level<T, INV, DIT, 10, CW>(s, lv, i, tw); break;
-    case 9: any_level<T, INV, DIT, 9, CW>(s, lv, i, tw); break;
-    case 8: any_level<T, INV, DIT, 8, CW>(s, lv, i, tw); break;
-    case 6: any_level<T, INV, DIT, 6, CW>(s, lv, i, tw); break;
-    case 5: any_level<T, INV, DIT, 5, CW>(s, lv, i, tw); break;
-    case 4: any_level<T, INV, DIT, 4, CW>(s, lv, i, tw); break;
-    case 3: any_level<T, INV, DIT, 3, CW>(s, lv, i, tw); break;
-    default: any_level<T, INV, DIT, 2, CW>(s, lv, i, tw); break;
-  }
+  any_radix(lv.r[i], [&](auto r) { any_level<T, INV, DIT, decltype(r)::value, CW>(s, lv, i, tw); });
 }
 
 // All levels: natural order in, digit order out (DIT: the other way round).  Level 0's twiddles
@@ -333,39 +292,14 @@ __global__ void __launch_bounds__(ANY_NT, 2)
 
 // ---------------------------------------------------------------- launches
 
-constexpr size_t ANY_SMEM = 224 * 1024;  // (and static arrays beside it)
-
 template <typename T>
 static LimbTab<T> any_tab(const FftPlan2D& p, const AnyLevels& lv, const void* t) {
   return LimbTraits<T>::tab(p, t, t, lv.ntw);
 }
 
-// Threads of a row's CTA: the fewest turns of a level's items over the CTAs that an SM holds at
-// once, by its registers (512 threads of lf3, 1024 of lf2), shared memory and the rows there are.
 template <typename T>
-static int any_row_threads(mlc_ctx* ctx, const AnyLevels& lv, size_t smem, int nrows) {
-  constexpr int RES = sizeof(T) == sizeof(lf3) ? 512 : 1024;
-  const int fit = std::max(1, std::min((int)(ANY_SMEM / (smem + 1024)), ceil_div(nrows, ctx->sm_count)));
-  int best = 0;
-  float least = 0.f;
-  for (int nt = 64; nt <= 512; nt += 32) {
-    int turns = 0;
-    for (int i = 0; i < lv.n; i++) turns += ceil_div(lv.L / lv.r[i], nt) * lv.r[i];
-    const float cost = (float)turns / std::min(fit, RES / nt);
-    if (!best || cost < least) best = nt, least = cost;
-  }
-  return best;
-}
-// Threads of a column strip's CTA: the number that leaves the fewest idle ones over the levels.
-static int any_col_threads(const AnyLevels& lv) {
-  int best = 0;
-  long least = 0;
-  for (int nt = 64; nt <= ANY_NT; nt += 32) {
-    long cost = 0;
-    for (int i = 0; i < lv.n; i++) cost += (long)ceil_div(lv.L / lv.r[i] * ANY_CW, nt) * nt * lv.r[i];
-    if (!best || cost <= least) best = nt, least = cost;
-  }
-  return best;
+static int any_limb_row_threads(mlc_ctx* ctx, const AnyLevels& lv, size_t smem, int nrows) {
+  return any_row_threads(ctx, lv, smem, nrows, sizeof(T) == sizeof(lf3) ? 512 : 1024);
 }
 
 template <typename T>
@@ -379,7 +313,7 @@ bool any_rows_c2r_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* in, void* o
   set_max_smem((const void*)k, smem);
   {
     MLC_KSCOPE(ctx, "fft_rows_c2r");
-    k<<<p.Ny, any_row_threads<T>(ctx, lv, smem, p.Ny), smem, ctx->stream>>>((const C2<S>*)in, p.Wp, (TO*)out, p.Nx, limb_twx<T>(p), lv,
+    k<<<p.Ny, any_limb_row_threads<T>(ctx, lv, smem, p.Ny), smem, ctx->stream>>>((const C2<S>*)in, p.Wp, (TO*)out, p.Nx, limb_twx<T>(p), lv,
                                                          any_tab<T>(p, lv, p.anyM_tw));
   }
   MLC_CHECK_LAUNCH();
@@ -392,11 +326,14 @@ bool any_rows_r2c_impl(mlc_ctx* ctx, const FftPlan2D& p, const Loader& ld, int n
   const AnyLevels& lv = p.anyM;
   const size_t smem = any_row_smem<T>(lv);
   if (lv.n < 1 || smem > ANY_SMEM) return false;
+  // one row per SM at most (a profile's): the FP64 loop's short code finishes first up to here
+  // (rows of 1200 points 30 us against 47, of 2160 points 55 either way, of 4500 points 102 against 70)
+  if (nrows <= ctx->sm_count && p.M <= 2000) return false;
   auto k = k_any_rows_r2c<S, T, Loader>;
   set_max_smem((const void*)k, smem);
   {
     MLC_KSCOPE(ctx, name);
-    k<<<nrows, any_row_threads<T>(ctx, lv, smem, nrows), smem, ctx->stream>>>(ld, (C2<S>*)out, p.Wp, limb_twx<T>(p), lv,
+    k<<<nrows, any_limb_row_threads<T>(ctx, lv, smem, nrows), smem, ctx->stream>>>(ld, (C2<S>*)out, p.Wp, limb_twx<T>(p), lv,
                                                           any_tab<T>(p, lv, p.anyM_tw));
   }
   MLC_CHECK_LAUNCH();
@@ -415,7 +352,7 @@ bool any_colpass_impl(mlc_ctx* ctx, const FftPlan2D& p, void* buf, char kind, in
   set_max_smem((const void*)k, smem);
   {
     MLC_KSCOPE(ctx, A ? "fft_col_A" : "fft_col_B");
-    k<<<dim3(ceil_div(p.Wc, ANY_CW), A ? p.N2 : p.N1), any_col_threads(lv), smem, ctx->stream>>>(
+    k<<<dim3(ceil_div(p.Wc, ANY_CW), A ? p.N2 : p.N1), any_col_threads(lv, ANY_CW, ANY_NT), smem, ctx->stream>>>(
         (C2<S>*)buf, p.Wp, A ? 1 : p.N2, A ? p.N2 : 1, limb_twy<T>(p), post_tw, lv,
         any_tab<T>(p, lv, A ? p.any1_tw : p.any2_tw));
   }
@@ -434,7 +371,7 @@ void any3_conv(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, void* out, co
   set_max_smem((const void*)k_any_conv, smem);
   {
     MLC_KSCOPE(ctx, "conv_fused_spectrum");
-    k_any_conv<<<dim3(ceil_div(p.Wc, ANY_CW), p.N1), any_col_threads(lv), smem, ctx->stream>>>(
+    k_any_conv<<<dim3(ceil_div(p.Wc, ANY_CW), p.N1), any_col_threads(lv, ANY_CW, ANY_NT), smem, ctx->stream>>>(
         (const C2<double>*)Fmap, (C2<double>*)out, p.Wp, rows, h, p.Ny, p.N1, limb_twy<lf3>(p), r, rexp, lv,
         any_tab<lf3>(p, lv, p.any2_tw));
   }

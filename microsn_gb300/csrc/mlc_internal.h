@@ -13,7 +13,7 @@
 
 namespace mlc {
 
-// An in-place transform of L points in shared memory by any radices (fft_limb_any.cu): level i
+// An in-place transform of L points in shared memory by any radices (fft_any.cuh): level i
 // works on blocks of r[0] ... r[i-1] parts, each of r[i] sub-blocks of bn[i] points that lie
 // tn[i] places apart; its twiddles [q - 1][m] start at entry tw[i] of the table.
 struct AnyLevels {
@@ -43,7 +43,7 @@ struct FftPlan2D {
   void* twy3 = nullptr;
   void* twl3 = nullptr;  // W_M^(m q), [q - 1][m]: level 0 of the limb row transforms (limb_first_radix)
   AnyLevels anyM{}, any1{}, any2{};  // M, N1 and N2 points by any radices, and their tables
-  void* anyM_tw = nullptr;           // (the arithmetic's own layout: float-float, or three limbs)
+  void* anyM_tw = nullptr;           // (in the plan's arithmetic, FP64 in three limbs)
   void* any1_tw = nullptr;
   void* any2_tw = nullptr;
   void* twl = nullptr;   // the same as twl3 for level 1 of FP32 three-level rows (row3_first_radix)

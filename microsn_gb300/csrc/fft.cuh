@@ -45,11 +45,12 @@ struct Dft<T, 3, INV> {
     const T h = (T)0.86602540378443864676372317075294;  // sin(2 pi / 3)
     C2<T> s = cadd(v[1], v[2]);
     C2<T> d = csub(v[1], v[2]);
-    C2<T> m = C2<T>{v[0].x - scale2(s.x, 0.5f), v[0].y - scale2(s.y, 0.5f)};
+    C2<T> m = csub(v[0], cscale2(s, 0.5f));
     C2<T> id = mul_mi<T, INV>(d);  // -i d (forward) / +i d (inverse)
     v[0] = cadd(v[0], s);
-    v[1] = C2<T>{m.x + h * id.x, m.y + h * id.y};
-    v[2] = C2<T>{m.x - h * id.x, m.y - h * id.y};
+    const C2<T> hd = crmul(h, id);
+    v[1] = cadd(m, hd);
+    v[2] = csub(m, hd);
   }
 };
 
@@ -79,11 +80,11 @@ struct Dft<T, 5, INV> {
     C2<T> sa = cadd(v[1], v[4]), da = csub(v[1], v[4]);
     C2<T> sb = cadd(v[2], v[3]), db = csub(v[2], v[3]);
     C2<T> t1 = cadd(sa, sb), t2 = csub(sa, sb);
-    C2<T> u = C2<T>{x0.x - scale2(t1.x, 0.25f), x0.y - scale2(t1.y, 0.25f)};
-    C2<T> m = C2<T>{b * t2.x, b * t2.y};
+    C2<T> u = csub(x0, cscale2(t1, 0.25f));
+    C2<T> m = crmul(b, t2);
     C2<T> p1 = cadd(u, m), p2 = csub(u, m);
-    C2<T> q1 = C2<T>{lin2(s1, da.x, s2, db.x), lin2(s1, da.y, s2, db.y)};
-    C2<T> q2 = C2<T>{lin2(s2, da.x, -s1, db.x), lin2(s2, da.y, -s1, db.y)};
+    C2<T> q1 = clin2(s1, da, s2, db);
+    C2<T> q2 = clin2(s2, da, -s1, db);
     C2<T> iq1 = mul_mi<T, INV>(q1), iq2 = mul_mi<T, INV>(q2);
     v[0] = cadd(x0, t1);
     v[1] = cadd(p1, iq1);
@@ -102,8 +103,7 @@ struct Dft<T, 8, INV> {
     Dft<T, 4, INV>::run(e);
     Dft<T, 4, INV>::run(o);
     // o[q] *= W8^q ; forward W8 = (1 - i)/sqrt2, inverse (1 + i)/sqrt2
-    C2<T> o1 = INV ? C2<T>{r * (o[1].x - o[1].y), r * (o[1].x + o[1].y)}
-                   : C2<T>{r * (o[1].x + o[1].y), r * (o[1].y - o[1].x)};
+    C2<T> o1 = crmul(r, INV ? C2<T>{o[1].x - o[1].y, o[1].x + o[1].y} : C2<T>{o[1].x + o[1].y, o[1].y - o[1].x});
     C2<T> o2 = mul_mi<T, INV>(o[2]);
     C2<T> o3 = INV ? C2<T>{-r * (o[3].x + o[3].y), r * (o[3].x - o[3].y)}
                    : C2<T>{r * (o[3].y - o[3].x), -r * (o[3].x + o[3].y)};

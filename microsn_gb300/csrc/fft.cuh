@@ -30,12 +30,14 @@ RadixList factor_radices(int L, int tw_stride);
 template <typename T, int R, bool INV>
 struct Dft;
 
+// (Radix 2 and 3 of float-float stay unpacked: values come as (hi, lo) pairs, and a stage of so
+// few additions does not pay for pairing them anew.  P1 of 540^2: 14.0 us, packed 15.0.)
 template <typename T, bool INV>
 struct Dft<T, 2, INV> {
   static __device__ __forceinline__ void run(C2<T>* v) {
     C2<T> a = v[0], b = v[1];
-    v[0] = cadd(a, b);
-    v[1] = csub(a, b);
+    v[0] = std::is_same<T, ff>::value ? cadd<T>(a, b) : cadd(a, b);
+    v[1] = std::is_same<T, ff>::value ? csub<T>(a, b) : csub(a, b);
   }
 };
 
@@ -43,14 +45,17 @@ template <typename T, bool INV>
 struct Dft<T, 3, INV> {
   static __device__ __forceinline__ void run(C2<T>* v) {
     const T h = (T)0.86602540378443864676372317075294;  // sin(2 pi / 3)
-    C2<T> s = cadd(v[1], v[2]);
-    C2<T> d = csub(v[1], v[2]);
-    C2<T> m = csub(v[0], cscale2(s, 0.5f));
+    constexpr bool FF = std::is_same<T, ff>::value;
+    auto add = [](C2<T> a, C2<T> b) { return FF ? cadd<T>(a, b) : cadd(a, b); };
+    auto sub = [](C2<T> a, C2<T> b) { return FF ? csub<T>(a, b) : csub(a, b); };
+    C2<T> s = add(v[1], v[2]);
+    C2<T> d = sub(v[1], v[2]);
+    C2<T> m = sub(v[0], cscale2(s, 0.5f));
     C2<T> id = mul_mi<T, INV>(d);  // -i d (forward) / +i d (inverse)
-    v[0] = cadd(v[0], s);
+    v[0] = add(v[0], s);
     const C2<T> hd = crmul(h, id);
-    v[1] = cadd(m, hd);
-    v[2] = csub(m, hd);
+    v[1] = add(m, hd);
+    v[2] = sub(m, hd);
   }
 };
 

@@ -184,10 +184,11 @@ constexpr int any_real_resident() {  // threads an SM holds by their registers
   return std::is_same<T, float>::value ? 1024 : 512;
 }
 
-// Four CTAs or fewer per SM (the rows of a profile, maps below 640^2): the Stockham loops' short
-// code and 512 threads a row finish first (profile rows of 3000 and 9000 points in float-float
-// 16 and 32 us against 42 and 54; rows of a 600^2 map 18 against 25).
-static bool any_real_many(mlc_ctx* ctx, long ctas) { return ctas > 4L * ctx->sm_count; }
+// Six CTAs or fewer per SM (the rows of a profile, small maps): the Stockham loops' short code and
+// 512 threads a row finish first.  Float-float profile rows of 1500 and 4500 points 16 and 32 us
+// against 42 and 54; six last passes of 810^2 174 against 208 us, of 1080^2 258 against 192; FP32
+// is equal at 810^2, and 10 against 8 us a column pass at 1000^2.
+static bool any_real_many(mlc_ctx* ctx, long ctas) { return ctas > 6L * ctx->sm_count; }
 
 template <typename T, typename Loader>
 bool any_real_r2c(mlc_ctx* ctx, const FftPlan2D& p, const Loader& ld, int nrows, void* out, const char* name) {

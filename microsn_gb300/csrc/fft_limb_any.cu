@@ -309,6 +309,9 @@ bool any_rows_c2r_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* in, void* o
   const AnyLevels& lv = p.anyM;
   const size_t smem = any_row_smem<T>(lv);
   if (lv.n < 1 || smem > ANY_SMEM) return false;
+  // lf2: four rows or fewer per SM take the float-float loop's short code (ten last passes of 540^2
+  // 161 us against 168, six of 810^2 150 against 113)
+  if (sizeof(T) == sizeof(lf2) && p.Ny <= 4 * ctx->sm_count) return false;
   auto k = k_any_rows_c2r<S, T, TO>;
   set_max_smem((const void*)k, smem);
   {

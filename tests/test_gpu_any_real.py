@@ -21,6 +21,13 @@ SIZES = [
     (36, 250),      # 18 (9 2), 10 x 25
     (24000, 96),    # 12000 (10 10 10 4 3), FP32 only: rows in float-float end at 13000
     (25600, 48),    # 12800 (10 10 8 8 2), FP32 only
+    # (fewer rows than six per SM keep the general kernel)
+    (108, 1500),    # 54 (9 6)
+    (64, 2048),     # 32 (8 4)
+    (36, 1000),     # 18 (9 2)
+    (20, 1080),     # 10: one level
+    (9216, 1024),   # 4608 (9 8 8 8)
+    (24000, 960),   # 12000, FP32 only
 ]
 
 

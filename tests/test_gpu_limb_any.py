@@ -22,6 +22,11 @@ SIZES = [
     (64, 32),       # 32 (8 4), 4 x 8
     (36, 250),      # 18 (9 2), 10 x 25
     (36, 125),      # odd
+    (108, 1500),    # 54 (9 6); two limbs take more than four rows per SM
+    (64, 2048),     # 32 (8 4)
+    (36, 1000),     # 18 (9 2)
+    (20, 1080),     # 10: one level
+    (9216, 1024),   # 4608 (9 8 8 8)
 ]
 
 

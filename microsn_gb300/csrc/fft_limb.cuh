@@ -722,9 +722,18 @@ __device__ __forceinline__ void limb_c2r_row(LV, const C2<S>* __restrict__ a, co
       LV{}, s, [&](C2<T> z) { return C2<TO>{limb_round(z.x, sc), limb_round(z.y, sc)}; }, put);
 }
 
+// CTAs per SM that the last pass's registers have to allow: lf2 rows of 2000 and 1000 points begin
+// with radix 4 in 64 registers and fill the SM with warps (2000^2: 31 -> 25 us, 4000^2 80 -> 76,
+// against first radices of 10 and 8 in 133 and 106 registers); 5000 points in 5 x 10 x 10 x 10
+// and 64 registers took 561 us against 492 at 10000^2.
+template <typename T, typename LV>
+constexpr int limb_row_ctas() {
+  return sizeof(T) == sizeof(lf3) ? 0 : LV::M == 2000 ? 4 : LV::M == 1000 ? 8 : 0;
+}
+
 // P3: one row per CTA, the pixels written from registers in thread order.
 template <typename S, typename T, typename TO, int NT, typename LV>
-__global__ void __launch_bounds__(NT) k_limb_rows_c2r(const C2<S>* __restrict__ in, long pitch, TO* __restrict__ out,
+__global__ void __launch_bounds__(NT, limb_row_ctas<T, LV>()) k_limb_rows_c2r(const C2<S>* __restrict__ in, long pitch, TO* __restrict__ out,
                                                       long ldo, LimbTab<T> twx, LimbTab<T> tab0) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ LimbSum<S> red[NT / 32];
@@ -736,7 +745,7 @@ __global__ void __launch_bounds__(NT) k_limb_rows_c2r(const C2<S>* __restrict__ 
 // P3 of four profiles with the interleave fused in, the cluster form of k_rows_c2r3_il
 // (fft_impl.cuh): the row of pixels is left rounded to TO in each CTA's shared memory.
 template <typename S, typename T, typename TO, int NT, typename LV>
-__global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(NT)
+__global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(NT, limb_row_ctas<T, LV>())
     k_limb_rows_c2r_il(const C2<S>* __restrict__ specs, long spec_stride, long pitch, int nm, TO* __restrict__ out,
                        int S_, LimbTab<T> twx, LimbTab<T> tab0, unsigned planar) {
   constexpr int M = LV::M, NX = 2 * M;
@@ -1013,8 +1022,14 @@ static bool limb_row_dispatch(int M, F f) {
   switch (M) {
     case 5000: f(Levels<10, 10, 10, 5>{}, integral_constant<int, F64 ? 512 : 256>{}); return true;
     case 4096: f(Levels<8, 8, 8, 8>{}, integral_constant<int, F64 ? 512 : 288>{}); return true;
-    case 2000: f(Levels<8, 10, 5, 5>{}, integral_constant<int, F64 ? 256 : 128>{}); return true;
-    case 1000: f(Levels<10, 10, 10>{}, integral_constant<int, 128>{}); return true;
+    case 2000:
+      if constexpr (F64) f(Levels<8, 10, 5, 5>{}, integral_constant<int, 256>{});
+      else f(Levels<4, 10, 10, 5>{}, integral_constant<int, 256>{});
+      return true;
+    case 1000:
+      if constexpr (F64) f(Levels<10, 10, 10>{}, integral_constant<int, 128>{});
+      else f(Levels<4, 10, 5, 5>{}, integral_constant<int, 128>{});
+      return true;
     default: return false;
   }
 }

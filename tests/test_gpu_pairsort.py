@@ -39,6 +39,23 @@ def _curves(kind, n, seed):
     return torch.as_tensor(c, device=DEV)
 
 
+# quotients in long runs of equal top bits whose keys alternate: 2, 64 and more than the 64 runs
+# that are sorted one by one, at the ends of the range and across tiles
+@pytest.mark.parametrize("runs", [2, 64, 150])
+def test_long_runs_out_of_order(ctx, runs):
+    import microsn_gb300 as mlc
+    n = 1200
+    rng = np.random.default_rng(runs)
+    v = np.linspace(1.0, 3.0, runs)[rng.integers(0, runs, n)]
+    A = torch.as_tensor(np.repeat((v * (1 + 2.0 ** -45 * rng.integers(0, 3, n)))[:, None], 3, 1), device=DEV)
+    B = torch.ones((n, 3), dtype=torch.float64, device=DEV)
+    rank, _, _ = mlc.setup_integral(ctx, A.contiguous(), B, mlc.bin_edges(10, 1e-3, 1e3))
+    _, order = torch.sort((A[:, 0][:, None] / B[:, 0][None, :]).reshape(-1), stable=True)
+    want = torch.empty_like(order)
+    want[order] = torch.arange(order.numel(), device=DEV)
+    assert torch.equal(rank.to(torch.int64) & 0xFFFFFFFF, want)
+
+
 # from 1024 pairs a side on the keys are sorted by the top of their range, 5600: chi2 and ranks
 # written through bins (above 3e7)
 @pytest.mark.parametrize("kind,n", [("integers", 300), ("extreme", 1100), ("smooth", 1500), ("integers", 1500),

@@ -290,14 +290,16 @@ void radix_sort_u64_u32(mlc_ctx* ctx, long n, uint64_t* keys, uint32_t* vals) {
 // sorted by its full keys, stably, by one thread: within tiles of the keys in shared memory
 // (k_fix_tiles), then across the tiles' edges (k_fix_edges).  Runs of equal keys are in order
 // as they stand, however long.  A run with a descent that is longer than FIX_RUN is noted
-// (long_run) and sorted as a range of its own: quotients of ray counts come in runs of 10^4
-// equal keys, and here and there two such runs share their top bits (8.5e7 of them, FP32
-// counts: 12.2 ms with all keys made and sorted anew by all bits, 5.9 with the few runs alone).
+// (long_run) and sorted by a CTA, or, beyond RUN_MAX keys, as a range of its own.  Quotients of
+// ray counts come in runs of 10^2 to 10^4 equal keys, and here and there two such runs share
+// their top bits: 8.5e7 of them, FP32 counts around 20, 12.2 ms with all keys made and sorted
+// anew by all bits where that happened, 5.9 as here.
 constexpr int FIX_TILE = 4096, FIX_THREADS = 256;
-constexpr int LONG_RUNS = 64;
+constexpr int RUN_SLOTS = 8192, RUN_MAX = 2048, BIG_RUNS = 64;
 struct LongRuns {
-  int scatter_err, full;  // full: more than LONG_RUNS runs, the order is not made
-  unsigned long long at[LONG_RUNS], end[LONG_RUNS];  // first key (~0: none) and end of each
+  int scatter_err, full, nbig;  // full: more runs than there is room for, the order is not made
+  unsigned long long at[RUN_SLOTS];  // first key of a noted run (~0: none), by a hash of it
+  unsigned long long big_at[BIG_RUNS], big_end[BIG_RUNS];
 };
 
 // First of the n keys, ordered by their top bits, whose top bits are at least tp.
@@ -312,20 +314,46 @@ __device__ __forceinline__ long lower_bound_top(const uint64_t* __restrict__ key
 }
 __device__ __noinline__ void long_run(const uint64_t* keys, long n, uint64_t lo, int sh, uint64_t tp, LongRuns* lr) {
   const unsigned long long b = (unsigned long long)lower_bound_top(keys, n, lo, sh, tp);
-  for (int r = 0; r < LONG_RUNS; r++) {
-    const unsigned long long was = atomicCAS(&lr->at[r], ~0ull, b);
+  const unsigned h = ((unsigned)b * 2654435761u) >> 16;
+  for (unsigned r = 0; r < 64; r++) {
+    const unsigned long long was = atomicCAS(&lr->at[(h + r) % RUN_SLOTS], ~0ull, b);
     if (was == ~0ull || was == b) return;
   }
   atomicExch(&lr->full, 1);
 }
-__global__ void __launch_bounds__(LONG_RUNS) k_long_run_ends(const uint64_t* __restrict__ keys, long n,
-                                                             const unsigned long long* __restrict__ range,
-                                                             LongRuns* __restrict__ lr) {
-  const unsigned long long b = lr->at[threadIdx.x];
+// A CTA per slot: the noted run stably sorted by counting the keys before each.
+__global__ void __launch_bounds__(256) k_sort_runs(uint64_t* __restrict__ keys, uint32_t* __restrict__ vals, long n,
+                                                   const unsigned long long* __restrict__ range,
+                                                   LongRuns* __restrict__ lr) {
+  __shared__ uint64_t ks[RUN_MAX];
+  __shared__ uint32_t vs[RUN_MAX];
+  __shared__ long end;
+  const unsigned long long b = lr->at[blockIdx.x];
   if (b == ~0ull) return;
-  const uint64_t lo = range[0];
-  const int sh = RangeDigit::base_shift(range);
-  lr->end[threadIdx.x] = (unsigned long long)lower_bound_top(keys, n, lo, sh, ((keys[b] - lo) >> sh) + 1);
+  if (threadIdx.x == 0) {
+    const uint64_t lo = range[0];
+    const int sh = RangeDigit::base_shift(range);
+    end = lower_bound_top(keys, n, lo, sh, ((keys[b] - lo) >> sh) + 1);
+  }
+  __syncthreads();
+  const long len = end - (long)b;
+  if (len > RUN_MAX) {
+    if (threadIdx.x == 0) {
+      const int r = atomicAdd(&lr->nbig, 1);
+      if (r < BIG_RUNS) lr->big_at[r] = b, lr->big_end[r] = (unsigned long long)end;
+      else atomicExch(&lr->full, 1);
+    }
+    return;
+  }
+  for (int i = threadIdx.x; i < len; i += blockDim.x) ks[i] = keys[b + i], vs[i] = vals[b + i];
+  __syncthreads();
+  for (int i = threadIdx.x; i < len; i += blockDim.x) {
+    const uint64_t k = ks[i];
+    int r = 0;
+    for (int j = 0; j < len; j++) r += ks[j] < k || (ks[j] == k && j < i);
+    keys[b + r] = k;
+    vals[b + r] = vs[i];
+  }
 }
 
 __global__ void __launch_bounds__(FIX_THREADS) k_fix_tiles(uint64_t* __restrict__ keys, uint32_t* __restrict__ vals,
@@ -427,18 +455,23 @@ bool radix_sort_range_u64_u32(mlc_ctx* ctx, long n, uint64_t* keys, uint32_t* va
     const long tiles = (n + FIX_TILE - 1) / FIX_TILE;
     k_fix_tiles<<<(unsigned)tiles, FIX_THREADS, 0, ctx->stream>>>(keys, vals, n, range, dl);
     k_fix_edges<<<(unsigned)((tiles + 255) / 256), 256, 0, ctx->stream>>>(keys, vals, n, range, dl);
-    k_long_run_ends<<<1, LONG_RUNS, 0, ctx->stream>>>(keys, n, range, dl);
+    k_sort_runs<<<RUN_SLOTS, 256, 0, ctx->stream>>>(keys, vals, n, range, dl);
   }
   MLC_CHECK_LAUNCH();
-  LongRuns h;
+  struct {
+    int scatter_err, full, nbig;
+  } h;
+  unsigned long long big[2 * BIG_RUNS];
   MLC_CUDA(cudaMemcpyAsync(&h, dl, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
+  MLC_CUDA(cudaMemcpyAsync(big, dl->big_at, sizeof big, cudaMemcpyDeviceToHost, ctx->stream));
   MLC_CUDA(cudaStreamSynchronize(ctx->stream));
   MLC_REQUIRE(h.scatter_err == 0, MLC_ERR_CUDA, "radix sort: scatter offset out of range (inconsistent digit counts)");
+  if (h.full) return false;
   unsigned long long total = 0;
-  for (int r = 0; r < LONG_RUNS && h.at[r] != ~0ull; r++) total += h.end[r] - h.at[r];
-  if (h.full || total > (unsigned long long)n / 2) return false;
-  for (int r = 0; r < LONG_RUNS && h.at[r] != ~0ull; r++)
-    radix_sort_u64_u32(ctx, (long)(h.end[r] - h.at[r]), keys + h.at[r], vals + h.at[r]);
+  for (int r = 0; r < h.nbig; r++) total += big[BIG_RUNS + r] - big[r];
+  if (total > (unsigned long long)n / 2) return false;
+  for (int r = 0; r < h.nbig; r++)
+    radix_sort_u64_u32(ctx, (long)(big[BIG_RUNS + r] - big[r]), keys + big[r], vals + big[r]);
   return true;
 }
 

@@ -39,9 +39,10 @@ def _curves(kind, n, seed):
     return torch.as_tensor(c, device=DEV)
 
 
-# quotients in long runs of equal top bits whose keys alternate: 2, 64 and more than the 64 runs
-# that are sorted one by one, at the ends of the range and across tiles
-@pytest.mark.parametrize("runs", [2, 64, 150])
+# quotients in long runs of equal top bits whose keys alternate: 2, 64 and more than the 64 large
+# runs that are sorted one by one, 1200 that a CTA each sorts, at the ends of the range and
+# across tiles
+@pytest.mark.parametrize("runs", [2, 64, 150, 1200])
 def test_long_runs_out_of_order(ctx, runs):
     import microsn_gb300 as mlc
     n = 1200

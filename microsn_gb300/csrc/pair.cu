@@ -17,7 +17,7 @@
 namespace mlc {
 
 void radix_sort_u64_u32(mlc_ctx* ctx, long n, uint64_t* keys, uint32_t* vals);
-bool radix_sort_range_u64_u32(mlc_ctx* ctx, long n, uint64_t* keys, uint32_t* vals, const unsigned long long* range);
+RangeSort radix_sort_range_u64_u32(mlc_ctx* ctx, long n, uint64_t* keys, uint32_t* vals, const unsigned long long* range);
 
 // The key of the reference's z sort (thrust::stable_sort_by_key on doubles, a radix sort):
 // the order of the bit patterns with the sign folded in, -0.0 taken as +0.0 (the radix sort
@@ -462,10 +462,9 @@ void pair_setup(mlc_ctx* ctx, int Nloc, int Nprof, const double* LCA, const doub
   make_keys();
   // by the top of the keys' range where the keys are many and that decides their order (8.5e7: 3.7
   // ms, by all bits 7.7); outliers, infinities or NaN may stretch the range: then by all bits
-  if (P < RANGE_SORT_FROM || !radix_sort_range_u64_u32(ctx, P, keys, idx, range)) {
-    if (P >= RANGE_SORT_FROM) make_keys();
-    radix_sort_u64_u32(ctx, P, keys, idx);
-  }
+  const RangeSort done = P < RANGE_SORT_FROM ? RangeSort::UNTOUCHED : radix_sort_range_u64_u32(ctx, P, keys, idx, range);
+  if (done == RangeSort::LOST) make_keys();
+  if (done != RangeSort::DONE) radix_sort_u64_u32(ctx, P, keys, idx);
   if (rank) put_by_index(ctx, "pair_rank", idx, LoadOwnIndex{}, P, rank);
   if (Nbins > 0) {
     double* dedge = (double*)ws_get(ctx, WS_SMALL, sizeof(double) * Nbins + sizeof(uint32_t) * Nbins);

@@ -23,6 +23,10 @@ struct ShiftDigit {
     return (unsigned)(k >> shift) & 0xffu;
   }
 };
+// What radix_sort_range_u64_u32 left: the sorted keys, the keys as they were, or keys in no order
+// (the last two have to be sorted by all their bits).
+enum class RangeSort { DONE, UNTOUCHED, LOST };
+
 // Byte `byte` of the top 32 bits of the keys' range: (key - lo) >> shift, lo and hi the least and
 // the largest key (range[0], ~range[1], as two minima gather them).
 struct RangeDigit {

@@ -10,10 +10,10 @@
 // twiddle tables need anyway), scales, transforms, and scales back on its stores.
 //
 // Measured at 10000^2, before (FP64, float-float) and with limbs:
-//   FP64         map rows 6.1 -> 1.5 ms, column pass 2.5 -> 0.72, P1 8.8 -> 2.0 (four Gaussians
+//   FP64         map rows 6.1 -> 1.5 ms, column pass 2.5 -> 0.70, P1 8.8 -> 1.9 (four Gaussians
 //                of 100 to 600 rows), P3 5.9 -> 1.5
-//   float-float  P1 from a cached profile spectrum 0.507 -> 0.378 ms (6.3 TB/s), P2 0.346 ->
-//                0.256 (6.0 TB/s), P3 of 16 profiles with the interleave 16.2 -> 10.4 ms
+//   float-float  P1 from a cached profile spectrum 0.507 -> 0.363 ms (6.6 TB/s), P2 0.346 ->
+//                0.256 (6.1 TB/s), P3 of 16 profiles with the interleave 16.2 -> 9.6 ms
 #pragma once
 
 #include <cooperative_groups.h>
@@ -307,7 +307,7 @@ __global__ void __launch_bounds__((L1 > L2 ? L1 : L2) * CW, 2)
 // P1 of FP32 maps' float-float plans, modes 0 and 2 of k_conv_fused2: the profile's forward half
 // in float-float as there (the same operations, so that its mode 1 makes the spectra of
 // mode 2), the product in float-float, the inverse half in lf2, scaled by the products' sum.
-// Mode 2 is bound by HBM: 2.4 GB at 10000^2 in 0.375 ms (6.3 TB/s; float-float 0.507 ms).
+// Mode 2 is bound by HBM: 2.4 GB at 10000^2 in 0.363 ms (6.6 TB/s; float-float 0.507 ms).
 template <int CW, int L1, int L2, int MODE>
 __global__ void __launch_bounds__((L1 > L2 ? L1 : L2) * CW, L1 + L2 > 20 ? 2 : 0)
     k_limb2_conv(const C2<ff>* __restrict__ Fmap, C2<ff>* __restrict__ out, long pitch, const C2<ff>* __restrict__ Kx,

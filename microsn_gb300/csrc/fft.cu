@@ -342,7 +342,7 @@ void conv_fused(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, const double
   if (p.prec == PREC_FFS) {  // P0-P2 to the half-spectrum, then P3 into FP32 pixels
     void* tmp = ws_get(ctx, WS_SPEC_TMP, p.spec_bytes());
     conv_fused_impl<ff>(ctx, p, Fmap, prof, pN, nullptr, tmp, WS_KX);
-    if (!limb2_rows_c2r(ctx, p, tmp, out)) rows_c2r_impl<ff, float>(ctx, p, tmp, out);
+    rows_c2r_impl<ff, float>(ctx, p, tmp, out);
   } else if (p.prec == PREC_FF) conv_fused_impl<ff>(ctx, p, Fmap, prof, pN, out);
   else if (p.prec == MLC_F64) conv_fused_impl<double>(ctx, p, Fmap, prof, pN, out);
   else conv_fused_impl<float>(ctx, p, Fmap, prof, pN, out);
@@ -381,7 +381,7 @@ void conv_cached(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, const void*
   if (p.prec == PREC_FFS) {
     void* tmp = ws_get(ctx, WS_SPEC_TMP, p.spec_bytes());
     conv_cached_impl<ff>(ctx, p, Fmap, ks, tmp);
-    if (!limb2_rows_c2r(ctx, p, tmp, out)) rows_c2r_impl<ff, float>(ctx, p, tmp, out);
+    rows_c2r_impl<ff, float>(ctx, p, tmp, out);
   } else if (p.prec == PREC_FF) conv_cached_real_impl<ff>(ctx, p, Fmap, ks, out);
   else if (p.prec == MLC_F64) conv_cached_real_impl<double>(ctx, p, Fmap, ks, out);
   else conv_cached_real_impl<float>(ctx, p, Fmap, ks, out);
@@ -394,7 +394,7 @@ bool rows_c2r_interleave_supported(const FftPlan2D& p) {
 bool rows_c2r_interleave(mlc_ctx* ctx, const FftPlan2D& p, const void* specs, long spec_stride, int nm, int S,
                          void* out, unsigned planar) {
   if (!rows_c2r_interleave_supported(p)) return false;
-  if (p.prec == PREC_FFS) return limb2_rows_c2r_il(ctx, p, specs, spec_stride, nm, S, out, planar);
+  if (p.prec == PREC_FFS) return c2r_interleave_impl<ff, float>(ctx, p, specs, spec_stride, nm, S, out, planar);
   if (p.prec == PREC_FF) return c2r_interleave_impl<ff>(ctx, p, specs, spec_stride, nm, S, out, planar);
   if (p.prec == MLC_F64) return limb3_rows_c2r_il(ctx, p, specs, spec_stride, nm, S, out, planar);
   return c2r_interleave_impl<float>(ctx, p, specs, spec_stride, nm, S, out, planar);

@@ -10,6 +10,7 @@ template bool any_real_r2c<ff, RealRows<ff, float>>(mlc_ctx*, const FftPlan2D&, 
 template bool any_real_r2c<ff, ProfileRows<ff>>(mlc_ctx*, const FftPlan2D&, const ProfileRows<ff>&, int, void*,
                                                   const char*);
 template bool any_real_c2r<ff, double>(mlc_ctx*, const FftPlan2D&, const void*, void*);
+template bool any_real_c2r<ff, float>(mlc_ctx*, const FftPlan2D&, const void*, void*);
 template bool any_real_colpass<ff, false>(mlc_ctx*, const FftPlan2D&, void*, char, int);
 template bool any_real_colpass<ff, true>(mlc_ctx*, const FftPlan2D&, void*, char, int);
 

@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(512) k_any_real_r2c(Loader ld, C2<T>* __restri
 
 // Inverse real transform of one row per CTA (k_rows_c2r's result).  The inputs of item j of
 // level 0, k = j + J q, have their partners M - k in item J - j: a thread forms and transforms
-// both (limb_c2r_first in fft_limb.cuh).
+// both.
 template <typename T, typename TO>
 __global__ void __launch_bounds__(512) k_any_real_c2r(const C2<T>* __restrict__ in, long pitch, TO* __restrict__ out,
                                                       long ldo, const C2<T>* __restrict__ twx,

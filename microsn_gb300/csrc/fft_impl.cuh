@@ -988,7 +988,7 @@ static void launch_rows_r2c(mlc_ctx* ctx, const FftPlan2D& p, const Loader& ld, 
 
 template <typename T, typename TO = typename RealOut<T>::type>
 static void launch_rows_c2r(mlc_ctx* ctx, const FftPlan2D& p, const void* in, void* out) {
-  if constexpr (!(std::is_same<T, ff>::value && std::is_same<TO, float>::value)) {  // (those: limb2_rows_c2r)
+  {
     using K3 = void (*)(const C2<T>*, long, TO*, long, const C2<T>*, const C2<T>*);
     K3 k3 = nullptr;
     int J = 0;
@@ -1011,7 +1011,7 @@ static void launch_rows_c2r(mlc_ctx* ctx, const FftPlan2D& p, const void* in, vo
       return;
     }
   }
-  if constexpr (!std::is_same<T, double>::value && std::is_same<TO, typename RealOut<T>::type>::value)
+  if constexpr (!std::is_same<T, double>::value)
     if (any_real_c2r<T, TO>(ctx, p, in, out)) return;
   size_t smem = 2 * (size_t)(p.M + 1) * sizeof(C2<T>);
   auto kern = k_rows_c2r<T, TO>;
@@ -1034,8 +1034,8 @@ constexpr int strip_width() {
 }
 
 // kind 'A': row sets {n2 + N2*j}, length N1; kind 'B': row blocks {k1*N2 + j}, length N2.
-// limbs: FP64 passes, and the inverse ones of FP32 maps' float-float plans, in limb arithmetic
-// where the length has a kernel (the plain convolution keeps the plan's own arithmetic).
+// limbs: FP64 passes in limb arithmetic where the length has a kernel (the plain convolution
+// keeps the plan's own arithmetic).
 template <typename T, bool INV>
 static void launch_colpass(mlc_ctx* ctx, const FftPlan2D& p, void* buf, char kind, int post_tw, bool limbs = true) {
   constexpr int CW = strip_width<T>();
@@ -1051,8 +1051,6 @@ static void launch_colpass(mlc_ctx* ctx, const FftPlan2D& p, void* buf, char kin
   if (L == 1 && !post_tw) return;
   if constexpr (std::is_same<T, double>::value)
     if (limbs && limb3_colpass(ctx, p, buf, kind, INV, post_tw)) return;
-  if constexpr (std::is_same<T, ff>::value && INV)
-    if (limbs && p.prec == PREC_FFS && limb2_colpass_inverse(ctx, p, buf, kind, post_tw)) return;
   // two-level register kernels for the lengths that split into two supported factors
   using K2 = void (*)(C2<T>*, long, long, long, const C2<T>*, int, int);
   K2 k2 = nullptr;
@@ -1110,7 +1108,7 @@ void forward_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* in, int in_dtype
 }
 
 // Workspace of P0's rows; FP64 keeps them in three limbs (24 bytes) beside the FP64 ones, with
-// an exponent per column (LimbProfileBuffer in fft_limb.cuh).
+// an exponent per column (limb3_profile_rows in fft_limb.cuh).
 template <typename T>
 static size_t profile_rows_bytes(const FftPlan2D& p, int rows) {
   const size_t n = (size_t)(rows > 0 ? rows : 1) * p.Wp;
@@ -1145,11 +1143,8 @@ void conv_fused_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, const d
   void* kx = ws_get(ctx, kx_slot, profile_rows_bytes<T>(p, 2 * h));
   void* tmp = spec_out ? spec_out : ws_get(ctx, WS_SPEC_TMP, p.spec_bytes());
   profile_rows<T>(ctx, p, prof, pN, kx);
-  {
-    bool done = false;
-    if constexpr (std::is_same<T, double>::value) done = limb3_conv(ctx, p, Fmap, tmp, kx, h);
-    if constexpr (std::is_same<T, ff>::value) done = p.prec == PREC_FFS && limb2_conv(ctx, p, Fmap, tmp, kx, h);
-    if (done) {
+  if constexpr (std::is_same<T, double>::value) {
+    if (limb3_conv(ctx, p, Fmap, tmp, kx, h)) {
       launch_colpass<T, true>(ctx, p, tmp, 'A', 0);
       if (!spec_out) real_rows<T>(ctx, p, tmp, out);
       return;
@@ -1273,22 +1268,18 @@ void conv_cached_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, const 
   if constexpr (std::is_same<T, double>::value) {
     limb3_conv_cached(ctx, p, Fmap, spec_out, ks);
   } else {
-    bool done = false;
-    if constexpr (std::is_same<T, ff>::value) done = p.prec == PREC_FFS && limb2_conv_cached(ctx, p, Fmap, spec_out, ks);
-    if (!done) {
-      int nthr = 0;
-      const auto k = p1_mode_kernel<T, 2>(p.N2, nthr);
-      const T scale = (T)(1.0 / ((double)p.Nx * (double)p.Ny));
-      const size_t smem = ((size_t)p.N2 * CW + p.N1 + 2 * (size_t)p.N2) * sizeof(C2<T>);
-      set_max_smem((const void*)k, smem);
-      {
-        MLC_KSCOPE(ctx, "conv_cached_spectrum");
-        k<<<dim3(ceil_div(p.Wc, CW), p.N1), nthr, smem, ctx->stream>>>((const C2<T>*)Fmap, (C2<T>*)spec_out, p.Wp,
-                                                                         nullptr, 0, p.Ny, p.N1, (const C2<T>*)p.twy,
-                                                                         scale, (C2<T>*)ks);
-      }
-      MLC_CHECK_LAUNCH();
+    int nthr = 0;
+    const auto k = p1_mode_kernel<T, 2>(p.N2, nthr);
+    const T scale = (T)(1.0 / ((double)p.Nx * (double)p.Ny));
+    const size_t smem = ((size_t)p.N2 * CW + p.N1 + 2 * (size_t)p.N2) * sizeof(C2<T>);
+    set_max_smem((const void*)k, smem);
+    {
+      MLC_KSCOPE(ctx, "conv_cached_spectrum");
+      k<<<dim3(ceil_div(p.Wc, CW), p.N1), nthr, smem, ctx->stream>>>((const C2<T>*)Fmap, (C2<T>*)spec_out, p.Wp,
+                                                                       nullptr, 0, p.Ny, p.N1, (const C2<T>*)p.twy,
+                                                                       scale, (C2<T>*)ks);
     }
+    MLC_CHECK_LAUNCH();
   }
   launch_colpass<T, true>(ctx, p, spec_out, 'A', 0);
 }

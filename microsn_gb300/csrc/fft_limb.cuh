@@ -1,19 +1,13 @@
-// The transform passes of fft_impl.cuh in fixed-grid limb arithmetic (limb.cuh):
+// The FP64 transform passes of fft_impl.cuh, forward and inverse, in fixed-grid limb arithmetic
+// (limb.cuh): storage S = double, arithmetic T = lf3.
 //
-//   FP64 plans (storage S = double, arithmetic T = lf3)   every pass, forward and inverse
-//   float-float plans of FP32 maps (S = ff, T = lf2)      the inverse passes P1 - P3
-//
-// What bounded them before: the FP64 passes the FP64 pipe (0.63 T operations/s; a P1 of
-// 10000^2 took 8.8 ms for 2.4 GB of traffic), the float-float ones the FP32 pipe, half of
-// it two-sums.  Each pass reads its inputs once into registers, sums |re| + |im| over every
-// transform it holds (one exchange through shared memory beside the barrier that the
+// What bounded them before: the FP64 pipe (0.63 T operations/s; a P1 of 10000^2 took 8.8 ms for
+// 2.4 GB of traffic).  Each pass reads its inputs once into registers, sums |re| + |im| over
+// every transform it holds (one exchange through shared memory beside the barrier that the
 // twiddle tables need anyway), scales, transforms, and scales back on its stores.
 //
-// Measured at 10000^2, before (FP64, float-float) and with limbs:
-//   FP64         map rows 6.1 -> 1.5 ms, column pass 2.5 -> 0.70, P1 8.8 -> 1.9 (four Gaussians
-//                of 100 to 600 rows), P3 5.9 -> 1.5
-//   float-float  P1 from a cached profile spectrum 0.507 -> 0.363 ms (6.6 TB/s), P2 0.346 ->
-//                0.256 (6.1 TB/s), P3 of 16 profiles with the interleave 16.2 -> 9.6 ms
+// Measured at 10000^2, FP64 arithmetic and limbs: map rows 6.1 and 1.5 ms, column pass 2.5 and
+// 0.70, P1 8.8 and 1.9 (four Gaussians of 100 to 600 rows), P3 5.9 and 1.5.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -34,7 +28,7 @@ __device__ __forceinline__ C2<T> limb_zero() {
 // exchanged through red while the tables are being filled.  Strips wider than the pitch's
 // 16-column granule mask the columns past it.
 template <typename S, typename T, int CW, int L1, int L2, bool INV>
-__global__ void __launch_bounds__((L1 > L2 ? L1 : L2) * CW, sizeof(T) == sizeof(lf3) ? 2 : L1 + L2 > 20 ? 2 : 4)
+__global__ void __launch_bounds__((L1 > L2 ? L1 : L2) * CW, 2)
     k_limb_colpass2(C2<S>* __restrict__ buf, long pitch, long set_mul, long j_mul, LimbTab<T> twy, int tw_stride,
                     int post_tw) {
   constexpr int L = L1 * L2;
@@ -71,8 +65,7 @@ __global__ void __launch_bounds__((L1 > L2 ? L1 : L2) * CW, sizeof(T) == sizeof(
     Dft<T, L1, INV>::run(v);
 #pragma unroll
     for (int k1 = 0; k1 < L1; k1++)
-      y.st((g * L1 + k1) * CW + c, k1 == 0 ? (sizeof(T) == sizeof(lf3) ? limb_cnorm(v[0]) : v[0])
-                                           : limb_tw<INV, false>(v[k1], wl.ld(g * k1)));
+      y.st((g * L1 + k1) * CW + c, k1 == 0 ? limb_cnorm(v[0]) : limb_tw<INV>(v[k1], wl.ld(g * k1)));
   }
   __syncthreads();
   if (g < L1) {
@@ -84,7 +77,7 @@ __global__ void __launch_bounds__((L1 > L2 ? L1 : L2) * CW, sizeof(T) == sizeof(
     for (int k2 = 0; k2 < L2; k2++) {
       const int j = g + L1 * k2;
       C2<T> val = u[k2];
-      if (post_tw) val = limb_tw<INV, false>(val, pw.ld(j));
+      if (post_tw) val = limb_tw<INV>(val, pw.ld(j));
       if (in) b[(long)j * j_mul * pitch] = limb_cout<S>(val, sc);
     }
   }
@@ -211,7 +204,7 @@ __global__ void __launch_bounds__((L1 > L2 ? L1 : L2) * CW, 2)
         }
         const C2<T> w = w1.ld(n1);
 #pragma unroll
-        for (int q = 0; q < E; q++) acc[q] = cadd(acc[q], limb_tw<false, true>(v[q], w));
+        for (int q = 0; q < E; q++) acc[q] = cadd(acc[q], limb_tw<false>(v[q], w));
       };
 #pragma unroll
       for (int q = 0; q < E; q++) {
@@ -225,7 +218,7 @@ __global__ void __launch_bounds__((L1 > L2 ? L1 : L2) * CW, 2)
 #pragma unroll
       for (int q = 0; q < E; q++) {
         const int n2 = g + G * (i + q);
-        y.st(n2 * CW + c, limb_tw<false, true>(acc[q], w2r.ld(n2)));
+        y.st(n2 * CW + c, limb_tw<false>(acc[q], w2r.ld(n2)));
       }
     }
     __syncthreads();
@@ -240,7 +233,7 @@ __global__ void __launch_bounds__((L1 > L2 ? L1 : L2) * CW, 2)
       if (g < L2) {
 #pragma unroll
         for (int k1 = 0; k1 < L1; k1++)
-          y.st((g * L1 + k1) * CW + c, k1 == 0 ? limb_cnorm(v[0]) : limb_tw<false, true>(v[k1], wl.ld(g * k1)));
+          y.st((g * L1 + k1) * CW + c, k1 == 0 ? limb_cnorm(v[0]) : limb_tw<false>(v[k1], wl.ld(g * k1)));
       }
     }
     __syncthreads();
@@ -276,13 +269,13 @@ __global__ void __launch_bounds__((L1 > L2 ? L1 : L2) * CW, 2)
 #pragma unroll
       for (int k2 = 0; k2 < L2; k2++) {
         const C2<T> fl = limb_cin(in ? f[(long)(L1 * k2) * pitch] : C2<double>{0.0, 0.0}, sc);
-        u[k2] = limb_tw<false, true>(fl, MODE == 0 ? limb_cnorm(u[k2]) : u[k2]);
+        u[k2] = limb_tw<false>(fl, MODE == 0 ? limb_cnorm(u[k2]) : u[k2]);
       }
       Dft<T, L2, true>::run(u);  // over k2 -> n2
       // (the thread rewrites exactly the entries of y it read above: no other thread's data)
 #pragma unroll
       for (int n2 = 0; n2 < L2; n2++)
-        y.st((n2 * L1 + g) * CW + c, n2 == 0 ? limb_cnorm(u[0]) : limb_tw<true, true>(u[n2], wl.ld(g * n2)));
+        y.st((n2 * L1 + g) * CW + c, n2 == 0 ? limb_cnorm(u[0]) : limb_tw<true>(u[n2], wl.ld(g * n2)));
     }
     sc.bad |= ke == LIMB_BAD;  // the scales multiply: exponents add
     sc.e += sc.bad ? 0 : ke;
@@ -297,140 +290,9 @@ __global__ void __launch_bounds__((L1 > L2 ? L1 : L2) * CW, 2)
 #pragma unroll
         for (int n1 = 0; n1 < L1; n1++) {
           const int n = g + L2 * n1;
-          out[((long)kk * N2 + n) * pitch + col] = limb_cout<double>(limb_tw<true, false>(v[n1], w2.ld(n)), sc);
+          out[((long)kk * N2 + n) * pitch + col] = limb_cout<double>(limb_tw<true>(v[n1], w2.ld(n)), sc);
         }
       }
-    }
-  }
-}
-
-// P1 of FP32 maps' float-float plans, modes 0 and 2 of k_conv_fused2: the profile's forward half
-// in float-float as there (the same operations, so that its mode 1 makes the spectra of
-// mode 2), the product in float-float, the inverse half in lf2, scaled by the products' sum.
-// Mode 2 is bound by HBM: 2.4 GB at 10000^2 in 0.363 ms (6.6 TB/s; float-float 0.507 ms).
-template <int CW, int L1, int L2, int MODE>
-__global__ void __launch_bounds__((L1 > L2 ? L1 : L2) * CW, L1 + L2 > 20 ? 2 : 0)
-    k_limb2_conv(const C2<ff>* __restrict__ Fmap, C2<ff>* __restrict__ out, long pitch, const C2<ff>* __restrict__ Kx,
-                 int h, int Ny, int N1, const C2<ff>* __restrict__ twy, ff scale, const C2<ff>* __restrict__ ks) {
-  constexpr int N2 = L1 * L2, G = L1 > L2 ? L1 : L2, NE = N2 / G;
-  static_assert(N2 % G == 0, "rows per thread");
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C2<ff>* a = reinterpret_cast<C2<ff>*>(smem_raw);   // [N2][CW]: the profile's sub-pass
-  C2<lf2>* y = reinterpret_cast<C2<lf2>*>(smem_raw);  // and the inverse half's transpose
-  C2<ff>* w2 = a + N2 * CW;                          // W_Ny^(n kk), n < N2
-  C2<ff>* wl = w2 + N2;                              // W_N2^m, m < N2
-  C2<ff>* w1 = wl + N2;                              // W_N1^(n1 kk), n1 < N1
-  __shared__ float red[L1][CW];
-  const int kk = blockIdx.y;
-  const long col0 = (long)blockIdx.x * CW;
-  const int c = threadIdx.x % CW, g = threadIdx.x / CW;
-  C2<ff> f[L2], kf[L2];
-  if constexpr (MODE == 2) {
-    if (g < L1) {
-#pragma unroll
-      for (int k2 = 0; k2 < L2; k2++) {
-        const long e = ((long)kk * N2 + g + L1 * k2) * pitch + col0 + c;
-        f[k2] = ldc(Fmap + e);
-        kf[k2] = ldc(ks + e);
-      }
-    }
-  } else {
-    // the map-spectrum tile is needed after the profile's forward half: into L2 now
-    constexpr int LINES = (int)(CW * sizeof(C2<ff>) / 128);
-    for (int n = threadIdx.x; n < N2 * LINES; n += blockDim.x)
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(Fmap + ((long)kk * N2 + n / LINES) * pitch + col0 +
-                                                    (n % LINES) * (128 / (int)sizeof(C2<ff>))));
-    for (int n1 = threadIdx.x; n1 < N1; n1 += blockDim.x) w1[n1] = ldc(twy + (long)((n1 * kk) % N1) * N2);
-  }
-  for (int n = threadIdx.x; n < N2; n += blockDim.x) {
-    w2[n] = ldc(twy + (long)n * kk);
-    wl[n] = ldc(twy + (long)n * N1);
-  }
-  if constexpr (MODE != 2) {
-    const C2<ff>* kx = Kx + col0 + c;
-    C2<ff> acc[NE];
-#pragma unroll
-    for (int i = 0; i < NE; i++) acc[i] = g + G * i < h ? ldc(kx + (long)(g + G * i) * pitch) : C2<ff>{ff(0), ff(0)};
-    __syncthreads();
-    const int tlo = (h + N2 - 1) / N2;
-#pragma unroll 1
-    for (int n1 = 1; n1 < tlo; n1++) {
-      const C2<ff> w = w1[n1];
-#pragma unroll
-      for (int i = 0; i < NE; i++) {
-        const int j = n1 * N2 + g + G * i;
-        if (j < h) acc[i] = cadd(acc[i], cmul(ldc(kx + (long)j * pitch), w));
-      }
-    }
-#pragma unroll 1
-    for (int n1 = max(N1 - tlo - 1, 0); n1 < N1; n1++) {
-      const C2<ff> w = w1[n1];
-#pragma unroll
-      for (int i = 0; i < NE; i++) {
-        const int j = n1 * N2 + g + G * i;  // kernel row
-        if (j >= Ny - h) acc[i] = cadd(acc[i], cmul(ldc(kx + (j - (Ny - 2L * h)) * pitch), w));
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < NE; i++) a[(g + G * i) * CW + c] = cmul(acc[i], w2[g + G * i]);
-    __syncthreads();
-    {
-      C2<ff> v[L1];
-      if (g < L2) {
-#pragma unroll
-        for (int n1 = 0; n1 < L1; n1++) v[n1] = a[(L2 * n1 + g) * CW + c];
-        Dft<ff, L1, false>::run(v);
-      }
-      __syncthreads();
-      if (g < L2) {
-#pragma unroll
-        for (int k1 = 0; k1 < L1; k1++) a[(g * L1 + k1) * CW + c] = k1 == 0 ? v[0] : cmul(v[k1], wl[g * k1]);
-      }
-    }
-    __syncthreads();
-    if (g < L1) {
-#pragma unroll
-      for (int n2 = 0; n2 < L2; n2++) kf[n2] = a[(n2 * L1 + g) * CW + c];
-      Dft<ff, L2, false>::run(kf);
-#pragma unroll
-      for (int k2 = 0; k2 < L2; k2++) {
-        f[k2] = ldc(Fmap + ((long)kk * N2 + g + L1 * k2) * pitch + col0 + c);
-        kf[k2] = cscale(kf[k2], scale);
-      }
-    }
-  }
-  if (g < L1) {
-#pragma unroll
-    for (int k2 = 0; k2 < L2; k2++) f[k2] = cmul(f[k2], kf[k2]);
-    red[g][c] = limb_sum<L2>(f).s;
-  }
-  __syncthreads();
-  float sum = red[0][c];
-#pragma unroll
-  for (int q = 1; q < L1; q++) sum = __fadd_rn(sum, red[q][c]);
-  const LimbScale<lf2> sc = limb_scale(LimbSum<ff>{sum}, 0);
-  auto tw = [](C2<ff> w) { return C2<lf2>{lf2(w.x.hi, w.x.lo), lf2(w.y.hi, w.y.lo)}; };
-  if (g < L1) {
-    C2<lf2> u[L2];
-#pragma unroll
-    for (int k2 = 0; k2 < L2; k2++) u[k2] = limb_cin(f[k2], sc);
-    Dft<lf2, L2, true>::run(u);  // over k2 -> n2
-    // (the thread rewrites exactly the entries it read above: no other thread's data)
-#pragma unroll
-    for (int n2 = 0; n2 < L2; n2++)
-      y[(n2 * L1 + g) * CW + c] = n2 == 0 ? u[0] : limb_tw<true, false>(u[n2], tw(wl[g * n2]));
-  }
-  __syncthreads();
-  // inverse stage B: thread (n2 = g, c) over k1 -> rows n2 + L2 n1
-  if (g < L2) {
-    C2<lf2> v[L1];
-#pragma unroll
-    for (int k1 = 0; k1 < L1; k1++) v[k1] = y[(g * L1 + k1) * CW + c];
-    Dft<lf2, L1, true>::run(v);
-#pragma unroll
-    for (int n1 = 0; n1 < L1; n1++) {
-      const int n = g + L2 * n1;
-      out[((long)kk * N2 + n) * pitch + col0 + c] = limb_cout<ff>(limb_tw<true, false>(v[n1], tw(w2[n])), sc);
     }
   }
 }
@@ -485,8 +347,7 @@ struct LevelPlace<Levels<R0, R1, R...>> {
 
 // One level but the last: NB blocks of LV, whose places come from `outer`; tw(q, m) is
 // W_{LV::M}^(m q).
-// lf3 products always carry; lf2 ones (and the output without a twiddle) where CARRY asks.
-template <typename T, bool INV, int NT, typename LV, int R0, int NB, bool CARRY, typename Place, typename Tw>
+template <typename T, bool INV, int NT, typename LV, int R0, int NB, typename Place, typename Tw>
 __device__ __forceinline__ void limb_level(const LimbArr<T>& s, Place outer, Tw tw) {
   constexpr int BN = LV::Next::M, TN = LV::TN;
   for (int it = threadIdx.x; it < NB * BN; it += NT) {
@@ -496,9 +357,9 @@ __device__ __forceinline__ void limb_level(const LimbArr<T>& s, Place outer, Tw 
 #pragma unroll
     for (int q = 0; q < R0; q++) u[q] = s.ld(p + q * TN);
     Dft<T, R0, INV>::run(u);
-    s.st(p, (CARRY || sizeof(T) == sizeof(lf3)) ? limb_cnorm(u[0]) : u[0]);
+    s.st(p, limb_cnorm(u[0]));
 #pragma unroll
-    for (int q = 1; q < R0; q++) s.st(p + q * TN, limb_tw<INV, CARRY>(u[q], tw(q, m)));
+    for (int q = 1; q < R0; q++) s.st(p + q * TN, limb_tw<INV>(u[q], tw(q, m)));
   }
   __syncthreads();
 }
@@ -533,8 +394,7 @@ __device__ __forceinline__ void limb_fill_deep(Levels<R0, R1, R...>, const LimbA
 }
 
 // All levels but the last, in order, from level DEPTH on; `at`: where the level's table starts
-// in w.  lf2 carries after levels 0 and 1 (a low limb that gathers over three radices rounds
-// at 2^-44 of the scale).
+// in w.
 template <typename T, bool INV, int NT, int DEPTH, int NB, typename Place, int R0>
 __device__ __forceinline__ void limb_levels(Levels<R0>, const LimbArr<T>&, const LimbArr<T>&, int, const LimbTab<T>&,
                                             Place) {}
@@ -543,7 +403,7 @@ __device__ __forceinline__ void limb_levels(Levels<R0, R1, R...>, const LimbArr<
                                             const LimbTab<T>& tab0, Place outer) {
   using LV = Levels<R0, R1, R...>;
   constexpr int BN = LV::Next::M;
-  limb_level<T, INV, NT, LV, R0, NB, DEPTH == 1>(s, outer, [&](int q, int m) {
+  limb_level<T, INV, NT, LV, R0, NB>(s, outer, [&](int q, int m) {
     if constexpr (DEPTH == 0) return tab0.ld((q - 1) * BN + m);
     else return w.ld(at + (q - 1) * BN + m);
   });
@@ -610,7 +470,7 @@ constexpr size_t limb_row_smem() {
 template <typename T>
 __device__ __forceinline__ void limb_c2r_pair(C2<T> xk, C2<T> xm, C2<T> w, C2<T>& bk, C2<T>& bm) {
   const C2<T> e = cadd(xk, xm);
-  const C2<T> o = limb_tw<true, false>(csub(xk, xm), w);  // (X - conj X') W^-k
+  const C2<T> o = limb_tw<true>(csub(xk, xm), w);  // (X - conj X') W^-k
   bk = C2<T>{e.x - o.y, e.y + o.x};
   bm = C2<T>{e.x + o.y, o.x - e.y};
 }
@@ -618,13 +478,10 @@ __device__ __forceinline__ void limb_c2r_pair(C2<T> xk, C2<T> xm, C2<T> w, C2<T>
 // The inverse real transform of one spectrum row (as k_rows_c2r: the input
 // b[k] = (X[k] + conj X[M-k]) + i (X[k] - conj X[M-k]) W_Nx^-k, then the inverse transform of
 // M points).  The row is read once into registers, both partners k and M - k by one thread.
-//
-// lf3: the input goes to shared memory, then level 0 (radix R0, J = M / R0 items) like the others.
 template <typename S, typename T, int NT, int R0, int... R>
-__device__ __forceinline__ LimbScale<T> limb_c2r_first(Levels<R0, R...>, std::integral_constant<bool, false>,
-                                                       const C2<S>* __restrict__ a, const LimbTab<T>& twx,
-                                                       const LimbTab<T>& tab0, const LimbArr<T>& s,
-                                                       const LimbArr<T>& w, LimbSum<S>* red) {
+__device__ __forceinline__ LimbScale<T> limb_c2r_first(Levels<R0, R...>, const C2<S>* __restrict__ a,
+                                                       const LimbTab<T>& twx, const LimbTab<T>& tab0,
+                                                       const LimbArr<T>& s, const LimbArr<T>& w, LimbSum<S>* red) {
   using LV = Levels<R0, R...>;
   constexpr int M = LV::M, NP = (M / 2 + 1 + NT - 1) / NT;
   const int tid = threadIdx.x;
@@ -637,7 +494,7 @@ __device__ __forceinline__ LimbScale<T> limb_c2r_first(Levels<R0, R...>, std::in
     x[2 * i + 1] = in ? ldc(a + (M - k)) : C2<S>{S(0.0), S(0.0)};
   }
   limb_fill_deep<T, NT, R0>(typename LV::Next{}, w, 0, twx);
-  // |b[k]| + |b[M-k]| <= 2 sqrt(2) (|X[k]| + |X[M-k]|), and lf3's scale leaves a bit
+  // |b[k]| + |b[M-k]| <= 2 sqrt(2) (|X[k]| + |X[M-k]|), and the scale leaves a bit
   const LimbScale<T> sc = limb_scale(limb_block_sum<S, NT>(limb_sum<2 * NP>(x), red), 1);
 #pragma unroll
   for (int i = 0; i < NP; i++) {
@@ -654,86 +511,19 @@ __device__ __forceinline__ LimbScale<T> limb_c2r_first(Levels<R0, R...>, std::in
   return sc;
 }
 
-// Powers w[1] .. w[R-1] of w[1], products at most four deep.
-template <int R, typename T>
-__device__ __forceinline__ void limb_powers(C2<T>* w) {
-#pragma unroll
-  for (int q = 2; q < R; q++) w[q] = limb_tw<false, false>(w[q / 2], w[q - q / 2]);
-}
-
-// lf2: level 0 straight from the registers.  The inputs of item j, k = j + J q, have their
-// partners M - k = (J - j) + J (R0 - 1 - q) in item J - j, so one thread forms and transforms
-// both items: no trip of the input through shared memory.  (Items 0 and J / 2 are their own
-// partners: their threads' second item is theirs again, and not stored.)  Level 0's twiddles
-// W_M^(j q) as powers of one loaded value.
-template <typename S, typename T, int NT, int R0, int... R>
-__device__ __forceinline__ LimbScale<T> limb_c2r_first(Levels<R0, R...>, std::integral_constant<bool, true>,
-                                                       const C2<S>* __restrict__ a, const LimbTab<T>& twx,
-                                                       const LimbTab<T>& tab0, const LimbArr<T>& s,
-                                                       const LimbArr<T>& w, LimbSum<S>* red) {
-  using LV = Levels<R0, R...>;
-  constexpr int M = LV::M, J = M / R0;
-  static_assert(J % 2 == 0 && J / 2 < NT, "one pair of items per thread");
-  const int j = threadIdx.x;
-  const bool act = j <= J / 2;
-  C2<S> xa[R0], xb[R0];
-#pragma unroll
-  for (int q = 0; q < R0; q++) {
-    xa[q] = act ? ldc(a + (j + J * q)) : C2<S>{S(0.0), S(0.0)};
-    xb[q] = act ? ldc(a + (J * (q + 1) - j)) : C2<S>{S(0.0), S(0.0)};
-  }
-  limb_fill_deep<T, NT, R0>(typename LV::Next{}, w, 0, twx);
-  // |b[k]| + |b[M-k]| <= 2 sqrt(2) (|X[k]| + |X[M-k]|): two more bits
-  const LimbScale<T> sc =
-      limb_scale(limb_block_sum<S, NT>(limb_sum_add(limb_sum<R0>(xa), limb_sum<R0>(xb)), red), 2);
-  if (act) {
-    C2<T> u[R0], v[R0];
-#pragma unroll
-    for (int q = 0; q < R0; q++)
-      limb_c2r_pair(limb_cin(xa[q], sc), cconj(limb_cin(xb[R0 - 1 - q], sc)), twx.ld(j + J * q), u[q], v[R0 - 1 - q]);
-#pragma unroll
-    for (int side = 0; side < 2; side++) {
-      C2<T>* z = side ? v : u;
-      const int m = side ? J - j : j;
-      if (side && (j == 0 || j == J / 2)) continue;
-      Dft<T, R0, true>::run(z);
-      C2<T> p[R0];
-      p[1] = twx.ld(2L * m);
-      limb_powers<R0>(p);
-      const int at = LevelPlace<typename LV::Next>::of(m);
-      s.st(at, limb_cnorm(z[0]));
-#pragma unroll
-      for (int q = 1; q < R0; q++) s.st(at + q * LV::TN, limb_tw<true, true>(z[q], p[q]));
-    }
-  }
-  __syncthreads();
-  limb_levels<T, true, NT, 1, R0>(typename LV::Next{}, s, w, 0, tab0, [](int blk) { return blk * LV::TN; });
-  return sc;
-}
-
 template <typename S, typename T, typename TO, int NT, bool BAR, typename Put, typename LV>
 __device__ __forceinline__ void limb_c2r_row(LV, const C2<S>* __restrict__ a, const LimbTab<T>& twx,
                                              const LimbTab<T>& tab0, unsigned char* smem, LimbSum<S>* red, Put put) {
   const LimbArr<T> s = LimbArr<T>::at(smem, LV::T);
   const LimbArr<T> w = LimbArr<T>::at(smem + LimbArr<T>::bytes(LV::T), DeepTwiddles<typename LV::Next>::n);
-  const LimbScale<T> sc = limb_c2r_first<S, T, NT>(
-      LV{}, std::integral_constant<bool, sizeof(T) == sizeof(lf2)>{}, a, twx, tab0, s, w, red);
+  const LimbScale<T> sc = limb_c2r_first<S, T, NT>(LV{}, a, twx, tab0, s, w, red);
   limb_last_level<T, true, NT, BAR, C2<TO>>(
       LV{}, s, [&](C2<T> z) { return C2<TO>{limb_round(z.x, sc), limb_round(z.y, sc)}; }, put);
 }
 
-// CTAs per SM that the last pass's registers have to allow: lf2 rows of 2000 and 1000 points begin
-// with radix 4 in 64 registers and fill the SM with warps (2000^2: 31 -> 25 us, 4000^2 80 -> 76,
-// against first radices of 10 and 8 in 133 and 106 registers); 5000 points in 5 x 10 x 10 x 10
-// and 64 registers took 561 us against 492 at 10000^2.
-template <typename T, typename LV>
-constexpr int limb_row_ctas() {
-  return sizeof(T) == sizeof(lf3) ? 0 : LV::M == 2000 ? 4 : LV::M == 1000 ? 8 : 0;
-}
-
 // P3: one row per CTA, the pixels written from registers in thread order.
 template <typename S, typename T, typename TO, int NT, typename LV>
-__global__ void __launch_bounds__(NT, limb_row_ctas<T, LV>()) k_limb_rows_c2r(const C2<S>* __restrict__ in, long pitch, TO* __restrict__ out,
+__global__ void __launch_bounds__(NT) k_limb_rows_c2r(const C2<S>* __restrict__ in, long pitch, TO* __restrict__ out,
                                                       long ldo, LimbTab<T> twx, LimbTab<T> tab0) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ LimbSum<S> red[NT / 32];
@@ -745,7 +535,7 @@ __global__ void __launch_bounds__(NT, limb_row_ctas<T, LV>()) k_limb_rows_c2r(co
 // P3 of four profiles with the interleave fused in, the cluster form of k_rows_c2r3_il
 // (fft_impl.cuh): the row of pixels is left rounded to TO in each CTA's shared memory.
 template <typename S, typename T, typename TO, int NT, typename LV>
-__global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(NT, limb_row_ctas<T, LV>())
+__global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(NT)
     k_limb_rows_c2r_il(const C2<S>* __restrict__ specs, long spec_stride, long pitch, int nm, TO* __restrict__ out,
                        int S_, LimbTab<T> twx, LimbTab<T> tab0, unsigned planar) {
   constexpr int M = LV::M, NX = 2 * M;
@@ -832,7 +622,7 @@ __global__ void __launch_bounds__(NT)
   for (int k = tid; k <= M / 2; k += NT) {
     const C2<T> zk = s.ld(k), zc = cconj(s.ld(k == 0 ? 0 : M - k));
     const C2<T> a = cadd(zk, zc);
-    const C2<T> wd = limb_tw<false, false>(csub(zk, zc), twx.ld(k));
+    const C2<T> wd = limb_tw<false>(csub(zk, zc), twx.ld(k));
     o[k] = limb_cout<S>(C2<T>{a.x + wd.y, a.y - wd.x}, half);
     if (k != M - k) o[M - k] = limb_cout<S>(C2<T>{a.x - wd.y, -wd.x - a.y}, half);
   }
@@ -844,12 +634,6 @@ __global__ void __launch_bounds__(NT)
 template <typename T>
 struct LimbTraits;
 template <>
-struct LimbTraits<lf2> {
-  using S = ff;
-  using TO = float;
-  static LimbTab<lf2> tab(const FftPlan2D&, const void* t, const void*, int) { return {(const float4*)t}; }
-};
-template <>
 struct LimbTraits<lf3> {
   using S = double;
   using TO = double;
@@ -858,7 +642,6 @@ struct LimbTraits<lf3> {
     return {(const float4*)t3, (const float2*)((const char*)t3 + (size_t)N * 16)};
   }
 };
-// (two-limb plans keep their tables in the float-float layout)
 template <typename T>
 static LimbTab<T> limb_twx(const FftPlan2D& p) { return LimbTraits<T>::tab(p, p.twx, p.twx3, p.Nx); }
 template <typename T>
@@ -868,13 +651,9 @@ static LimbTab<T> limb_tab0(const FftPlan2D& p) {
 template <typename T>
 static LimbTab<T> limb_twy(const FftPlan2D& p) { return LimbTraits<T>::tab(p, p.twy, p.twy3, p.Ny); }
 
-// Columns per CTA for factors whose larger one is g.  lf2 passes are bound by HBM: 16 columns,
-// whole warps for every pair of factors.  lf3 passes are bound by the FP32 pipe and fetch long
-// unrolled code: wide CTAs, two per SM.
-template <typename T>
-constexpr int limb_cw(int g) {
-  return sizeof(T) == sizeof(lf2) || g == 16 ? 16 : 32;
-}
+// Columns per CTA for factors whose larger one is g.  The passes are bound by the FP32 pipe and
+// fetch long unrolled code: wide CTAs, two per SM.
+constexpr int limb_cw(int g) { return g == 16 ? 16 : 32; }
 
 // The same passes for other lengths (fft_limb_any.cu).
 template <bool INV>
@@ -897,18 +676,16 @@ bool limb_colpass_impl(mlc_ctx* ctx, const FftPlan2D& p, void* buf, char kind, i
   K k = nullptr;
   int g = 0;
   switch (L) {
-    case 100: k = k_limb_colpass2<S, T, limb_cw<T>(10), 10, 10, INV>; g = 10; break;
-    case 128: k = k_limb_colpass2<S, T, limb_cw<T>(16), 8, 16, INV>; g = 16; break;
-    case 64: k = k_limb_colpass2<S, T, limb_cw<T>(8), 8, 8, INV>; g = 8; break;
-    case 80: k = k_limb_colpass2<S, T, limb_cw<T>(10), 8, 10, INV>; g = 10; break;
-    case 50: k = k_limb_colpass2<S, T, limb_cw<T>(10), 5, 10, INV>; g = 10; break;
-    case 40: k = k_limb_colpass2<S, T, limb_cw<T>(8), 5, 8, INV>; g = 8; break;
+    case 100: k = k_limb_colpass2<S, T, limb_cw(10), 10, 10, INV>; g = 10; break;
+    case 128: k = k_limb_colpass2<S, T, limb_cw(16), 8, 16, INV>; g = 16; break;
+    case 64: k = k_limb_colpass2<S, T, limb_cw(8), 8, 8, INV>; g = 8; break;
+    case 80: k = k_limb_colpass2<S, T, limb_cw(10), 8, 10, INV>; g = 10; break;
+    case 50: k = k_limb_colpass2<S, T, limb_cw(10), 5, 10, INV>; g = 10; break;
+    case 40: k = k_limb_colpass2<S, T, limb_cw(8), 5, 8, INV>; g = 8; break;
     default:
-      // (lf2: the float-float kernel is as fast, 42 and 53 us at 2400^2)
-      if constexpr (sizeof(T) == sizeof(lf3)) return any_colpass_impl<INV>(ctx, p, buf, kind, post_tw);
-      return false;
+      return any_colpass_impl<INV>(ctx, p, buf, kind, post_tw);
   }
-  const int cw = limb_cw<T>(g);
+  const int cw = limb_cw(g);
   const size_t smem = LimbArr<T>::bytes(L * cw) + 2 * LimbArr<T>::bytes(L);
   set_max_smem((const void*)k, smem);
   {
@@ -934,16 +711,16 @@ bool limb3_conv_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, void* o
   K k = nullptr;
   int g = 0;
   switch (p.N2) {
-    case 100: k = k_limb3_conv<limb_cw<lf3>(10), 10, 10, MODE>; g = 10; break;
-    case 128: k = k_limb3_conv<limb_cw<lf3>(16), 8, 16, MODE>; g = 16; break;
+    case 100: k = k_limb3_conv<limb_cw(10), 10, 10, MODE>; g = 10; break;
+    case 128: k = k_limb3_conv<limb_cw(16), 8, 16, MODE>; g = 16; break;
     default: break;
   }
   if constexpr (MODE == 0) {
     switch (p.N2) {
-      case 64: k = k_limb3_conv<limb_cw<lf3>(8), 8, 8, MODE>; g = 8; break;
-      case 80: k = k_limb3_conv<limb_cw<lf3>(10), 8, 10, MODE>; g = 10; break;
-      case 50: k = k_limb3_conv<limb_cw<lf3>(10), 5, 10, MODE>; g = 10; break;
-      case 40: k = k_limb3_conv<limb_cw<lf3>(8), 5, 8, MODE>; g = 8; break;
+      case 64: k = k_limb3_conv<limb_cw(8), 8, 8, MODE>; g = 8; break;
+      case 80: k = k_limb3_conv<limb_cw(10), 8, 10, MODE>; g = 10; break;
+      case 50: k = k_limb3_conv<limb_cw(10), 5, 10, MODE>; g = 10; break;
+      case 40: k = k_limb3_conv<limb_cw(8), 5, 8, MODE>; g = 8; break;
       default: break;
     }
   }
@@ -966,7 +743,7 @@ bool limb3_conv_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, void* o
     any3_conv(ctx, p, Fmap, out, rows, h, r, -e);
     return true;
   }
-  const int cw = limb_cw<lf3>(g);
+  const int cw = limb_cw(g);
   const size_t smem = LimbArr<lf3>::bytes(p.N2 * cw) + 3 * LimbArr<lf3>::bytes(p.N2) + LimbArr<lf3>::bytes(p.N1);
   set_max_smem((const void*)k, smem);
   {
@@ -979,57 +756,16 @@ bool limb3_conv_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, void* o
   return true;
 }
 
-template <int MODE>
-bool limb2_conv_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, void* out, const void* kx, int h,
-                     const void* ks, const char* name) {
-  constexpr int CW = 16;
-  using K = void (*)(const C2<ff>*, C2<ff>*, long, const C2<ff>*, int, int, int, const C2<ff>*, ff, const C2<ff>*);
-  K k = nullptr;
-  int g = 0;
-  switch (p.N2) {
-    case 100: k = k_limb2_conv<CW, 10, 10, MODE>; g = 10; break;
-    case 128: k = k_limb2_conv<CW, 8, 16, MODE>; g = 16; break;
-    default: break;
-  }
-  if constexpr (MODE == 0) {
-    switch (p.N2) {
-      case 64: k = k_limb2_conv<CW, 8, 8, MODE>; g = 8; break;
-      case 80: k = k_limb2_conv<CW, 8, 10, MODE>; g = 10; break;
-      case 50: k = k_limb2_conv<CW, 5, 10, MODE>; g = 10; break;
-      case 40: k = k_limb2_conv<CW, 5, 8, MODE>; g = 8; break;
-      default: break;
-    }
-  }
-  if (!k) return false;
-  const size_t smem = ((size_t)p.N2 * CW + 2 * (size_t)p.N2 + p.N1) * sizeof(C2<ff>);
-  set_max_smem((const void*)k, smem);
-  {
-    MLC_KSCOPE(ctx, name);
-    k<<<dim3(ceil_div(p.Wc, CW), p.N1), g * CW, smem, ctx->stream>>>(
-        (const C2<ff>*)Fmap, (C2<ff>*)out, p.Wp, (const C2<ff>*)kx, h, p.Ny, p.N1, (const C2<ff>*)p.twy,
-        ff(1.0 / ((double)p.Nx * (double)p.Ny)), (const C2<ff>*)ks);
-  }
-  MLC_CHECK_LAUNCH();
-  return true;
-}
-
 // Row lengths with a limb kernel (limb_first_radix lists them too), their radices and threads:
-// f(levels, threads).  The last pass of lf2 needs a thread per pair of level-0 items.
-template <typename T, typename F>
+// f(levels, threads).
+template <typename F>
 static bool limb_row_dispatch(int M, F f) {
-  constexpr bool F64 = sizeof(T) == sizeof(lf3);
   using std::integral_constant;
   switch (M) {
-    case 5000: f(Levels<10, 10, 10, 5>{}, integral_constant<int, F64 ? 512 : 256>{}); return true;
-    case 4096: f(Levels<8, 8, 8, 8>{}, integral_constant<int, F64 ? 512 : 288>{}); return true;
-    case 2000:
-      if constexpr (F64) f(Levels<8, 10, 5, 5>{}, integral_constant<int, 256>{});
-      else f(Levels<4, 10, 10, 5>{}, integral_constant<int, 256>{});
-      return true;
-    case 1000:
-      if constexpr (F64) f(Levels<10, 10, 10>{}, integral_constant<int, 128>{});
-      else f(Levels<4, 10, 5, 5>{}, integral_constant<int, 128>{});
-      return true;
+    case 5000: f(Levels<10, 10, 10, 5>{}, integral_constant<int, 512>{}); return true;
+    case 4096: f(Levels<8, 8, 8, 8>{}, integral_constant<int, 512>{}); return true;
+    case 2000: f(Levels<8, 10, 5, 5>{}, integral_constant<int, 256>{}); return true;
+    case 1000: f(Levels<10, 10, 10>{}, integral_constant<int, 128>{}); return true;
     default: return false;
   }
 }
@@ -1038,7 +774,7 @@ template <typename T>
 bool limb_rows_c2r_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* in, void* out) {
   using S = typename LimbTraits<T>::S;
   using TO = typename LimbTraits<T>::TO;
-  const bool done = limb_row_dispatch<T>(p.M, [&](auto lv, auto nt) {
+  const bool done = limb_row_dispatch(p.M, [&](auto lv, auto nt) {
     using LV = decltype(lv);
     auto k = k_limb_rows_c2r<S, T, TO, decltype(nt)::value, LV>;
     const size_t smem = limb_row_smem<T, LV>();
@@ -1057,7 +793,7 @@ bool limb_rows_c2r_il_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* specs, 
                            void* out, unsigned planar) {
   using S = typename LimbTraits<T>::S;
   using TO = typename LimbTraits<T>::TO;
-  return limb_row_dispatch<T>(p.M, [&](auto lv, auto nt) {
+  return limb_row_dispatch(p.M, [&](auto lv, auto nt) {
     using LV = decltype(lv);
     auto k = k_limb_rows_c2r_il<S, T, TO, decltype(nt)::value, LV>;
     const size_t smem = limb_row_smem<T, LV>();
@@ -1074,7 +810,7 @@ bool limb_rows_c2r_il_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* specs, 
 template <typename T, typename Loader>
 bool limb_rows_r2c_impl(mlc_ctx* ctx, const FftPlan2D& p, const Loader& ld, int nrows, void* out, const char* name) {
   using S = typename LimbTraits<T>::S;
-  const bool done = limb_row_dispatch<T>(p.M, [&](auto lv, auto nt) {
+  const bool done = limb_row_dispatch(p.M, [&](auto lv, auto nt) {
     using LV = decltype(lv);
     auto k = k_limb_rows_r2c<S, T, decltype(nt)::value, LV, Loader>;
     const size_t smem = limb_row_smem<T, LV>();

@@ -27,14 +27,14 @@ __device__ __forceinline__ void any_level(const LimbArr<T>& s, const AnyLevels& 
       u[0] = limb_cnorm(u[0]);
       if (!last) {
 #pragma unroll
-        for (int q = 1; q < R; q++) u[q] = limb_tw<INV, true>(u[q], tw((q - 1) * bn + m));
+        for (int q = 1; q < R; q++) u[q] = limb_tw<INV>(u[q], tw((q - 1) * bn + m));
       }
     }
     Dft<T, R, INV>::run(u);
     if (!DIT && !last) {
       s.st(p, limb_cnorm(u[0]));
 #pragma unroll
-      for (int q = 1; q < R; q++) s.st(p + q * tn, limb_tw<INV, true>(u[q], tw((q - 1) * bn + m)));
+      for (int q = 1; q < R; q++) s.st(p + q * tn, limb_tw<INV>(u[q], tw((q - 1) * bn + m)));
     } else {
 #pragma unroll
       for (int q = 0; q < R; q++) s.st(p + q * tn, u[q]);
@@ -76,8 +76,6 @@ __device__ __forceinline__ LimbSum<S> any_block_sum(LimbSum<S> v, LimbSum<S>* re
 }
 template <typename S>
 __device__ __forceinline__ LimbSum<S> limb_sum_zero();
-template <>
-__device__ __forceinline__ LimbSum<ff> limb_sum_zero() { return LimbSum<ff>{0.f}; }
 template <>
 __device__ __forceinline__ LimbSum<double> limb_sum_zero() { return LimbSum<double>{0, 0.f}; }
 
@@ -123,8 +121,8 @@ __global__ void __launch_bounds__(512)
     }
   }
   any_fill_deep(w, lv, tab);
-  // |b[k]| + |b[M-k]| <= 2 sqrt(2) (|X[k]| + |X[M-k]|); lf3's scale leaves one of the two bits
-  const LimbScale<T> sc = limb_scale(any_block_sum(sum, red), sizeof(T) == sizeof(lf3) ? 1 : 2);
+  // |b[k]| + |b[M-k]| <= 2 sqrt(2) (|X[k]| + |X[M-k]|), and the scale leaves a bit
+  const LimbScale<T> sc = limb_scale(any_block_sum(sum, red), 1);
   for (int k = tid; k <= M / 2; k += NT) {
     C2<T> bk, bm;
     const int pk = any_inner(lv, 0, k), pm = k > 0 ? any_inner(lv, 0, M - k) : 0;
@@ -177,7 +175,7 @@ __global__ void __launch_bounds__(512)
   for (int k = tid; k <= M / 2; k += NT) {
     const C2<T> zk = s.ld(any_output(lv, k)), zc = cconj(s.ld(k == 0 ? any_output(lv, 0) : any_output(lv, M - k)));
     const C2<T> a = cadd(zk, zc);
-    const C2<T> wd = limb_tw<false, false>(csub(zk, zc), twx.ld(k));
+    const C2<T> wd = limb_tw<false>(csub(zk, zc), twx.ld(k));
     o[k] = limb_cout<S>(C2<T>{a.x + wd.y, a.y - wd.x}, half);
     if (k != M - k) o[M - k] = limb_cout<S>(C2<T>{a.x - wd.y, -wd.x - a.y}, half);
   }
@@ -200,7 +198,7 @@ __device__ __forceinline__ LimbSum<S> any_column_sum(LimbSum<S> v, LimbSum<S> (*
 }
 
 template <typename S, typename T, bool INV>
-__global__ void __launch_bounds__(ANY_NT, sizeof(T) == sizeof(lf3) ? 2 : 3)
+__global__ void __launch_bounds__(ANY_NT, 2)
     k_any_colpass(C2<S>* __restrict__ buf, long pitch, long set_mul, long j_mul, LimbTab<T> twy, int post_tw,
                   const __grid_constant__ AnyLevels lv, LimbTab<T> tab) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -231,7 +229,7 @@ __global__ void __launch_bounds__(ANY_NT, sizeof(T) == sizeof(lf3) ? 2 : 3)
   any_transform<T, INV, false, false, ANY_CW>(s, lv, tab, w);
   for (int j = g; j < L; j += G) {
     C2<T> v = s.ld(any_output(lv, j) * ANY_CW + c);
-    if (post_tw) v = limb_tw<INV, false>(v, twy.ld((long)set * j));  // set*j < Ny
+    if (post_tw) v = limb_tw<INV>(v, twy.ld((long)set * j));  // set*j < Ny
     b[(long)j * j_mul * pitch] = limb_cout<S>(v, sc);
   }
 }
@@ -266,19 +264,19 @@ __global__ void __launch_bounds__(ANY_NT, 2)
     C2<T> acc = n2 < h ? kx.ld((long)n2 * pitch + col) : limb_zero<T>();  // weight W^0 = 1
 #pragma unroll 1
     for (int n1 = 1; n1 * N2 + n2 < h; n1++)
-      acc = cadd(acc, limb_tw<false, true>(kx.ld((long)(n1 * N2 + n2) * pitch + col), twy.ld((long)((n1 * kk) % N1) * N2)));
+      acc = cadd(acc, limb_tw<false>(kx.ld((long)(n1 * N2 + n2) * pitch + col), twy.ld((long)((n1 * kk) % N1) * N2)));
 #pragma unroll 1
     for (int n1 = max((Ny - h - n2 + N2 - 1) / N2, 0); n1 < N1; n1++)
-      acc = cadd(acc, limb_tw<false, true>(kx.ld((n1 * N2 + n2 - (Ny - 2L * h)) * pitch + col),
+      acc = cadd(acc, limb_tw<false>(kx.ld((n1 * N2 + n2 - (Ny - 2L * h)) * pitch + col),
                                            twy.ld((long)((n1 * kk) % N1) * N2)));
     const C2<T> t = twy.ld((long)n2 * kk);
-    s.st(n2 * ANY_CW + c, limb_tw<false, true>(acc, limb_cnorm(C2<T>{r * t.x, r * t.y})));
+    s.st(n2 * ANY_CW + c, limb_tw<false>(acc, limb_cnorm(C2<T>{r * t.x, r * t.y})));
   }
   const LimbScale<T> sf = limb_scale(any_column_sum(sum, red), 0);  // (its barrier also ends the writes of s and w)
   any_transform<T, false, false, false, ANY_CW>(s, lv, tab, w);
   for (int k2 = g; k2 < N2; k2 += G) {
     const int p = any_output(lv, k2) * ANY_CW + c;
-    s.st(p, limb_tw<false, true>(limb_cin(ldc(f + (long)k2 * pitch), sf), limb_cnorm(s.ld(p))));
+    s.st(p, limb_tw<false>(limb_cin(ldc(f + (long)k2 * pitch), sf), limb_cnorm(s.ld(p))));
   }
   __syncthreads();
   any_transform<T, true, true, false, ANY_CW>(s, lv, tab, w);
@@ -287,7 +285,7 @@ __global__ void __launch_bounds__(ANY_NT, 2)
   sc.e += sc.bad ? 0 : ke;
   for (int n2 = g; n2 < N2; n2 += G)
     out[((long)kk * N2 + n2) * pitch + col] =
-        limb_cout<double>(limb_tw<true, true>(s.ld(n2 * ANY_CW + c), twy.ld((long)n2 * kk)), sc);
+        limb_cout<double>(limb_tw<true>(s.ld(n2 * ANY_CW + c), twy.ld((long)n2 * kk)), sc);
 }
 
 // ---------------------------------------------------------------- launches
@@ -299,7 +297,7 @@ static LimbTab<T> any_tab(const FftPlan2D& p, const AnyLevels& lv, const void* t
 
 template <typename T>
 static int any_limb_row_threads(mlc_ctx* ctx, const AnyLevels& lv, size_t smem, int nrows) {
-  return any_row_threads(ctx, lv, smem, nrows, sizeof(T) == sizeof(lf3) ? 512 : 1024);
+  return any_row_threads(ctx, lv, smem, nrows, 512);
 }
 
 template <typename T>
@@ -309,9 +307,6 @@ bool any_rows_c2r_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* in, void* o
   const AnyLevels& lv = p.anyM;
   const size_t smem = any_row_smem<T>(lv);
   if (lv.n < 1 || smem > ANY_SMEM) return false;
-  // lf2: four rows or fewer per SM take the float-float loop's short code (ten last passes of 540^2
-  // 161 us against 168, six of 810^2 150 against 113)
-  if (sizeof(T) == sizeof(lf2) && p.Ny <= 4 * ctx->sm_count) return false;
   auto k = k_any_rows_c2r<S, T, TO>;
   set_max_smem((const void*)k, smem);
   {
@@ -384,7 +379,6 @@ void any3_conv(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, void* out, co
 template bool any_colpass_impl<false>(mlc_ctx*, const FftPlan2D&, void*, char, int);
 template bool any_colpass_impl<true>(mlc_ctx*, const FftPlan2D&, void*, char, int);
 template bool any_rows_c2r_impl<lf3>(mlc_ctx*, const FftPlan2D&, const void*, void*);
-template bool any_rows_c2r_impl<lf2>(mlc_ctx*, const FftPlan2D&, const void*, void*);
 template bool any_rows_r2c_impl<lf3, RealRows<double, double>>(mlc_ctx*, const FftPlan2D&,
                                                                const RealRows<double, double>&, int, void*, const char*);
 template bool any_rows_r2c_impl<lf3, RealRows<double, float>>(mlc_ctx*, const FftPlan2D&,

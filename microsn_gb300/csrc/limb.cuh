@@ -1,22 +1,18 @@
-// Fixed-grid sums of two or three FP32 numbers ("limbs") for the transforms.
+// Fixed-grid sums of three FP32 numbers ("limbs") for FP64 transforms.
 //
 // GB300 issues FP32 about sixty times faster than FP64 (measured: 39 against 0.63 T
-// operations/s), and a Fourier transform is mostly additions.  A float-float sum needs the
-// two-sum (8 FP32 operations) because its parts float: where the exponents of the operands
-// are not known, the rounding error of the high parts has to be recovered.  Here every value
-// of one transform is first scaled by one power of two so that |x| < 1, and its high limb
-// is a multiple of one fixed grid, 2^-22.  High limbs then add exactly in a single FP32
-// addition, and a sum costs one addition per limb:
-//
-//   lf2  h (multiple of 2^-22) + l                          two limbs, about 46 bits
-//   lf3  h (multiple of 2^-22) + m (multiple of 2^-39) + l   three limbs, about 62 bits
+// operations/s), and a Fourier transform is mostly additions.  A sum of floating parts needs
+// two-sums (8 FP32 operations each), because the rounding error of the high parts has to be
+// recovered where the exponents of the operands are not known.  Here every value of one
+// transform is first scaled by one power of two so that |x| < 1, and its high limbs are
+// multiples of fixed grids: h of 2^-22, m of 2^-39, and l the rest, about 62 bits.  High limbs
+// then add exactly in a single FP32 addition, and a sum costs one addition per limb.
 //
 // Why |x| < 1 holds throughout a transform: the scale comes from S, the sum of |re| + |im|
 // over all of its inputs, and every intermediate value of an FFT is a sum of distinct inputs
 // times factors of modulus one, so its modulus is at most S -- whatever the inputs.  The
-// absolute error of an operation is about 2^-46 S (lf2) or 2^-62 S (lf3); against the
-// rms of the values that is about 2^-40 and 2^-56 in the passes here, so lf2 results
-// rounded to FP32 and lf3 results rounded to FP64 carry the rounding of the last step.
+// absolute error of an operation is about 2^-62 S.  (Two limbs, 46 bits, in place of
+// float-float lost the faint pixels of FP32 maps: 2^-30 of the map's rms at 10000^2.)
 //
 // Products return to the grid with the additive constant 3 = 1.5 * 2: t = 3 + x c is
 // rounded to 2^-22 (t lies in [2, 4)), t - 3 is the high limb, and fma(x, c, -(t - 3)) is the
@@ -31,13 +27,6 @@ namespace mlc {
 constexpr float LIMB_G1 = 3.0f;         // 1.5 * 2: rounds to multiples of 2^-22
 constexpr float LIMB_G2 = 0x1.8p-16f;   // rounds to multiples of 2^-39
 constexpr float LIMB_G3 = 0x1.8p-39f;   // rounds to multiples of 2^-62
-
-struct lf2 {
-  float h, l;
-  lf2() = default;
-  __host__ __device__ constexpr lf2(float h_, float l_) : h(h_), l(l_) {}
-  __host__ __device__ constexpr lf2(double d) : h((float)d), l((float)(d - (double)(float)d)) {}
-};
 
 // A constant's high limb is cut to multiples of 2^-24, so that its product with a value's
 // high limb leaves an exact remainder.
@@ -60,55 +49,6 @@ struct C2<lf3> {
   lf3 x, y;
 };
 
-template <typename T>
-struct is_limb {
-  static constexpr bool value = false;
-};
-template <>
-struct is_limb<lf2> {
-  static constexpr bool value = true;
-};
-template <>
-struct is_limb<lf3> {
-  static constexpr bool value = true;
-};
-
-// ---------------------------------------------------------------- lf2
-
-__device__ __forceinline__ lf2 operator+(lf2 a, lf2 b) { return lf2(__fadd_rn(a.h, b.h), __fadd_rn(a.l, b.l)); }
-__device__ __forceinline__ lf2 operator-(lf2 a, lf2 b) { return lf2(__fsub_rn(a.h, b.h), __fsub_rn(a.l, b.l)); }
-__device__ __forceinline__ lf2 operator-(lf2 a) { return lf2(-a.h, -a.l); }
-__device__ __forceinline__ lf2 operator*(lf2 a, lf2 b) {
-  const float h = __fsub_rn(__fmaf_rn(a.h, b.h, LIMB_G1), LIMB_G1);
-  float e = __fmaf_rn(a.h, b.h, -h);
-  e = __fmaf_rn(a.h, b.l, e);
-  return lf2(h, __fmaf_rn(a.l, b.h, e));
-}
-__device__ __forceinline__ lf2 scale2(lf2 a, float s) {
-  const float h = __fsub_rn(__fmaf_rn(a.h, s, LIMB_G1), LIMB_G1);
-  return lf2(h, __fmaf_rn(a.l, s, __fmaf_rn(a.h, s, -h)));
-}
-// c x + d y with one trip over the grid (12 operations).  NORM carries what has gathered in
-// the low limb back into the high one (3 more).
-template <bool NORM>
-__device__ __forceinline__ lf2 limb_lin2(lf2 c, lf2 x, lf2 d, lf2 y) {
-  const float t1 = __fmaf_rn(c.h, x.h, LIMB_G1), t2 = __fmaf_rn(d.h, y.h, t1);
-  float e = __fmaf_rn(c.h, x.h, -__fsub_rn(t1, LIMB_G1));
-  float f = __fmaf_rn(d.h, y.h, -__fsub_rn(t2, t1));
-  e = __fmaf_rn(c.l, x.h, e);
-  f = __fmaf_rn(d.l, y.h, f);
-  e = __fmaf_rn(c.h, x.l, e);
-  f = __fmaf_rn(d.h, y.l, f);
-  e = __fadd_rn(e, f);
-  if (!NORM) return lf2(__fsub_rn(t2, LIMB_G1), e);
-  const float t3 = __fadd_rn(t2, e);
-  return lf2(__fsub_rn(t3, LIMB_G1), __fsub_rn(e, __fsub_rn(t3, t2)));
-}
-__device__ __forceinline__ lf2 limb_norm(lf2 a) {
-  const float q = __fsub_rn(__fadd_rn(a.l, LIMB_G1), LIMB_G1);
-  return lf2(__fadd_rn(a.h, q), __fsub_rn(a.l, q));
-}
-
 // ---------------------------------------------------------------- lf3
 
 __device__ __forceinline__ lf3 operator+(lf3 a, lf3 b) {
@@ -129,13 +69,6 @@ __device__ __forceinline__ lf3 operator*(lf3 a, lf3 b) {
   f = __fmaf_rn(a.l, b.h, f);
   e = __fmaf_rn(a.m, b.m, e);
   return lf3(h, __fsub_rn(u2, LIMB_G2), __fadd_rn(e, f));
-}
-// s a power of two, at least 2^-16: the remainder of the high limb is on the second grid.
-__device__ __forceinline__ lf3 scale2(lf3 a, float s) {
-  const float h = __fsub_rn(__fmaf_rn(a.h, s, LIMB_G1), LIMB_G1);
-  const float r = __fmaf_rn(a.h, s, -h);
-  const float p = __fsub_rn(__fmaf_rn(a.m, s, LIMB_G2), LIMB_G2);
-  return lf3(h, __fadd_rn(r, p), __fmaf_rn(a.l, s, __fmaf_rn(a.m, s, -p)));
 }
 // c x + d y (34 operations).  NORM carries the lower limbs' excess upwards (6 more): between
 // two carries a limb may gather up to 2^7 of its own grid steps, the exact range of an FP32
@@ -163,13 +96,6 @@ __device__ __forceinline__ lf3 limb_lin2(lf3 c, lf3 x, lf3 d, lf3 y) {
   const float m = __fsub_rn(u5, LIMB_G2), t3 = __fadd_rn(t2, m);
   return lf3(__fsub_rn(t3, LIMB_G1), __fsub_rn(m, __fsub_rn(t3, t2)), __fsub_rn(e, __fsub_rn(u5, u4)));
 }
-__device__ __forceinline__ lf3 limb_norm(lf3 a) {
-  const float q = __fsub_rn(__fadd_rn(a.l, LIMB_G2), LIMB_G2);
-  const float m = __fadd_rn(a.m, q);
-  const float p = __fsub_rn(__fadd_rn(m, LIMB_G1), LIMB_G1);
-  return lf3(__fadd_rn(a.h, p), __fsub_rn(m, p), __fsub_rn(a.l, q));
-}
-
 // ---------------------------------------------------------------- complex products
 
 // a x + b y of the small DFTs' constants: the limb forms make one trip over the grid.
@@ -177,7 +103,6 @@ template <typename T>
 __device__ __forceinline__ T lin2(T a, T x, T b, T y) {
   return a * x + b * y;
 }
-__device__ __forceinline__ lf2 lin2(lf2 a, lf2 x, lf2 b, lf2 y) { return limb_lin2<false>(a, x, b, y); }
 __device__ __forceinline__ lf3 lin2(lf3 a, lf3 x, lf3 b, lf3 y) { return limb_lin2<false>(a, x, b, y); }
 
 // Complex forms on both components.
@@ -231,17 +156,6 @@ __device__ __forceinline__ f32p pfma(f32p a, f32p b, f32p c) {
 template <typename T>
 struct Packed;
 template <>
-struct Packed<lf2> {
-  f32p h, l;
-  static __device__ __forceinline__ Packed of(lf2 x, lf2 y) { return Packed{pk(x.h, y.h), pk(x.l, y.l)}; }
-  __device__ __forceinline__ C2<lf2> c() const {
-    C2<lf2> r;
-    unpk(h, r.x.h, r.y.h);
-    unpk(l, r.x.l, r.y.l);
-    return r;
-  }
-};
-template <>
 struct Packed<lf3> {
   f32p h, m, l;
   static __device__ __forceinline__ Packed of(lf3 x, lf3 y) {
@@ -266,19 +180,10 @@ struct Packed<ff> {
     return r;
   }
 };
-using P2 = Packed<lf2>;
 using P3 = Packed<lf3>;
 template <typename T>
 __device__ __forceinline__ Packed<T> pc(C2<T> a) { return Packed<T>::of(a.x, a.y); }
 
-__device__ __forceinline__ C2<lf2> cadd(C2<lf2> a, C2<lf2> b) {
-  const P2 x = pc(a), y = pc(b);
-  return P2{x.h + y.h, x.l + y.l}.c();
-}
-__device__ __forceinline__ C2<lf2> csub(C2<lf2> a, C2<lf2> b) {
-  const P2 x = pc(a), y = pc(b);
-  return P2{x.h - y.h, x.l - y.l}.c();
-}
 __device__ __forceinline__ C2<lf3> cadd(C2<lf3> a, C2<lf3> b) {
   const P3 x = pc(a), y = pc(b);
   return P3{x.h + y.h, x.m + y.m, x.l + y.l}.c();
@@ -288,12 +193,6 @@ __device__ __forceinline__ C2<lf3> csub(C2<lf3> a, C2<lf3> b) {
   return P3{x.h - y.h, x.m - y.m, x.l - y.l}.c();
 }
 // (the operations of the scalar forms above, one for one; -(t - G) as G - t)
-__device__ __forceinline__ P2 pmul(P2 a, P2 b) {
-  const f32p G = pk(LIMB_G1), t = pfma(a.h, b.h, G);
-  f32p e = pfma(a.h, b.h, G - t);
-  e = pfma(a.h, b.l, e);
-  return P2{t - G, pfma(a.l, b.h, e)};
-}
 __device__ __forceinline__ P3 pmul(P3 a, P3 b) {
   const f32p G1 = pk(LIMB_G1), G2 = pk(LIMB_G2), t = pfma(a.h, b.h, G1);
   const f32p r = pfma(a.h, b.h, G1 - t);
@@ -305,16 +204,6 @@ __device__ __forceinline__ P3 pmul(P3 a, P3 b) {
   f = pfma(a.l, b.h, f);
   e = pfma(a.m, b.m, e);
   return P3{t - G1, u2 - G2, e + f};
-}
-__device__ __forceinline__ P2 plin2(P2 c, P2 x, P2 d, P2 y) {
-  const f32p G = pk(LIMB_G1), t1 = pfma(c.h, x.h, G), t2 = pfma(d.h, y.h, t1);
-  f32p e = pfma(c.h, x.h, G - t1);
-  f32p f = pfma(d.h, y.h, t1 - t2);
-  e = pfma(c.l, x.h, e);
-  f = pfma(d.l, y.h, f);
-  e = pfma(c.h, x.l, e);
-  f = pfma(d.h, y.l, f);
-  return P2{t2 - G, e + f};
 }
 __device__ __forceinline__ P3 plin2(P3 c, P3 x, P3 d, P3 y) {
   const f32p G1 = pk(LIMB_G1), G2 = pk(LIMB_G2);
@@ -335,19 +224,11 @@ __device__ __forceinline__ P3 plin2(P3 c, P3 x, P3 d, P3 y) {
   f = pfma(d.h, y.l, f);
   return P3{t2 - G1, u4 - G2, e + f};
 }
-__device__ __forceinline__ C2<lf2> crmul(lf2 c, C2<lf2> a) { return pmul(P2::of(c, c), pc(a)).c(); }
 __device__ __forceinline__ C2<lf3> crmul(lf3 c, C2<lf3> a) { return pmul(P3::of(c, c), pc(a)).c(); }
-__device__ __forceinline__ C2<lf2> clin2(lf2 a, C2<lf2> x, lf2 b, C2<lf2> y) {
-  return plin2(P2::of(a, a), pc(x), P2::of(b, b), pc(y)).c();
-}
 __device__ __forceinline__ C2<lf3> clin2(lf3 a, C2<lf3> x, lf3 b, C2<lf3> y) {
   return plin2(P3::of(a, a), pc(x), P3::of(b, b), pc(y)).c();
 }
-__device__ __forceinline__ C2<lf2> cscale2(C2<lf2> a, float s) {
-  const P2 x = pc(a);
-  const f32p G = pk(LIMB_G1), S = pk(s), t = pfma(x.h, S, G);
-  return P2{t - G, pfma(x.l, S, pfma(x.h, S, G - t))}.c();
-}
+// s a power of two, at least 2^-16: the remainder of the high limb is on the second grid.
 __device__ __forceinline__ C2<lf3> cscale2(C2<lf3> a, float s) {
   const P3 x = pc(a);
   const f32p G1 = pk(LIMB_G1), G2 = pk(LIMB_G2), S = pk(s), t = pfma(x.h, S, G1), u = pfma(x.m, S, G2);
@@ -370,35 +251,24 @@ __device__ __forceinline__ C2<ff> csub(C2<ff> a, C2<ff> b) {
 }
 __device__ __forceinline__ C2<ff> clin2(ff a, C2<ff> x, ff b, C2<ff> y) { return cadd(crmul(a, x), crmul(b, y)); }
 
-// v w or v conj(w) with the carry of limb_lin2 where NORM (lf3: always).
-template <bool CONJ, bool NORM, typename T>
+// v w or v conj(w); every product carries.
+template <bool CONJ, typename T>
 __device__ __forceinline__ C2<T> limb_tw(C2<T> v, C2<T> w) {
-  constexpr bool N = NORM || sizeof(T) == sizeof(lf3);
-  if (CONJ) return C2<T>{limb_lin2<N>(w.x, v.x, w.y, v.y), limb_lin2<N>(w.x, v.y, -w.y, v.x)};
-  return C2<T>{limb_lin2<N>(w.x, v.x, -w.y, v.y), limb_lin2<N>(w.x, v.y, w.y, v.x)};
+  if (CONJ) return C2<T>{limb_lin2<true>(w.x, v.x, w.y, v.y), limb_lin2<true>(w.x, v.y, -w.y, v.x)};
+  return C2<T>{limb_lin2<true>(w.x, v.x, -w.y, v.y), limb_lin2<true>(w.x, v.y, w.y, v.x)};
 }
-template <typename T>
-__device__ __forceinline__ C2<T> limb_cnorm(C2<T> v) {
-  const Packed<T> a = pc(v);
-  if constexpr (sizeof(T) == sizeof(lf2)) {
-    const f32p G = pk(LIMB_G1), q = (a.l + G) - G;
-    return Packed<T>{a.h + q, a.l - q}.c();
-  } else {
-    const f32p G1 = pk(LIMB_G1), G2 = pk(LIMB_G2), q = (a.l + G2) - G2, m = a.m + q, p = (m + G1) - G1;
-    return Packed<T>{a.h + p, m - p, a.l - q}.c();
-  }
+__device__ __forceinline__ C2<lf3> limb_cnorm(C2<lf3> v) {
+  const P3 a = pc(v);
+  const f32p G1 = pk(LIMB_G1), G2 = pk(LIMB_G2), q = (a.l + G2) - G2, m = a.m + q, p = (m + G1) - G1;
+  return P3{a.h + p, m - p, a.l - q}.c();
 }
 
 // ---------------------------------------------------------------- scale of one transform
 
-// Partial sum of |re| + |im| over the inputs of one transform.  FP64: s 2^(e - 1023) with
-// the exponent field e kept apart (in place, bits 20..30), s from the high words alone.
+// Partial sum of |re| + |im| over the inputs of one transform: s 2^(e - 1023) with the exponent
+// field e kept apart (in place, bits 20..30), s from the high words alone.
 template <typename S>
 struct LimbSum;
-template <>
-struct LimbSum<ff> {
-  float s;
-};
 template <>
 struct LimbSum<double> {
   int e;
@@ -408,13 +278,6 @@ struct LimbSum<double> {
 // 2^(a - b) for exponent fields a <= b in place (bits 20..30); 0 where it underflows FP32.
 __device__ __forceinline__ float limb_pow_diff(int a, int b) {
   return __int_as_float(max(a - b + (127 << 20), 0) << 3);
-}
-template <int N>
-__device__ __forceinline__ LimbSum<ff> limb_sum(const C2<ff>* v) {
-  float s = 0.f;
-#pragma unroll
-  for (int i = 0; i < N; i++) s = __fadd_rn(s, __fadd_rn(fabsf(v[i].x.hi), fabsf(v[i].y.hi)));
-  return LimbSum<ff>{s};
 }
 template <int N>
 __device__ __forceinline__ LimbSum<double> limb_sum(const C2<double>* v) {
@@ -431,17 +294,9 @@ __device__ __forceinline__ LimbSum<double> limb_sum(const C2<double>* v) {
   }
   return LimbSum<double>{e, s};
 }
-__device__ __forceinline__ LimbSum<ff> limb_sum_add(LimbSum<ff> a, LimbSum<ff> b) {
-  return LimbSum<ff>{__fadd_rn(a.s, b.s)};
-}
 __device__ __forceinline__ LimbSum<double> limb_sum_add(LimbSum<double> a, LimbSum<double> b) {
   const int e = max(a.e, b.e);
   return LimbSum<double>{e, __fmaf_rn(a.s, limb_pow_diff(a.e, e), __fmul_rn(b.s, limb_pow_diff(b.e, e)))};
-}
-__device__ __forceinline__ LimbSum<ff> limb_sum_warp(LimbSum<ff> a) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) a.s = __fadd_rn(a.s, __shfl_xor_sync(0xffffffffu, a.s, o));
-  return a;
 }
 __device__ __forceinline__ LimbSum<double> limb_sum_warp(LimbSum<double> a) {
   const int e = __reduce_max_sync(0xffffffffu, a.e);
@@ -452,28 +307,18 @@ __device__ __forceinline__ LimbSum<double> limb_sum_warp(LimbSum<double> a) {
   return a;
 }
 
-// The power of two that brings a transform below 1/2 and back.  lf2: two FP32 factors;
-// lf3: the exponent fields to add to a double before its conversion to a 62-bit fixed-point
-// integer and after the way back.  A sum that is not finite makes every output NaN.
+// The power of two that brings a transform below 1/2 and back: the exponent fields to add to a
+// double before its conversion to a 62-bit fixed-point integer and after the way back.  A sum
+// that is not finite makes every output NaN.
 template <typename T>
 struct LimbScale;
-template <>
-struct LimbScale<lf2> {
-  float down, up;
-};
 template <>
 struct LimbScale<lf3> {
   int e;  // x < 2^(e - 1)
   bool bad;
 };
-// extra: the transform's values may grow to 2^extra times the sum.  lf2 takes the least power of
-// two above the sum; lf3 one more, as limb_out needs |x| < 1 and the sum is cut to high words.
-__device__ __forceinline__ LimbScale<lf2> limb_scale(LimbSum<ff> a, int extra) {
-  const int b = __float_as_int(a.s) >> 23;  // (a.s >= 0, so no sign bit)
-  if (b >= 255) return LimbScale<lf2>{__int_as_float(0x7fffffff), __int_as_float(0x7fffffff)};
-  const int e = min(max(b - 127 + 1 + extra, -100), 126);
-  return LimbScale<lf2>{__int_as_float((127 - e) << 23), __int_as_float((127 + e) << 23)};
-}
+// extra: the transform's values may grow to 2^extra times the sum.  One more than the least
+// power of two above the sum, as limb_out needs |x| < 1 and the sum is cut to high words.
 // (values below 2^-1022 of a transform whose sum is below 2^-960 count as zero)
 __device__ __forceinline__ LimbScale<lf3> limb_scale(LimbSum<double> a, int extra) {
   const int e = (a.e >> 20) - 1023 + ((__float_as_int(a.s) >> 23) - 127) + 2 + extra;
@@ -481,16 +326,6 @@ __device__ __forceinline__ LimbScale<lf3> limb_scale(LimbSum<double> a, int extr
 }
 
 // ---------------------------------------------------------------- in and out
-
-__device__ __forceinline__ lf2 limb_in(ff v, LimbScale<lf2> s) {
-  const float hi = __fmul_rn(v.hi, s.down);
-  const float h = __fsub_rn(__fadd_rn(hi, LIMB_G1), LIMB_G1);
-  return lf2(h, __fmaf_rn(v.lo, s.down, __fsub_rn(hi, h)));
-}
-__device__ __forceinline__ ff limb_out(lf2 v, LimbScale<lf2> s) {
-  return ff(__fmul_rn(v.h, s.up), __fmul_rn(v.l, s.up));
-}
-__device__ __forceinline__ float limb_round(lf2 v, LimbScale<lf2> s) { return __fmul_rn(__fadd_rn(v.h, v.l), s.up); }
 
 // FP64 in: the exponent moved by an integer addition, one conversion to a fixed-point
 // integer of 62 fractional bits, and its bit fields 22 | 17 | 23 as the three limbs.
@@ -533,22 +368,10 @@ __device__ __forceinline__ C2<S> limb_cout(C2<T> v, LimbScale<T> s) {
 
 // ---------------------------------------------------------------- arrays of limbs
 
-// Complex limbs in shared memory: lf2 as one 16-byte word, lf3 as 16 bytes (high and middle
-// limbs) and 8 bytes (low limbs) in two planes, so that every access is one aligned vector.
+// Complex limbs in shared memory: 16 bytes (high and middle limbs) and 8 bytes (low limbs) in
+// two planes, so that every access is one aligned vector.
 template <typename T>
-struct LimbArr {
-  C2<T>* p;
-  static __host__ __device__ constexpr size_t bytes(long n) { return (size_t)n * sizeof(C2<T>); }
-  static __device__ __forceinline__ LimbArr at(unsigned char* raw, long) { return LimbArr{reinterpret_cast<C2<T>*>(raw)}; }
-  // (as (h, h, l, l): the register pairs of the packed operations)
-  __device__ __forceinline__ C2<T> ld(int i) const {
-    const float4 u = reinterpret_cast<const float4*>(p)[i];
-    return C2<T>{T(u.x, u.z), T(u.y, u.w)};
-  }
-  __device__ __forceinline__ void st(int i, C2<T> v) const {
-    reinterpret_cast<float4*>(p)[i] = make_float4(v.x.h, v.y.h, v.x.l, v.y.l);
-  }
-};
+struct LimbArr;
 template <>
 struct LimbArr<lf3> {
   float4* a;
@@ -568,25 +391,9 @@ struct LimbArr<lf3> {
   }
 };
 
-// Twiddle tables in global memory: the float-float table for ff and lf2, two planes for lf3.
+// Twiddle tables in global memory: two planes likewise.
 template <typename T>
 struct LimbTab;
-template <>
-struct LimbTab<ff> {
-  const float4* p;
-  __device__ __forceinline__ C2<ff> ld(long i) const {
-    const float4 v = __ldg(p + i);
-    return C2<ff>{ff(v.x, v.y), ff(v.z, v.w)};
-  }
-};
-template <>
-struct LimbTab<lf2> {
-  const float4* p;
-  __device__ __forceinline__ C2<lf2> ld(long i) const {
-    const float4 v = __ldg(p + i);
-    return C2<lf2>{lf2(v.x, v.y), lf2(v.z, v.w)};
-  }
-};
 template <>
 struct LimbTab<lf3> {
   const float4* a;

@@ -280,9 +280,8 @@ bool c2r_interleave_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* specs, lo
 template <typename T, typename TO>
 void rows_c2r_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* spec, void* out);
 
-// The passes in fixed-grid limb arithmetic (fft_limb.cuh): FP64 plans in three limbs, the
-// inverse passes of FP32 maps' float-float plans in two.  Each returns false, with nothing
-// launched, where it has no kernel for the plan's sizes.
+// The passes of FP64 plans in fixed-grid limb arithmetic (fft_limb.cuh).  Each returns false,
+// with nothing launched, where it has no kernel for the plan's sizes.
 bool limb3_rows_r2c_map(mlc_ctx* ctx, const FftPlan2D& p, const void* in, int in_dtype, void* out);
 bool limb3_rows_r2c_profile(mlc_ctx* ctx, const FftPlan2D& p, const double* prof, int pN, void* out);
 bool limb3_rows_c2r(mlc_ctx* ctx, const FftPlan2D& p, const void* in, void* out);
@@ -293,12 +292,6 @@ bool limb3_conv(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, void* out, v
 bool limb3_conv_profile(mlc_ctx* ctx, const FftPlan2D& p, void* kx, int h, void* ks);
 size_t limb3_profile_spectrum_bytes(const FftPlan2D& p);  // of ks
 bool limb3_conv_cached(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, void* out, const void* ks);
-bool limb2_colpass_inverse(mlc_ctx* ctx, const FftPlan2D& p, void* buf, char kind, int post_tw);
-bool limb2_conv(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, void* out, const void* kx, int h);
-bool limb2_conv_cached(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, void* out, const void* ks);
-bool limb2_rows_c2r(mlc_ctx* ctx, const FftPlan2D& p, const void* in, void* out);
-bool limb2_rows_c2r_il(mlc_ctx* ctx, const FftPlan2D& p, const void* specs, long spec_stride, int nm, int S,
-                       void* out, unsigned planar);
 
 // Host profile rasters (profile.cpp)
 int profile_dims(const mlc_profile& p);

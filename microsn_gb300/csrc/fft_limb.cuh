@@ -732,11 +732,12 @@ bool limb3_conv_impl(mlc_ctx* ctx, const FftPlan2D& p, const void* Fmap, void* o
                                                                            rows.b, rows.e);
   }
   MLC_CHECK_LAUNCH();
-  // 1 / (Nx Ny) = r 2^-rexp with r in (1/2, 1]
+  // 1 / (Nx Ny) = r 2^-rexp with r in (1/2, 1]; its high limb a multiple of 2^-22, as a value's, for the
+  // products with twiddles (both cut to 2^-24 only, their remainder had 25 bits: r W was off by 2^-49)
   const long double inv = 1.0L / ((long double)p.Nx * p.Ny);
   int e = 0;
   long double m = frexpl(inv, &e);
-  const float a = (float)(rintl(m * 16777216.0L) / 16777216.0L);
+  const float a = (float)(rintl(m * 4194304.0L) / 4194304.0L);
   const float b = (float)(m - (long double)a);
   const lf3 r(a, b, (float)(m - (long double)a - (long double)b));
   if (!k) {

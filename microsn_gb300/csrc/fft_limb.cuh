@@ -57,7 +57,7 @@ __global__ void __launch_bounds__((L1 > L2 ? L1 : L2) * CW, 2)
   LimbSum<S> sum = red[0][c];
 #pragma unroll
   for (int q = 1; q < L2; q++) sum = limb_sum_add(sum, red[q][c]);
-  const LimbScale<T> sc = limb_scale(sum, 0);
+  const LimbScale<T> sc = limb_scale(sum);
   if (g < L2) {
     C2<T> v[L1];
 #pragma unroll
@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(256) k_limb_profile_columns(const C2<double>* 
   sum = red[0][c];
 #pragma unroll
   for (int q = 1; q < G; q++) sum = limb_sum_add(sum, red[q][c]);
-  const LimbScale<lf3> sc = limb_scale(sum, 0);
+  const LimbScale<lf3> sc = limb_scale(sum);
   if (g == 0) kexp[col] = sc.bad ? LIMB_BAD : sc.e;
   for (int r = g; r < rows; r += G) {
     const long i = r * pitch + col;
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__((L1 > L2 ? L1 : L2) * CW, 2)
     LimbSum<double> sum = red[0][c];
 #pragma unroll
     for (int q = 1; q < L1; q++) sum = limb_sum_add(sum, red[q][c]);
-    LimbScale<T> sc = limb_scale(sum, 0);
+    LimbScale<T> sc = limb_scale(sum);
     // product with the map spectrum: thread (k1 = g, c) holds frequencies k1 + L1 k2
     if (g < L1) {
 #pragma unroll
@@ -347,8 +347,9 @@ struct LevelPlace<Levels<R0, R1, R...>> {
 
 // One level but the last: NB blocks of LV, whose places come from `outer`; tw(q, m) is
 // W_{LV::M}^(m q).
+// grow: the factor to the level's scale, 1 where it stays.
 template <typename T, bool INV, int NT, typename LV, int R0, int NB, typename Place, typename Tw>
-__device__ __forceinline__ void limb_level(const LimbArr<T>& s, Place outer, Tw tw) {
+__device__ __forceinline__ void limb_level(const LimbArr<T>& s, float grow, Place outer, Tw tw) {
   constexpr int BN = LV::Next::M, TN = LV::TN;
   for (int it = threadIdx.x; it < NB * BN; it += NT) {
     const int blk = it / BN, m = it - blk * BN;
@@ -356,6 +357,10 @@ __device__ __forceinline__ void limb_level(const LimbArr<T>& s, Place outer, Tw 
     C2<T> u[R0];
 #pragma unroll
     for (int q = 0; q < R0; q++) u[q] = s.ld(p + q * TN);
+    if (grow != 1.f) {
+#pragma unroll
+      for (int q = 0; q < R0; q++) u[q] = cscale2(u[q], grow);
+    }
     Dft<T, R0, INV>::run(u);
     s.st(p, limb_cnorm(u[0]));
 #pragma unroll
@@ -397,25 +402,25 @@ __device__ __forceinline__ void limb_fill_deep(Levels<R0, R1, R...>, const LimbA
 // in w.
 template <typename T, bool INV, int NT, int DEPTH, int NB, typename Place, int R0>
 __device__ __forceinline__ void limb_levels(Levels<R0>, const LimbArr<T>&, const LimbArr<T>&, int, const LimbTab<T>&,
-                                            Place) {}
+                                            LimbGrow&, Place) {}
 template <typename T, bool INV, int NT, int DEPTH, int NB, typename Place, int R0, int R1, int... R>
 __device__ __forceinline__ void limb_levels(Levels<R0, R1, R...>, const LimbArr<T>& s, const LimbArr<T>& w, int at,
-                                            const LimbTab<T>& tab0, Place outer) {
+                                            const LimbTab<T>& tab0, LimbGrow& grow, Place outer) {
   using LV = Levels<R0, R1, R...>;
   constexpr int BN = LV::Next::M;
-  limb_level<T, INV, NT, LV, R0, NB>(s, outer, [&](int q, int m) {
+  limb_level<T, INV, NT, LV, R0, NB>(s, DEPTH == 0 ? 1.f : grow.next(R0), outer, [&](int q, int m) {
     if constexpr (DEPTH == 0) return tab0.ld((q - 1) * BN + m);
     else return w.ld(at + (q - 1) * BN + m);
   });
   limb_levels<T, INV, NT, DEPTH + 1, NB * R0>(
-      typename LV::Next{}, s, w, DEPTH == 0 ? 0 : at + (R0 - 1) * BN, tab0,
+      typename LV::Next{}, s, w, DEPTH == 0 ? 0 : at + (R0 - 1) * BN, tab0, grow,
       [=](int blk) { return outer(blk / R0) + (blk % R0) * LV::TN; });
 }
 
 // The last level of a row transform from the padded places in s.  Its results go through cvt,
 // then -- with BAR after a barrier, so that put may write over s -- to put(n, v).
 template <typename T, bool INV, int NT, bool BAR, typename V, typename Cvt, typename Put, int R0, int... R>
-__device__ __forceinline__ void limb_last_level(Levels<R0, R...>, const LimbArr<T>& s, Cvt cvt, Put put) {
+__device__ __forceinline__ void limb_last_level(Levels<R0, R...>, const LimbArr<T>& s, float grow, Cvt cvt, Put put) {
   using LV = Levels<R0, R...>;
   constexpr int LAST = LV::LAST, NI = LV::M / LAST, PER = (NI + NT - 1) / NT;
   V out[PER][LAST];
@@ -427,6 +432,10 @@ __device__ __forceinline__ void limb_last_level(Levels<R0, R...>, const LimbArr<
       C2<T> u[LAST];
 #pragma unroll
       for (int q = 0; q < LAST; q++) u[q] = s.ld(p + q);
+      if (grow != 1.f) {
+#pragma unroll
+        for (int q = 0; q < LAST; q++) u[q] = cscale2(u[q], grow);
+      }
       Dft<T, LAST, INV>::run(u);
 #pragma unroll
       for (int q = 0; q < LAST; q++) out[i][q] = cvt(u[q]);
@@ -449,15 +458,15 @@ __device__ __forceinline__ void limb_last_level(Levels<R0, R...>, const LimbArr<
   }
 }
 
-template <typename S, int NT>
-__device__ __forceinline__ LimbSum<S> limb_block_sum(LimbSum<S> v, LimbSum<S>* red) {
-  v = limb_sum_warp(v);
+template <int NT>
+__device__ __forceinline__ LimbPeak limb_block_peak(LimbPeak v, LimbPeak* red) {
+  v = limb_peak_warp(v);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
-  LimbSum<S> sum = red[0];
+  LimbPeak all = red[0];
 #pragma unroll
-  for (int w = 1; w < NT / 32; w++) sum = limb_sum_add(sum, red[w]);
-  return sum;
+  for (int w = 1; w < NT / 32; w++) all = limb_peak_add(all, red[w]);
+  return all;
 }
 
 template <typename T, typename LV>
@@ -479,9 +488,9 @@ __device__ __forceinline__ void limb_c2r_pair(C2<T> xk, C2<T> xm, C2<T> w, C2<T>
 // b[k] = (X[k] + conj X[M-k]) + i (X[k] - conj X[M-k]) W_Nx^-k, then the inverse transform of
 // M points).  The row is read once into registers, both partners k and M - k by one thread.
 template <typename S, typename T, int NT, int R0, int... R>
-__device__ __forceinline__ LimbScale<T> limb_c2r_first(Levels<R0, R...>, const C2<S>* __restrict__ a,
+__device__ __forceinline__ LimbGrow limb_c2r_first(Levels<R0, R...>, const C2<S>* __restrict__ a,
                                                        const LimbTab<T>& twx, const LimbTab<T>& tab0,
-                                                       const LimbArr<T>& s, const LimbArr<T>& w, LimbSum<S>* red) {
+                                                       const LimbArr<T>& s, const LimbArr<T>& w, LimbPeak* red) {
   using LV = Levels<R0, R...>;
   constexpr int M = LV::M, NP = (M / 2 + 1 + NT - 1) / NT;
   const int tid = threadIdx.x;
@@ -494,8 +503,9 @@ __device__ __forceinline__ LimbScale<T> limb_c2r_first(Levels<R0, R...>, const C
     x[2 * i + 1] = in ? ldc(a + (M - k)) : C2<S>{S(0.0), S(0.0)};
   }
   limb_fill_deep<T, NT, R0>(typename LV::Next{}, w, 0, twx);
-  // |b[k]| + |b[M-k]| <= 2 sqrt(2) (|X[k]| + |X[M-k]|), and the scale leaves a bit
-  const LimbScale<T> sc = limb_scale(limb_block_sum<S, NT>(limb_sum<2 * NP>(x), red), 1);
+  // |b[k]| + |b[M-k]| <= 2 sqrt(2) (|X[k]| + |X[M-k]|), and each of them <= 2 (|X[k]| + |X[M-k]|)
+  LimbGrow grow = LimbGrow::of(limb_block_peak<NT>(limb_peak<2 * NP, 2>(x), red), 2.82843f, 2.f);
+  const LimbScale<T> sc = grow.first(R0);
 #pragma unroll
   for (int i = 0; i < NP; i++) {
     const int k = tid + i * NT;
@@ -507,18 +517,20 @@ __device__ __forceinline__ LimbScale<T> limb_c2r_first(Levels<R0, R...>, const C
     }
   }
   __syncthreads();
-  limb_levels<T, true, NT, 0, 1>(LV{}, s, w, 0, tab0, [](int) { return 0; });
-  return sc;
+  limb_levels<T, true, NT, 0, 1>(LV{}, s, w, 0, tab0, grow, [](int) { return 0; });
+  return grow;
 }
 
 template <typename S, typename T, typename TO, int NT, bool BAR, typename Put, typename LV>
 __device__ __forceinline__ void limb_c2r_row(LV, const C2<S>* __restrict__ a, const LimbTab<T>& twx,
-                                             const LimbTab<T>& tab0, unsigned char* smem, LimbSum<S>* red, Put put) {
+                                             const LimbTab<T>& tab0, unsigned char* smem, LimbPeak* red, Put put) {
   const LimbArr<T> s = LimbArr<T>::at(smem, LV::T);
   const LimbArr<T> w = LimbArr<T>::at(smem + LimbArr<T>::bytes(LV::T), DeepTwiddles<typename LV::Next>::n);
-  const LimbScale<T> sc = limb_c2r_first<S, T, NT>(LV{}, a, twx, tab0, s, w, red);
+  LimbGrow grow = limb_c2r_first<S, T, NT>(LV{}, a, twx, tab0, s, w, red);
+  const float last = grow.next(LV::LAST);
+  const LimbScale<T> sc = grow.scale();
   limb_last_level<T, true, NT, BAR, C2<TO>>(
-      LV{}, s, [&](C2<T> z) { return C2<TO>{limb_round(z.x, sc), limb_round(z.y, sc)}; }, put);
+      LV{}, s, last, [&](C2<T> z) { return C2<TO>{limb_round(z.x, sc), limb_round(z.y, sc)}; }, put);
 }
 
 // P3: one row per CTA, the pixels written from registers in thread order.
@@ -526,7 +538,7 @@ template <typename S, typename T, typename TO, int NT, typename LV>
 __global__ void __launch_bounds__(NT) k_limb_rows_c2r(const C2<S>* __restrict__ in, long pitch, TO* __restrict__ out,
                                                       long ldo, LimbTab<T> twx, LimbTab<T> tab0) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ LimbSum<S> red[NT / 32];
+  __shared__ LimbPeak red[NT / 32];
   C2<TO>* dst = reinterpret_cast<C2<TO>*>(out + (long)blockIdx.x * ldo);
   limb_c2r_row<S, T, TO, NT, false>(LV{}, in + (long)blockIdx.x * pitch, twx, tab0, smem_raw, red,
                                     [&](int n, C2<TO> z) { dst[n] = z; });
@@ -542,7 +554,7 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(NT)
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ LimbSum<S> red[NT / 32];
+  __shared__ LimbPeak red[NT / 32];
   TO* px = reinterpret_cast<TO*>(smem_raw);
   C2<TO>* pz = reinterpret_cast<C2<TO>*>(smem_raw);
   const int row = blockIdx.y;
@@ -591,7 +603,7 @@ __global__ void __launch_bounds__(NT)
     k_limb_rows_r2c(Loader ld, C2<S>* __restrict__ out, long pitch, LimbTab<T> twx, LimbTab<T> tab0) {
   constexpr int M = LV::M, NV = (M + NT - 1) / NT;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ LimbSum<S> red[NT / 32];
+  __shared__ LimbPeak red[NT / 32];
   const LimbArr<T> s = LimbArr<T>::at(smem_raw, LV::T);
   const LimbArr<T> w = LimbArr<T>::at(smem_raw + LimbArr<T>::bytes(LV::T), DeepTwiddles<typename LV::Next>::n);
   const int tid = threadIdx.x, row = blockIdx.x;
@@ -602,29 +614,28 @@ __global__ void __launch_bounds__(NT)
     x[i] = n < M ? ld.pair(row, n) : C2<S>{S(0.0), S(0.0)};
   }
   limb_fill_deep<T, NT, LV::M / LV::Next::M>(typename LV::Next{}, w, 0, twx);
-  // the split's sums may double the transform's values: one more bit
-  const LimbScale<T> sc = limb_scale(limb_block_sum<S, NT>(limb_sum<NV>(x), red), 1);
+  LimbGrow grow = LimbGrow::of(limb_block_peak<NT>(limb_peak<NV, 1>(x), red), 1.f, 1.f);
+  const LimbScale<T> sc = grow.first(LV::M / LV::Next::M);
 #pragma unroll
   for (int i = 0; i < NV; i++) {
     const int n = tid + i * NT;
     if (n < M) s.st(LevelPlace<LV>::of(n), limb_cin(x[i], sc));
   }
   __syncthreads();
-  limb_levels<T, false, NT, 0, 1>(LV{}, s, w, 0, tab0, [](int) { return 0; });
+  limb_levels<T, false, NT, 0, 1>(LV{}, s, w, 0, tab0, grow, [](int) { return 0; });
   limb_last_level<T, false, NT, true, C2<T>>(
-      LV{}, s, [](C2<T> z) { return z; }, [&](int n, C2<T> z) { s.st(n, z); });
+      LV{}, s, grow.next(LV::LAST), [](C2<T> z) { return z; }, [&](int n, C2<T> z) { s.st(n, z); });
   __syncthreads();
-  // X[k] = (s - i W^k d) / 2 with s = Z[k] + conj Z[M-k], d = Z[k] - conj Z[M-k]; for M - k,
-  // s' = conj s and W^(M-k) d' = conj (W^k d): X[M-k] = (conj s - i conj (W^k d)) / 2
+  // X[k] = s - i W^k d with s = (Z[k] + conj Z[M-k]) / 2, d = (Z[k] - conj Z[M-k]) / 2, which the scale
+  // of Z holds for; for M - k, s' = conj s and W^(M-k) d' = conj (W^k d): X[M-k] = conj s - i conj (W^k d)
   C2<S>* o = out + (long)row * pitch;
-  LimbScale<T> half = sc;
-  half.e -= 1;
+  const LimbScale<T> so = grow.scale();
   for (int k = tid; k <= M / 2; k += NT) {
-    const C2<T> zk = s.ld(k), zc = cconj(s.ld(k == 0 ? 0 : M - k));
+    const C2<T> zk = cscale2(s.ld(k), 0.5f), zc = cconj(cscale2(s.ld(k == 0 ? 0 : M - k), 0.5f));
     const C2<T> a = cadd(zk, zc);
     const C2<T> wd = limb_tw<false>(csub(zk, zc), twx.ld(k));
-    o[k] = limb_cout<S>(C2<T>{a.x + wd.y, a.y - wd.x}, half);
-    if (k != M - k) o[M - k] = limb_cout<S>(C2<T>{a.x - wd.y, -wd.x - a.y}, half);
+    o[k] = limb_cout<S>(C2<T>{a.x + wd.y, a.y - wd.x}, so);
+    if (k != M - k) o[M - k] = limb_cout<S>(C2<T>{a.x - wd.y, -wd.x - a.y}, so);
   }
   for (int k = M + 1 + tid; k < pitch; k += NT) o[k] = C2<S>{S(0.0), S(0.0)};
 }

@@ -10,8 +10,9 @@ namespace mlc {
 
 // Level i, radix R, over CW interleaved columns.  DIT false: the small transform, then the
 // twiddles; true (the way back, levels in the opposite order): conjugate twiddles, then it.
+// grow: the factor to the level's scale (rows), 1 where it stays.
 template <typename T, bool INV, bool DIT, int R, int CW, typename Tw>
-__device__ __forceinline__ void any_level(const LimbArr<T>& s, const AnyLevels& lv, int i, Tw tw) {
+__device__ __forceinline__ void any_level(const LimbArr<T>& s, const AnyLevels& lv, int i, float grow, Tw tw) {
   const int bn = lv.bn[i], tn = lv.tn[i] * CW, items = lv.L / R * CW;
   const bool last = i == lv.n - 1;
   const uint32_t mbn = lv.mbn[i];
@@ -23,6 +24,10 @@ __device__ __forceinline__ void any_level(const LimbArr<T>& s, const AnyLevels& 
     C2<T> u[R];
 #pragma unroll
     for (int q = 0; q < R; q++) u[q] = s.ld(p + q * tn);
+    if (CW == 1 && grow != 1.f) {
+#pragma unroll
+      for (int q = 0; q < R; q++) u[q] = cscale2(u[q], grow);
+    }
     if (DIT) {
       u[0] = limb_cnorm(u[0]);
       if (!last) {
@@ -44,35 +49,42 @@ __device__ __forceinline__ void any_level(const LimbArr<T>& s, const AnyLevels& 
 }
 
 template <typename T, bool INV, bool DIT, int CW, typename Tw>
-__device__ __forceinline__ void any_level_r(const LimbArr<T>& s, const AnyLevels& lv, int i, Tw tw) {
-  any_radix(lv.r[i], [&](auto r) { any_level<T, INV, DIT, decltype(r)::value, CW>(s, lv, i, tw); });
+__device__ __forceinline__ void any_level_r(const LimbArr<T>& s, const AnyLevels& lv, int i, float grow, Tw tw) {
+  any_radix(lv.r[i], [&](auto r) { any_level<T, INV, DIT, decltype(r)::value, CW>(s, lv, i, grow, tw); });
 }
 
 // All levels: natural order in, digit order out (DIT: the other way round).  Level 0's twiddles
-// straight from the table where DEEP (rows: w holds the deeper levels'), else all from w.
-template <typename T, bool INV, bool DIT, bool DEEP, int CW>
-__device__ __forceinline__ void any_transform(const LimbArr<T>& s, const AnyLevels& lv, const LimbTab<T>& tab,
-                                              const LimbArr<T>& w) {
-  const int w0 = DEEP && lv.n > 1 ? lv.tw[1] : 0;
+// straight from the table for rows (w holds the deeper levels'), else all from w.
+template <typename T, bool INV>
+__device__ __forceinline__ void any_row_transform(const LimbArr<T>& s, const AnyLevels& lv, const LimbTab<T>& tab,
+                                                  const LimbArr<T>& w, LimbGrow& grow) {
+  const int w0 = lv.n > 1 ? lv.tw[1] : 0;
+#pragma unroll 1
+  for (int i = 0; i < lv.n; i++) {
+    const int at = lv.tw[i];
+    if (i == 0) any_level_r<T, INV, false, 1>(s, lv, i, 1.f, [&](int e) { return tab.ld(e); });
+    else any_level_r<T, INV, false, 1>(s, lv, i, grow.next(lv.r[i]), [&](int e) { return w.ld(at - w0 + e); });
+  }
+}
+template <typename T, bool INV, bool DIT, int CW>
+__device__ __forceinline__ void any_transform(const LimbArr<T>& s, const AnyLevels& lv, const LimbArr<T>& w) {
 #pragma unroll 1
   for (int l = 0; l < lv.n; l++) {
     const int i = DIT ? lv.n - 1 - l : l;
     const int at = lv.tw[i];
-    if (DEEP && i == 0) any_level_r<T, INV, DIT, CW>(s, lv, i, [&](int e) { return tab.ld(e); });
-    else any_level_r<T, INV, DIT, CW>(s, lv, i, [&](int e) { return w.ld(at - w0 + e); });
+    any_level_r<T, INV, DIT, CW>(s, lv, i, 1.f, [&](int e) { return w.ld(at + e); });
   }
 }
 
 // ---------------------------------------------------------------- rows
 
-template <typename S>
-__device__ __forceinline__ LimbSum<S> any_block_sum(LimbSum<S> v, LimbSum<S>* red) {
-  v = limb_sum_warp(v);
+__device__ __forceinline__ LimbPeak any_block_peak(LimbPeak v, LimbPeak* red) {
+  v = limb_peak_warp(v);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
-  LimbSum<S> sum = red[0];
-  for (int w = 1; w < (int)(blockDim.x >> 5); w++) sum = limb_sum_add(sum, red[w]);
-  return sum;
+  LimbPeak all = red[0];
+  for (int w = 1; w < (int)(blockDim.x >> 5); w++) all = limb_peak_add(all, red[w]);
+  return all;
 }
 template <typename S>
 __device__ __forceinline__ LimbSum<S> limb_sum_zero();
@@ -94,12 +106,12 @@ __global__ void __launch_bounds__(512)
     k_any_rows_c2r(const C2<S>* __restrict__ in, long pitch, TO* __restrict__ out, long ldo, LimbTab<T> twx,
                    const __grid_constant__ AnyLevels lv, LimbTab<T> tab) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ LimbSum<S> red[512 / 32];
+  __shared__ LimbPeak red[512 / 32];
   const int M = lv.L, tid = threadIdx.x, NT = blockDim.x;
   const LimbArr<T> s = LimbArr<T>::at(smem_raw, lv.places);
   const LimbArr<T> w = LimbArr<T>::at(smem_raw + LimbArr<T>::bytes(lv.places), lv.n > 1 ? lv.ntw - lv.tw[1] : 0);
   const C2<S>* a = in + (long)blockIdx.x * pitch;
-  LimbSum<S> sum = limb_sum_zero<S>();
+  LimbPeak peak{0, 0.f, 0.f};
   C2<S>* raw = reinterpret_cast<C2<S>*>(smem_raw);  // 16 bytes a value, as the limbs' first plane
   C2<S> top{S(0.0), S(0.0)};                        // X[M], beside X[0] of thread 0
   for (int k0 = tid; k0 <= M / 2; k0 += 2 * NT) {  // (the loads of a round are in flight together)
@@ -110,7 +122,7 @@ __global__ void __launch_bounds__(512)
       v[2 * i] = k <= M / 2 ? ldc(a + k) : C2<S>{S(0.0), S(0.0)};
       v[2 * i + 1] = k <= M / 2 ? ldc(a + (M - k)) : C2<S>{S(0.0), S(0.0)};
     }
-    sum = limb_sum_add(sum, limb_sum<4>(v));
+    peak = limb_peak_add(peak, limb_peak<4, 2>(v));
 #pragma unroll
     for (int i = 0; i < 2; i++) {
       const int k = k0 + i * NT;
@@ -121,8 +133,9 @@ __global__ void __launch_bounds__(512)
     }
   }
   any_fill_deep(w, lv, tab);
-  // |b[k]| + |b[M-k]| <= 2 sqrt(2) (|X[k]| + |X[M-k]|), and the scale leaves a bit
-  const LimbScale<T> sc = limb_scale(any_block_sum(sum, red), 1);
+  // |b[k]| + |b[M-k]| <= 2 sqrt(2) (|X[k]| + |X[M-k]|), and each of them <= 2 (|X[k]| + |X[M-k]|)
+  LimbGrow grow = LimbGrow::of(any_block_peak(peak, red), 2.82843f, 2.f);
+  const LimbScale<T> sc = grow.first(lv.r[0]);
   for (int k = tid; k <= M / 2; k += NT) {
     C2<T> bk, bm;
     const int pk = any_inner(lv, 0, k), pm = k > 0 ? any_inner(lv, 0, M - k) : 0;
@@ -131,11 +144,12 @@ __global__ void __launch_bounds__(512)
     if (k > 0 && k != M - k) s.st(pm, bm);
   }
   __syncthreads();
-  any_transform<T, true, false, true, 1>(s, lv, tab, w);
+  any_row_transform<T, true>(s, lv, tab, w, grow);
+  const LimbScale<T> so = grow.scale();
   C2<TO>* dst = reinterpret_cast<C2<TO>*>(out + (long)blockIdx.x * ldo);
   for (int n = tid; n < M; n += NT) {
     const C2<T> z = s.ld(any_output(lv, n));
-    dst[n] = C2<TO>{limb_round(z.x, sc), limb_round(z.y, sc)};
+    dst[n] = C2<TO>{limb_round(z.x, so), limb_round(z.y, so)};
   }
 }
 
@@ -144,40 +158,40 @@ __global__ void __launch_bounds__(512)
     k_any_rows_r2c(Loader ld, C2<S>* __restrict__ out, long pitch, LimbTab<T> twx,
                    const __grid_constant__ AnyLevels lv, LimbTab<T> tab) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ LimbSum<S> red[512 / 32];
+  __shared__ LimbPeak red[512 / 32];
   const int M = lv.L, tid = threadIdx.x, NT = blockDim.x, row = blockIdx.x;
   const LimbArr<T> s = LimbArr<T>::at(smem_raw, lv.places);
   const LimbArr<T> w = LimbArr<T>::at(smem_raw + LimbArr<T>::bytes(lv.places), lv.n > 1 ? lv.ntw - lv.tw[1] : 0);
-  LimbSum<S> sum = limb_sum_zero<S>();
+  LimbPeak peak{0, 0.f, 0.f};
   C2<S>* raw = reinterpret_cast<C2<S>*>(smem_raw);
   for (int n0 = tid; n0 < M; n0 += 4 * NT) {  // (the loads of a round are in flight together)
     C2<S> v[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) v[i] = n0 + i * NT < M ? ld.pair(row, n0 + i * NT) : C2<S>{S(0.0), S(0.0)};
-    sum = limb_sum_add(sum, limb_sum<4>(v));
+    peak = limb_peak_add(peak, limb_peak<4, 1>(v));
 #pragma unroll
     for (int i = 0; i < 4; i++)
       if (n0 + i * NT < M) raw[any_inner(lv, 0, n0 + i * NT)] = v[i];
   }
   any_fill_deep(w, lv, tab);
-  // the split's sums may double the transform's values: one more bit
-  const LimbScale<T> sc = limb_scale(any_block_sum(sum, red), 1);
+  LimbGrow grow = LimbGrow::of(any_block_peak(peak, red), 1.f, 1.f);
+  const LimbScale<T> sc = grow.first(lv.r[0]);
   for (int n = tid; n < M; n += NT) {
     const int p = any_inner(lv, 0, n);
     s.st(p, limb_cin(raw[p], sc));
   }
   __syncthreads();
-  any_transform<T, false, false, true, 1>(s, lv, tab, w);
+  any_row_transform<T, false>(s, lv, tab, w, grow);
   // the split of k_limb_rows_r2c
   C2<S>* o = out + (long)row * pitch;
-  LimbScale<T> half = sc;
-  half.e -= 1;
+  const LimbScale<T> so = grow.scale();
   for (int k = tid; k <= M / 2; k += NT) {
-    const C2<T> zk = s.ld(any_output(lv, k)), zc = cconj(s.ld(k == 0 ? any_output(lv, 0) : any_output(lv, M - k)));
+    const C2<T> zk = cscale2(s.ld(any_output(lv, k)), 0.5f);
+    const C2<T> zc = cconj(cscale2(s.ld(k == 0 ? any_output(lv, 0) : any_output(lv, M - k)), 0.5f));
     const C2<T> a = cadd(zk, zc);
     const C2<T> wd = limb_tw<false>(csub(zk, zc), twx.ld(k));
-    o[k] = limb_cout<S>(C2<T>{a.x + wd.y, a.y - wd.x}, half);
-    if (k != M - k) o[M - k] = limb_cout<S>(C2<T>{a.x - wd.y, -wd.x - a.y}, half);
+    o[k] = limb_cout<S>(C2<T>{a.x + wd.y, a.y - wd.x}, so);
+    if (k != M - k) o[M - k] = limb_cout<S>(C2<T>{a.x - wd.y, -wd.x - a.y}, so);
   }
   for (int k = M + 1 + tid; k < pitch; k += NT) o[k] = C2<S>{S(0.0), S(0.0)};
 }
@@ -223,10 +237,10 @@ __global__ void __launch_bounds__(ANY_NT, 2)
       if (j0 + i * G < L) raw[(j0 + i * G) * ANY_CW + c] = v[i];
   }
   for (int e = threadIdx.x; e < lv.ntw; e += blockDim.x) w.st(e, tab.ld(e));
-  const LimbScale<T> sc = limb_scale(any_column_sum(sum, red), 0);
+  const LimbScale<T> sc = limb_scale(any_column_sum(sum, red));
   for (int j = g; j < L; j += G) s.st(j * ANY_CW + c, limb_cin(raw[j * ANY_CW + c], sc));
   __syncthreads();
-  any_transform<T, INV, false, false, ANY_CW>(s, lv, tab, w);
+  any_transform<T, INV, false, ANY_CW>(s, lv, w);
   for (int j = g; j < L; j += G) {
     C2<T> v = s.ld(any_output(lv, j) * ANY_CW + c);
     if (post_tw) v = limb_tw<INV>(v, twy.ld((long)set * j));  // set*j < Ny
@@ -272,14 +286,14 @@ __global__ void __launch_bounds__(ANY_NT, 2)
     const C2<T> t = twy.ld((long)n2 * kk);
     s.st(n2 * ANY_CW + c, limb_tw<false>(acc, limb_cnorm(C2<T>{r * t.x, r * t.y})));
   }
-  const LimbScale<T> sf = limb_scale(any_column_sum(sum, red), 0);  // (its barrier also ends the writes of s and w)
-  any_transform<T, false, false, false, ANY_CW>(s, lv, tab, w);
+  const LimbScale<T> sf = limb_scale(any_column_sum(sum, red));  // (its barrier also ends the writes of s and w)
+  any_transform<T, false, false, ANY_CW>(s, lv, w);
   for (int k2 = g; k2 < N2; k2 += G) {
     const int p = any_output(lv, k2) * ANY_CW + c;
     s.st(p, limb_tw<false>(limb_cin(ldc(f + (long)k2 * pitch), sf), limb_cnorm(s.ld(p))));
   }
   __syncthreads();
-  any_transform<T, true, true, false, ANY_CW>(s, lv, tab, w);
+  any_transform<T, true, true, ANY_CW>(s, lv, w);
   LimbScale<T> sc = sf;
   sc.bad |= ke == LIMB_BAD;  // the scales multiply: exponents add
   sc.e += sc.bad ? 0 : ke;

@@ -10,9 +10,16 @@
 //
 // Why |x| < 1 holds throughout a transform: the scale comes from S, the sum of |re| + |im|
 // over all of its inputs, and every intermediate value of an FFT is a sum of distinct inputs
-// times factors of modulus one, so its modulus is at most S -- whatever the inputs.  The
-// absolute error of an operation is about 2^-62 S.  (Two limbs, 46 bits, in place of
-// float-float lost the faint pixels of FP32 maps: 2^-30 of the map's rms at 10000^2.)
+// times factors of modulus one, so its modulus is at most S -- whatever the inputs.
+//
+// An operation's error is absolute, about 2^-62 of the scale, and S is far above the values of a
+// long transform until its last levels: rows of 5000 points under the scale of S throughout
+// kept 2^-47.7 of their rms (forward) and 2^-49.4 (back), where FP64 keeps 2^-51.8.  The rows
+// therefore start under a scale from their largest input and go over to a larger one from
+// level to level, as far as the radices since then can have made the values grow (LimbGrow):
+// 2^-52.7 and 2^-51.7.  Columns, of 128 points or so, gain nothing from that.
+// (Two limbs, 46 bits, in place of float-float lost the faint pixels of FP32 maps: 2^-30 of
+// the map's rms at 10000^2.)
 //
 // Products return to the grid with the additive constant 3 = 1.5 * 2: t = 3 + x c is
 // rounded to 2^-22 (t lies in [2, 4)), t - 3 is the high limb, and fma(x, c, -(t - 3)) is the
@@ -307,23 +314,96 @@ __device__ __forceinline__ LimbSum<double> limb_sum_warp(LimbSum<double> a) {
   return a;
 }
 
-// The power of two that brings a transform below 1/2 and back: the exponent fields to add to a
+// The same with the largest |re| + |im| of a value, or of the G values that one input of the
+// transform is made of: p 2^(e - 1023).
+struct LimbPeak {
+  int e;
+  float s, p;
+};
+template <int N, int G>
+__device__ __forceinline__ LimbPeak limb_peak(const C2<double>* v) {
+  static_assert(N % G == 0, "whole groups");
+  int top = 0;
+#pragma unroll
+  for (int i = 0; i < N; i++)
+    top = max(top, max(__double2hiint(v[i].x) & 0x7fffffff, __double2hiint(v[i].y) & 0x7fffffff));
+  const int e = top & 0x7ff00000;
+  float s = 0.f, p = 0.f;
+#pragma unroll
+  for (int i = 0; i < N; i += G) {
+    float g = 0.f;
+#pragma unroll
+    for (int k = 0; k < G; k++) {
+      g = __fadd_rn(g, limb_pow_diff(__double2hiint(v[i + k].x) & 0x7fffffff, e));
+      g = __fadd_rn(g, limb_pow_diff(__double2hiint(v[i + k].y) & 0x7fffffff, e));
+    }
+    s = __fadd_rn(s, g);
+    p = fmaxf(p, g);
+  }
+  return LimbPeak{e, s, p};
+}
+__device__ __forceinline__ LimbPeak limb_peak_add(LimbPeak a, LimbPeak b) {
+  const int e = max(a.e, b.e);
+  const float fa = limb_pow_diff(a.e, e), fb = limb_pow_diff(b.e, e);
+  return LimbPeak{e, __fmaf_rn(a.s, fa, __fmul_rn(b.s, fb)), fmaxf(__fmul_rn(a.p, fa), __fmul_rn(b.p, fb))};
+}
+__device__ __forceinline__ LimbPeak limb_peak_warp(LimbPeak a) {
+  const int e = __reduce_max_sync(0xffffffffu, a.e);
+  const float f = limb_pow_diff(a.e, e);
+  a.s = __fmul_rn(a.s, f);
+  a.p = __int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(__fmul_rn(a.p, f))));  // (p >= 0)
+  a.e = e;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) a.s = __fadd_rn(a.s, __shfl_xor_sync(0xffffffffu, a.s, o));
+  return a;
+}
+
+// The power of two that brings a transform below 1 and back: the exponent fields to add to a
 // double before its conversion to a 62-bit fixed-point integer and after the way back.  A sum
 // that is not finite makes every output NaN.
 template <typename T>
 struct LimbScale;
 template <>
 struct LimbScale<lf3> {
-  int e;  // x < 2^(e - 1)
+  int e;  // |x| < 2^e
   bool bad;
 };
-// extra: the transform's values may grow to 2^extra times the sum.  One more than the least
-// power of two above the sum, as limb_out needs |x| < 1 and the sum is cut to high words.
-// (values below 2^-1022 of a transform whose sum is below 2^-960 count as zero)
-__device__ __forceinline__ LimbScale<lf3> limb_scale(LimbSum<double> a, int extra) {
-  const int e = (a.e >> 20) - 1023 + ((__float_as_int(a.s) >> 23) - 127) + 2 + extra;
-  return LimbScale<lf3>{max(e, -960), a.e >= 0x7ff00000};
+// Least e with s 2^(field - 1023) < 2^e; the margin covers the cut to high words and the
+// rounding of some ten thousand FP32 additions.
+__device__ __forceinline__ int limb_above(int field, float s) {
+  return (field >> 20) - 1023 + ((__float_as_int(__fmul_rn(s, 1.f + 0x1p-17f)) >> 23) - 127) + 1;
 }
+// (values below 2^-1022 of a transform whose sum is below 2^-960 count as zero)
+__device__ __forceinline__ LimbScale<lf3> limb_scale(LimbSum<double> a) {
+  return LimbScale<lf3>{max(limb_above(a.e, a.s), -960), a.e >= 0x7ff00000};
+}
+
+// The scales of a row transform's levels: the values are at most p r_0 ... r_i in level i, p the
+// largest of the inputs, and at most the sum s.  first(): the scale of the inputs, for level 0
+// of radix r; next(): the factor that takes the values over to the scale of a level of radix r.
+struct LimbGrow {
+  int field, top, e;
+  float p;
+  bool bad;
+  // bs, bp: what the transform's sum and its largest input are at most, in s and p of a
+  static __device__ __forceinline__ LimbGrow of(LimbPeak a, float bs, float bp) {
+    return LimbGrow{a.e, max(limb_above(a.e, __fmul_rn(a.s, bs)), -960), 0, __fmul_rn(a.p, bp), a.e >= 0x7ff00000};
+  }
+  __device__ __forceinline__ int level(int r) {
+    p = __fmul_rn(p, (float)r);
+    return max(min(top, limb_above(field, p)), -960);
+  }
+  __device__ __forceinline__ LimbScale<lf3> first(int r) {
+    e = level(r);
+    return LimbScale<lf3>{e, bad};
+  }
+  __device__ __forceinline__ float next(int r) {
+    const int was = e;
+    e = level(r);
+    return __int_as_float((127 + was - e) << 23);
+  }
+  __device__ __forceinline__ LimbScale<lf3> scale() const { return LimbScale<lf3>{e, bad}; }
+};
 
 // ---------------------------------------------------------------- in and out
 

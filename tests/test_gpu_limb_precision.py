@@ -19,8 +19,9 @@ def _map(Ny, Nx, sd, seed):
     return (m / m.mean()).contiguous()
 
 
-# rows of 600 points by run-time radices and of 1000 points unrolled
-@pytest.mark.parametrize("Ny,Nx", [(1200, 1200), (2000, 2000)])
+# rows of 600, 1000, 1500, 2000, 3000, 4096 and 5000 points, by run-time radices and unrolled
+@pytest.mark.parametrize("Ny,Nx", [(1200, 1200), (2000, 2000), (2000, 3000), (4000, 4000), (3000, 6000), (4096, 8192),
+                                   (10000, 10000)])
 @pytest.mark.parametrize("sd", [0.8, 2.0])
 def test_fp64_convolution_keeps_fp64_precision(ctx, Ny, Nx, sd):
     import microsn_gb300 as mlc

@@ -430,10 +430,11 @@ __device__ __forceinline__ double limb_out(lf3 v, LimbScale<lf3> s) {
   const long long q = ((long long)ih << 40) + ((long long)im << 23) + il;
   const double d = __ll2double_rn(q);
   if (s.bad) return __longlong_as_double(0x7ff8000000000000ll);
-  const int hi = __double2hiint(d), ex = hi & 0x7ff00000, r = ex + ((s.e - 62) << 20);
-  if (ex == 0 || r <= 0) return 0.0;
-  if (r >= 0x7ff00000) return __hiloint2double((hi & 0x80000000) | 0x7ff00000, 0);
-  return __hiloint2double(hi + ((s.e - 62) << 20), __double2loint(d));
+  const int hi = __double2hiint(d), lo = __double2loint(d), ef = (hi >> 20) & 0x7ff, sh = s.e - 62, r = ef + sh;
+  if (ef == 0 || (unsigned)(r - 1) >= 2046u) {  // zero, or beyond the exponents: zero below, infinite above
+    return ef == 0 || r <= 0 ? 0.0 : __hiloint2double((hi & 0x80000000) | 0x7ff00000, 0);
+  }
+  return __hiloint2double(hi + (int)((unsigned)sh << 20), lo);
 }
 __device__ __forceinline__ double limb_round(lf3 v, LimbScale<lf3> s) { return limb_out(v, s); }
 

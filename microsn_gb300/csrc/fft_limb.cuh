@@ -60,8 +60,9 @@ __global__ void __launch_bounds__((L1 > L2 ? L1 : L2) * CW, 2)
   const LimbScale<T> sc = limb_scale(sum);
   if (g < L2) {
     C2<T> v[L1];
+    const LimbScale<T> si = limb_lift<L1>(raw, sc);
 #pragma unroll
-    for (int n1 = 0; n1 < L1; n1++) v[n1] = limb_cin(raw[n1], sc);
+    for (int n1 = 0; n1 < L1; n1++) v[n1] = limb_cin(raw[n1], si);
     Dft<T, L1, INV>::run(v);
 #pragma unroll
     for (int k1 = 0; k1 < L1; k1++)
@@ -112,7 +113,9 @@ __global__ void __launch_bounds__(256) k_limb_profile_columns(const C2<double>* 
   if (g == 0) kexp[col] = sc.bad ? LIMB_BAD : sc.e;
   for (int r = g; r < rows; r += G) {
     const long i = r * pitch + col;
-    const C2<lf3> v = limb_cin(ldc(kx + i), sc);
+    C2<double> raw = ldc(kx + i);
+    const LimbScale<lf3> si = limb_lift<1>(&raw, sc);
+    const C2<lf3> v = limb_cin(raw, si);
     la[i] = make_float4(v.x.h, v.y.h, v.x.m, v.y.m);
     lb[i] = make_float2(v.x.l, v.y.l);
   }
@@ -268,7 +271,9 @@ __global__ void __launch_bounds__((L1 > L2 ? L1 : L2) * CW, 2)
     if (g < L1) {
 #pragma unroll
       for (int k2 = 0; k2 < L2; k2++) {
-        const C2<T> fl = limb_cin(in ? f[(long)(L1 * k2) * pitch] : C2<double>{0.0, 0.0}, sc);
+        C2<double> raw = in ? f[(long)(L1 * k2) * pitch] : C2<double>{0.0, 0.0};
+        const LimbScale<T> si = limb_lift<1>(&raw, sc);
+        const C2<T> fl = limb_cin(raw, si);
         u[k2] = limb_tw<false>(fl, MODE == 0 ? limb_cnorm(u[k2]) : u[k2]);
       }
       Dft<T, L2, true>::run(u);  // over k2 -> n2
@@ -505,7 +510,7 @@ __device__ __forceinline__ LimbGrow limb_c2r_first(Levels<R0, R...>, const C2<S>
   limb_fill_deep<T, NT, R0>(typename LV::Next{}, w, 0, twx);
   // |b[k]| + |b[M-k]| <= 2 sqrt(2) (|X[k]| + |X[M-k]|), and each of them <= 2 (|X[k]| + |X[M-k]|)
   LimbGrow grow = LimbGrow::of(limb_block_peak<NT>(limb_peak<2 * NP, 2>(x), red), 2.82843f, 2.f);
-  const LimbScale<T> sc = grow.first(R0);
+  const LimbScale<T> sc = limb_lift<2 * NP>(x, grow.first(R0));
 #pragma unroll
   for (int i = 0; i < NP; i++) {
     const int k = tid + i * NT;
@@ -615,7 +620,7 @@ __global__ void __launch_bounds__(NT)
   }
   limb_fill_deep<T, NT, LV::M / LV::Next::M>(typename LV::Next{}, w, 0, twx);
   LimbGrow grow = LimbGrow::of(limb_block_peak<NT>(limb_peak<NV, 1>(x), red), 1.f, 1.f);
-  const LimbScale<T> sc = grow.first(LV::M / LV::Next::M);
+  const LimbScale<T> sc = limb_lift<NV>(x, grow.first(LV::M / LV::Next::M));
 #pragma unroll
   for (int i = 0; i < NV; i++) {
     const int n = tid + i * NT;

@@ -139,7 +139,9 @@ __global__ void __launch_bounds__(512)
   for (int k = tid; k <= M / 2; k += NT) {
     C2<T> bk, bm;
     const int pk = any_inner(lv, 0, k), pm = k > 0 ? any_inner(lv, 0, M - k) : 0;
-    limb_c2r_pair(limb_cin(raw[pk], sc), cconj(limb_cin(k > 0 ? raw[pm] : top, sc)), twx.ld(k), bk, bm);
+    C2<S> x[2] = {raw[pk], k > 0 ? raw[pm] : top};
+    const LimbScale<T> si = limb_lift<2>(x, sc);
+    limb_c2r_pair(limb_cin(x[0], si), cconj(limb_cin(x[1], si)), twx.ld(k), bk, bm);
     s.st(pk, bk);
     if (k > 0 && k != M - k) s.st(pm, bm);
   }
@@ -178,7 +180,9 @@ __global__ void __launch_bounds__(512)
   const LimbScale<T> sc = grow.first(lv.r[0]);
   for (int n = tid; n < M; n += NT) {
     const int p = any_inner(lv, 0, n);
-    s.st(p, limb_cin(raw[p], sc));
+    C2<S> x = raw[p];
+    const LimbScale<T> si = limb_lift<1>(&x, sc);
+    s.st(p, limb_cin(x, si));
   }
   __syncthreads();
   any_row_transform<T, false>(s, lv, tab, w, grow);
@@ -238,7 +242,11 @@ __global__ void __launch_bounds__(ANY_NT, 2)
   }
   for (int e = threadIdx.x; e < lv.ntw; e += blockDim.x) w.st(e, tab.ld(e));
   const LimbScale<T> sc = limb_scale(any_column_sum(sum, red));
-  for (int j = g; j < L; j += G) s.st(j * ANY_CW + c, limb_cin(raw[j * ANY_CW + c], sc));
+  for (int j = g; j < L; j += G) {
+    C2<S> x = raw[j * ANY_CW + c];
+    const LimbScale<T> si = limb_lift<1>(&x, sc);
+    s.st(j * ANY_CW + c, limb_cin(x, si));
+  }
   __syncthreads();
   any_transform<T, INV, false, ANY_CW>(s, lv, w);
   for (int j = g; j < L; j += G) {
@@ -290,7 +298,9 @@ __global__ void __launch_bounds__(ANY_NT, 2)
   any_transform<T, false, false, ANY_CW>(s, lv, w);
   for (int k2 = g; k2 < N2; k2 += G) {
     const int p = any_output(lv, k2) * ANY_CW + c;
-    s.st(p, limb_tw<false>(limb_cin(ldc(f + (long)k2 * pitch), sf), limb_cnorm(s.ld(p))));
+    C2<double> x = ldc(f + (long)k2 * pitch);
+    const LimbScale<T> si = limb_lift<1>(&x, sf);
+    s.st(p, limb_tw<false>(limb_cin(x, si), limb_cnorm(s.ld(p))));
   }
   __syncthreads();
   any_transform<T, true, true, ANY_CW>(s, lv, w);

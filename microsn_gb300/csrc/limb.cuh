@@ -373,9 +373,8 @@ struct LimbScale<lf3> {
 __device__ __forceinline__ int limb_above(int field, float s) {
   return (field >> 20) - 1023 + ((__float_as_int(__fmul_rn(s, 1.f + 0x1p-17f)) >> 23) - 127) + 1;
 }
-// (values below 2^-1022 of a transform whose sum is below 2^-960 count as zero)
 __device__ __forceinline__ LimbScale<lf3> limb_scale(LimbSum<double> a) {
-  return LimbScale<lf3>{max(limb_above(a.e, a.s), -960), a.e >= 0x7ff00000};
+  return LimbScale<lf3>{limb_above(a.e, a.s), a.e >= 0x7ff00000};
 }
 
 // The scales of a row transform's levels: the values are at most p r_0 ... r_i in level i, p the
@@ -387,11 +386,11 @@ struct LimbGrow {
   bool bad;
   // bs, bp: what the transform's sum and its largest input are at most, in s and p of a
   static __device__ __forceinline__ LimbGrow of(LimbPeak a, float bs, float bp) {
-    return LimbGrow{a.e, max(limb_above(a.e, __fmul_rn(a.s, bs)), -960), 0, __fmul_rn(a.p, bp), a.e >= 0x7ff00000};
+    return LimbGrow{a.e, limb_above(a.e, __fmul_rn(a.s, bs)), 0, __fmul_rn(a.p, bp), a.e >= 0x7ff00000};
   }
   __device__ __forceinline__ int level(int r) {
     p = __fmul_rn(p, (float)r);
-    return max(min(top, limb_above(field, p)), -960);
+    return min(top, limb_above(field, p));
   }
   __device__ __forceinline__ LimbScale<lf3> first(int r) {
     e = level(r);
@@ -408,9 +407,10 @@ struct LimbGrow {
 // ---------------------------------------------------------------- in and out
 
 // FP64 in: the exponent moved by an integer addition, one conversion to a fixed-point
-// integer of 62 fractional bits, and its bit fields 22 | 17 | 23 as the three limbs.
+// integer of 62 fractional bits, and its bit fields 22 | 17 | 23 as the three limbs.  Subnormal
+// values count as zero: where the sum is so small that they matter, limb_lift comes first.
 __device__ __forceinline__ lf3 limb_in(double v, LimbScale<lf3> s) {
-  const int hi = __double2hiint(v), d = (62 - s.e) << 20;
+  const int hi = __double2hiint(v), d = (62 - s.e) * (1 << 20);
   const int ex = hi & 0x7ff00000;
   const bool z = ex == 0 || ex + d <= 0;
   const long long q = __double2ll_rn(z ? 0.0 : __hiloint2double(hi + d, __double2loint(v)));
@@ -431,8 +431,10 @@ __device__ __forceinline__ double limb_out(lf3 v, LimbScale<lf3> s) {
   const double d = __ll2double_rn(q);
   if (s.bad) return __longlong_as_double(0x7ff8000000000000ll);
   const int hi = __double2hiint(d), lo = __double2loint(d), ef = (hi >> 20) & 0x7ff, sh = s.e - 62, r = ef + sh;
-  if (ef == 0 || (unsigned)(r - 1) >= 2046u) {  // zero, or beyond the exponents: zero below, infinite above
-    return ef == 0 || r <= 0 ? 0.0 : __hiloint2double((hi & 0x80000000) | 0x7ff00000, 0);
+  if (ef == 0 || (unsigned)(r - 1) >= 2046u) {  // zero; beyond the exponents: infinite; below: rounded to a subnormal
+    if (ef == 0 || r < -60) return 0.0;
+    if (r > 0) return __hiloint2double((hi & 0x80000000) | 0x7ff00000, 0);
+    return __dmul_rn(__hiloint2double(hi + (sh + 64) * (1 << 20), lo), 0x1p-64);
   }
   return __hiloint2double(hi + (int)((unsigned)sh << 20), lo);
 }
@@ -445,6 +447,21 @@ __device__ __forceinline__ C2<T> limb_cin(C2<S> v, LimbScale<T> s) {
 template <typename S, typename T>
 __device__ __forceinline__ C2<S> limb_cout(C2<T> v, LimbScale<T> s) {
   return C2<S>{limb_out(v.x, s), limb_out(v.y, s)};
+}
+
+// The inputs of a transform and its scale, times 2^128 where the sum is below 2^-880: subnormal
+// inputs become normal.  (Asked once for all of them: asked for in every conversion it cost 7 %.)
+template <int N>
+__device__ __forceinline__ LimbScale<lf3> limb_lift(C2<double>* v, LimbScale<lf3> s) {
+  if (s.e < -880) {
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      v[i].x = __dmul_rn(v[i].x, 0x1p128);
+      v[i].y = __dmul_rn(v[i].y, 0x1p128);
+    }
+    s.e += 128;
+  }
+  return s;
 }
 
 // ---------------------------------------------------------------- arrays of limbs

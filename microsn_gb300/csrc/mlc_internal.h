@@ -136,6 +136,20 @@ struct mlc_ctx {
   std::map<std::string, std::string> tune_name;  // the choice as the report prints it
 };
 
+namespace mlc {
+// A host buffer to the device on the context's stream (a plain cudaMemcpy goes through the legacy
+// default stream, which streams of the caller's own do not wait for, nor it for them).  The
+// buffer may be reused at once where it is pageable; a caller's own may be page-locked.
+inline void upload(mlc_ctx* ctx, void* dst, const void* src, size_t bytes) {
+  MLC_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
+}
+// Device results to the host, there when it returns.
+inline void download(mlc_ctx* ctx, void* dst, const void* src, size_t bytes) {
+  MLC_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+  MLC_CUDA(cudaStreamSynchronize(ctx->stream));
+}
+}  // namespace mlc
+
 struct mlc_map {
   mlc_ctx* ctx = nullptr;
   int device = 0;  // kept here so that destroying a map never touches its context

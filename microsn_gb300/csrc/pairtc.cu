@@ -698,7 +698,7 @@ static int pd_epilogue_choice(mlc_ctx* ctx, int nkb, bool out, int nbins, long l
       MLC_CUDA(cudaEventRecord(b, ctx->stream));
       MLC_CUDA(cudaEventSynchronize(b));
       unsigned hc[4];
-      MLC_CUDA(cudaMemcpy(hc, counters, 16, cudaMemcpyDeviceToHost));
+      download(ctx, hc, counters, 16);
       MLC_REQUIRE(hc[2] == 0, MLC_ERR_TIMEOUT, "tensor-core pair kernel: a pipeline wait timed out");
       float t = 0.f;
       MLC_CUDA(cudaEventElapsedTime(&t, a, b));
@@ -761,7 +761,7 @@ static void pairdiff_core(mlc_ctx* ctx, int method, const float* A, const float*
     const double expect = (double)k * (double)S / (double)P;
     const long rank = std::min<long>(S - 1, (long)std::ceil(4.0 * expect) + 16);
     uint64_t u = 0;
-    MLC_CUDA(cudaMemcpy(&u, sk + rank, 8, cudaMemcpyDeviceToHost));
+    download(ctx, &u, sk + rank, 8);
     double v;
     std::memcpy(&v, &u, 8);
     thr = v;
@@ -857,7 +857,7 @@ static void pairdiff_core(mlc_ctx* ctx, int method, const float* A, const float*
           MLC_CUDA(cudaMemcpyAsync(hc.data(), chunk, sizeof(double) * hc.size(), cudaMemcpyDeviceToHost, ctx->stream));
           MLC_CUDA(cudaStreamSynchronize(ctx->stream));
           std::vector<float> hf(hc.begin(), hc.end());
-          MLC_CUDA(cudaMemcpy(out + r0 * NB, hf.data(), sizeof(float) * hf.size(), cudaMemcpyHostToDevice));
+          upload(ctx, out + r0 * NB, hf.data(), sizeof(float) * hf.size());
         }
         const long n = nr * NB;
         const size_t hsm = sizeof(uint32_t) * (nbins + 2);
@@ -902,10 +902,10 @@ static void pairdiff_core(mlc_ctx* ctx, int method, const float* A, const float*
     }
     break;
   }
-  if (hist_host) MLC_CUDA(cudaMemcpy(hist_host, hist, 8 * (size_t)nbins, cudaMemcpyDeviceToHost));
+  if (hist_host) download(ctx, hist_host, hist, 8 * (size_t)nbins);
   {
     unsigned long long oor[2];
-    MLC_CUDA(cudaMemcpy(oor, hist + nbins, sizeof oor, cudaMemcpyDeviceToHost));
+    download(ctx, oor, hist + nbins, sizeof oor);
     res.below = (long long)oor[0];
     res.above = (long long)oor[1];
   }
@@ -938,9 +938,9 @@ static void pairdiff_core(mlc_ctx* ctx, int method, const float* A, const float*
     // the first k + 1024 by value; order ties by pair index on the host
     std::vector<float> hv(m);
     std::vector<int> hi_(m), hj(m);
-    MLC_CUDA(cudaMemcpy(hv.data(), gv, 4 * (size_t)m, cudaMemcpyDeviceToHost));
-    MLC_CUDA(cudaMemcpy(hi_.data(), gi, 4 * (size_t)m, cudaMemcpyDeviceToHost));
-    MLC_CUDA(cudaMemcpy(hj.data(), gj, 4 * (size_t)m, cudaMemcpyDeviceToHost));
+    download(ctx, hv.data(), gv, 4 * (size_t)m);
+    download(ctx, hi_.data(), gi, 4 * (size_t)m);
+    download(ctx, hj.data(), gj, 4 * (size_t)m);
     const unsigned ncand_used = m;
     std::vector<uint32_t> idx(ncand_used);
     for (unsigned q = 0; q < ncand_used; q++) idx[q] = q;

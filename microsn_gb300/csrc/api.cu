@@ -348,9 +348,8 @@ static const double* upload_profile(mlc_ctx* ctx, const mlc_profile& pr, int* pN
   std::vector<double> h((size_t)N * N);
   MLC_REQUIRE(profile_raster(pr, h.data(), (long)h.size()) == N, MLC_ERR_ARG, "profile raster failed");
   double* d = (double*)ws_get(ctx, WS_PROFILE, sizeof(double) * h.size());
-  // synchronous copy: the host buffer dies with this function
   MLC_CUDA(cudaStreamSynchronize(ctx->stream));
-  MLC_CUDA(cudaMemcpy(d, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice));
+  upload(ctx, d, h.data(), sizeof(double) * h.size());
   *pN = N;
   return d;
 }
@@ -578,9 +577,9 @@ int mlc_chi2_offset(mlc_ctx* ctx, int precision, int ncurves, int T, const void*
   if (!(W > 0)) return fail(ctx, MLC_ERR_ARG, "weights must sum to a positive number");
   return guarded(ctx, [&] {
     double* buf = (double*)ws_get(ctx, WS_SMALL, sizeof(double) * 2 * T);
+    upload(ctx, buf, obs_host, sizeof(double) * T);
+    upload(ctx, buf + T, w_host, sizeof(double) * T);
     MLC_CUDA(cudaStreamSynchronize(ctx->stream));
-    MLC_CUDA(cudaMemcpy(buf, obs_host, sizeof(double) * T, cudaMemcpyHostToDevice));
-    MLC_CUDA(cudaMemcpy(buf + T, w_host, sizeof(double) * T, cudaMemcpyHostToDevice));
     chi2_offset(ctx, precision, ncurves, T, m, buf, buf + T, W, chi2, dm);
   });
 }
@@ -681,9 +680,9 @@ int mlc_pair_chi2_magdiff_list(mlc_ctx* ctx, int NA, int NB, int T, const float*
     for (int t = 0; t < T; t++) W += w_host[t];
     MLC_REQUIRE(W > 0, MLC_ERR_ARG, "weights sum to zero");
     double* buf = (double*)ws_get(ctx, WS_SMALL, sizeof(double) * 2 * T);
+    upload(ctx, buf, w_host, sizeof(double) * T);
+    if (d_host) upload(ctx, buf + T, d_host, sizeof(double) * T);
     MLC_CUDA(cudaStreamSynchronize(ctx->stream));
-    MLC_CUDA(cudaMemcpy(buf, w_host, sizeof(double) * T, cudaMemcpyHostToDevice));
-    if (d_host) MLC_CUDA(cudaMemcpy(buf + T, d_host, sizeof(double) * T, cudaMemcpyHostToDevice));
     pairdiff_plain(ctx, A, B, NA, NB, T, buf, d_host ? buf + T : nullptr, W, offset, npairs, (const long*)ia,
                    (const long*)ib, chi2);
   });

@@ -325,6 +325,8 @@ FftPlan2D* plan_get(mlc_ctx* ctx, int Nx, int Ny, int prec) {
   p->anyM_tw = upload_any(p->anyM, prec);
   p->any1_tw = upload_any(p->any1, prec);
   p->any2_tw = upload_any(p->any2, prec);
+  // (the tables' copies went through the legacy default stream: they are there for any stream)
+  MLC_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
   FftPlan2D* raw = p.get();
   ctx->plans[key] = std::move(p);
   return raw;

@@ -243,7 +243,7 @@ void radius_stack(mlc_ctx* ctx, mlc_map* map, int K, const double* radii, double
   }
   double* dprof = (double*)ws_get(ctx, WS_PROFILE, h.size() * sizeof(double));
   MLC_CUDA(cudaStreamSynchronize(ctx->stream));
-  MLC_CUDA(cudaMemcpy(dprof, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice));
+  upload(ctx, dprof, h.data(), h.size() * sizeof(double));
   const long npix = (long)map->Nx * map->Ny;
   const size_t es = map->prec == MLC_F64 ? 8 : 4;
   constexpr int G = 4;  // radii per group: 16 convolved maps, then one interleave pass

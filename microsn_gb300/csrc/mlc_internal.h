@@ -123,6 +123,7 @@ struct mlc_ctx {
   std::map<std::string, std::pair<double, long>> ktimes;  // name -> (ms, launches)
   void* ws_ptr[mlc::WS_NSLOTS] = {};
   size_t ws_size[mlc::WS_NSLOTS] = {};
+  const double* exp_table = nullptr;  // WS_EXP_TAB, once its values are there
   std::map<std::tuple<int, int, int>, std::unique_ptr<mlc::FftPlan2D>> plans;
   mlc::BatchIO* batch = nullptr;
   // launch autotuner: key -> choice (-1: FFT form; >= 0: direct tile shape), candidate timings

@@ -212,15 +212,17 @@ __device__ __forceinline__ double exp_neg_half(double c, const double* tab) {
   return __hiloint2double(__double2hiint(e) + ((ki >> 12) << 20), __double2loint(e));
 }
 
-// 2^(j/4096) on the device, made once per context.
+// 2^(j/4096) on the device, made once per context (and there for any stream it is given later).
 static const double* exp_table(mlc_ctx* ctx) {
-  if (!ctx->ws_ptr[WS_EXP_TAB]) {
+  if (!ctx->exp_table) {
     std::vector<double> h(EXP_TAB);
     for (int j = 0; j < EXP_TAB; j++) h[j] = (double)exp2l((long double)j / EXP_TAB);
     void* d = ws_get(ctx, WS_EXP_TAB, sizeof(double) * EXP_TAB);
-    MLC_CUDA(cudaMemcpy(d, h.data(), sizeof(double) * EXP_TAB, cudaMemcpyHostToDevice));
+    upload(ctx, d, h.data(), sizeof(double) * EXP_TAB);
+    MLC_CUDA(cudaStreamSynchronize(ctx->stream));
+    ctx->exp_table = (const double*)d;
   }
-  return (const double*)ctx->ws_ptr[WS_EXP_TAB];
+  return ctx->exp_table;
 }
 __device__ __forceinline__ void load_exp_table(const double* __restrict__ src, double* dst) {
   for (int i = threadIdx.x; i < EXP_TAB / 2; i += blockDim.x)
@@ -538,7 +540,7 @@ static Interp build_interp(mlc_ctx* ctx, int Njp, const int* indA, const int* in
   int* hi = reinterpret_cast<int*>(hd + 6 * Njp);
   std::copy(indA, indA + Njp, hi);
   std::copy(indB, indB + Njp, hi + Njp);
-  MLC_CUDA(cudaMemcpy(fA, h.data(), h.size(), cudaMemcpyHostToDevice));
+  upload(ctx, fA, h.data(), h.size());
   if (n > 0) {
     {
       MLC_KSCOPE(ctx, "pair_interp");

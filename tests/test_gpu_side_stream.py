@@ -21,6 +21,57 @@ def side():
     c.close()
 
 
+def _vars(d, s):
+    import microsn_gb300 as mlc
+    return mlc.Chi2Vars(3, np.array([0, 1, -1], np.int32), np.array([1, -1, 0], np.int32), np.array([0.3, 0.6, 0.0]),
+                        np.array([0.2, 0.0, 0.9]), np.array(d), np.array(s), 0.0)
+
+
+def test_ratio_chi2_of_two_calls_in_a_row(ctx, side):
+    import microsn_gb300 as mlc
+    c, s, busy = side
+    rng = np.random.default_rng(3)
+    A, B = (torch.as_tensor(np.exp(rng.normal(0, 0.5, (300, 3))), device=DEV) for _ in range(2))
+    dA, dB = torch.diff(A, dim=1).contiguous(), torch.diff(B, dim=1).contiguous()
+    both = [_vars([0.7, 1.2, 1.1], [0.1, 0.15, 0.3]), _vars([1.7, 0.4, 0.9], [0.2, 0.05, 0.6])]
+    want = [mlc.calculate_chi2(ctx, v, A, dA, B, dB).clone() for v in both]
+    edges = mlc.bin_edges(50, 1e-2, 1e2)
+    fused = [mlc.pair_bin_fused(ctx, v, A, dA, B, dB, edges) for v in both]
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        mlc.calculate_chi2(c, both[0], A, dA, B, dB)  # (workspaces made)
+        s.synchronize()
+        busy()
+        got = [mlc.calculate_chi2(c, v, A, dA, B, dB) for v in both]
+        busy()
+        binned = [mlc.pair_bin_fused(c, v, A, dA, B, dB, edges) for v in both]
+    s.synchronize()
+    for w, g in zip(want, got):
+        assert torch.equal(w, g)
+    for w, g in zip(fused, binned):
+        assert np.array_equal(w[2], g[2])
+        for k in range(2):
+            np.testing.assert_allclose(g[k], w[k], rtol=1e-13)  # (sums of 90000 values in no fixed order)
+
+
+def test_convolution_of_two_profiles_in_a_row(ctx, side):
+    import microsn_gb300 as mlc
+    c, s, busy = side
+    mp = torch.rand((360, 360), dtype=torch.float64, device=DEV)
+    profs = [mlc.profile("gaussian", 3.0, 1.0, ref_compat=False), mlc.profile("gaussian", 4.0, 1.0, ref_compat=False)]
+    m = mlc.Map(ctx, mp, "f64")
+    want = [mlc.convolve(ctx, m, p).clone() for p in profs]
+    m.close()
+    with torch.cuda.stream(s):
+        m = mlc.Map(c, mp, "f64")
+        busy()
+        got = [mlc.convolve(c, m, p) for p in profs]
+        s.synchronize()
+        m.close()
+    for w, g in zip(want, got):
+        assert torch.equal(w, g)
+
+
 @pytest.mark.parametrize("k", [50, 3000])
 def test_best_pairs(ctx, side, k):
     import microsn_gb300 as mlc
@@ -36,3 +87,19 @@ def test_best_pairs(ctx, side, k):
             got = mlc.pair_chi2_magdiff(c, A, B, w, None, True, nbins=100, lo=-1.0, hi=9.0, k=k)
         for name in ("hist", "topk_val", "topk_i", "topk_j"):
             assert np.array_equal(np.asarray(want[name]), np.asarray(got[name])), name
+
+
+def test_offset_chi2_of_two_calls_in_a_row(ctx, side):
+    import microsn_gb300 as mlc
+    c, s, busy = side
+    m = torch.rand((500, 30), dtype=torch.float64, device=DEV)
+    obs = [np.linspace(0, 1, 30), np.linspace(1, -1, 30)]
+    w = [np.full(30, 9.0), np.linspace(1, 4, 30)]
+    want = [mlc.chi2_offset(ctx, m, o, x) for o, x in zip(obs, w)]
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        busy()
+        got = [mlc.chi2_offset(c, m, o, x) for o, x in zip(obs, w)]
+    s.synchronize()
+    for a, b in zip(want, got):
+        assert all(torch.equal(p, q) for p, q in zip(a, b))

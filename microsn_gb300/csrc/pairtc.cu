@@ -224,6 +224,10 @@ __global__ void __launch_bounds__(Epi<EPIW>::threads, 1) k_pairdiff_tc(const __g
     *abort_s = 1;
     atomicExch(P.err, 1);
   };
+  // For whole warps: one answer for all lanes (their own reads of the flag, or their own waits, may
+  // differ, and lanes that leave a loop are missed by the votes and barriers inside it).
+  auto warp_aborted = [&]() { return __shfl_sync(0xffffffffu, *abort_s, 0) != 0; };
+  auto warp_wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, tc::mbar_wait(bar, parity)) != 0; };
 
   if (warp == 0 && lane == 0) {
     // ------------------------------------------------ TMA producer
@@ -254,14 +258,13 @@ __global__ void __launch_bounds__(Epi<EPIW>::threads, 1) k_pairdiff_tc(const __g
     // base + offset is the base descriptor plus offset >> 4 in its low word (no carry).
     const uint64_t dA = tc::desc_sw128(tc::smem_u32(A_s)), dB = tc::desc_sw128(tc::smem_u32(B_s));
     const uint32_t a_hi = (uint32_t)(dA >> 32), a_lo = (uint32_t)dA, b_hi = (uint32_t)(dB >> 32), b_lo = (uint32_t)dB;
-    for (int it = blockIdx.x; it < P.nitems && !*abort_s; it += gridDim.x, n++) {
+    for (int it = blockIdx.x; it < P.nitems && !warp_aborted(); it += gridDim.x, n++) {
       const int jc = it % P.njc;
       const int j0 = jc * P.jchunk, j1 = min(P.nj, j0 + P.jchunk);
-      if (!__all_sync(0xffffffffu, tc::mbar_wait(a_full, n & 1))) { fail(); break; }
+      if (!warp_wait(a_full, n & 1)) { fail(); break; }
       for (int jt = j0; jt < j1; jt++, cB++, ct++) {
         const uint32_t s = cB & 1, u = cB >> 1, tb = ct & 1, tu = ct >> 1;
-        if (!__all_sync(0xffffffffu, !*abort_s && tc::mbar_wait(b_full + s, u & 1) &&
-                                         tc::mbar_wait(t_empty + tb, (tu & 1) ^ 1))) {
+        if (warp_aborted() || !warp_wait(b_full + s, u & 1) || !warp_wait(t_empty + tb, (tu & 1) ^ 1)) {
           fail();
           break;
         }
@@ -330,7 +333,7 @@ __global__ void __launch_bounds__(Epi<EPIW>::threads, 1) k_pairdiff_tc(const __g
       fetch(j0);
       for (int jt = j0; jt < j1; jt++, ct++) {
         const uint32_t tb = ct & 1, tu = ct >> 1;
-        if (*abort_s) break;
+        if (warp_aborted()) break;
         // (the previous tile's reads of cv ended at the __syncwarp closing it)
         if (lane < WCOLS) {
           float* bp = cv + lane / 2 * 8 + (lane & 1);
@@ -340,7 +343,7 @@ __global__ void __launch_bounds__(Epi<EPIW>::threads, 1) k_pairdiff_tc(const __g
         }
         fetch(jt + 1);
         __syncwarp();
-        if (!tc::mbar_wait(t_full + tb, tu & 1)) {
+        if (!warp_wait(t_full + tb, tu & 1)) {
           fail();
           break;
         }

@@ -114,18 +114,22 @@ __global__ void k_upper_bound(const uint64_t* __restrict__ sorted, long P, const
 }
 
 // m[i*Nloc + a] = LC[a*Nprof + ind_i] + fac_i * DLC[a*(Nprof-1) + ind_i], or 1 (ind_i = -1).
-// The B side (rho given) as rho_i / m, rho_i = rho[i] + rho[Njp + i], rounded once: one division
-// per (epoch, location) instead of one per pair.
+// The B side (rho given): B_i = rho_i / m, rho_i = rho[i] + rho[Njp + i], rounded once: one division
+// per (epoch, location) instead of one per pair; and 1 / m in inv.  *plain is set where a B_i
+// is beyond the exponents that 1 / m still has (m near the ends of FP64).
 __global__ void k_interp(const double* __restrict__ LC, const double* __restrict__ DLC, int Nloc, int Nprof,
                          int Njp, const int* __restrict__ ind, const double* __restrict__ fac,
-                         const double* __restrict__ rho, double* __restrict__ m) {
+                         const double* __restrict__ rho, double* __restrict__ m, double* __restrict__ inv,
+                         int* __restrict__ plain) {
   const long n = (long)Nloc * Njp;
   for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) {
     const int i = (int)(q / Nloc), a = (int)(q % Nloc);
     const int k = ind[i];
     double v = (k == -1) ? 1.0 : LC[(long)a * Nprof + k] + fac[i] * DLC[(long)a * (Nprof - 1) + k];
     if (rho) {
+      inv[q] = 1.0 / v;
       const double h = rho[i] / v, r = __fma_rn(-h, v, rho[i]) + rho[Njp + i];
+      if (v != 0.0 && isfinite(v) && !(fabs(h) >= 0x1p-960 && fabs(h) <= 0x1p960)) *plain = 1;
       // (a quotient that is 0, infinite or NaN has no residual)
       v = isfinite(h) && h != 0.0 && isfinite(r) ? h + r / v : h;
     }
@@ -149,38 +153,47 @@ __global__ void k_zvalues(const double* __restrict__ LC, int Nloc, int Nprof, in
 // (to twice the precision).  d_i/s_i is rounded, but rho_i follows it, so that t = rho_i (d_i -
 // mA_i/mB_i) with the one rounding of B_i inside the difference -- as 1/mB_i's would be -- and
 // a factor rho_i within one ulp of 1/s_i.  Where d_i or s_i is zero, not finite or of an extreme
-// exponent (PLAIN) the terms are (d_i - mA_i RN(1/mB_i)) RN(1/s_i).
-template <bool PLAIN>
+// exponent, or a B_i would be, the terms are (d_i - mA_i RN(1/mB_i)) RN(1/s_i) (*plain).
 struct RatioChi2 {
   const double* mA;
-  const double* iB;
-  const double* d;   // ds_i, or d_i
-  const double* is;  // 1 / s_i (PLAIN)
+  const double* iB;   // B_i
+  const double* inv;  // 1 / mB_i
+  const double* ds;
+  const double* d;
+  const double* is;  // 1 / s_i
+  const int* plain;
   int Nloc, Njp;
-  __device__ __forceinline__ double operator()(int a, int b) const {
+  __device__ __forceinline__ double operator()(int a, int b, bool pl) const {
+    const double* A = mA + a;
     double c = 0.0;
-    for (int i = 0; i < Njp; i++) {
-      double t = __fma_rn(-__ldg(mA + (long)i * Nloc + a), __ldg(iB + (long)i * Nloc + b), __ldg(d + i));
-      if (PLAIN) t *= __ldg(is + i);
-      c = __fma_rn(t, t, c);
+    if (!pl) {
+      for (int i = 0; i < Njp; i++) {
+        const double t = __fma_rn(-__ldg(A + (long)i * Nloc), __ldg(iB + (long)i * Nloc + b), __ldg(ds + i));
+        c = __fma_rn(t, t, c);
+      }
+    } else {
+#pragma unroll 1
+      for (int i = 0; i < Njp; i++) {
+        const double t = __fma_rn(-__ldg(A + (long)i * Nloc), __ldg(inv + (long)i * Nloc + b), __ldg(d + i)) * __ldg(is + i);
+        c = __fma_rn(t, t, c);
+      }
     }
     return c;
   }
   __device__ __forceinline__ double operator()(long p) const {  // pair index a Nloc + b, below 2^32
     const uint32_t a = (uint32_t)p / (uint32_t)Nloc;
-    return (*this)((int)a, (int)((uint32_t)p - a * (uint32_t)Nloc));
+    return (*this)((int)a, (int)((uint32_t)p - a * (uint32_t)Nloc), __ldg(plain) != 0);
   }
 };
 
 // One pair per thread, in pair order, or at its rank.
-template <bool PLAIN>
-__global__ void __launch_bounds__(256) k_pair_chi2_ratio(RatioChi2<PLAIN> f, const uint32_t* __restrict__ rank,
+__global__ void __launch_bounds__(256) k_pair_chi2_ratio(RatioChi2 f, const uint32_t* __restrict__ rank,
                                                          double* __restrict__ chi2) {
   const int b = blockIdx.x * 32 + (threadIdx.x & 31);
   const int a = blockIdx.y * 8 + (threadIdx.x >> 5);
   if (a >= f.Nloc || b >= f.Nloc) return;
   const long p = (long)a * f.Nloc + b;
-  chi2[rank ? rank[p] : p] = f(a, b);
+  chi2[rank ? rank[p] : p] = f(a, b, __ldg(f.plain) != 0);
 }
 
 // Bin means of the rank-ordered chi2 (bin_chi2_GPU): every bin's slice is cut into pieces
@@ -326,8 +339,7 @@ __device__ __forceinline__ int edge_search(const double* e, int nb, double z) {
   return lo;
 }
 
-template <bool PLAIN>
-__global__ void __launch_bounds__(256) k_pair_bin_fused(RatioChi2<PLAIN> f, FusedSide A, FusedSide B, int na, int nb,
+__global__ void __launch_bounds__(256) k_pair_bin_fused(RatioChi2 f, FusedSide A, FusedSide B, int na, int nb,
                                                         const double* __restrict__ edges,
                                                         const double* __restrict__ etab, int copies,
                                                         double* __restrict__ gsum, double* __restrict__ gexp,
@@ -344,6 +356,7 @@ __global__ void __launch_bounds__(256) k_pair_bin_fused(RatioChi2<PLAIN> f, Fuse
     atomicAdd(gexp + copy + bin, se);
     atomicAdd(gcnt + copy + bin, (unsigned long long)cn);
   };
+  const bool plain = __ldg(f.plain) != 0;
   const int b = blockIdx.x * 256 + threadIdx.x;
   if (b < f.Nloc) {
     const float zb = __ldg(B.zf + b);
@@ -388,7 +401,7 @@ __global__ void __launch_bounds__(256) k_pair_bin_fused(RatioChi2<PLAIN> f, Fuse
         above = fminf(above, 0x1p100f);
       }
       if (bin >= nb) continue;
-      const double c = f(a, b);
+      const double c = f(a, b, plain);
       sc += c;
       se += exp_neg_half(c, tab);
       cn++;
@@ -488,20 +501,12 @@ void pair_setup(mlc_ctx* ctx, int Nloc, int Nprof, const double* LCA, const doub
   }
 }
 
-struct Interp {
-  double* mA;
-  double* iB;  // B_i (see RatioChi2), 1 / mB_i where plain
-  double* d;
-  double* is;
-  bool plain;
-};
-
 static bool moderate_host(double v) {
   int e = 0;
   return std::isfinite(v) && v != 0.0 && (std::frexp(v, &e), e > -400 && e < 400);
 }
 
-static Interp build_interp(mlc_ctx* ctx, int Njp, const int* indA, const int* indB, const double* facA,
+static RatioChi2 build_interp(mlc_ctx* ctx, int Njp, const int* indA, const int* indB, const double* facA,
                            const double* facB, const double* d, const double* s, int Nloc, int Nprof,
                            const double* LCA, const double* DLCA, const double* LCB, const double* DLCB) {
   const long n = (long)Nloc * Njp;
@@ -509,74 +514,69 @@ static Interp build_interp(mlc_ctx* ctx, int Njp, const int* indA, const int* in
     MLC_REQUIRE(indA[i] >= -1 && indA[i] < Nprof - 1 && indB[i] >= -1 && indB[i] < Nprof - 1, MLC_ERR_ARG,
                 "interpolation index out of the profile range");
   }
-  // small tables: fac A/B, d (ds), 1/s, rho (two rows); ind A/B (int)
-  size_t small = sizeof(double) * 6 * Njp + sizeof(int) * 2 * Njp + 64;
-  char* sm = (char*)ws_get(ctx, WS_LOC, sizeof(double) * 2 * n + small);
-  Interp I;
-  I.mA = (double*)sm;
-  I.iB = I.mA + n;
-  double* fA = I.iB + n;
+  // small tables: fac A/B, ds, d, 1/s, rho (two rows); ind A/B, plain (int)
+  const size_t nd = 7 * (size_t)Njp, ni = 2 * (size_t)Njp + 1;
+  char* sm = (char*)ws_get(ctx, WS_LOC, sizeof(double) * (3 * n + nd) + sizeof(int) * ni + 64);
+  double* mA = (double*)sm;
+  double* iB = mA + n;
+  double* inv = iB + n;
+  double* fA = inv + n;
   double* fB = fA + Njp;
-  I.d = fB + Njp;
-  I.is = I.d + Njp;
-  double* rho = I.is + Njp;
-  int* iA = reinterpret_cast<int*>(rho + 2 * Njp);
-  int* iB = iA + Njp;
-  I.plain = false;
-  for (int i = 0; i < Njp; i++) I.plain |= !moderate_host(d[i]) || !moderate_host(s[i]);
-  std::vector<char> h(sizeof(double) * 6 * Njp + sizeof(int) * 2 * Njp);
+  double* rho = fB + 4 * Njp;
+  int* iA = reinterpret_cast<int*>(fA + nd);
+  int* iBx = iA + Njp;
+  int* plain = iBx + Njp;
+  bool pl = false;
+  for (int i = 0; i < Njp; i++) pl |= !moderate_host(d[i]) || !moderate_host(s[i]);
+  std::vector<char> h(sizeof(double) * nd + sizeof(int) * ni);
   double* hd = reinterpret_cast<double*>(h.data());
   std::copy(facA, facA + Njp, hd);
   std::copy(facB, facB + Njp, hd + Njp);
   for (int i = 0; i < Njp; i++) {
     const double ds = d[i] / s[i];
-    hd[2 * Njp + i] = I.plain ? d[i] : ds;
-    hd[3 * Njp + i] = 1.0 / s[i];
+    hd[2 * Njp + i] = ds;
+    hd[3 * Njp + i] = d[i];
+    hd[4 * Njp + i] = 1.0 / s[i];
     // rho = ds / d to twice the precision: its rounding, then the exact residual over d
-    const double rh = I.plain ? 1.0 : ds / d[i];
-    hd[4 * Njp + i] = rh;
-    hd[5 * Njp + i] = I.plain ? 0.0 : std::fma(-rh, d[i], ds) / d[i];
+    const double rh = pl ? 1.0 : ds / d[i];
+    hd[5 * Njp + i] = rh;
+    hd[6 * Njp + i] = pl ? 0.0 : std::fma(-rh, d[i], ds) / d[i];
   }
-  int* hi = reinterpret_cast<int*>(hd + 6 * Njp);
+  int* hi = reinterpret_cast<int*>(hd + nd);
   std::copy(indA, indA + Njp, hi);
   std::copy(indB, indB + Njp, hi + Njp);
+  hi[2 * Njp] = pl;
   upload(ctx, fA, h.data(), h.size());
   if (n > 0) {
     {
       MLC_KSCOPE(ctx, "pair_interp");
-      k_interp<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(LCA, DLCA, Nloc, Nprof, Njp, iA, fA, nullptr, I.mA);
+      k_interp<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(LCA, DLCA, Nloc, Nprof, Njp, iA, fA, nullptr, mA, nullptr,
+                                                          nullptr);
     }
     MLC_CHECK_LAUNCH();
     {
       MLC_KSCOPE(ctx, "pair_interp");
-      k_interp<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(LCB, DLCB, Nloc, Nprof, Njp, iB, fB, rho, I.iB);
+      k_interp<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(LCB, DLCB, Nloc, Nprof, Njp, iBx, fB, rho, iB, inv, plain);
     }
     MLC_CHECK_LAUNCH();
   }
-  return I;
-}
-
-template <bool PLAIN>
-static void pair_chi2_run(mlc_ctx* ctx, const Interp& I, int Nloc, int Njp, const uint32_t* rank, double* chi2) {
-  const RatioChi2<PLAIN> f{I.mA, I.iB, I.d, I.is, Nloc, Njp};
-  if (rank && (long)Nloc * Nloc <= 0xFFFFFFFFl) {
-    put_by_index(ctx, "pair_chi2_ratio", rank, f, (long)Nloc * Nloc, chi2);
-    return;
-  }
-  {
-    MLC_KSCOPE(ctx, "pair_chi2_ratio");
-    k_pair_chi2_ratio<PLAIN><<<dim3(ceil_div(Nloc, 32), ceil_div(Nloc, 8)), 256, 0, ctx->stream>>>(f, rank, chi2);
-  }
-  MLC_CHECK_LAUNCH();
+  return RatioChi2{mA, iB, inv, fB + Njp, fB + 2 * Njp, fB + 3 * Njp, plain, Nloc, Njp};
 }
 
 void pair_chi2_ratio(mlc_ctx* ctx, int Njp, const int* indA, const int* indB, const double* facA,
                      const double* facB, const double* d, const double* s, int Nloc, int Nprof, const double* LCA,
                      const double* DLCA, const double* LCB, const double* DLCB, const uint32_t* rank, double* chi2) {
   if (Nloc <= 0) return;
-  Interp I = build_interp(ctx, Njp, indA, indB, facA, facB, d, s, Nloc, Nprof, LCA, DLCA, LCB, DLCB);
-  if (I.plain) pair_chi2_run<true>(ctx, I, Nloc, Njp, rank, chi2);
-  else pair_chi2_run<false>(ctx, I, Nloc, Njp, rank, chi2);
+  const RatioChi2 f = build_interp(ctx, Njp, indA, indB, facA, facB, d, s, Nloc, Nprof, LCA, DLCA, LCB, DLCB);
+  if (rank && (long)Nloc * Nloc <= 0xFFFFFFFFl) {
+    put_by_index(ctx, "pair_chi2_ratio", rank, f, (long)Nloc * Nloc, chi2);
+    return;
+  }
+  {
+    MLC_KSCOPE(ctx, "pair_chi2_ratio");
+    k_pair_chi2_ratio<<<dim3(ceil_div(Nloc, 32), ceil_div(Nloc, 8)), 256, 0, ctx->stream>>>(f, rank, chi2);
+  }
+  MLC_CHECK_LAUNCH();
 }
 
 void bin_chi2(mlc_ctx* ctx, int Nbins, const uint32_t* lower_host, const uint32_t* nper_host,
@@ -642,14 +642,13 @@ void pair_bin_fused(mlc_ctx* ctx, int Njp, const int* indA, const int* indB, con
     k_zvalues<<<grid_for(ctx, Nloc), 256, 0, ctx->stream>>>(LCB, Nloc, Nprof, 1, z + N, zf + N);
   }
   MLC_CHECK_LAUNCH();
-  Interp I = build_interp(ctx, Njp, indA, indB, facA, facB, d, s, Nloc, Nprof, LCA, DLCA, LCB, DLCB);
+  const RatioChi2 f = build_interp(ctx, Njp, indA, indB, facA, facB, d, s, Nloc, Nprof, LCA, DLCA, LCB, DLCB);
   MLC_CUDA(cudaMemcpyAsync(de, edges_host, sizeof(double) * Nbins, cudaMemcpyHostToDevice, ctx->stream));
   MLC_CUDA(cudaMemsetAsync(gs, 0, 8 * 3 * NC, ctx->stream));
   const size_t smem = sizeof(double) * EXP_TAB + sizeof(float) * Nbins;
   const double* etab = exp_table(ctx);
   if (Nloc > 0) {
-    const void* k = I.plain ? (const void*)k_pair_bin_fused<true> : (const void*)k_pair_bin_fused<false>;
-    set_max_smem(k, smem);
+    set_max_smem((const void*)k_pair_bin_fused, smem);
     // A places per CTA: as many as leave four CTAs for every SM
     const int cols = ceil_div(Nloc, 256);
     const int na = (int)std::max<long>(4, std::min<long>(FUSED_A, (long)Nloc * cols / (4 * ctx->sm_count)));
@@ -657,12 +656,7 @@ void pair_bin_fused(mlc_ctx* ctx, int Njp, const int* indA, const int* indB, con
     const FusedSide A{z, zf}, B{z + N, zf + N};
     {
       MLC_KSCOPE(ctx, "pair_bin_fused");
-      if (I.plain)
-        k_pair_bin_fused<true><<<grid, 256, smem, ctx->stream>>>(RatioChi2<true>{I.mA, I.iB, I.d, I.is, Nloc, Njp}, A, B,
-                                                                 na, Nbins, de, etab, copies, gs, ge, gc);
-      else
-        k_pair_bin_fused<false><<<grid, 256, smem, ctx->stream>>>(RatioChi2<false>{I.mA, I.iB, I.d, I.is, Nloc, Njp},
-                                                                  A, B, na, Nbins, de, etab, copies, gs, ge, gc);
+      k_pair_bin_fused<<<grid, 256, smem, ctx->stream>>>(f, A, B, na, Nbins, de, etab, copies, gs, ge, gc);
     }
     MLC_CHECK_LAUNCH();
     MLC_KSCOPE(ctx, "pair_bin_combine");

@@ -14,8 +14,8 @@
 //
 // f/df is rounded, but rho follows it, so t = rho (f - mu1/mu2) with the one rounding of B inside
 // the difference, as 1/mu2 would have, and a factor rho within 2^-24 of 1/df.  (f = 0: rho =
-// RN(1/df).)  Few locations, or an f or df that is not of moderate size: t = (f - mu1 RN(1/mu2))
-// RN(1/df), three operations.
+// RN(1/df).)  Few locations, or an f or df that is not of moderate size, or a B beyond the exponents that
+// 1/mu2 still has: t = (f - mu1 RN(1/mu2)) RN(1/df), three operations.
 // exp(-chi2) is summed per thread relative to its smallest chi2 (FP32 terms, one FP64-range
 // exp per thread), per CTA in FP64, and the CTA sums are added in a fixed order
 // (deterministic).  chi2 is stored only when asked for.
@@ -194,10 +194,11 @@ __global__ void __launch_bounds__(256) k_flux_ratio(const float* __restrict__ mu
 }
 
 // mu1 and B in the order [k][location] with Np locations a row (zeros past N), 32 x 32 values per
-// CTA through shared memory.  blockIdx.z: 0 mu1, 1 B.
+// CTA through shared memory.  blockIdx.z: 0 mu1, 1 B.  *beyond is set where a B of an ordinary
+// mu2 is near or past the ends of FP32.
 __global__ void __launch_bounds__(256) k_flux_layout(const float* __restrict__ mu1, const float* __restrict__ mu2,
                                                      FluxTables tab, int N, int Np, int K, float* __restrict__ a,
-                                                     float* __restrict__ b) {
+                                                     float* __restrict__ b, int* __restrict__ beyond) {
   __shared__ float t[32][33];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int l0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
@@ -208,7 +209,11 @@ __global__ void __launch_bounds__(256) k_flux_layout(const float* __restrict__ m
     float v = 0.f;
     if (loc < N && k < K) {
       v = __ldg(src + (long)loc * K + k);
-      if (side) v = tab.b(k, v);
+      if (side) {
+        const float m = v;
+        v = tab.b(k, m);
+        if (m != 0.f && isfinite(m) && !(fabsf(v) >= 0x1p-110f && fabsf(v) <= 0x1p110f)) *beyond = 1;
+      }
     }
     t[l][lane] = v;
   }
@@ -311,18 +316,10 @@ __global__ void __launch_bounds__(1024) k_sum_partials(const double* __restrict_
   }
 }
 
-void flux_ratio_chi2(mlc_ctx* ctx, const float* f_obs_host, const float* df_obs_host, const float* mu1,
-                     const float* mu2, int N, int F, int T, float* chi2, double* likelihood_host) {
-  MLC_REQUIRE(N >= 1 && F >= 1 && T >= 1, MLC_ERR_ARG, "need N, F, T >= 1");
-  MLC_REQUIRE(N <= 200000, MLC_ERR_LIMIT, "N <= 200000 locations");
-  const int K = F * T;
-  // 128 x 128 tiles once they fill every SM twice, two operations per term where the scaled values
-  // stay in range (a size within 2^16 either way keeps B in range with mu2)
-  const int nb = (N + FR_BIG - 1) / FR_BIG;
-  bool big = (long)nb * nb >= 2L * 2 * ctx->sm_count;
-  auto moderate = [](float v) { return std::isfinite(v) && std::fabs(v) >= 0x1p-16f && std::fabs(v) <= 0x1p16f; };
-  for (int k = 0; k < K && big; k++)
-    big = moderate(df_obs_host[k]) && (f_obs_host[k] == 0.f || moderate(f_obs_host[k]));
+// One of the two forms; false where a B is beyond the exponents that 1/mu2 still has (big), and the
+// results are not to be used.
+static bool flux_ratio_run(mlc_ctx* ctx, const float* f_obs_host, const float* df_obs_host, const float* mu1,
+                           const float* mu2, int N, int K, float* chi2, double* likelihood_host, bool big) {
   std::vector<float> h(4 * (size_t)K);
   for (int k = 0; k < K; k++) {
     const float f = f_obs_host[k], df = df_obs_host[k];
@@ -334,14 +331,19 @@ void flux_ratio_chi2(mlc_ctx* ctx, const float* f_obs_host, const float* df_obs_
     h[2 * (size_t)K + k] = (float)rho;
     h[3 * (size_t)K + k] = (float)(rho - (double)(float)rho);
   }
-  const int nt = big ? nb : (N + FR_TILE - 1) / FR_TILE;
+  const int nb = (N + FR_BIG - 1) / FR_BIG, nt = big ? nb : (N + FR_TILE - 1) / FR_TILE;
   const long nblk = (long)nt * nt;
   const size_t hb = round_up((long)(4 * K * sizeof(float)), 256);
   char* ws = (char*)ws_get(ctx, WS_SMALL, hb + (size_t)nblk * sizeof(double) + 256);
   float* d_tab = (float*)ws;
   double* d_part = (double*)(ws + hb);
-  double* d_like = d_part + nblk;
+  struct Result {
+    double like;
+    int beyond;
+  };
+  Result* d_res = (Result*)(d_part + nblk);
   MLC_CUDA(cudaMemcpyAsync(d_tab, h.data(), (big ? 4 : 2) * (size_t)K * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
+  MLC_CUDA(cudaMemsetAsync(d_res, 0, sizeof(Result), ctx->stream));
   const FluxTables tab{d_tab, K};
   if (big) {
     const int Np = nb * FR_BIG;
@@ -349,7 +351,8 @@ void flux_ratio_chi2(mlc_ctx* ctx, const float* f_obs_host, const float* df_obs_
     float* db = da + (size_t)K * Np;
     {
       MLC_KSCOPE(ctx, "flux_layout");
-      k_flux_layout<<<dim3(Np / 32, ceil_div(K, 32), 2), 256, 0, ctx->stream>>>(mu1, mu2, tab, N, Np, K, da, db);
+      k_flux_layout<<<dim3(Np / 32, ceil_div(K, 32), 2), 256, 0, ctx->stream>>>(mu1, mu2, tab, N, Np, K, da, db,
+                                                                                &d_res->beyond);
     }
     MLC_CHECK_LAUNCH();
     MLC_KSCOPE(ctx, "flux_ratio_chi2");
@@ -361,11 +364,29 @@ void flux_ratio_chi2(mlc_ctx* ctx, const float* f_obs_host, const float* df_obs_
   MLC_CHECK_LAUNCH();
   {
     MLC_KSCOPE(ctx, "flux_ratio_sum");
-    k_sum_partials<<<1, 1024, 0, ctx->stream>>>(d_part, nblk, d_like);
+    k_sum_partials<<<1, 1024, 0, ctx->stream>>>(d_part, nblk, &d_res->like);
   }
   MLC_CHECK_LAUNCH();
-  MLC_CUDA(cudaMemcpyAsync(likelihood_host, d_like, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-  MLC_CUDA(cudaStreamSynchronize(ctx->stream));
+  Result r;
+  download(ctx, &r, d_res, sizeof r);
+  *likelihood_host = r.like;
+  return !r.beyond;
+}
+
+void flux_ratio_chi2(mlc_ctx* ctx, const float* f_obs_host, const float* df_obs_host, const float* mu1,
+                     const float* mu2, int N, int F, int T, float* chi2, double* likelihood_host) {
+  MLC_REQUIRE(N >= 1 && F >= 1 && T >= 1, MLC_ERR_ARG, "need N, F, T >= 1");
+  MLC_REQUIRE(N <= 200000, MLC_ERR_LIMIT, "N <= 200000 locations");
+  const int K = F * T;
+  // 128 x 128 tiles once they fill every SM twice, two operations per term where the scaled values
+  // stay in range (f and df within 2^16 of 1; B is looked at where it is formed)
+  const int nb = (N + FR_BIG - 1) / FR_BIG;
+  bool big = (long)nb * nb >= 2L * 2 * ctx->sm_count;
+  auto moderate = [](float v) { return std::isfinite(v) && std::fabs(v) >= 0x1p-16f && std::fabs(v) <= 0x1p16f; };
+  for (int k = 0; k < K && big; k++)
+    big = moderate(df_obs_host[k]) && (f_obs_host[k] == 0.f || moderate(f_obs_host[k]));
+  if (big && flux_ratio_run(ctx, f_obs_host, df_obs_host, mu1, mu2, N, K, chi2, likelihood_host, true)) return;
+  flux_ratio_run(ctx, f_obs_host, df_obs_host, mu1, mu2, N, K, chi2, likelihood_host, false);
 }
 
 }  // namespace mlc

@@ -49,6 +49,17 @@ void* ws_get(mlc_ctx* ctx, int slot, size_t bytes) {
   return p;
 }
 
+bool ws_try(mlc_ctx* ctx, int slot, size_t bytes) {
+  try {
+    ws_get(ctx, slot, bytes);
+  } catch (const Error& e) {
+    if (e.code != MLC_ERR_OOM) throw;
+    cudaGetLastError();  // (the failed allocation is dealt with)
+    return false;
+  }
+  return true;
+}
+
 }  // namespace mlc
 
 using namespace mlc;

@@ -380,11 +380,13 @@ void flux_ratio_chi2(mlc_ctx* ctx, const float* f_obs_host, const float* df_obs_
   const int K = F * T;
   // 128 x 128 tiles once they fill every SM twice, two operations per term where the scaled values
   // stay in range (f and df within 2^16 of 1; B is looked at where it is formed)
+  // and there is room for them (they take as much as mu1 and mu2)
   const int nb = (N + FR_BIG - 1) / FR_BIG;
   bool big = (long)nb * nb >= 2L * 2 * ctx->sm_count;
   auto moderate = [](float v) { return std::isfinite(v) && std::fabs(v) >= 0x1p-16f && std::fabs(v) <= 0x1p16f; };
   for (int k = 0; k < K && big; k++)
     big = moderate(df_obs_host[k]) && (f_obs_host[k] == 0.f || moderate(f_obs_host[k]));
+  big = big && ws_try(ctx, WS_SORT_KEYS, 2 * (size_t)K * nb * FR_BIG * sizeof(float));
   if (big && flux_ratio_run(ctx, f_obs_host, df_obs_host, mu1, mu2, N, K, chi2, likelihood_host, true)) return;
   flux_ratio_run(ctx, f_obs_host, df_obs_host, mu1, mu2, N, K, chi2, likelihood_host, false);
 }

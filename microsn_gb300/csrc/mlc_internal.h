@@ -198,6 +198,7 @@ struct DeviceGuard {
 };
 
 void* ws_get(mlc_ctx* ctx, int slot, size_t bytes);
+bool ws_try(mlc_ctx* ctx, int slot, size_t bytes);  // false where the device has no room
 
 // Scope around one kernel launch: counts it and, when the context's timing is on,
 // brackets it with CUDA events on the context's stream.

@@ -233,6 +233,7 @@ static void scatter(mlc_ctx* ctx, const char* name, const K* kin, Load load, K* 
 // by bin, whose places of out (1/256 of it) stay in L2 until their sectors are whole; one
 // more trip of index and value through memory, in order.  8.5e7 values: ranks (4 bytes) 2.77
 // ms directly, 1.27 ms; chi2 (8 bytes, with the FP64 arithmetic that makes them) 3.23 ms, 2.67 ms.
+// Where the bins' 8 or 12 bytes a value do not fit the device, each value is written by itself.
 // 4.2e7: 1.00 and 0.64; 1.46 and 1.33.  2.7e7: 0.33 and 0.41; 0.83 and 0.87.
 template <typename V>
 static __global__ void __launch_bounds__(256) k_put(const uint32_t* __restrict__ idx, const V* __restrict__ val, long n,
@@ -256,7 +257,9 @@ constexpr long BINNED_PUT_FROM = 30'000'000;
 template <typename V, typename Load>
 static void put_by_index(mlc_ctx* ctx, const char* name, const uint32_t* idx, Load load, long n, V* out) {
   if (n <= 0) return;
-  if (n < BINNED_PUT_FROM) {
+  const int ntiles = (int)((n + SORT_TILE - 1) / SORT_TILE);
+  if (n < BINNED_PUT_FROM || !ws_try(ctx, WS_SORT_KEYS, sizeof(V) * n) || !ws_try(ctx, WS_SORT_VALS, sizeof(uint32_t) * n) ||
+      !ws_try(ctx, WS_SORT_HIST, sizeof(uint32_t) * 256 * (size_t)ntiles * 2 + 256 * 8 + 64)) {
     {
       MLC_KSCOPE(ctx, name);
       const int grid = (int)std::max<long>(1, std::min<long>((n + 255) / 256, (long)ctx->sm_count * 16));
@@ -265,7 +268,6 @@ static void put_by_index(mlc_ctx* ctx, const char* name, const uint32_t* idx, Lo
     MLC_CHECK_LAUNCH();
     return;
   }
-  const int ntiles = (int)((n + SORT_TILE - 1) / SORT_TILE);
   int shift = 0;
   while (((n - 1) >> shift) > 255) shift++;
   V* val = (V*)ws_get(ctx, WS_SORT_KEYS, sizeof(V) * n);

@@ -146,7 +146,8 @@ __device__ __forceinline__ void digit_places(uint32_t (*wcnt)[256], uint32_t* ba
 // One tile into digit order and out: key K with its digit, payload V from load(i) for element
 // i of the input.  8.5e7 keys of 8 + 4 bytes: 2.37 ms a pass when every thread wrote the
 // keys it had ranked (tiles of 4096: runs of 16 keys in random order), 0.64 ms in digit order
-// from shared memory.  Two CTAs of 512 threads per SM.
+// from shared memory.  Two CTAs of 512 threads per SM.  A place of n or more is not written and sets
+// *err, where there is one.
 template <typename K, typename V, typename D, typename Load>
 __global__ void __launch_bounds__(SORT_THREADS, 2) k_scatter(const K* __restrict__ kin, Load load, K* __restrict__ kout,
                                                              V* __restrict__ vout, long n, int ntiles, D digit,
@@ -193,7 +194,7 @@ __global__ void __launch_bounds__(SORT_THREADS, 2) k_scatter(const K* __restrict
       const K k = ks[i];
       dst[q] = gofs[dg(k)] + (uint32_t)i;
       if (dst[q] < un) kout[dst[q]] = k;
-      else atomicExch(err, 1);
+      else if (err) atomicExch(err, 1);
     }
   }
   __syncthreads();
@@ -259,7 +260,7 @@ static void put_by_index(mlc_ctx* ctx, const char* name, const uint32_t* idx, Lo
   if (n <= 0) return;
   const int ntiles = (int)((n + SORT_TILE - 1) / SORT_TILE);
   if (n < BINNED_PUT_FROM || !ws_try(ctx, WS_SORT_KEYS, sizeof(V) * n) || !ws_try(ctx, WS_SORT_VALS, sizeof(uint32_t) * n) ||
-      !ws_try(ctx, WS_SORT_HIST, sizeof(uint32_t) * 256 * (size_t)ntiles * 2 + 256 * 8 + 64)) {
+      !ws_try(ctx, WS_SORT_HIST, sizeof(uint32_t) * 256 * (size_t)ntiles * 2 + 256 * 8)) {
     {
       MLC_KSCOPE(ctx, name);
       const int grid = (int)std::max<long>(1, std::min<long>((n + 255) / 256, (long)ctx->sm_count * 16));
@@ -272,10 +273,9 @@ static void put_by_index(mlc_ctx* ctx, const char* name, const uint32_t* idx, Lo
   while (((n - 1) >> shift) > 255) shift++;
   V* val = (V*)ws_get(ctx, WS_SORT_KEYS, sizeof(V) * n);
   uint32_t* key = (uint32_t*)ws_get(ctx, WS_SORT_VALS, sizeof(uint32_t) * n);
-  uint32_t* hist = (uint32_t*)ws_get(ctx, WS_SORT_HIST, sizeof(uint32_t) * 256 * (size_t)ntiles * 2 + 256 * 8 + 64);
+  uint32_t* hist = (uint32_t*)ws_get(ctx, WS_SORT_HIST, sizeof(uint32_t) * 256 * (size_t)ntiles * 2 + 256 * 8);
   uint32_t* offs = hist + (size_t)256 * ntiles;
   unsigned long long* dtot = reinterpret_cast<unsigned long long*>(offs + (size_t)256 * ntiles);
-  int* derr = reinterpret_cast<int*>(dtot + 256);
   {
     MLC_KSCOPE(ctx, name);
     k_tile_hist<uint32_t, ShiftDigit><<<ntiles, SORT_THREADS, 0, ctx->stream>>>(idx, n, ntiles, ShiftDigit{shift}, hist);
@@ -283,7 +283,8 @@ static void put_by_index(mlc_ctx* ctx, const char* name, const uint32_t* idx, Lo
     k_scan_digit<<<256, 1024, 0, ctx->stream>>>(hist, ntiles, dtot, offs);
   }
   MLC_CHECK_LAUNCH();
-  scatter(ctx, name, idx, load, key, val, n, ntiles, ShiftDigit{shift}, offs, derr);
+  // (no error word: the places are counts of the same idx, below n whatever its values)
+  scatter(ctx, name, idx, load, key, val, n, ntiles, ShiftDigit{shift}, offs, nullptr);
   {
     MLC_KSCOPE(ctx, name);
     k_put<V><<<(unsigned)((n + 2047) / 2048), 256, 0, ctx->stream>>>(key, val, n, out);

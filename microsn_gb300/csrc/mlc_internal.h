@@ -86,7 +86,7 @@ enum WsSlot {
   WS_BATCH_MAPS,  // convolved maps of one profile group (mlc_convolve_sample_tracks)
   WS_BATCH_IMAP,  // their profile-interleaved copy
   WS_SAMPLE_ORDER,  // the sampler's epoch chunks in map-cell order
-  WS_EXP_TAB,       // 2^(j/4096) of the pair stage's exponentials
+  WS_EXP_TAB,       // 2^(j/2048) of the pair stage's exponentials
   WS_NSLOTS
 };
 
@@ -123,7 +123,7 @@ struct mlc_ctx {
   std::map<std::string, std::pair<double, long>> ktimes;  // name -> (ms, launches)
   void* ws_ptr[mlc::WS_NSLOTS] = {};
   size_t ws_size[mlc::WS_NSLOTS] = {};
-  const double* exp_table = nullptr;  // WS_EXP_TAB, once its values are there
+  const void* exp_table = nullptr;  // WS_EXP_TAB, once its values are there
   std::map<std::tuple<int, int, int>, std::unique_ptr<mlc::FftPlan2D>> plans;
   mlc::BatchIO* batch = nullptr;
   // launch autotuner: key -> choice (-1: FFT form; >= 0: direct tile shape), candidate timings

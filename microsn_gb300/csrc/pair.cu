@@ -203,43 +203,49 @@ __global__ void __launch_bounds__(256) k_pair_chi2_ratio(RatioChi2 f, const uint
 // per bin left most SMs idle behind the largest bins).
 //
 // exp(-c/2), the FP64 pipe's largest part of this kernel, from a table: exp(-c/2) =
-// 2^(k/4096) e^r with k = RN(-c 2048/ln 2) and |r| <= ln 2/8192, where three terms of the
-// series for e^r - 1 leave less than 2^-58; 2^(j/4096) for the 4096 fractions lies in shared
-// memory.  Eight FP64 operations, within 1.02 ulp (bin means of 8.5e7 pairs 3.24 -> 2.03 ms); outside [0, 1400] (NaN, results near or
-// below the smallest normal) the library's exp, and 0 where that underflows.
-constexpr int EXP_TAB = 4096;
-__device__ __forceinline__ double exp_neg_half(double c, const double* tab) {
+// 2^(k/2048) e^r with k = RN(-c 1024/ln 2) and |r| <= ln 2/4096, where three terms of the
+// series for e^r - 1, the fourth folded into the second where it is least off, leave 2^-57;
+// 2^(j/2048) for the 2048 fractions lies in shared memory, rounded, with the relative rest.  Eight
+// FP64 operations, within 0.53 ulp (the library's within 0.51; 4096 entries without the rest
+// were within one ulp); outside [0, 1400] (NaN, results
+// near or below the smallest normal) the library's exp, and 0 where that underflows.
+constexpr int EXP_TAB = 2048;
+__device__ __forceinline__ double exp_neg_half(double c, const double2* tab) {
   // (compared by its high word: FP64 comparisons run on the FP64 pipe, and a negative or NaN c
   // has a larger one)
   const unsigned hi = (unsigned)__double2hiint(c);
   if (hi >= 0x4095E000u) return hi - 0x40977000u < 0x7FF00000u - 0x40977000u ? 0.0 : exp(-0.5 * c);  // 1400; 1500 to below inf
-  const double magic = 6755399441055744.0;                  // 1.5 * 2^52: the sum's low word is k
-  const double t = __fma_rn(c, -2954.639443740597, magic);  // 2048 / ln 2
+  const double magic = 6755399441055744.0;                   // 1.5 * 2^52: the sum's low word is k
+  const double t = __fma_rn(c, -1477.3197218702985, magic);  // 1024 / ln 2
   const double k = __dsub_rn(t, magic);
-  double r = __fma_rn(k, 0x1.62e42fe8p-12, c);  // r' = -2 r = c + k ln 2/2048; 30 bits of it: exact
-  r = __fma_rn(k, 0x1.e8e7bcd5e4f1ep-42, r);
+  double r = __fma_rn(k, 0x1.62e42fe8p-11, c);  // r' = -2 r = c + k ln 2/1024; 30 bits of it: exact
+  r = __fma_rn(k, 0x1.e8e7bcd5e4f1ep-41, r);
   const int ki = __double2loint(t);
-  const double p = __fma_rn(r, __fma_rn(r, -1.0 / 48.0, 0.125), -0.5);
-  const double s = tab[ki & (EXP_TAB - 1)];
-  const double e = __fma_rn(s, __dmul_rn(r, p), s);
-  return __hiloint2double(__double2hiint(e) + ((ki >> 12) << 20), __double2loint(e));
+  // e^r - 1 = r' (-1/2 + r'/8 - r'^2/48 + r'^3/384), r'^4 as 0.828 (ln 2/2048)^2 r'^2
+  const double p = __fma_rn(r, __fma_rn(r, -1.0 / 48.0, 0.125 + 0.828427 / 384.0 * (0x1.62e42fefa39efp-12 * 0x1.62e42fefa39efp-12)), -0.5);
+  const double2 s = tab[ki & (EXP_TAB - 1)];
+  const double e = __fma_rn(s.x, __fma_rn(r, p, s.y), s.x);
+  return __hiloint2double(__double2hiint(e) + ((ki >> 11) << 20), __double2loint(e));
 }
 
-// 2^(j/4096) on the device, made once per context (and there for any stream it is given later).
-static const double* exp_table(mlc_ctx* ctx) {
+// 2^(j/2048) on the device, made once per context (and there for any stream it is given later).
+static const double2* exp_table(mlc_ctx* ctx) {
   if (!ctx->exp_table) {
-    std::vector<double> h(EXP_TAB);
-    for (int j = 0; j < EXP_TAB; j++) h[j] = (double)exp2l((long double)j / EXP_TAB);
-    void* d = ws_get(ctx, WS_EXP_TAB, sizeof(double) * EXP_TAB);
-    upload(ctx, d, h.data(), sizeof(double) * EXP_TAB);
+    std::vector<double2> h(EXP_TAB);
+    for (int j = 0; j < EXP_TAB; j++) {
+      const long double v = exp2l((long double)j / EXP_TAB);
+      h[j].x = (double)v;
+      h[j].y = (double)(v / h[j].x - 1.0L);
+    }
+    void* d = ws_get(ctx, WS_EXP_TAB, sizeof(double2) * EXP_TAB);
+    upload(ctx, d, h.data(), sizeof(double2) * EXP_TAB);
     MLC_CUDA(cudaStreamSynchronize(ctx->stream));
-    ctx->exp_table = (const double*)d;
+    ctx->exp_table = d;
   }
-  return ctx->exp_table;
+  return (const double2*)ctx->exp_table;
 }
-__device__ __forceinline__ void load_exp_table(const double* __restrict__ src, double* dst) {
-  for (int i = threadIdx.x; i < EXP_TAB / 2; i += blockDim.x)
-    reinterpret_cast<double2*>(dst)[i] = __ldg(reinterpret_cast<const double2*>(src) + i);
+__device__ __forceinline__ void load_exp_table(const double2* __restrict__ src, double2* dst) {
+  for (int i = threadIdx.x; i < EXP_TAB; i += blockDim.x) dst[i] = __ldg(src + i);
 }
 constexpr uint32_t BIN_PIECE = 1u << 15;
 struct BinPiece {
@@ -248,9 +254,9 @@ struct BinPiece {
 
 __global__ void __launch_bounds__(256) k_bin_piece_sums(const double* __restrict__ chi2,
                                                         const BinPiece* __restrict__ pieces, int npieces,
-                                                        const double* __restrict__ etab, double* __restrict__ psum,
+                                                        const double2* __restrict__ etab, double* __restrict__ psum,
                                                         double* __restrict__ pexp) {
-  __shared__ __align__(16) double tab[EXP_TAB];
+  __shared__ double2 tab[EXP_TAB];
   __shared__ double r1[8], r2[8];
   load_exp_table(etab, tab);
   __syncthreads();
@@ -341,11 +347,11 @@ __device__ __forceinline__ int edge_search(const double* e, int nb, double z) {
 
 __global__ void __launch_bounds__(256) k_pair_bin_fused(RatioChi2 f, FusedSide A, FusedSide B, int na, int nb,
                                                         const double* __restrict__ edges,
-                                                        const double* __restrict__ etab, int copies,
+                                                        const double2* __restrict__ etab, int copies,
                                                         double* __restrict__ gsum, double* __restrict__ gexp,
                                                         unsigned long long* __restrict__ gcnt) {
   extern __shared__ __align__(16) double sm[];
-  double* tab = sm;
+  double2* tab = reinterpret_cast<double2*>(sm);
   float* ef_s = reinterpret_cast<float*>(tab + EXP_TAB);
   load_exp_table(etab, tab);
   for (int i = threadIdx.x; i < nb; i += blockDim.x) ef_s[i] = (float)edges[i];
@@ -604,7 +610,7 @@ void bin_chi2(mlc_ctx* ctx, int Nbins, const uint32_t* lower_host, const uint32_
     MLC_CUDA(cudaMemcpyAsync(dp, pieces.data(), sizeof(BinPiece) * pieces.size(), cudaMemcpyHostToDevice, ctx->stream));
   MLC_CUDA(cudaMemcpyAsync(dfirst, pfirst.data(), sizeof(uint32_t) * (Nbins + 1), cudaMemcpyHostToDevice, ctx->stream));
   MLC_CUDA(cudaMemcpyAsync(dn, nper.data(), sizeof(uint32_t) * Nbins, cudaMemcpyHostToDevice, ctx->stream));
-  const double* etab = exp_table(ctx);
+  const double2* etab = exp_table(ctx);
   if (!pieces.empty()) {
     MLC_KSCOPE(ctx, "pair_bin_means");
     const unsigned grid = (unsigned)std::min<size_t>(pieces.size(), (size_t)ctx->sm_count * 6);
@@ -645,8 +651,8 @@ void pair_bin_fused(mlc_ctx* ctx, int Njp, const int* indA, const int* indB, con
   const RatioChi2 f = build_interp(ctx, Njp, indA, indB, facA, facB, d, s, Nloc, Nprof, LCA, DLCA, LCB, DLCB);
   MLC_CUDA(cudaMemcpyAsync(de, edges_host, sizeof(double) * Nbins, cudaMemcpyHostToDevice, ctx->stream));
   MLC_CUDA(cudaMemsetAsync(gs, 0, 8 * 3 * NC, ctx->stream));
-  const size_t smem = sizeof(double) * EXP_TAB + sizeof(float) * Nbins;
-  const double* etab = exp_table(ctx);
+  const size_t smem = sizeof(double2) * EXP_TAB + sizeof(float) * Nbins;
+  const double2* etab = exp_table(ctx);
   if (Nloc > 0) {
     set_max_smem((const void*)k_pair_bin_fused, smem);
     // A places per CTA: as many as leave four CTAs for every SM

@@ -10,8 +10,8 @@
 // digit be skipped.  Then one pass per remaining digit: (1) per-tile counts of that
 // digit in the keys' current order (the up-front counts serve the first pass only,
 // since each scatter permutes the keys); (2) k_scan_digit turns them into scatter
-// offsets; (3) k_scatter ranks each key inside its tile with __match_any_sync in
-// element order (stable), puts the tile in digit order in shared memory and writes it
+// offsets; (3) k_scatter ranks each key inside its tile in element order (stable; one
+// vote per bit of the digit), puts the tile in digit order in shared memory and writes it
 // from there: the keys of one digit are consecutive, 32 on average in a tile of 8192, so
 // a warp writes a few whole runs (writing each key from the thread that ranked it cost
 // 2.4 ms a pass for 8.5e7 keys, this 0.64; see k_scatter).  Every scatter address is checked against
@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(SORT_THREADS) k_digit_hist(const uint64_t* __r
   }
 }
 
-// The longest run of keys with equal sorted bits that one thread puts in order.
+// The longest run of keys with equal sorted bits that one thread or warp puts in order.
 constexpr int FIX_RUN = 64;
 
 // Insertion of elements [b, e): a key passes only larger ones.
@@ -99,6 +99,37 @@ __device__ __forceinline__ int run_of_descent(const uint64_t* ks, int i, uint64_
 constexpr int SMALL_THREADS = 1024, SMALL_WARPS = SMALL_THREADS / 32, SMALL_MAX_ITEMS = 16;
 constexpr long SMALL_MAX = (long)SMALL_THREADS * SMALL_MAX_ITEMS;
 
+// One stable pass by the digit at `shift` over the CTA's THREADS x ITEMS keys and values in shared
+// memory; item q of a thread is element e0 + 32 q.
+template <int ITEMS, int THREADS>
+__device__ __forceinline__ void cta_pass(uint64_t* ks, uint32_t* vs, uint64_t (&key)[ITEMS], uint32_t (*wcnt)[256],
+                                         uint32_t* base, uint32_t* wsum, int e0, int shift) {
+  constexpr int WARPS = THREADS / 32;
+  const int warp = threadIdx.x >> 5;
+  const unsigned lt = (1u << (threadIdx.x & 31)) - 1u;
+  for (int i = threadIdx.x; i < WARPS * 256; i += THREADS) (&wcnt[0][0])[i] = 0;
+#pragma unroll
+  for (int q = 0; q < ITEMS; q++) key[q] = ks[e0 + 32 * q];
+  __syncthreads();
+  uint32_t pos[ITEMS];
+#pragma unroll
+  for (int q = 0; q < ITEMS; q++) pos[q] = warp_digit_rank((unsigned)(key[q] >> shift) & 0xffu, true, wcnt[warp], lt);
+  __syncthreads();
+  digit_places<WARPS>(wcnt, base, wsum);
+#pragma unroll
+  for (int q = 0; q < ITEMS; q++) {
+    pos[q] += wcnt[warp][(unsigned)(key[q] >> shift) & 0xffu];
+    ks[pos[q]] = key[q];
+  }
+  uint32_t v[ITEMS];
+#pragma unroll
+  for (int q = 0; q < ITEMS; q++) v[q] = vs[e0 + 32 * q];
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < ITEMS; q++) vs[pos[q]] = v[q];
+  __syncthreads();
+}
+
 template <int ITEMS, bool F64>
 __global__ void __launch_bounds__(SMALL_THREADS) k_sort_small(uint64_t* __restrict__ keys, uint32_t* __restrict__ vals,
                                                               int n) {
@@ -113,7 +144,6 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_sort_small(uint64_t* __restri
   __shared__ unsigned long long differ;
   __shared__ int nlist, too_long;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
   const int e0 = warp * (ITEMS * 32) + lane;  // item q is element e0 + 32 q
   if (threadIdx.x == 0) differ = 0, nlist = 0, too_long = 0;
   __syncthreads();
@@ -136,29 +166,7 @@ __global__ void __launch_bounds__(SMALL_THREADS) k_sort_small(uint64_t* __restri
   if (m) atomicOr(&differ, (unsigned long long)m);
   __syncthreads();
   const uint64_t diff = differ;
-  auto pass = [&](int shift) {
-    for (int i = threadIdx.x; i < SMALL_WARPS * 256; i += SMALL_THREADS) (&wcnt[0][0])[i] = 0;
-#pragma unroll
-    for (int q = 0; q < ITEMS; q++) key[q] = ks[e0 + 32 * q];
-    __syncthreads();
-    uint32_t pos[ITEMS];
-#pragma unroll
-    for (int q = 0; q < ITEMS; q++) pos[q] = warp_digit_rank((unsigned)(key[q] >> shift) & 0xffu, true, wcnt[warp], lt);
-    __syncthreads();
-    digit_places<SMALL_WARPS>(wcnt, base, wsum);
-#pragma unroll
-    for (int q = 0; q < ITEMS; q++) {
-      pos[q] += wcnt[warp][(unsigned)(key[q] >> shift) & 0xffu];
-      ks[pos[q]] = key[q];
-    }
-    uint32_t v[ITEMS];
-#pragma unroll
-    for (int q = 0; q < ITEMS; q++) v[q] = vs[e0 + 32 * q];
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < ITEMS; q++) vs[pos[q]] = v[q];
-    __syncthreads();
-  };
+  auto pass = [&](int shift) { cta_pass<ITEMS, SMALL_THREADS>(ks, vs, key, wcnt, base, wsum, e0, shift); };
   const int sh = diff ? max(0, 32 - __clzll((long long)diff)) : 64;  // the lowest sorted bit
 #pragma unroll 1
   for (int shift = sh; shift < min(64, sh + 32); shift += 8)
@@ -290,12 +298,17 @@ void radix_sort_u64_u32(mlc_ctx* ctx, long n, uint64_t* keys, uint32_t* vals) {
 // sorted by its full keys, stably, by one thread: within tiles of the keys in shared memory
 // (k_fix_tiles), then across the tiles' edges (k_fix_edges).  Runs of equal keys are in order
 // as they stand, however long.  A run with a descent that is longer than FIX_RUN is noted
-// (long_run) and sorted by a CTA, or, beyond RUN_MAX keys, as a range of its own.  Quotients of
-// ray counts come in runs of 10^2 to 10^4 equal keys, and here and there two such runs share
-// their top bits: 8.5e7 of them, FP32 counts around 20, 12.2 ms with all keys made and sorted
-// anew by all bits where that happened, 5.9 as here.
+// (long_run) and sorted by a CTA, up to RUN_MAX keys in shared memory (k_sort_runs), longer ones
+// through the second buffers (k_sort_big), by its keys less the least of them: a digit or two.  A
+// few beyond BIG_MAX are sorted as ranges of their own.  Quotients of ray counts come in runs
+// of 10^2 to 10^4 equal keys, and equal fractions of different counts share their top bits.  Rank
+// of 1500 and 2200 locations with counts around 300: 0.51 and 0.93 ms by all bits, 0.82 and
+// 1.68 with long runs sorted by comparison or one by one from the host, 0.40 and 0.55 as here.
 constexpr int FIX_TILE = 4096, FIX_THREADS = 256;
-constexpr int RUN_SLOTS = 8192, RUN_MAX = 2048, BIG_RUNS = 64;
+constexpr int RUN_SLOTS = 8192, BIG_RUNS = 1024, HOST_RUNS = 8;
+constexpr int RUN_THREADS = 256, RUN_ITEMS = 8, RUN_MAX = RUN_THREADS * RUN_ITEMS;
+constexpr int BIG_THREADS = 1024, BIG_ITEMS = 8, BIG_TILE = BIG_THREADS * BIG_ITEMS;
+constexpr unsigned long long BIG_MAX = 1 << 18;
 struct LongRuns {
   int scatter_err, full, nbig;  // full: more runs than there is room for, the order is not made
   unsigned long long at[RUN_SLOTS];  // first key of a noted run (~0: none), by a hash of it
@@ -312,8 +325,10 @@ __device__ __forceinline__ long lower_bound_top(const uint64_t* __restrict__ key
   }
   return b;
 }
-__device__ __noinline__ void long_run(const uint64_t* keys, long n, uint64_t lo, int sh, uint64_t tp, LongRuns* lr) {
-  const unsigned long long b = (unsigned long long)lower_bound_top(keys, n, lo, sh, tp);
+// start: the run's first place, -1 where it has to be searched for.
+__device__ __noinline__ void long_run(const uint64_t* keys, long n, uint64_t lo, int sh, uint64_t tp, long start,
+                                      LongRuns* lr) {
+  const unsigned long long b = (unsigned long long)(start >= 0 ? start : lower_bound_top(keys, n, lo, sh, tp));
   const unsigned h = ((unsigned)b * 2654435761u) >> 16;
   for (unsigned r = 0; r < 64; r++) {
     const unsigned long long was = atomicCAS(&lr->at[(h + r) % RUN_SLOTS], ~0ull, b);
@@ -321,39 +336,191 @@ __device__ __noinline__ void long_run(const uint64_t* keys, long n, uint64_t lo,
   }
   atomicExch(&lr->full, 1);
 }
-// A CTA per slot: the noted run stably sorted by counting the keys before each.
-__global__ void __launch_bounds__(256) k_sort_runs(uint64_t* __restrict__ keys, uint32_t* __restrict__ vals, long n,
-                                                   const unsigned long long* __restrict__ range,
-                                                   LongRuns* __restrict__ lr) {
+// A CTA per slot: the noted run, stably sorted by its keys less the least of them.
+__global__ void __launch_bounds__(RUN_THREADS) k_sort_runs(uint64_t* keys, uint32_t* vals, long n,
+                                                           const unsigned long long* __restrict__ range,
+                                                           LongRuns* __restrict__ lr) {
   __shared__ uint64_t ks[RUN_MAX];
   __shared__ uint32_t vs[RUN_MAX];
-  __shared__ long end;
+  __shared__ uint32_t wcnt[RUN_THREADS / 32][256];
+  __shared__ uint32_t base[256], wsum[32];
+  __shared__ unsigned long long least, most;
+  __shared__ int len_s;
   const unsigned long long b = lr->at[blockIdx.x];
   if (b == ~0ull) return;
-  if (threadIdx.x == 0) {
-    const uint64_t lo = range[0];
-    const int sh = RangeDigit::base_shift(range);
-    end = lower_bound_top(keys, n, lo, sh, ((keys[b] - lo) >> sh) + 1);
+  if (threadIdx.x == 0) least = ~0ull, most = 0, len_s = 0;
+  __syncthreads();
+  const uint64_t lo = range[0];
+  const int sh = RangeDigit::base_shift(range);
+  const uint64_t tp = (keys[b] - lo) >> sh;
+  const long rest = n - (long)b;
+  const int e0 = (threadIdx.x >> 5) * (RUN_ITEMS * 32) + (threadIdx.x & 31);
+  uint64_t key[RUN_ITEMS], kmin = ~0ull, kmax = 0;
+  int in = 0;
+#pragma unroll
+  for (int q = 0; q < RUN_ITEMS; q++) {
+    const int e = e0 + 32 * q;
+    if (e < rest) {
+      const uint64_t k = keys[b + e];
+      if ((k - lo) >> sh == tp) {
+        key[q] = k;
+        vs[e] = vals[b + e];
+        kmin = min(kmin, k);
+        kmax = max(kmax, k);
+        in++;
+      }
+    }
+  }
+  if (in) {
+    atomicAdd(&len_s, in);
+    atomicMin(&least, (unsigned long long)kmin);
+    atomicMax(&most, (unsigned long long)kmax);
   }
   __syncthreads();
-  const long len = end - (long)b;
-  if (len > RUN_MAX) {
+  const int len = len_s;
+  if (len == RUN_MAX && rest > RUN_MAX && (keys[b + RUN_MAX] - lo) >> sh == tp) {
     if (threadIdx.x == 0) {
       const int r = atomicAdd(&lr->nbig, 1);
-      if (r < BIG_RUNS) lr->big_at[r] = b, lr->big_end[r] = (unsigned long long)end;
+      if (r < BIG_RUNS) lr->big_at[r] = b, lr->big_end[r] = b + lower_bound_top(keys + b, rest, lo, sh, tp + 1);
       else atomicExch(&lr->full, 1);
     }
     return;
   }
-  for (int i = threadIdx.x; i < len; i += blockDim.x) ks[i] = keys[b + i], vs[i] = vals[b + i];
+  const uint64_t k0 = least, spread = most - k0;
+  // (places past the run: all bits set, and after the others of their digit, so they stay there)
+#pragma unroll
+  for (int q = 0; q < RUN_ITEMS; q++) ks[e0 + 32 * q] = e0 + 32 * q < len ? key[q] - k0 : ~0ull;
   __syncthreads();
-  for (int i = threadIdx.x; i < len; i += blockDim.x) {
-    const uint64_t k = ks[i];
-    int r = 0;
-    for (int j = 0; j < len; j++) r += ks[j] < k || (ks[j] == k && j < i);
-    keys[b + r] = k;
-    vals[b + r] = vs[i];
+#pragma unroll 1
+  for (int shift = 0; shift < 64 && spread >> shift; shift += 8)
+    cta_pass<RUN_ITEMS, RUN_THREADS>(ks, vs, key, wcnt, base, wsum, e0, shift);
+#pragma unroll
+  for (int q = 0; q < RUN_ITEMS; q++) {
+    const int e = e0 + 32 * q;
+    if (e < len) {
+      keys[b + e] = ks[e] + k0;
+      vals[b + e] = vs[e];
+    }
   }
+}
+
+// The same for runs beyond RUN_MAX (a CTA each, up to BIG_MAX keys): tile by tile from one buffer
+// to the other, each digit's next place in shared memory.
+__global__ void __launch_bounds__(BIG_THREADS) k_sort_big(uint64_t* keys, uint32_t* vals, uint64_t* k2, uint32_t* v2,
+                                                          const LongRuns* __restrict__ lr) {
+  constexpr int WARPS = BIG_THREADS / 32;
+  __shared__ uint32_t wcnt[WARPS][256];
+  __shared__ uint32_t base[256], next[256], wsum[32];
+  __shared__ unsigned long long least, most;
+  const unsigned long long b = lr->big_at[blockIdx.x], all = lr->big_end[blockIdx.x] - b;
+  if (all > BIG_MAX) return;
+  const int len = (int)all, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, e0 = warp * (BIG_ITEMS * 32) + lane;
+  const unsigned lt = (1u << lane) - 1u;
+  uint64_t *ka = keys + b, *kb = k2 + b;
+  uint32_t *va = vals + b, *vb = v2 + b;
+  if (threadIdx.x == 0) least = ~0ull, most = 0;
+  __syncthreads();
+  // few digits occur, so that one atomic per warp and digit does
+  auto count = [&](int n, auto at) {
+    for (int i0 = 0; i0 < n; i0 += BIG_THREADS) {
+      const int i = i0 + threadIdx.x;
+      const unsigned d = i < n ? at(i) : 256u, peers = __match_any_sync(0xffffffffu, d);
+      if (d < 256 && (peers & lt) == 0) atomicAdd(&next[d], (uint32_t)__popc(peers));
+    }
+  };
+  uint64_t kmin = ~0ull, kmax = 0;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < len; i += BIG_THREADS) {
+    const uint64_t k = ka[i];
+    kmin = min(kmin, k);
+    kmax = max(kmax, k);
+  }
+  atomicMin(&least, (unsigned long long)kmin);
+  atomicMax(&most, (unsigned long long)kmax);
+  __syncthreads();
+  const uint64_t k0 = least, spread = most - k0;
+#pragma unroll 1
+  for (int shift = 0; shift < 64 && spread >> shift; shift += 8) {
+    auto digit = [&](uint64_t k) { return (unsigned)((k - k0) >> shift) & 0xffu; };
+    if (threadIdx.x < 256) next[threadIdx.x] = 0;
+    __syncthreads();
+    count(len, [&](int i) { return digit(ka[i]); });
+    __syncthreads();
+    uint32_t agg;
+    const uint32_t ex = block_exclusive_sum(threadIdx.x < 256 ? next[threadIdx.x] : 0u, &agg, wsum);
+    __syncthreads();
+    if (threadIdx.x < 256) next[threadIdx.x] = ex;
+#pragma unroll 1
+    for (int t0 = 0; t0 < len; t0 += BIG_TILE) {
+      const int cnt = min(BIG_TILE, len - t0);
+      for (int i = threadIdx.x; i < WARPS * 256; i += BIG_THREADS) (&wcnt[0][0])[i] = 0;
+      __syncthreads();
+      uint64_t key[BIG_ITEMS];
+      uint32_t pos[BIG_ITEMS];
+#pragma unroll
+      for (int q = 0; q < BIG_ITEMS; q++) key[q] = e0 + 32 * q < cnt ? ka[t0 + e0 + 32 * q] : 0ull;
+#pragma unroll
+      for (int q = 0; q < BIG_ITEMS; q++)
+        pos[q] = warp_digit_rank(digit(key[q]), e0 + 32 * q < cnt, wcnt[warp], lt);
+      __syncthreads();
+      digit_places<WARPS>(wcnt, base, wsum);
+#pragma unroll
+      for (int q = 0; q < BIG_ITEMS; q++)
+        if (e0 + 32 * q < cnt) {
+          const unsigned d = digit(key[q]);
+          const uint32_t dst = next[d] + pos[q] + wcnt[warp][d] - base[d];  // (below len)
+          kb[dst] = key[q];
+          vb[dst] = va[t0 + e0 + 32 * q];
+        }
+      __syncthreads();
+      if (threadIdx.x < 256) next[threadIdx.x] += (threadIdx.x < 255 ? base[threadIdx.x + 1] : cnt) - base[threadIdx.x];
+      __syncthreads();
+    }
+    uint64_t* tk = ka;
+    ka = kb;
+    kb = tk;
+    uint32_t* tv = va;
+    va = vb;
+    vb = tv;
+  }
+  if (ka != keys + b)
+    for (int i = threadIdx.x; i < len; i += BIG_THREADS) {
+      kb[i] = ka[i];
+      vb[i] = va[i];
+    }
+}
+
+// A run of up to 32 KPL keys, stably sorted by one warp that counts the keys before each.  (A
+// thread's insertions move keys and values in memory one after another: 160 us where a run of
+// 60 was among them.)
+constexpr int THREAD_RUN = 8;  // keys of a run that one thread sorts by insertion
+template <int KPL>
+__device__ __forceinline__ void warp_run(uint64_t* keys, uint32_t* vals, int len) {
+  const int lane = threadIdx.x & 31;
+  uint64_t k[KPL];
+  uint32_t v[KPL];
+  int r[KPL];
+#pragma unroll
+  for (int q = 0; q < KPL; q++) {
+    const bool in = lane + 32 * q < len;
+    k[q] = in ? keys[lane + 32 * q] : ~0ull;
+    v[q] = in ? vals[lane + 32 * q] : 0u;
+    r[q] = 0;
+  }
+#pragma unroll
+  for (int p = 0; p < KPL; p++)
+    for (int l = 0; l < 32 && 32 * p + l < len; l++) {
+      const uint64_t o = __shfl_sync(0xffffffffu, k[p], l);
+#pragma unroll
+      for (int q = 0; q < KPL; q++) r[q] += o < k[q] || (o == k[q] && 32 * p + l < lane + 32 * q);
+    }
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < KPL; q++)
+    if (lane + 32 * q < len) {
+      keys[r[q]] = k[q];
+      vals[r[q]] = v[q];
+    }
 }
 
 __global__ void __launch_bounds__(FIX_THREADS) k_fix_tiles(uint64_t* __restrict__ keys, uint32_t* __restrict__ vals,
@@ -361,20 +528,22 @@ __global__ void __launch_bounds__(FIX_THREADS) k_fix_tiles(uint64_t* __restrict_
                                                            LongRuns* __restrict__ lr) {
   __shared__ uint64_t ks[FIX_TILE];
   __shared__ uint16_t list[FIX_TILE / 2];  // first elements of the runs to sort (two keys or more each)
-  __shared__ int nlist;
+  __shared__ uint32_t wide[FIX_TILE / THREAD_RUN];  // those of more than THREAD_RUN keys: first element and length
+  __shared__ int nlist, nwide;
   const uint64_t lo = range[0];
   const int sh = RangeDigit::base_shift(range);
   const long t0 = (long)blockIdx.x * FIX_TILE;
   const int cnt = (int)min((long)FIX_TILE, n - t0);
-  if (threadIdx.x == 0) nlist = 0;
+  if (threadIdx.x == 0) nlist = nwide = 0;
   for (int i = threadIdx.x; i < cnt; i += FIX_THREADS) ks[i] = keys[t0 + i];
   __syncthreads();
   auto top = [&](uint64_t k) { return (k - lo) >> sh; };
   for (int i = threadIdx.x; i + 1 < cnt; i += FIX_THREADS) {
     if (!(ks[i] > ks[i + 1])) continue;  // (a descent has equal top bits: the keys are in their order)
-    const int b = run_of_descent(ks, i, lo, sh);
+    int b = run_of_descent(ks, i, lo, sh);
+    // (a long run may be listed for each descent that has none in the FIX_RUN keys before it)
+    if (b == -2) b = (int)lower_bound_top(ks, i, lo, sh, top(ks[i]));
     if (b >= 0) list[atomicAdd(&nlist, 1)] = (uint16_t)b;
-    else if (b == -2) long_run(keys, n, lo, sh, top(ks[i]), lr);
   }
   __syncthreads();
   for (int r = threadIdx.x; r < nlist; r += FIX_THREADS) {
@@ -383,34 +552,52 @@ __global__ void __launch_bounds__(FIX_THREADS) k_fix_tiles(uint64_t* __restrict_
     int e = b + 1;
     while (e < cnt && e - b <= FIX_RUN && top(ks[e]) == tp) e++;
     if (e - b > FIX_RUN) {
-      long_run(keys, n, lo, sh, tp, lr);
+      long_run(keys, n, lo, sh, tp, b > 0 ? t0 + b : -1, lr);
       continue;
     }
     // (a run that goes on in a neighbouring tile is k_fix_edges')
     if ((b == 0 && t0 > 0 && top(keys[t0 - 1]) == tp) || (e == cnt && t0 + e < n && top(keys[t0 + e]) == tp)) continue;
+    if (e - b > THREAD_RUN) {
+      wide[atomicAdd(&nwide, 1)] = (uint32_t)b | (uint32_t)(e - b) << 16;
+      continue;
+    }
     fix_run(ks, vals + t0, b, e);
     for (int i = b; i < e; i++) keys[t0 + i] = ks[i];
   }
+  __syncthreads();
+  for (int r = threadIdx.x >> 5; r < nwide; r += FIX_THREADS / 32) {
+    const uint32_t w = wide[r];
+    warp_run<2>(keys + t0 + (w & 0xffffu), vals + t0 + (w & 0xffffu), (int)(w >> 16));
+  }
 }
 
-// The runs across the edge at the start of tile 1, 2, ...: a thread each.
+// The runs across the edge at the start of tile 1, 2, ...: a warp each, whose lanes look at the keys
+// on both sides at once (one thread's walk through a long run took 40 us).
 __global__ void __launch_bounds__(256) k_fix_edges(uint64_t* __restrict__ keys, uint32_t* __restrict__ vals, long n,
                                                    const unsigned long long* __restrict__ range,
                                                    LongRuns* __restrict__ lr) {
+  static_assert(FIX_RUN == 64, "two keys a lane");
   const uint64_t lo = range[0];
-  const int sh = RangeDigit::base_shift(range);
-  const long j = ((long)blockIdx.x * blockDim.x + threadIdx.x + 1) * FIX_TILE;
-  if (j >= n) return;
+  const int sh = RangeDigit::base_shift(range), lane = threadIdx.x & 31;
+  const long j = (((long)blockIdx.x * blockDim.x + threadIdx.x) / 32 + 1) * FIX_TILE;
+  if (j >= n) return;  // (a whole warp)
   const uint64_t tp = (keys[j] - lo) >> sh;
-  long b = j, e = j;
-  while (b > 0 && j - b <= FIX_RUN && ((keys[b - 1] - lo) >> sh) == tp) b--;
-  while (e < n && e - j <= FIX_RUN && ((keys[e] - lo) >> sh) == tp) e++;
-  if (b == j) return;
+  auto same = [&](long i) { return i >= 0 && i < n && (keys[i] - lo) >> sh == tp; };
+  // keys of the run from place i on in steps of dir, counted up to FIX_RUN + 1
+  auto length = [&](long i, int dir) {
+    const unsigned a = __ballot_sync(0xffffffffu, same(i + dir * lane)), b = __ballot_sync(0xffffffffu, same(i + dir * (32 + lane)));
+    if (a != ~0u) return __ffs(~a) - 1;
+    if (b != ~0u) return 32 + __ffs(~b) - 1;
+    return same(i + dir * 64) ? 65 : 64;
+  };
+  const int before = length(j - 1, -1), after = length(j, 1);
+  if (before == 0) return;
+  const long b = j - before, e = j + after;
   bool descent = false;
-  for (long i = b; i + 1 < e; i++) descent |= keys[i] > keys[i + 1];
-  if (!descent) return;
-  if (j - b > FIX_RUN || e - j > FIX_RUN) long_run(keys, n, lo, sh, tp, lr);
-  else fix_run(keys + b, vals + b, 0, (int)(e - b));
+  for (long i = b + lane; i + 1 < e; i += 32) descent |= keys[i] > keys[i + 1];
+  if (!__any_sync(0xffffffffu, descent)) return;
+  if (before <= FIX_RUN && after <= FIX_RUN) warp_run<4>(keys + b, vals + b, (int)(e - b));
+  else if (lane == 0) long_run(keys, n, lo, sh, tp, before <= FIX_RUN ? b : -1, lr);
 }
 
 // An even sample of the keys, and how many neighbours of the sorted sample are unequal but share
@@ -497,22 +684,32 @@ RangeSort radix_sort_range_u64_u32(mlc_ctx* ctx, long n, uint64_t* keys, uint32_
     MLC_KSCOPE(ctx, "sort_fix");
     const long tiles = (n + FIX_TILE - 1) / FIX_TILE;
     k_fix_tiles<<<(unsigned)tiles, FIX_THREADS, 0, ctx->stream>>>(keys, vals, n, range, dl);
-    k_fix_edges<<<(unsigned)((tiles + 255) / 256), 256, 0, ctx->stream>>>(keys, vals, n, range, dl);
-    k_sort_runs<<<RUN_SLOTS, 256, 0, ctx->stream>>>(keys, vals, n, range, dl);
+    k_fix_edges<<<(unsigned)((tiles + 7) / 8), 256, 0, ctx->stream>>>(keys, vals, n, range, dl);
+    k_sort_runs<<<RUN_SLOTS, RUN_THREADS, 0, ctx->stream>>>(keys, vals, n, range, dl);
   }
   MLC_CHECK_LAUNCH();
   struct {
     int scatter_err, full, nbig;
   } h;
-  unsigned long long big[2 * BIG_RUNS];
   MLC_CUDA(cudaMemcpyAsync(&h, dl, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
-  MLC_CUDA(cudaMemcpyAsync(big, dl->big_at, sizeof big, cudaMemcpyDeviceToHost, ctx->stream));
   MLC_CUDA(cudaStreamSynchronize(ctx->stream));
   MLC_REQUIRE(h.scatter_err == 0, MLC_ERR_CUDA, "radix sort: scatter offset out of range (inconsistent digit counts)");
   if (h.full) return RangeSort::LOST;
-  // (their keys agree in most digits, whose passes are skipped)
+  if (h.nbig == 0) return RangeSort::DONE;
+  {
+    MLC_KSCOPE(ctx, "sort_big_runs");
+    k_sort_big<<<h.nbig, BIG_THREADS, 0, ctx->stream>>>(keys, vals, k2, v2, dl);
+  }
+  MLC_CHECK_LAUNCH();
+  std::vector<unsigned long long> big(2 * BIG_RUNS);
+  MLC_CUDA(cudaMemcpyAsync(big.data(), dl->big_at, sizeof dl->big_at + sizeof dl->big_end, cudaMemcpyDeviceToHost, ctx->stream));
+  MLC_CUDA(cudaStreamSynchronize(ctx->stream));
+  std::vector<int> host;
   for (int r = 0; r < h.nbig; r++)
-    radix_sort_u64_u32(ctx, (long)(big[BIG_RUNS + r] - big[r]), keys + big[r], vals + big[r]);
+    if (big[BIG_RUNS + r] - big[r] > BIG_MAX) host.push_back(r);
+  if ((int)host.size() > HOST_RUNS) return RangeSort::LOST;
+  // (their keys agree in most digits, whose passes are skipped)
+  for (int r : host) radix_sort_u64_u32(ctx, (long)(big[BIG_RUNS + r] - big[r]), keys + big[r], vals + big[r]);
   return RangeSort::DONE;
 }
 

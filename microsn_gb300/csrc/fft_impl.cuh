@@ -268,12 +268,25 @@ __global__ void __launch_bounds__(256) k_rows_c2r3(const C2<T>* __restrict__ in,
   C2<T>* s = reinterpret_cast<C2<T>*>(smem_raw);
   const int row = blockIdx.x;
   C2<TO>* dst = reinterpret_cast<C2<TO>*>(out + (long)row * ldo);
+  // Float-float to FP64 through shared memory: the conversions run on the FP64 pipe, and the L1 L2 threads
+  // of level 3 leave parts of it idle (80 of 256 at 2000 points: 4000^2 334 us from registers, 250
+  // so); other results from the registers.
+  constexpr bool spread = std::is_same<T, ff>::value && std::is_same<TO, double>::value;
   c2r3_row<T, L1, L2, L3>(in + (long)row * pitch, twx, tw1, s, [&](bool act, int n0, const C2<T>* w) {
+    if (spread) __syncthreads();
     if (act) {
 #pragma unroll
-      for (int n3 = 0; n3 < L3; n3++) dst[n0 + L1 * L2 * n3] = C2<TO>{out_cvt<TO>(w[n3].x), out_cvt<TO>(w[n3].y)};
+      for (int n3 = 0; n3 < L3; n3++) {
+        if constexpr (spread) s[n0 + L1 * L2 * n3] = w[n3];
+        else dst[n0 + L1 * L2 * n3] = C2<TO>{out_cvt<TO>(w[n3].x), out_cvt<TO>(w[n3].y)};
+      }
     }
   });
+  if constexpr (spread) {
+    __syncthreads();
+    for (int n = threadIdx.x; n < L1 * L2 * L3; n += blockDim.x)
+      dst[n] = C2<TO>{out_cvt<TO>(s[n].x), out_cvt<TO>(s[n].y)};
+  }
 }
 
 // P3 of four profiles with the interleave fused in.  A cluster of four CTAs takes one row

@@ -71,3 +71,28 @@ def test_faint_pixels_from_cached_spectra(ctx):
         for k, ref in enumerate(refs):
             assert _excess(out[k], ref) <= LIMIT
     m.close()
+
+
+@pytest.mark.parametrize("N", [2000, 4000, 10000])
+def test_fp64_pixels_cost_their_bytes(ctx, N):
+    """The last pass of a float-float convolution into FP64 pixels against FP32 ones: twice the pixels'
+    bytes and the conversions on the FP64 pipe, which all warps share, are less than twice the time."""
+    import microsn_gb300 as mlc
+    p = mlc.profile("exponential", 16.0, 1.0, ref_compat=False)
+    ms = []
+    ctx.set_timing(True)
+    try:
+        for prec, dt in (("f32", torch.float32), ("f64", torch.float64)):
+            m = mlc.Map(ctx, torch.rand((N, N), dtype=dt, device=DEV) + 0.5, prec)
+            m.set_fft("f32x2")
+            out = mlc.convolve(ctx, m, p)
+            times = []
+            for _ in range(7):
+                ctx.kernel_times()
+                mlc.convolve(ctx, m, p, out=out)
+                times.append(ctx.kernel_times()["fft_rows_c2r"][0])
+            ms.append(sorted(times)[3])
+            m.close()
+    finally:
+        ctx.set_timing(False)
+    assert ms[1] <= 1.75 * ms[0]

@@ -642,7 +642,12 @@ void pair_bin_fused(mlc_ctx* ctx, int Njp, const int* indA, const int* indB, con
                     double* bchi2_host, double* bexp_host, uint32_t* nper_host) {
   MLC_REQUIRE(Nbins > 0 && Nbins <= 6000, MLC_ERR_LIMIT, "fused pair binning supports 1..6000 bins");
   // edges, sums, counts; both sides' FP64 and FP32 point-source values
-  const int copies = std::max(16, std::min(1024, (1 << 19) / Nbins));
+  // A places per CTA: as many as leave four CTAs for every SM
+  const int cols = ceil_div(Nloc, 256);
+  const int na = (int)std::max<long>(4, std::min<long>(FUSED_A, (long)Nloc * cols / (4 * ctx->sm_count)));
+  const dim3 grid(cols, ceil_div(Nloc, na));
+  // (no more copies than CTAs: 10 locations spent 20 us on adding up 1024 of them)
+  const int copies = (int)std::max<long>(1, std::min<long>(std::max(16, std::min(1024, (1 << 19) / Nbins)), (long)grid.x * grid.y));
   const size_t N = (size_t)Nloc, NC = (size_t)copies * Nbins;
   char* sm = (char*)ws_get(ctx, WS_PAIR_ACC, 8 * (3 * NC + Nbins) + 2 * (8 + 4) * N + 512);
   double* de = (double*)sm;
@@ -664,10 +669,6 @@ void pair_bin_fused(mlc_ctx* ctx, int Njp, const int* indA, const int* indB, con
   const double2* etab = exp_table(ctx);
   if (Nloc > 0) {
     set_max_smem((const void*)k_pair_bin_fused, smem);
-    // A places per CTA: as many as leave four CTAs for every SM
-    const int cols = ceil_div(Nloc, 256);
-    const int na = (int)std::max<long>(4, std::min<long>(FUSED_A, (long)Nloc * cols / (4 * ctx->sm_count)));
-    dim3 grid(cols, ceil_div(Nloc, na));
     const FusedSide A{z, zf}, B{z + N, zf + N};
     {
       MLC_KSCOPE(ctx, "pair_bin_fused");

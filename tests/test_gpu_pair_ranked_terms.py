@@ -37,3 +37,25 @@ def test_more_epochs_in_rank_order(ctx):
         ctx.set_timing(False)
         ms[terms] = sorted(times)[3]
     assert ms[6] <= 1.1 * ms[5] and ms[8] <= 1.15 * ms[5]
+
+
+def test_few_locations_add_up_few_copies(ctx):
+    """The fused bins of 10 locations: as many copies of the accumulators as CTAs, whose sum takes less
+    than the pairs' kernel (1024 copies took half as long again)."""
+    import microsn_gb300 as mlc
+    r = np.random.default_rng(2)
+    A, B = (torch.as_tensor(np.exp(r.normal(0, 1, (10, 3))), device=DEV) for _ in range(2))
+    dA, dB = torch.diff(A, dim=1).contiguous(), torch.diff(B, dim=1).contiguous()
+    edges = mlc.bin_edges(300, 1e-4, 300.0)
+    v = _vars(3)
+    mlc.pair_bin_fused(ctx, v, A, dA, B, dB, edges)
+    ctx.set_timing(True)
+    times = {"pair_bin_combine": [], "pair_bin_fused": []}
+    for _ in range(9):
+        ctx.kernel_times()
+        mlc.pair_bin_fused(ctx, v, A, dA, B, dB, edges)
+        t = ctx.kernel_times()
+        for k in times:
+            times[k].append(t[k][0])
+    ctx.set_timing(False)
+    assert sorted(times["pair_bin_combine"])[4] <= sorted(times["pair_bin_fused"])[4]

@@ -27,27 +27,45 @@ RadixList factor_radices(int L, int tw_stride);
 
 // ---------------------------------------------------------------- small DFTs
 
-template <typename T, int R, bool INV>
+// PK: float-float additions of the real and the imaginary part as one packed operation; false is for
+// short loops with few warps, where pairing the values anew costs more than it saves (Stockham
+// passes of 600^2: a last pass 16.4 us, packed 18.4).
+template <typename T, int R, bool INV, bool PK = true>
 struct Dft;
+
+template <bool PK, typename T>
+__device__ __forceinline__ C2<T> dadd(C2<T> a, C2<T> b) {
+  if constexpr (std::is_same<T, ff>::value && !PK) return cadd<T>(a, b);
+  else return cadd(a, b);
+}
+template <bool PK, typename T>
+__device__ __forceinline__ C2<T> dsub(C2<T> a, C2<T> b) {
+  if constexpr (std::is_same<T, ff>::value && !PK) return csub<T>(a, b);
+  else return csub(a, b);
+}
+template <bool PK, typename T>
+__device__ __forceinline__ C2<T> dlin2(T a, C2<T> x, T b, C2<T> y) {
+  if constexpr (std::is_same<T, ff>::value && !PK) return clin2<T>(a, x, b, y);
+  else return clin2(a, x, b, y);
+}
 
 // (Radix 2 and 3 of float-float stay unpacked: values come as (hi, lo) pairs, and a stage of so
 // few additions does not pay for pairing them anew.  P1 of 540^2: 14.0 us, packed 15.0.)
-template <typename T, bool INV>
-struct Dft<T, 2, INV> {
+template <typename T, bool INV, bool PK>
+struct Dft<T, 2, INV, PK> {
   static __device__ __forceinline__ void run(C2<T>* v) {
     C2<T> a = v[0], b = v[1];
-    v[0] = std::is_same<T, ff>::value ? cadd<T>(a, b) : cadd(a, b);
-    v[1] = std::is_same<T, ff>::value ? csub<T>(a, b) : csub(a, b);
+    v[0] = dadd<false>(a, b);
+    v[1] = dsub<false>(a, b);
   }
 };
 
-template <typename T, bool INV>
-struct Dft<T, 3, INV> {
+template <typename T, bool INV, bool PK>
+struct Dft<T, 3, INV, PK> {
   static __device__ __forceinline__ void run(C2<T>* v) {
     const T h = (T)0.86602540378443864676372317075294;  // sin(2 pi / 3)
-    constexpr bool FF = std::is_same<T, ff>::value;
-    auto add = [](C2<T> a, C2<T> b) { return FF ? cadd<T>(a, b) : cadd(a, b); };
-    auto sub = [](C2<T> a, C2<T> b) { return FF ? csub<T>(a, b) : csub(a, b); };
+    auto add = [](C2<T> a, C2<T> b) { return dadd<false>(a, b); };
+    auto sub = [](C2<T> a, C2<T> b) { return dsub<false>(a, b); };
     C2<T> s = add(v[1], v[2]);
     C2<T> d = sub(v[1], v[2]);
     C2<T> m = sub(v[0], cscale2(s, 0.5f));
@@ -59,15 +77,15 @@ struct Dft<T, 3, INV> {
   }
 };
 
-template <typename T, bool INV>
-struct Dft<T, 4, INV> {
+template <typename T, bool INV, bool PK>
+struct Dft<T, 4, INV, PK> {
   static __device__ __forceinline__ void run(C2<T>* v) {
-    C2<T> a0 = cadd(v[0], v[2]), a1 = csub(v[0], v[2]);
-    C2<T> a2 = cadd(v[1], v[3]), a3 = mul_mi<T, INV>(csub(v[1], v[3]));
-    v[0] = cadd(a0, a2);
-    v[2] = csub(a0, a2);
-    v[1] = cadd(a1, a3);
-    v[3] = csub(a1, a3);
+    C2<T> a0 = dadd<PK>(v[0], v[2]), a1 = dsub<PK>(v[0], v[2]);
+    C2<T> a2 = dadd<PK>(v[1], v[3]), a3 = mul_mi<T, INV>(dsub<PK>(v[1], v[3]));
+    v[0] = dadd<PK>(a0, a2);
+    v[2] = dsub<PK>(a0, a2);
+    v[1] = dadd<PK>(a1, a3);
+    v[3] = dsub<PK>(a1, a3);
   }
 };
 
@@ -75,57 +93,57 @@ struct Dft<T, 4, INV> {
 // u +/- m with u = x0 + (c1 + c2)/2 (sa + sb), m = (c1 - c2)/2 (sa - sb), where
 // (c1 + c2)/2 = -1/4 exactly (an exact scaling) and (c1 - c2)/2 = sqrt(5)/4: one general
 // product per component instead of four.
-template <typename T, bool INV>
-struct Dft<T, 5, INV> {
+template <typename T, bool INV, bool PK>
+struct Dft<T, 5, INV, PK> {
   static __device__ __forceinline__ void run(C2<T>* v) {
     const T b = (T)0.55901699437494742410229341718282;    // (cos(2 pi/5) - cos(4 pi/5)) / 2
     const T s1 = (T)0.95105651629515357211643933337938;   // sin(2 pi/5)
     const T s2 = (T)0.58778525229247312916870595463907;   // sin(4 pi/5)
     C2<T> x0 = v[0];
-    C2<T> sa = cadd(v[1], v[4]), da = csub(v[1], v[4]);
-    C2<T> sb = cadd(v[2], v[3]), db = csub(v[2], v[3]);
-    C2<T> t1 = cadd(sa, sb), t2 = csub(sa, sb);
-    C2<T> u = csub(x0, cscale2(t1, 0.25f));
+    C2<T> sa = dadd<PK>(v[1], v[4]), da = dsub<PK>(v[1], v[4]);
+    C2<T> sb = dadd<PK>(v[2], v[3]), db = dsub<PK>(v[2], v[3]);
+    C2<T> t1 = dadd<PK>(sa, sb), t2 = dsub<PK>(sa, sb);
+    C2<T> u = dsub<PK>(x0, cscale2(t1, 0.25f));
     C2<T> m = crmul(b, t2);
-    C2<T> p1 = cadd(u, m), p2 = csub(u, m);
-    C2<T> q1 = clin2(s1, da, s2, db);
-    C2<T> q2 = clin2(s2, da, -s1, db);
+    C2<T> p1 = dadd<PK>(u, m), p2 = dsub<PK>(u, m);
+    C2<T> q1 = dlin2<PK>(s1, da, s2, db);
+    C2<T> q2 = dlin2<PK>(s2, da, -s1, db);
     C2<T> iq1 = mul_mi<T, INV>(q1), iq2 = mul_mi<T, INV>(q2);
-    v[0] = cadd(x0, t1);
-    v[1] = cadd(p1, iq1);
-    v[4] = csub(p1, iq1);
-    v[2] = cadd(p2, iq2);
-    v[3] = csub(p2, iq2);
+    v[0] = dadd<PK>(x0, t1);
+    v[1] = dadd<PK>(p1, iq1);
+    v[4] = dsub<PK>(p1, iq1);
+    v[2] = dadd<PK>(p2, iq2);
+    v[3] = dsub<PK>(p2, iq2);
   }
 };
 
-template <typename T, bool INV>
-struct Dft<T, 8, INV> {
+template <typename T, bool INV, bool PK>
+struct Dft<T, 8, INV, PK> {
   static __device__ __forceinline__ void run(C2<T>* v) {
     const T r = (T)0.70710678118654752440084436210485;
     C2<T> e[4] = {v[0], v[2], v[4], v[6]};
     C2<T> o[4] = {v[1], v[3], v[5], v[7]};
-    Dft<T, 4, INV>::run(e);
-    Dft<T, 4, INV>::run(o);
+    Dft<T, 4, INV, PK>::run(e);
+    Dft<T, 4, INV, PK>::run(o);
     // o[q] *= W8^q ; forward W8 = (1 - i)/sqrt2, inverse (1 + i)/sqrt2
     C2<T> o1 = crmul(r, INV ? C2<T>{o[1].x - o[1].y, o[1].x + o[1].y} : C2<T>{o[1].x + o[1].y, o[1].y - o[1].x});
     C2<T> o2 = mul_mi<T, INV>(o[2]);
     C2<T> o3 = INV ? C2<T>{-r * (o[3].x + o[3].y), r * (o[3].x - o[3].y)}
                    : C2<T>{r * (o[3].y - o[3].x), -r * (o[3].x + o[3].y)};
-    v[0] = cadd(e[0], o[0]);
-    v[4] = csub(e[0], o[0]);
-    v[1] = cadd(e[1], o1);
-    v[5] = csub(e[1], o1);
-    v[2] = cadd(e[2], o2);
-    v[6] = csub(e[2], o2);
-    v[3] = cadd(e[3], o3);
-    v[7] = csub(e[3], o3);
+    v[0] = dadd<PK>(e[0], o[0]);
+    v[4] = dsub<PK>(e[0], o[0]);
+    v[1] = dadd<PK>(e[1], o1);
+    v[5] = dsub<PK>(e[1], o1);
+    v[2] = dadd<PK>(e[2], o2);
+    v[6] = dsub<PK>(e[2], o2);
+    v[3] = dadd<PK>(e[3], o3);
+    v[7] = dsub<PK>(e[3], o3);
   }
 };
 
 // Radix 2 over two half-length DFTs: X[k] = E[k] + W^k O[k], X[k + R/2] = E[k] - W^k O[k],
 // W = exp(-/+ 2 pi i / R); wr[k], wi[k] = cos, sin(2 pi k / R).
-template <typename T, int H, bool INV>
+template <typename T, int H, bool INV, bool PK>
 __device__ __forceinline__ void dft_split2(C2<T>* v, const T* wr, const T* wi) {
   C2<T> e[H], o[H];
 #pragma unroll
@@ -133,17 +151,17 @@ __device__ __forceinline__ void dft_split2(C2<T>* v, const T* wr, const T* wi) {
     e[i] = v[2 * i];
     o[i] = v[2 * i + 1];
   }
-  Dft<T, H, INV>::run(e);
-  Dft<T, H, INV>::run(o);
-  v[0] = cadd(e[0], o[0]);  // W^0 = 1
-  v[H] = csub(e[0], o[0]);
+  Dft<T, H, INV, PK>::run(e);
+  Dft<T, H, INV, PK>::run(o);
+  v[0] = dadd<PK>(e[0], o[0]);  // W^0 = 1
+  v[H] = dsub<PK>(e[0], o[0]);
 #pragma unroll
   for (int k = 1; k < H; k++) {
     // W^k o with W^k = (wr, -wi) forward, (wr, wi) inverse
     const T sr = INV ? -wi[k] : wi[k];
     const C2<T> t = C2<T>{lin2(wr[k], o[k].x, sr, o[k].y), lin2(wr[k], o[k].y, -sr, o[k].x)};
-    v[k] = cadd(e[k], t);
-    v[k + H] = csub(e[k], t);
+    v[k] = dadd<PK>(e[k], t);
+    v[k + H] = dsub<PK>(e[k], t);
   }
 }
 
@@ -151,18 +169,18 @@ __device__ __forceinline__ void dft_split2(C2<T>* v, const T* wr, const T* wi) {
 // with n = (5 n1 + 2 n2) mod 10 and k = (5 k1 + 6 k2) mod 10, W10^(n k) = W2^(n1 k1) W5^(n2 k2),
 // so five DFT2 over n1, then two DFT5 over n2 (84 real additions and 32 multiplications,
 // against 94 and 52 for the radix-2 split with its twiddles).
-template <typename T, bool INV>
-struct Dft<T, 10, INV> {
+template <typename T, bool INV, bool PK>
+struct Dft<T, 10, INV, PK> {
   static __device__ __forceinline__ void run(C2<T>* v) {
     C2<T> a[5], b[5];
 #pragma unroll
     for (int n2 = 0; n2 < 5; n2++) {
       const C2<T> x0 = v[(2 * n2) % 10], x1 = v[(5 + 2 * n2) % 10];
-      a[n2] = cadd(x0, x1);  // k1 = 0
-      b[n2] = csub(x0, x1);  // k1 = 1
+      a[n2] = dadd<PK>(x0, x1);  // k1 = 0
+      b[n2] = dsub<PK>(x0, x1);  // k1 = 1
     }
-    Dft<T, 5, INV>::run(a);
-    Dft<T, 5, INV>::run(b);
+    Dft<T, 5, INV, PK>::run(a);
+    Dft<T, 5, INV, PK>::run(b);
 #pragma unroll
     for (int k2 = 0; k2 < 5; k2++) {
       v[(6 * k2) % 10] = a[k2];
@@ -172,18 +190,18 @@ struct Dft<T, 10, INV> {
 };
 
 // 6 points by the prime-factor split 6 = 2 x 3: n = (3 n1 + 2 n2) mod 6, k = (3 k1 + 4 k2) mod 6.
-template <typename T, bool INV>
-struct Dft<T, 6, INV> {
+template <typename T, bool INV, bool PK>
+struct Dft<T, 6, INV, PK> {
   static __device__ __forceinline__ void run(C2<T>* v) {
     C2<T> a[3], b[3];
 #pragma unroll
     for (int n2 = 0; n2 < 3; n2++) {
       const C2<T> x0 = v[(2 * n2) % 6], x1 = v[(3 + 2 * n2) % 6];
-      a[n2] = cadd(x0, x1);
-      b[n2] = csub(x0, x1);
+      a[n2] = dadd<PK>(x0, x1);
+      b[n2] = dsub<PK>(x0, x1);
     }
-    Dft<T, 3, INV>::run(a);
-    Dft<T, 3, INV>::run(b);
+    Dft<T, 3, INV, PK>::run(a);
+    Dft<T, 3, INV, PK>::run(b);
 #pragma unroll
     for (int k2 = 0; k2 < 3; k2++) {
       v[(4 * k2) % 6] = a[k2];
@@ -193,8 +211,8 @@ struct Dft<T, 6, INV> {
 };
 
 // 9 points as 3 x 3: DFT3 over n1 of x[3 n1 + n2], twiddle W9^(n2 k1), DFT3 over n2 -> X[k1 + 3 k2].
-template <typename T, bool INV>
-struct Dft<T, 9, INV> {
+template <typename T, bool INV, bool PK>
+struct Dft<T, 9, INV, PK> {
   static __device__ __forceinline__ void run(C2<T>* v) {
     // cos, sin(2 pi m / 9), m = 1, 2, 4
     const T cr[3] = {(T)0.76604444311897803520239265055541668, (T)0.17364817766693034885171662676931480,
@@ -206,7 +224,7 @@ struct Dft<T, 9, INV> {
     for (int n2 = 0; n2 < 3; n2++) {
 #pragma unroll
       for (int n1 = 0; n1 < 3; n1++) y[n2][n1] = v[3 * n1 + n2];
-      Dft<T, 3, INV>::run(y[n2]);
+      Dft<T, 3, INV, PK>::run(y[n2]);
 #pragma unroll
       for (int k1 = 1; k1 < 3; k1++) {
         if (n2 == 0) continue;
@@ -219,40 +237,40 @@ struct Dft<T, 9, INV> {
 #pragma unroll
     for (int k1 = 0; k1 < 3; k1++) {
       C2<T> u[3] = {y[0][k1], y[1][k1], y[2][k1]};
-      Dft<T, 3, INV>::run(u);
+      Dft<T, 3, INV, PK>::run(u);
 #pragma unroll
       for (int k2 = 0; k2 < 3; k2++) v[k1 + 3 * k2] = u[k2];
     }
   }
 };
 
-template <typename T, bool INV>
-struct Dft<T, 16, INV> {
+template <typename T, bool INV, bool PK>
+struct Dft<T, 16, INV, PK> {
   static __device__ __forceinline__ void run(C2<T>* v) {
     const T c1 = (T)0.92387953251128675612818318939679, s1 = (T)0.38268343236508977172845998403040;
     const T r = (T)0.70710678118654752440084436210485;
     const T wr[8] = {(T)1, c1, r, s1, (T)0, -s1, -r, -c1};
     const T wi[8] = {(T)0, s1, r, c1, (T)1, c1, r, s1};
-    dft_split2<T, 8, INV>(v, wr, wi);
+    dft_split2<T, 8, INV, PK>(v, wr, wi);
   }
 };
 
-template <typename T, bool INV>
-struct Dft<T, 20, INV> {
+template <typename T, bool INV, bool PK>
+struct Dft<T, 20, INV, PK> {
   static __device__ __forceinline__ void run(C2<T>* v) {
     // cos, sin(2 pi k / 20), k = 0..9
     const T a = (T)0.95105651629515357211643933337938214, b = (T)0.30901699437494742410229341718281906;
     const T c = (T)0.80901699437494742410229341718281906, d = (T)0.58778525229247312916870595463907277;
     const T wr[10] = {(T)1, a, c, d, b, (T)0, -b, -d, -c, -a};
     const T wi[10] = {(T)0, b, d, c, a, (T)1, a, c, d, b};
-    dft_split2<T, 10, INV>(v, wr, wi);
+    dft_split2<T, 10, INV, PK>(v, wr, wi);
   }
 };
 
 // 25 points as 5 x 5 (four-step in registers): DFT5 over n1 of x[5 n1 + n2], twiddle
 // W25^(n2 k1), DFT5 over n2 -> X[k1 + 5 k2].
-template <typename T, bool INV>
-struct Dft<T, 25, INV> {
+template <typename T, bool INV, bool PK>
+struct Dft<T, 25, INV, PK> {
   static __device__ __forceinline__ void run(C2<T>* v) {
     // cos, sin(2 pi m / 25), m = 0..16
     const T cr[17] = {(T)1,
@@ -278,7 +296,7 @@ struct Dft<T, 25, INV> {
     for (int n2 = 0; n2 < 5; n2++) {
 #pragma unroll
       for (int n1 = 0; n1 < 5; n1++) y[n2][n1] = v[5 * n1 + n2];
-      Dft<T, 5, INV>::run(y[n2]);
+      Dft<T, 5, INV, PK>::run(y[n2]);
 #pragma unroll
       for (int k1 = 1; k1 < 5; k1++) {
         if (n2 == 0) continue;
@@ -293,7 +311,7 @@ struct Dft<T, 25, INV> {
       C2<T> u[5];
 #pragma unroll
       for (int n2 = 0; n2 < 5; n2++) u[n2] = y[n2][k1];
-      Dft<T, 5, INV>::run(u);
+      Dft<T, 5, INV, PK>::run(u);
 #pragma unroll
       for (int k2 = 0; k2 < 5; k2++) v[k1 + 5 * k2] = u[k2];
     }
@@ -332,7 +350,7 @@ __device__ __forceinline__ void stockham_stage(const C2<T>* __restrict__ src, C2
         if (i + 1 < R) w = cmul(w, w1);
       }
     }
-    Dft<T, R, INV>::run(v);
+    Dft<T, R, INV, !std::is_same<T, ff>::value>::run(v);
     const int d = q * Ns * R + k;
 #pragma unroll
     for (int i = 0; i < R; i++) dst[(d + i * Ns) * CW + c] = v[i];
@@ -366,7 +384,7 @@ __device__ __forceinline__ void stockham_stage_st(const C2<T>* __restrict__ src,
 #pragma unroll
       for (int i = 1; i < R; i++) v[i] = INV ? cmulc(v[i], w[i - 1]) : cmul(v[i], w[i - 1]);
     }
-    Dft<T, R, INV>::run(v);
+    Dft<T, R, INV, !std::is_same<T, ff>::value>::run(v);
     const int d = q * Ns * R + k;
 #pragma unroll
     for (int i = 0; i < R; i++) dst[(d + i * Ns) * CW + c] = v[i];

@@ -115,7 +115,7 @@ int mlc_ctx_autotune_report(mlc_ctx* ctx, char* buf, int cap);
  * the autotuner is on), e.g. to compare variants or to fix a run's kernels:
  *   "conv f32 <Nx>x<Ny> N<pN>[ spectrum]": -1 FFT form, 0..3 direct tile shape;
  *   "conv P1 <arithmetic> <Nx>x<Ny>[ two-chain]": 0 map spectrum prefetched into L2, 1
- *     staged in shared memory (float-float transforms of FP64 maps); " two-chain" is the
+ *     staged in shared memory (float-float transforms); " two-chain" is the
  *     batched step's key, where the second convolution chain runs alongside (not timed:
  *     0 unless pinned);
  *   "pairdiff_tc K<64|128>[ matrix] bins<1024|4096> pairs~4^<k>": epilogue warps 12, 16
@@ -134,8 +134,8 @@ int mlc_ctx_tune_set(mlc_ctx* ctx, const char* key, int choice);
  * convolution then skips the profile's transform (P0 and the forward half of P1; the same
  * operations on the same values otherwise, so the same results bit for bit).  They take
  * nprof x (Ny x (Nx/2+1) complex) of the map's transform arithmetic: 800 MB per profile at
- * 10000^2 in float-float, 1.2 GB in FP64 (three FP32 limbs, 24 bytes per value).  max_bytes: -1 (default) a quarter of the device memory, 0 never
- * cache, else the limit; lists that do not fit are convolved without the cache.  Map sizes
+ * 10000^2 in float-float, 1.2 GB in FP64 (three FP32 limbs, 24 bytes per value).  max_bytes:
+ * -1 (default) a quarter of the device memory, 0 never cache, else the limit; lists that do not fit are convolved without the cache.  Map sizes
  * whose column split has N2 = 100 or 128 (e.g. 2000^2 ... 10000^2, 8192^2). */
 int mlc_ctx_set_profile_cache(mlc_ctx* ctx, long long max_bytes);
 int mlc_ctx_kernel_times(mlc_ctx* ctx, char* names_host, int name_cap, double* ms_host, long* launches_host,

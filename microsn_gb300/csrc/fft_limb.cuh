@@ -6,7 +6,7 @@
 // every transform it holds (one exchange through shared memory beside the barrier that the
 // twiddle tables need anyway), scales, transforms, and scales back on its stores.
 //
-// Measured at 10000^2, FP64 arithmetic and limbs: map rows 6.1 and 1.5 ms, column pass 2.5 and
+// Measured at 10000^2, FP64 arithmetic and limbs: map rows 6.1 and 1.7 ms, column pass 2.5 and
 // 0.70, P1 8.8 and 1.9 (four Gaussians of 100 to 600 rows), P3 5.9 and 1.5.
 #pragma once
 

@@ -130,9 +130,8 @@ __device__ __forceinline__ C2<T> clin2(T a, C2<T> x, T b, C2<T> y) {
 
 // The real and imaginary limbs of a complex value as one register pair: packed FP32
 // instructions do the same roundings on both halves for one issue slot.  The small transforms
-// use them (10000^2: P3 of 16 profiles 10.26 -> 9.55 ms, P1 of FP64 8.1 -> 7.7); twiddle products
-// stay scalar, as the swap of one factor's components took back what the packing gave
-// (10.29 ms and 7.8).
+// use them (P1 of FP64 at 10000^2: 8.1 -> 7.7 ms); twiddle products stay scalar, as the swap of one
+// factor's components took back what the packing gave (7.8 ms).
 struct f32p {
   unsigned long long v;
 };

@@ -8,7 +8,7 @@
 //     x = p.q = 2^32 X0 + 2^24 X1 + 2^16 X2 + 2^8 X3 + X4   exactly,
 // and chi2 = |P|^2 + |Q|^2 - 2^(ei+ej+1) x is formed from the per-curve norms (natural
 // units, float-float) and the exactly scaled accumulators: in FP32 summed from the largest
-// term down (within 4e-6 relative) where chi2 >= 2^-14 (|P|^2+|Q|^2), in float-float
+// term down (to some 4e-6 relative) where chi2 >= 2^-14 (|P|^2+|Q|^2), in float-float
 // arithmetic below that.  Top-k
 // candidates, pairs whose chi2 is below 1e-7 of |P|^2 + |Q|^2 (where the float-float
 // rounding could matter) and, with a matrix requested, every pair whose quantisation error
@@ -29,7 +29,7 @@
 //               candidates below a threshold, refinement list, optional matrix
 // Every barrier wait is bounded; a timeout sets the error flag and all roles unwind.
 //
-// Measured, 10^10 pairs of 128 epochs: 15.8 ms.  The MMAs alone take 12.6 ms (loads and waits
+// Measured, 10^10 pairs of 128 epochs: 15.0 ms.  The MMAs alone take 12.6 ms (loads and waits
 // kept, the arithmetic after them left out; 9.7 ms at the tensor pipe's rate), the epilogue is
 // the rest: 34 instructions a pair.  One MMA per slice pair (N = 48, 72 a tile, issued by a
 // lone thread) took 33.5 ms, bound by the issue of an MMA, some 50 cycles whatever its shape;
@@ -377,8 +377,10 @@ __global__ void __launch_bounds__(Epi<EPIW>::threads, 1) k_pairdiff_tc(const __g
             // FP32 assembly from the largest term down: ab + e = |P|^2 + |Q|^2 (high parts)
             // exactly; s0 X0 is exact (integer < 2^24 times a power of two), so ab + s0 X0 is
             // rounded once, relative to itself, then the X1 term, then the small rest.  Error
-            // about 3 2^-24 chi2 + 2^-32 (|P|^2+|Q|^2) (the left-out X4 term below 2^-30 of it):
-            // within 4e-6 of chi2 whenever chi2 >= 2^-14 (|P|^2+|Q|^2)
+            // about 3 2^-24 chi2 + 2^-32 (|P|^2+|Q|^2), and the left-out X4 term: digits of
+            // either sign add up to 2^-33 of the norms or so, within 4e-6 of chi2 whenever
+            // chi2 >= 2^-14 (|P|^2+|Q|^2).  That is no bound: low digits all near 127 and alike
+            // in both curves, beside one large value, would make it 2^-23.
             const f2 s0 = f2_mul(npa, bz);
             const f2 ab = f2_add(ax, bx), bb = f2_sub(ab, ax);
             const f2 e = f2_add(f2_sub(ax, f2_sub(ab, bb)), f2_sub(bx, bb));

@@ -295,7 +295,7 @@ void radix_sort_u64_u32(mlc_ctx* ctx, long n, uint64_t* keys, uint32_t* vals) {
 // decide the order: of 8.5e7 quotients over some twenty octaves about one key in six has a
 // neighbour of the same 32 bits.  Four stable passes order the keys by them; where two
 // neighbours of the same top bits then stand in the wrong order (a descent), their run is
-// sorted by its full keys, stably, by one thread: within tiles of the keys in shared memory
+// sorted by its full keys, stably, by a thread or a warp: within tiles of the keys in shared memory
 // (k_fix_tiles), then across the tiles' edges (k_fix_edges).  Runs of equal keys are in order
 // as they stand, however long.  A run with a descent that is longer than FIX_RUN is noted
 // (long_run) and sorted by a CTA, up to RUN_MAX keys in shared memory (k_sort_runs), longer ones

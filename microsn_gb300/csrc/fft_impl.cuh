@@ -48,12 +48,12 @@ struct ProfileRows {
 
 // Spectrum value k <= M of a real row from Z = FFT_M(x[2n] + i x[2n+1]):
 // X[k] = (Z[k] + conj Z[M-k]) / 2 - i W_Nx^k (Z[k] - conj Z[M-k]) / 2, Z[M] = Z[0].
-template <typename T>
+template <bool PK = true, typename T>
 __device__ __forceinline__ C2<T> r2c_split(const C2<T>* Z, int M, const C2<T>* __restrict__ twx, int k) {
   const C2<T> zk = Z[k == M ? 0 : k];
   const C2<T> zc = cconj(Z[k == 0 ? 0 : M - k]);
-  const C2<T> s = cadd(zk, zc);
-  const C2<T> wd = cmul(ldc(twx + k), csub(zk, zc));  // W_Nx^k (Z - conj Z')
+  const C2<T> s = dadd<PK>(zk, zc);
+  const C2<T> wd = cmul(ldc(twx + k), dsub<PK>(zk, zc));  // W_Nx^k (Z - conj Z')
   return C2<T>{(T)0.5 * (s.x + wd.y), (T)0.5 * (s.y - wd.x)};
 }
 
@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(512) k_rows_r2c(Loader ld, C2<T>* __restrict__
   __syncthreads();
   C2<T>* Z = fft_smem<T, false, 1>(a, b, rl, twx);
   C2<T>* o = out + (long)row * pitch;
-  for (int k = threadIdx.x; k <= M; k += blockDim.x) o[k] = cfin(r2c_split(Z, M, twx, k));
+  for (int k = threadIdx.x; k <= M; k += blockDim.x) o[k] = cfin(r2c_split<!std::is_same<T, ff>::value>(Z, M, twx, k));
   for (int k = M + 1 + threadIdx.x; k < pitch; k += blockDim.x) o[k] = C2<T>{(T)0, (T)0};
 }
 
@@ -185,8 +185,8 @@ __global__ void __launch_bounds__(512) k_rows_c2r(const C2<T>* __restrict__ in, 
   for (int k = threadIdx.x; k < M; k += blockDim.x) {
     C2<T> xk = a[k];
     C2<T> xm = cconj(a[M - k]);
-    C2<T> e = cadd(xk, xm);
-    C2<T> o = cmulc(csub(xk, xm), ldc(twx + k));  // (X - conj X') W^-k
+    C2<T> e = dadd<false>(xk, xm);
+    C2<T> o = cmulc(dsub<false>(xk, xm), ldc(twx + k));  // (X - conj X') W^-k
     b[k] = C2<T>{e.x - o.y, e.y + o.x};
   }
   __syncthreads();
@@ -695,13 +695,13 @@ __global__ void __launch_bounds__(256) k_conv_fused(const C2<T>* __restrict__ Fm
     C2<T> acc{(T)0, (T)0};
     for (int n1 = 0; n1 * N2 + n2 < h; n1++) {
       const long j = (long)n1 * N2 + n2;
-      acc = cadd(acc, cmul(Kx[j * pitch + col0 + c], w1[n1]));
+      acc = dadd<false>(acc, cmul(Kx[j * pitch + col0 + c], w1[n1]));
     }
     int n1s = (lo - n2 + N2 - 1) / N2;
     if (n1s < 0) n1s = 0;
     for (int n1 = n1s; n1 < N1; n1++) {
       const long j = (long)n1 * N2 + n2 - (Ny - 2L * h);
-      acc = cadd(acc, cmul(Kx[j * pitch + col0 + c], w1[n1]));
+      acc = dadd<false>(acc, cmul(Kx[j * pitch + col0 + c], w1[n1]));
     }
     a[idx] = cmul(acc, w2[n2]);
   }
